@@ -6,13 +6,19 @@
 //                   token tiles of at most BN rows (device-side, no host round trip)
 //   moe_tc_gather   xs[pos] = fp16(x[pair / S]) in sorted order (the TMA-loadable "B" operand)
 //   moe_tc_ffn      persistent, one CTA per SM walking (token tile, 128 weight rows) work items:
-//        warp 0      TMA producer for the token tiles (cp.async.bulk.tensor, 128-byte swizzle, 8-stage ring)
+//        warp 0      TMA producer for the token tiles (cp.async.bulk.tensor, 128-byte swizzle)
 //        warp 1      tensor-memory owner and tcgen05.mma issuer (kind::f16, fp16 x fp16 -> fp32 in TMEM,
 //                    A = weights read from tensor memory, B = tokens read from shared memory)
-//        warps 2-9   weight converters: stream the expert's NVFP4 / FP8-block / Q4_K / BF16 rows from HBM
+//        warps 2-17  weight converters: stream the expert's NVFP4 / FP8-block / Q4_K / BF16 rows from HBM
 //                    exactly once into registers, expand them to fp16 (group / block scale folded in) and
 //                    write them with tcgen05.st into a ring of operand stages in tensor memory
-//        warps 10-13 epilogue (tcgen05.ld -> SwiGLU(+clamp) -> fp16, or -> fp32 / bf16 rows, or NVLink stores)
+//        warp 22     TMA producer for the raw weight bytes
+//        warps 18-21 epilogue (tcgen05.ld -> SwiGLU(+clamp) -> fp16, or -> fp32 / bf16 rows, or NVLink stores)
+//     With few rows per expert the kernel is bound by the converters' instructions and by what the roles spend on barriers, not by DRAM or the
+//     tensor cores.  Measured (gate/up, down) with one converter set, a single thread walking the issue loop and 64 elements per operand
+//     stage: 32 rows x top-8 of 288 + 1 shared NVFP4 experts of 4096 x 2048 (169 hit) 773 and 590 us, 2048 rows 1508 and 1221 us, 777 rows
+//     over 256 FP8 experts of 7168 x 2048 2310 and 1717 us; as it is now 375 and 271, 920 and 633, 1373 and 867 us (weights at DRAM's rate:
+//     244 and 122, 417 and 208, 1153 and 577 us).
 //     gate and up tiles share one token tile and accumulate into two TMEM regions, so SwiGLU is
 //     fused and the [tokens, 2F] intermediate never exists.
 // Per-tensor NVFP4 scales are applied in the epilogue in fp32.  Every wait is bounded and reports
@@ -106,33 +112,31 @@ __device__ __forceinline__ uint32_t h2_bits(const __half2& h) { return *reinterp
 
 // Weight path of the grouped GEMM:  HBM --TMA--> raw ring in shared memory --ld.shared--> registers --convert-->
 // tcgen05.st --> operand ring in tensor memory --> tcgen05.mma (A from TMEM).
-// A pipeline stage is 64 reduction elements of 128 weight rows per matrix = one TMA box of SBYTES x 128 bytes of the
-// [slot][row][byte] view of the arena, written with the swizzle mode of width SBYTES.  One converter thread owns one
-// weight row (TMEM lane = row) and 64 / NH consecutive elements of the stage: it reads its 16-byte chunks from the
+// A pipeline stage is 64 reduction elements of 128 weight rows per matrix, SBYTES of every row.  What travels is a box of 128 bytes of
+// every row (SUB stages) of the [slot][row][byte] view of the arena, written with the 128-byte swizzle: whole DRAM lines, and one barrier
+// round trip of the converters for all of them.  One converter thread owns one
+// weight row (TMEM lane = row) and 64 / NH consecutive elements of a stage: it reads its 16-byte chunks from the
 // swizzled box (conflict free: the 8 lanes of a quarter-warp phase hit 8 different 16-byte bank groups), expands
 // them to fp16 pairs with the group / block scale folded in and writes them into its TMEM lane with one tcgen05.st.
 // The converted operand never exists in shared memory, which carries only raw bytes (once in, once out) and the
 // token tiles; staging fp16 weight tiles there would cost about four times the shared-memory bandwidth.
 //   RowConv<FMT, NH>::SBYTES                   raw bytes per row and stage
 //   stage_x(it)                                byte offset of stage `it` inside a weight row
-//   fetch(raw, tile, r, h)                     read this thread's chunks of row r (part h of NH) from the box at `tile`
+//   fetch(raw, tile, r, h, sub)                read this thread's chunks of row r (part h of NH) of stage `sub` of the box at `tile`
 //   convert(raw, out, k0, h)                   expand to 32 / NH packed fp16 pairs
 constexpr float kFp8Unscale = 1.f / 256.f;
-template <int SBYTES> __device__ __forceinline__ uint32_t swz_chunk(uint32_t tile, int r, int c) {
-    if (SBYTES == 128) return tile + (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4));
-    if (SBYTES == 64) return tile + (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
-    return tile + (uint32_t)(r * 32 + ((c ^ ((r >> 2) & 1)) << 4));
-}
+constexpr int kBoxBytes = 128;
+__device__ __forceinline__ uint32_t swz_chunk(uint32_t tile, int r, int c) { return tile + (uint32_t)(r * kBoxBytes + ((c ^ (r & 7)) << 4)); }
 template <int FMT, int NH> struct RowConv;
 
 template <int NH> struct RowConv<2, NH> {     // NVFP4: 32 bytes per row-stage; 4 group scales in one word
-    static constexpr int SBYTES = 32, NV = 2 / NH, AUX = 512;              // AUX: the stage's 128 x 4 scale atom
+    static constexpr int SBYTES = 32, NV = 2 / NH, AUX = 512;              // AUX: a stage's 128 x 4 scale atom
     struct Raw { uint4 v[NV]; uint32_t sc; };
     static __device__ __forceinline__ int pitch(int K) { return K >> 1; }
     static __device__ __forceinline__ int stage_x(int it) { return it * 32; }
-    static __device__ __forceinline__ void fetch(Raw& r, uint32_t tile, int row, int h) {
+    static __device__ __forceinline__ void fetch(Raw& r, uint32_t tile, int row, int h, int sub) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) r.v[i] = ld_shared_16(swz_chunk<32>(tile, row, h * NV + i));
+        for (int i = 0; i < NV; ++i) r.v[i] = ld_shared_16(swz_chunk(tile, row, sub * 2 + h * NV + i));
     }
     static __device__ __forceinline__ void convert(const Raw& r, uint32_t* out, int, int h) {
 #pragma unroll
@@ -156,9 +160,9 @@ template <int NH> struct RowConv<1, NH> {     // FP8 e4m3 with 128 x 128 block s
     struct Raw { uint4 v[NV]; float sc; };
     static __device__ __forceinline__ int pitch(int K) { return K; }
     static __device__ __forceinline__ int stage_x(int it) { return it * 64; }
-    static __device__ __forceinline__ void fetch(Raw& r, uint32_t tile, int row, int h) {
+    static __device__ __forceinline__ void fetch(Raw& r, uint32_t tile, int row, int h, int sub) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) r.v[i] = ld_shared_16(swz_chunk<64>(tile, row, h * NV + i));
+        for (int i = 0; i < NV; ++i) r.v[i] = ld_shared_16(swz_chunk(tile, row, sub * 4 + h * NV + i));
     }
     static __device__ __forceinline__ void convert(const Raw& r, uint32_t* out, int, int) {
         // block scales of small weights sit near the bottom of the fp16 range: carry them times 2^8 (exact)
@@ -181,9 +185,9 @@ template <int NH> struct RowConv<3, NH> {     // GGUF Q4_K: a stage = 32 quant b
     struct Raw { uint4 hdr; uint4 q[2]; };
     static __device__ __forceinline__ int pitch(int K) { return (K >> 8) * 144; }
     static __device__ __forceinline__ int stage_x(int it) { return (it >> 2) * 144 + 16 + (it & 3) * 32; }
-    static __device__ __forceinline__ void fetch(Raw& r, uint32_t tile, int row, int) {
-        r.q[0] = ld_shared_16(swz_chunk<32>(tile, row, 0));
-        r.q[1] = ld_shared_16(swz_chunk<32>(tile, row, 1));
+    static __device__ __forceinline__ void fetch(Raw& r, uint32_t tile, int row, int, int sub) {
+        r.q[0] = ld_shared_16(swz_chunk(tile, row, sub * 2));
+        r.q[1] = ld_shared_16(swz_chunk(tile, row, sub * 2 + 1));
     }
     static __device__ __forceinline__ void convert(const Raw& r, uint32_t* out, int k0, int h) {
         const __half2 dd = *reinterpret_cast<const __half2*>(&r.hdr.x);
@@ -217,9 +221,9 @@ template <int NH> struct RowConv<0, NH> {     // BF16: 128 bytes per row-stage
     struct Raw { uint4 v[NV]; };
     static __device__ __forceinline__ int pitch(int K) { return K * 2; }
     static __device__ __forceinline__ int stage_x(int it) { return it * 128; }
-    static __device__ __forceinline__ void fetch(Raw& r, uint32_t tile, int row, int h) {
+    static __device__ __forceinline__ void fetch(Raw& r, uint32_t tile, int row, int h, int) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) r.v[i] = ld_shared_16(swz_chunk<128>(tile, row, h * NV + i));
+        for (int i = 0; i < NV; ++i) r.v[i] = ld_shared_16(swz_chunk(tile, row, h * NV + i));
     }
     static __device__ __forceinline__ void convert(const Raw& r, uint32_t* out, int, int) {
 #pragma unroll
@@ -254,46 +258,52 @@ template <int FMT, int BN, bool GATEUP> struct MoeTcCfg {
     static constexpr int A_TILES = GATEUP ? 2 : 1;
     static constexpr int NH = GATEUP ? 1 : 2;                             // converter threads per (row, stage): gate/up = one per matrix
     using CV = RowConv<FMT, NH>;
-    static constexpr int B_BYTES = BN * kTBK * 2;
-
+    static constexpr int B_BYTES = BN * kTBK * 2;                         // token tile of a sub-stage
+    // An operand stage is KS sub-stages of 64 reduction elements behind one pair of barriers: the issuing warp's waits and commit cost a few
+    // hundred cycles a stage beside the converters' instruction streams, which is more than the MMAs of 64 elements of a small token tile take.
+#ifndef LSB_MOE_KS_GU
+#define LSB_MOE_KS_GU 2
+#endif
+#ifndef LSB_MOE_KS_DN
+#define LSB_MOE_KS_DN 4
+#endif
+    static constexpr int KS = GATEUP ? LSB_MOE_KS_GU : (BN <= 64 ? LSB_MOE_KS_DN : 2);
     static constexpr int ACC_COLS = A_TILES * BN;                         // one accumulator set (gate [+ up])
     // Tensor memory (512 columns): accumulator sets first, then the ring of converted weight stages
-    // (32 columns = 64 fp16 per matrix and stage).  Two accumulator sets let the epilogue of one item overlap the
+    // (32 columns = 64 fp16 per matrix and sub-stage).  Two accumulator sets let the epilogue of one item overlap the
     // main loop of the next; at ACC_COLS = 256 only one fits beside the weight ring.
 #ifndef LSB_MOE_NBUF1_COLS
 #define LSB_MOE_NBUF1_COLS 128
 #endif
     static constexpr int NBUF = ACC_COLS > LSB_MOE_NBUF1_COLS ? 1 : 2;
-    static constexpr int A_COLS = 32 * A_TILES;
+    static constexpr int A_COLS = 32 * A_TILES * KS;
     static constexpr int A_BASE = NBUF * ACC_COLS;
-    static constexpr int SA_FIT = (512 - A_BASE) / A_COLS;
-    static constexpr int SA = SA_FIT > 8 ? 8 : SA_FIT;                    // converted weight stages in TMEM
-    static constexpr int SB = 4;                                          // token-tile ring (shared memory, TMA)
+    static constexpr int S_FIT = (512 - A_BASE) / A_COLS;
+    static constexpr int S = S_FIT > 3 ? 3 : S_FIT;                       // operand stages: weights in tensor memory, tokens in shared memory
     static constexpr int TMEM_COLS = 512;
-    // 8 converter warps cover one stage (4 lane quarters x 2 parts); CONV_GROUPS such sets take the stages round-robin, so
-    // a warp has CONV_GROUPS stage times for its serial wait -> read -> convert -> store -> signal chain.
-#ifndef LSB_MOE_CONV_GROUPS
-#define LSB_MOE_CONV_GROUPS 1
-#endif
-    static constexpr int CONV_GROUPS = LSB_MOE_CONV_GROUPS;
-    static constexpr int STAGE_WARPS = 8;
-    static constexpr int CONV_WARPS = STAGE_WARPS * CONV_GROUPS;
+    // 8 converter warps cover one sub-stage (4 lane quarters x 2 parts); two sets of them take the sub-stages in turns, so that a warp has
+    // two sub-stage times for its serial read -> convert -> store chain
+    static constexpr int CONV_SETS = 2;
+    static constexpr int SET_WARPS = 8;
+    static constexpr int CONV_WARPS = SET_WARPS * CONV_SETS;
+    static_assert(KS % CONV_SETS == 0, "both sets have part in every operand stage");
     static constexpr int EPI_WARPS = 4;
     static constexpr int RAW_WARP = 2 + CONV_WARPS + EPI_WARPS;           // last warp: TMA producer of the raw weight ring
     static constexpr int THREADS = (RAW_WARP + 1) * 32;
-    // raw weight ring (shared memory): per stage one SBYTES x 128 box per matrix (+ the NVFP4 scale atoms)
-    static constexpr int W_TILE = kTBM * CV::SBYTES;
-    static constexpr int RAW_STAGE = A_TILES * (W_TILE + CV::AUX);
+    // raw weight ring (shared memory): per entry a box of SUB stages per matrix (+ the NVFP4 scale atoms of these)
+    static constexpr int SUB = kBoxBytes / CV::SBYTES;
+    static constexpr int W_TILE = kTBM * kBoxBytes;
+    static constexpr int RAW_STAGE = A_TILES * (W_TILE + SUB * CV::AUX);
     static constexpr int BAR_BYTES = 512;
-    static constexpr int RAW_BUDGET = 224 * 1024 - SB * B_BYTES - BAR_BYTES - 1024;
+    static constexpr int RAW_BUDGET = 224 * 1024 - S * KS * B_BYTES - BAR_BYTES - 1024;
     static constexpr int RD_FIT = (RAW_BUDGET > 144 * 1024 ? 144 * 1024 : RAW_BUDGET) / RAW_STAGE;
     static constexpr int RD = RD_FIT > 12 ? 12 : RD_FIT;
     // One CTA per SM by construction (the CTA owns all of tensor memory): ask for more than half of the SM's shared memory.
-    static constexpr int SMEM_NEED = SB * B_BYTES + RD * RAW_STAGE + BAR_BYTES + 1024;
+    static constexpr int SMEM_NEED = S * KS * B_BYTES + RD * RAW_STAGE + BAR_BYTES + 1024;
     static constexpr int SMEM = SMEM_NEED < 120 * 1024 ? 120 * 1024 : SMEM_NEED;
-    static_assert(SA >= 3 && A_BASE + SA * A_COLS <= 512, "tensor memory budget");
+    static_assert(S >= 2 && A_BASE + S * A_COLS <= 512, "tensor memory budget");
     static_assert(RD >= 3 && SMEM <= 227 * 1024, "shared memory budget");
-    static_assert((2 * SA + 2 * SB + 2 * RD + 4) * 8 + 8 <= BAR_BYTES, "barrier area");
+    static_assert((3 * S + 2 * RD + 4) * 8 + 8 <= BAR_BYTES, "barrier area");
 };
 constexpr int kMaxSlots = 1 << 16;
 // Role-level time breakdown for tuning builds (-DLSB_MOE_PROFILE): block 0 accumulates the cycles each role spends
@@ -327,21 +337,27 @@ __device__ __forceinline__ void work_item(int w, int ntiles, int NT, int& t, int
 // Persistent kernel: one CTA per SM walks the work list (token tile x 128-row weight tile); the rings, their barrier
 // phases and the accumulator sets carry over from one work item to the next, so the producers run ahead across
 // item boundaries.
+// Position in a ring of N entries and the parity of the round.
+template <int N> struct RingPos {
+    uint32_t i = 0, ph = 0;
+    __device__ __forceinline__ void next() { if (++i == N) { i = 0; ph ^= 1u; } }
+    __device__ __forceinline__ void skip(uint32_t n) { i += n; if (i >= N) { i -= N; ph ^= 1u; } }       // n <= N
+};
+
 template <int FMT, int BN, bool GATEUP>
-__global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS) moe_tc_ffn_kernel(const __grid_constant__ CUtensorMap map_b,
+__global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS, 1) moe_tc_ffn_kernel(const __grid_constant__ CUtensorMap map_b,
                                                                                        const __grid_constant__ CUtensorMap map_w0,
                                                                                        const __grid_constant__ CUtensorMap map_w1, MoeTcParams p) {
     using C = MoeTcCfg<FMT, BN, GATEUP>;
     using CV = typename C::CV;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* smem_b = smem;                                   // [SB] token tiles
-    uint8_t* smem_r = smem + C::SB * C::B_BYTES;              // [RD] raw weight stages
+    uint8_t* smem_b = smem;                                   // [S][KS] token tiles
+    uint8_t* smem_r = smem + C::S * C::KS * C::B_BYTES;       // [RD] raw weight entries
     uint64_t* full_a = reinterpret_cast<uint64_t*>(smem_r + C::RD * C::RAW_STAGE);
-    uint64_t* empty_a = full_a + C::SA;
-    uint64_t* full_b = empty_a + C::SA;
-    uint64_t* empty_b = full_b + C::SB;
-    uint64_t* full_r = empty_b + C::SB;
+    uint64_t* full_b = full_a + C::S;
+    uint64_t* empty = full_b + C::S;             // both operands of a stage
+    uint64_t* full_r = empty + C::S;
     uint64_t* empty_r = full_r + C::RD;
     uint64_t* acc_full = empty_r + C::RD;        // [NBUF]
     uint64_t* acc_empty = acc_full + 2;          // [NBUF]
@@ -352,12 +368,11 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS) moe_tc_ffn
     const int K = GATEUP || up ? p.ef.H : p.ef.F;          // reduction length
     const int NOUT = GATEUP || up ? p.ef.F : p.ef.H;       // weight rows
     const int NT = NOUT / kTBM;
-    const int nkb = K / kTBK;
+    const int nkb = K / kTBK, nops = (nkb + C::KS - 1) / C::KS;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::SA; ++s) { mbar_init(&full_a[s], C::STAGE_WARPS); mbar_init(&empty_a[s], 1); }
-        for (int s = 0; s < C::SB; ++s) { mbar_init(&full_b[s], 1); mbar_init(&empty_b[s], 1); }
-        for (int s = 0; s < C::RD; ++s) { mbar_init(&full_r[s], 1); mbar_init(&empty_r[s], C::STAGE_WARPS); }
+        for (int s = 0; s < C::S; ++s) { mbar_init(&full_a[s], C::CONV_WARPS); mbar_init(&full_b[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < C::RD; ++s) { mbar_init(&full_r[s], 1); mbar_init(&empty_r[s], C::SUB == 1 ? C::SET_WARPS : C::CONV_WARPS); }
         for (int b = 0; b < C::NBUF; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], C::EPI_WARPS); }
         fence_barrier_init();
         fence_proxy_async();
@@ -386,6 +401,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS) moe_tc_ffn
     if (warp == 0) {
         if (lane == 0) {
             // ---------------- TMA producer: token tiles ----------------
+            RingPos<C::S> r;
             uint32_t g = 0;
             bool ok = true;
             PROF_DECL();
@@ -398,18 +414,19 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS) moe_tc_ffn
                     continue;
                 }
                 const int row0 = p.tile_row0[t];
-                for (int it = 0; it < nkb; ++it, ++g) {
-                    const int s = g % C::SB;
-                    PROF_SCOPE(0, ok = mbar_wait(&empty_b[s], ((g / C::SB) & 1) ^ 1, p.err, 11));
+                for (int o = 0; o < nops; ++o, ++g, r.next()) {
+                    PROF_SCOPE(0, ok = mbar_wait(&empty[r.i], r.ph ^ 1, p.err, 11));
                     if (!ok) break;
-                    mbar_expect_tx(&full_b[s], C::B_BYTES);
-                    tma_load_2d(smem_b + s * C::B_BYTES, &map_b, &full_b[s], it * kTBK, row0);
+                    const int n = min(C::KS, nkb - o * C::KS);
+                    mbar_expect_tx(&full_b[r.i], (uint32_t)(n * C::B_BYTES));
+                    for (int j = 0; j < n; ++j)
+                        tma_load_2d(smem_b + (r.i * C::KS + j) * C::B_BYTES, &map_b, &full_b[r.i], (o * C::KS + j) * kTBK, row0);
                 }
             }
             PROF_FLUSH(0, 1);
             if (!ok) {
                 // loads in flight still write this CTA's shared memory: let them land (bounded, no error code)
-                for (uint32_t i = g > (uint32_t)C::SB ? g - C::SB : 0; i < g; ++i) mbar_wait(&full_b[i % C::SB], (i / C::SB) & 1, nullptr, 0);
+                for (uint32_t i = g > (uint32_t)C::S ? g - C::S : 0; i < g; ++i) mbar_wait(&full_b[i % C::S], (i / C::S) & 1, nullptr, 0);
             }
         }
     } else if (warp == C::RAW_WARP) {
@@ -427,19 +444,21 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS) moe_tc_ffn
                 const uint8_t* sf0 = base + (GATEUP ? p.ef.off_sg : (up ? p.ef.off_su : p.ef.off_sd));
                 const uint8_t* sf1 = base + p.ef.off_su;
                 const int gtiles = ((K >> 4) + 3) >> 2;        // NVFP4: 512-byte scale atoms per 128-row tile
-                for (int it = 0; it < nkb; ++it, ++g) {
+                for (int it = 0; it < nkb; it += C::SUB, ++g) {
                     const int s = g % C::RD;
                     PROF_SCOPE(0, ok = mbar_wait(&empty_r[s], ((g / C::RD) & 1) ^ 1, p.err, 16));
                     if (!ok) break;
                     uint8_t* dst = smem_r + s * C::RAW_STAGE;
-                    mbar_expect_tx(&full_r[s], C::RAW_STAGE);
+                    // (a row's last box may reach past the row: zeros, never read; its scale atoms are those of the stages that are left)
+                    const uint32_t aux = (uint32_t)(min(C::SUB, nkb - it) * CV::AUX);
+                    mbar_expect_tx(&full_r[s], C::A_TILES * (C::W_TILE + aux));
                     const int x = CV::stage_x(it);
                     tma_load_3d(dst, &map_w0, &full_r[s], x, jn * kTBM, slot);
                     if (GATEUP) tma_load_3d(dst + C::W_TILE, &map_w1, &full_r[s], x, jn * kTBM, slot);
                     if (CV::AUX) {
                         const size_t so = ((size_t)jn * gtiles + it) * 512;
-                        bulk_load_1d(dst + C::A_TILES * C::W_TILE, sf0 + so, 512, &full_r[s]);
-                        if (GATEUP) bulk_load_1d(dst + C::A_TILES * C::W_TILE + 512, sf1 + so, 512, &full_r[s]);
+                        bulk_load_1d(dst + C::A_TILES * C::W_TILE, sf0 + so, aux, &full_r[s]);
+                        if (GATEUP) bulk_load_1d(dst + C::A_TILES * C::W_TILE + C::SUB * CV::AUX, sf1 + so, aux, &full_r[s]);
                     }
                 }
             }
@@ -449,55 +468,69 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS) moe_tc_ffn
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // ---------------- MMA issuer: A (weights) from tensor memory, B (tokens) from shared memory ----------------
-            constexpr uint32_t idesc = idesc_f16(kTBM, BN, 0);
-            uint32_t g = 0, lt = 0;
-            bool ok = true;
-            PROF_DECL();
-            for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
-                int t, jn;
-                work_item(w, ntiles, NT, t, jn);
-                if (!slot_ok(p.slot_of[p.tile_expert[t]])) continue;
-                const uint32_t buf = lt % C::NBUF;
-                PROF_SCOPE(0, ok = mbar_wait(&acc_empty[buf], ((lt / C::NBUF) & 1u) ^ 1u, p.err, 15));   // epilogue has drained this accumulator set
+        // ---------------- MMA issuer: A (weights) from tensor memory, B (tokens) from shared memory ----------------
+        // The whole warp walks the list (loop bounds and ring positions stay warp-uniform, so the operands of the instructions are uniform
+        // registers) and one elected lane issues.
+        constexpr uint32_t idesc = idesc_f16(kTBM, BN, 0);
+        const int utotal = __reduce_max_sync(0xffffffffu, total), untiles = __reduce_max_sync(0xffffffffu, ntiles);
+        const uint32_t ut = __reduce_max_sync(0xffffffffu, tmem_d);
+        RingPos<C::S> r;
+        uint32_t lt = 0;
+        bool ok = true;
+        PROF_DECL();
+        for (int w = blockIdx.x; w < utotal && ok; w += gridDim.x) {
+            int t, jn;
+            work_item(w, untiles, NT, t, jn);
+            if (!__reduce_or_sync(0xffffffffu, slot_ok(p.slot_of[p.tile_expert[t]]) ? 1u : 0u)) continue;
+            const uint32_t buf = lt % C::NBUF;
+            PROF_SCOPE(0, ok = mbar_wait(&acc_empty[buf], ((lt / C::NBUF) & 1u) ^ 1u, p.err, 15));   // epilogue has drained this accumulator set
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t acc = ut + buf * C::ACC_COLS;
+            for (int o = 0; o < nops; ++o, r.next()) {
+                PROF_SCOPE(1, ok = mbar_wait(&full_b[r.i], r.ph, p.err, 12));
+                if (ok) PROF_SCOPE(2, ok = mbar_wait(&full_a[r.i], r.ph, p.err, 12));
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t acc = tmem_d + buf * C::ACC_COLS;
-                for (int it = 0; it < nkb; ++it, ++g) {
-                    const int sa = g % C::SA, sb = g % C::SB;
-                    PROF_SCOPE(1, ok = mbar_wait(&full_b[sb], (g / C::SB) & 1, p.err, 12));
-                    if (ok) PROF_SCOPE(2, ok = mbar_wait(&full_a[sa], (g / C::SA) & 1, p.err, 12));
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t a_t = tmem_d + C::A_BASE + sa * C::A_COLS;
-                    const uint64_t db = smem_desc_sw128(smem_b + sb * C::B_BYTES);
-                    PROF_SCOPE(3, {
+                const uint32_t a_t = ut + C::A_BASE + r.i * C::A_COLS;
+                const uint64_t db = smem_desc_sw128(smem_b + r.i * C::KS * C::B_BYTES);
+                const int n = min(C::KS, nkb - o * C::KS);
+                PROF_SCOPE(3, {
+                if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < kTBK / 16; ++k) {
-                        const uint32_t accum = (it > 0 || k > 0) ? 1u : 0u;
-                        umma_f16_ts(acc, a_t + 8 * k, db + 2 * k, idesc, accum);
-                        if (GATEUP) umma_f16_ts(acc + BN, a_t + 32 + 8 * k, db + 2 * k, idesc, accum);
+                    for (int j = 0; j < C::KS; ++j) {
+                        if (j > 0 && j >= n) break;
+#pragma unroll
+                        for (int k = 0; k < kTBK / 16; ++k) {
+                            const uint32_t accum = (o > 0 || j > 0 || k > 0) ? 1u : 0u;
+                            const uint64_t b = db + (uint64_t)(j * (C::B_BYTES >> 4) + 2 * k);
+                            umma_f16_ts(acc, a_t + j * 32 * C::A_TILES + 8 * k, b, idesc, accum);
+                            if (GATEUP) umma_f16_ts(acc + BN, a_t + j * 32 * C::A_TILES + 32 + 8 * k, b, idesc, accum);
+                        }
                     }
-                    umma_commit(&empty_a[sa]);
-                    umma_commit(&empty_b[sb]); });
+                    umma_commit(&empty[r.i]);
                 }
-                if (ok) umma_commit(&acc_full[buf]);
-                ++lt;
+                __syncwarp(); });
             }
-            PROF_FLUSH(0, 4); PROF_FLUSH(1, 2); PROF_FLUSH(2, 3); PROF_FLUSH(3, 14); PROF_TOTAL(5);
+            if (ok && elect_one()) umma_commit(&acc_full[buf]);
+            __syncwarp();
+            ++lt;
         }
+        if (lane == 0) { PROF_FLUSH(0, 4); PROF_FLUSH(1, 2); PROF_FLUSH(2, 3); PROF_FLUSH(3, 14); PROF_TOTAL(5); }
     } else if (warp < 2 + C::CONV_WARPS) {
         // ---------------- weight converters ----------------
         constexpr int NC = 32 / C::NH;
         const int q = warp & 3;                                // TMEM lane quarter this warp may access
         const int part = ((warp - 2) >> 2) & 1;                // gate/up: matrix (0 gate, 1 up); down: half of the stage's K range
-        const int grp = (warp - 2) >> 3;                       // this warp converts the stages with g % CONV_GROUPS == grp
+        const int set = (warp - 2) >> 3;                       // this warp converts the sub-stages `it` with it % CONV_SETS == set
         const int row = q * 32 + lane;                         // row of the 128-row weight tile = TMEM lane
         const int h = GATEUP ? 0 : part;
         const int mat = GATEUP ? part : 0;
         const uint32_t t_lane = tmem_d + C::A_BASE + ((uint32_t)(q * 32) << 16) + (GATEUP ? part * 32 : part * NC);
-        uint32_t g = 0;
+        RingPos<C::S> ra;                                      // operand stages
+        RingPos<C::RD> rr;                                     // raw entries
         bool ok = true;
         PROF_DECL();
         for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
@@ -511,57 +544,80 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS) moe_tc_ffn
             const int n = jn * kTBM + row;                     // weight row in the expert matrix
             // side data that does not travel through the ring: the FP8 block scale (one float per 128 x 128 block, the
             // same for the whole tile) and the Q4_K super-block header (16 bytes per row and 256 elements), both read
-            // one handled stage ahead of their use
+            // one stage ahead of their use
             const float* fsc = reinterpret_cast<const float*>(sf) + (size_t)(n >> 7) * ((K + 127) >> 7);
             const uint8_t* qrow = wm + (size_t)n * CV::pitch(K);
-            const int it_first = (int)((grp + C::CONV_GROUPS - g % C::CONV_GROUPS) % C::CONV_GROUPS);   // first stage of this item that is ours
             float sc_next = 0.f;
             uint4 hdr_next = make_uint4(0, 0, 0, 0);
-            if (FMT == 1 && it_first < nkb) sc_next = __ldg(fsc + (it_first >> 1));
-            if (FMT == 3 && it_first < nkb) hdr_next = __ldg(reinterpret_cast<const uint4*>(qrow + (size_t)(it_first >> 2) * 144));
+            if (FMT == 1) sc_next = __ldg(fsc);
+            if (FMT == 3) hdr_next = __ldg(reinterpret_cast<const uint4*>(qrow));
+            const int nent = (nkb + C::SUB - 1) / C::SUB;
+            typename CV::Raw raw;
+            // Straight-line code for the sub-stages of whole entries and whole operand stages: the instructions around a sub-stage (ring
+            // positions, which barrier is due) cost as much as its conversion when they are decided at run time.
+            constexpr int BLK = C::SUB > C::KS ? C::SUB : C::KS;
+            int okw = 1;
 #pragma unroll 1
-            for (int it = 0; it < nkb && ok; ++it) {
-                if ((int)(g % C::CONV_GROUPS) != grp) { ++g; continue; }
-                typename CV::Raw raw;
-                const int itn = it + C::CONV_GROUPS;               // next stage of this item that is ours
-                if constexpr (FMT == 1) {
-                    raw.sc = sc_next;
-                    if (itn < nkb) sc_next = __ldg(fsc + (itn >> 1));
+            for (int b0 = 0; b0 < nkb && ok; b0 += BLK) {
+#pragma unroll
+                for (int i = 0; i < BLK / C::CONV_SETS; ++i) {
+                    const int l0 = i * C::CONV_SETS, l = l0 + set;       // sub-stages of both sets; this warp's
+                    if (b0 + l0 >= nkb) break;
+                    const bool mine = C::SUB > 1 || b0 + l < nkb;        // (past an odd end: zeros into columns that no MMA reads, or no entry at all)
+                    RingPos<C::RD> re = rr;
+                    if (C::SUB == 1) re.skip(l);
+                    if (C::SUB == 1 || l0 % C::SUB == 0) {
+                        if constexpr (FMT == 1) {
+                            raw.sc = sc_next;
+                            const int e = (b0 + l0) / C::SUB + 1;
+                            if (e < nent) sc_next = __ldg(fsc + e);
+                        }
+                        if constexpr (FMT == 3) {
+                            raw.hdr = hdr_next;
+                            const int e = (b0 + l0) / C::SUB + 1;
+                            if (e < nent) hdr_next = __ldg(reinterpret_cast<const uint4*>(qrow + (size_t)e * 144));
+                        }
+                        // one lane polls the barrier, the warp sleeps at the sync: waiting warps leave the issue slots alone
+                        if (lane == 0 && mine) { if (warp == 2) PROF_SCOPE(0, okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0); else okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0; }
+                        ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
+                        if (!ok) break;
+                    }
+                    uint32_t out[NC];
+                    if (mine) {
+                        const uint32_t entry = smem_u32(smem_r + re.i * C::RAW_STAGE);
+                        const int sub = l % C::SUB;
+                        CV::fetch(raw, entry + mat * C::W_TILE, row, h, sub);
+                        if constexpr (FMT == 2) {
+                            // scale atom of the 128-row tile: word (row % 32) * 4 + row / 32
+                            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(raw.sc) : "r"(entry + C::A_TILES * C::W_TILE + (mat * C::SUB + sub) * 512 + lane * 16 + q * 4) : "memory");
+                        }
+                        CV::convert(raw, out, (b0 + l) * kTBK, h);       // consumes every byte read above
+                    }
+                    if (C::SUB == 1 || (l0 + C::CONV_SETS) % C::SUB == 0 || b0 + l0 + C::CONV_SETS >= nkb) {
+                        __syncwarp();
+                        if (lane == 0 && mine) mbar_arrive(&empty_r[re.i]);        // the raw entry may be refilled
+                        if (C::SUB > 1) rr.next();
+                    }
+                    if (l0 % C::KS == 0) {
+                        if (lane == 0) { if (warp == 2) PROF_SCOPE(1, okw = mbar_wait(&empty[ra.i], ra.ph ^ 1, p.err, 13) ? 1 : 0); else okw = mbar_wait(&empty[ra.i], ra.ph ^ 1, p.err, 13) ? 1 : 0; }
+                        ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
+                        if (!ok) break;
+                        tc_fence_after();                      // the MMAs that read this operand stage have completed
+                    }
+                    if (mine) {
+                        const uint32_t dst = t_lane + ra.i * C::A_COLS + (l % C::KS) * 32 * C::A_TILES;
+                        if (NC == 32) tmem_st32(dst, out);
+                        else tmem_st16(dst, out);
+                    }
+                    if ((l0 + C::CONV_SETS) % C::KS == 0 || b0 + l0 + C::CONV_SETS >= nkb) {
+                        PROF_SCOPE(3, tmem_wait_st());
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&full_a[ra.i]);
+                        ra.next();
+                    }
                 }
-                if constexpr (FMT == 3) {
-                    raw.hdr = hdr_next;
-                    if (itn < nkb) hdr_next = __ldg(reinterpret_cast<const uint4*>(qrow + (size_t)(itn >> 2) * 144));
-                }
-                const int rs = g % C::RD, s = g % C::SA;
-                // one lane polls the barrier, the warp sleeps at the sync: waiting warps leave the issue slots alone
-                int okw = 1;
-                if (lane == 0) { if (warp == 2) PROF_SCOPE(0, okw = mbar_wait(&full_r[rs], (g / C::RD) & 1, p.err, 17) ? 1 : 0); else okw = mbar_wait(&full_r[rs], (g / C::RD) & 1, p.err, 17) ? 1 : 0; }
-                ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
-                if (!ok) break;
-                const uint32_t stage = smem_u32(smem_r + rs * C::RAW_STAGE);
-                CV::fetch(raw, stage + mat * C::W_TILE, row, h);
-                if constexpr (FMT == 2) {
-                    // scale atom of the 128-row tile: word (row % 32) * 4 + row / 32
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(raw.sc) : "r"(stage + C::A_TILES * C::W_TILE + mat * 512 + lane * 16 + q * 4) : "memory");
-                }
-                uint32_t out[NC];
-                CV::convert(raw, out, it * kTBK, h);           // consumes every byte read above
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&empty_r[rs]);                 // the raw stage may be refilled
-                    if (warp == 2) PROF_SCOPE(1, okw = mbar_wait(&empty_a[s], ((g / C::SA) & 1) ^ 1, p.err, 13) ? 1 : 0); else okw = mbar_wait(&empty_a[s], ((g / C::SA) & 1) ^ 1, p.err, 13) ? 1 : 0;
-                }
-                ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
-                if (!ok) break;
-                tc_fence_after();                              // the MMAs that read this operand stage have completed
-                PROF_SCOPE(3, {
-                    if (NC == 32) tmem_st32(t_lane + s * C::A_COLS, out);
-                    else tmem_st16(t_lane + s * C::A_COLS, out);
-                    tmem_wait_st(); });
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full_a[s]);
-                ++g;
+                if (C::SUB == 1) rr.skip(min(BLK, nkb - b0));
             }
         }
         if (warp == 2 && lane == 0) { PROF_FLUSH(0, 6); PROF_FLUSH(1, 8); PROF_FLUSH(2, 7); PROF_FLUSH(3, 9); PROF_TOTAL(10); }
@@ -648,19 +704,19 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS) moe_tc_ffn
 
 int make_map_bytes_3d(CUtensorMap* map, const void* ptr, uint64_t pitch, uint64_t rows, uint64_t slot_stride, uint64_t nslots,
                       uint32_t box_bytes, uint32_t box_rows);
-static int cached_map_w(CUtensorMap* out, const void* ptr, uint64_t pitch, uint64_t rows, uint64_t sstride, uint64_t nslots, int sbytes) {
+static int cached_map_w(CUtensorMap* out, const void* ptr, uint64_t pitch, uint64_t rows, uint64_t sstride, uint64_t nslots) {
     struct Key {
-        const void* p; uint64_t pitch, rows, ss, ns; int sb;
-        bool operator<(const Key& o) const { return std::tie(p, pitch, rows, ss, ns, sb) < std::tie(o.p, o.pitch, o.rows, o.ss, o.ns, o.sb); }
+        const void* p; uint64_t pitch, rows, ss, ns;
+        bool operator<(const Key& o) const { return std::tie(p, pitch, rows, ss, ns) < std::tie(o.p, o.pitch, o.rows, o.ss, o.ns); }
     };
     static std::map<Key, CUtensorMap> cache;
     static std::mutex mu;
     std::lock_guard<std::mutex> g(mu);
-    const Key k{ptr, pitch, rows, sstride, nslots, sbytes};
+    const Key k{ptr, pitch, rows, sstride, nslots};
     auto it = cache.find(k);
     if (it != cache.end()) { *out = it->second; return 0; }
     CUtensorMap m;
-    const int rc = make_map_bytes_3d(&m, ptr, pitch, rows, sstride, nslots, (uint32_t)sbytes, (uint32_t)kTBM);
+    const int rc = make_map_bytes_3d(&m, ptr, pitch, rows, sstride, nslots, (uint32_t)kBoxBytes, (uint32_t)kTBM);
     if (rc) return rc;
     if (cache.size() > 65536) cache.clear();
     cache[k] = m;
@@ -680,7 +736,6 @@ static int sm_count() {
 
 template <int FMT, int BN, bool GATEUP>
 static int launch_moe_tc(const CUtensorMap& mb, const MoeTcParams& p, int nout, int max_tiles, cudaStream_t st) {
-    using CVt = typename MoeTcCfg<FMT, BN, GATEUP>::CV;
     const int Kred = GATEUP || p.up ? p.ef.H : p.ef.F;
     CUtensorMap mw0, mw1;
     {
@@ -689,9 +744,9 @@ static int launch_moe_tc(const CUtensorMap& mb, const MoeTcParams& p, int nout, 
         const bool dense = p.ef.stride == 0;
         const uint64_t sstride = dense ? pitch * (uint64_t)nout : (uint64_t)p.ef.stride;
         const uint64_t nslots = dense ? 1 : (uint64_t)kMaxSlots;
-        int rc = cached_map_w(&mw0, p.arena + (GATEUP ? p.ef.off_gate : (p.up ? p.ef.off_up : p.ef.off_down)), pitch, (uint64_t)nout, sstride, nslots, CVt::SBYTES);
+        int rc = cached_map_w(&mw0, p.arena + (GATEUP ? p.ef.off_gate : (p.up ? p.ef.off_up : p.ef.off_down)), pitch, (uint64_t)nout, sstride, nslots);
         if (rc) return rc;
-        if (GATEUP) { rc = cached_map_w(&mw1, p.arena + p.ef.off_up, pitch, (uint64_t)nout, sstride, nslots, CVt::SBYTES); if (rc) return rc; }
+        if (GATEUP) { rc = cached_map_w(&mw1, p.arena + p.ef.off_up, pitch, (uint64_t)nout, sstride, nslots); if (rc) return rc; }
         else mw1 = mw0;
     }
     using C = MoeTcCfg<FMT, BN, GATEUP>;

@@ -109,3 +109,37 @@ def test_engine_prefill_uses_grouped_path_and_matches_oracle():
             outs.append(lg)
             eng.free_sequence(sid)
         assert float((outs[0] - outs[1]).abs().max() / outs[1].abs().max()) < 2e-2
+
+
+@pytest.mark.parametrize("fmt,H,F", [("nvfp4", 128, 128), ("nvfp4", 384, 640), ("nvfp4", 1152, 128), ("fp8_e4m3", 128, 384), ("fp8_e4m3", 640, 128), ("bf16", 128, 384),
+                                     ("bf16", 1152, 128), ("gguf_q4_k", 256, 768), ("gguf_q4_k", 1280, 256)])
+@pytest.mark.parametrize("BN", [32, 64, 128])
+def test_widths_that_end_inside_boxes_and_operand_stages(fmt, H, F, BN):
+    """Reduction lengths shorter than a weight box, that end inside one, inside an operand stage, and that wrap the rings; more work items than CTAs."""
+    from layerstorm_b200.ops import _native as nat
+    dev = torch.device("cuda")
+    E, R = 20, 2 * BN + 1
+    arena, ref = _setup(fmt, H, F, E, n_missing=0, seed=3)
+    g = torch.Generator(device="cpu").manual_seed(4)
+    x = torch.randn(R, H, generator=g).to(torch.bfloat16).to(dev)
+    ids = torch.stack([torch.full((R,), E - 1), torch.arange(R) % (E - 1)], 1).int().to(dev).contiguous()
+    P, tiles = R * 2, R * 2 // BN + E + 1
+    i32 = dict(dtype=torch.int32, device=dev)
+    srt, te, tr, tn, cnt, err = (torch.zeros(n, **i32) for n in (P, tiles, tiles, tiles, 2, 1))
+    xs, act = torch.zeros(P, H, dtype=torch.float16, device=dev), torch.zeros(P, F, dtype=torch.float16, device=dev)
+    y = torch.full((P, H), float("nan"), device=dev)
+    efp = ctypes.addressof(arena.ef)
+    nat.call("lsb_moe_tc_sort", ids, P, E, BN, srt, te, tr, tn, cnt)
+    nat.call("lsb_moe_tc_gather", x, srt, cnt, xs, P, 2, H)
+    nat.call("lsb_moe_tc_ffn", 1, xs, P, arena.data, arena.slot_of, efp, te, tr, tn, cnt, srt, act, BN, tiles, 0.0, None, err, None)
+    nat.call("lsb_moe_tc_ffn", 0, act, P, arena.data, arena.slot_of, efp, te, tr, tn, cnt, srt, y, BN, tiles, 0.0, None, err, None)
+    torch.cuda.synchronize()
+    assert int(err) == 0
+    xd, idc, got = x.double().cpu(), ids.cpu(), y.double().cpu()
+    for e in range(E):
+        gate, up, down = ref[e]
+        r, k = (idc == e).nonzero(as_tuple=True)
+        want = (torch.nn.functional.silu(xd[r] @ gate.T) * (xd[r] @ up.T)) @ down.T
+        # a hidden value rounded to fp16, at most 2^-11 relative per term (NVFP4, FP8 and bf16 weights are exact in fp16).  Q4_K weights are d sc v - dmin m
+        # with both products rounded to fp16, 2^-11 of terms up to 15 d sc and 8 d sc in size around weights of 4.6 d sc rms: 2.4e-3 at most
+        assert float((got[r * 2 + k] - want).norm() / want.norm()) < (3e-3 if fmt == "gguf_q4_k" else 1e-3), e
