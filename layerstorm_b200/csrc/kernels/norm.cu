@@ -358,6 +358,182 @@ __global__ void __launch_bounds__(512) mhc_finalize_kernel(bf16* __restrict__ ou
 }
 
 
+// ---- many-row variant: one launch ---------------------------------------------------------------------------------------
+// A block owns RPB whole rows, a warp each.  Per step of 128 hidden columns a warp updates its row's streams (16 values a lane, stored and
+// put into shared memory beside the next tile of `fn`, which cp.async brings a step ahead), then the block adds the step's 512 products to
+// the RPB x 24 mixing logits: a warp takes a slice of the 512, eight lanes a quarter of it, a lane RPB / 2 rows x 6 logits, so that 14 16-byte
+// shared reads feed 192 FMAs (of RPB = 16), and nothing is summed across lanes before the last step.  The gates, the contraction and the norm follow in the same launch.
+// Bound by the streams' traffic (read, written, read again from L2 for the contraction) and `fn` out of L2 once per block.  The two launches
+// it replaces for these rows (partials by 128-column blocks, one block per row to finish) computed the update in each of four warps and
+// summed seven values across lanes per row and 128 columns.  2048 rows of 4 x 4096: 371 -> 168 us (traffic at DRAM's rate: 49 us).
+constexpr int kHrCols = 128, kHrLd = kHcMax * kHrCols + 4;                // tile stride in floats: 16-byte aligned, rows four banks apart
+template <int RPB> struct HrCfg {
+    static constexpr int RES = RPB * kHrLd, FN = kHcOut * kHrLd;          // floats
+    static constexpr int SMEM = (RES + 2 * FN) * 4;
+    static_assert(RPB * RPB * kHcOut <= 2 * FN, "logit partials fit the tiles");
+};
+
+__device__ __forceinline__ void hr_cp_async(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+template <int RPB>
+__global__ void __launch_bounds__(RPB * 32, 1) mhc_rows_kernel(bf16* __restrict__ out, float* residual, const float* __restrict__ x, float* __restrict__ post,
+                                                               float* __restrict__ comb, const float* __restrict__ fn, const float* __restrict__ hc_scale,
+                                                               const float* __restrict__ hc_base, const float* __restrict__ norm_w, int rows, int hidden, int mode,
+                                                               int iters, float hc_eps, float rms_eps, float post_mult) {
+    constexpr int N = kHcMax, RL = RPB / 2, QW = N * kHrCols / 4 / RPB;    // rows per lane, quads per warp and step
+    extern __shared__ __align__(16) float hsm[];
+    float* s_res = hsm;
+    float* s_fn = hsm + HrCfg<RPB>::RES;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kq = lane >> 3, rg = (lane >> 2) & 1, og = lane & 3;
+    const int r = blockIdx.x * RPB + warp, steps = hidden / kHrCols;
+    auto fetch_fn = [&](int c) {
+        float* dst = s_fn + (c & 1) * HrCfg<RPB>::FN;
+        for (int i = threadIdx.x; i < kHcOut * N * (kHrCols / 4); i += RPB * 32) {
+            const int oj = i / (kHrCols / 4), q = i % (kHrCols / 4);
+            hr_cp_async(dst + (oj / N) * kHrLd + (oj % N) * kHrCols + q * 4, fn + (size_t)oj * hidden + c * kHrCols + q * 4);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch_fn(0);
+    pdl_wait();
+    pdl_launch_dependents();
+    const bool live = r < rows;
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    float* rp = residual + (size_t)r * N * hidden + lane * 4;
+    const float* xp = x + (size_t)r * hidden + lane * 4;
+    float pj[N], cj[N][N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        pj[j] = live && mode ? post[r * N + j] : 1.f;                      // mode 0: every stream starts as x
+#pragma unroll
+        for (int i = 0; i < N; ++i) cj[i][j] = live && mode ? comb[(r * N + i) * N + j] : 0.f;
+    }
+    float4 xv = z4, old[N];
+    auto load = [&](int c) {
+        if (live) xv = *reinterpret_cast<const float4*>(xp + c * kHrCols);
+#pragma unroll
+        for (int i = 0; i < N; ++i) old[i] = live && mode ? *reinterpret_cast<const float4*>(rp + (size_t)i * hidden + c * kHrCols) : z4;
+    };
+    load(0);
+    float acc[RL][6], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < RL; ++i)
+#pragma unroll
+        for (int q = 0; q < 6; ++q) acc[i][q] = 0.f;
+    for (int c = 0; c < steps; ++c) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            float4 a = make_float4(pj[j] * xv.x, pj[j] * xv.y, pj[j] * xv.z, pj[j] * xv.w);
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                a.x += cj[i][j] * old[i].x; a.y += cj[i][j] * old[i].y; a.z += cj[i][j] * old[i].z; a.w += cj[i][j] * old[i].w;
+            }
+            if (live) *reinterpret_cast<float4*>(rp + (size_t)j * hidden + c * kHrCols) = a;
+            *reinterpret_cast<float4*>(s_res + warp * kHrLd + j * kHrCols + lane * 4) = a;
+            ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+        }
+        if (c + 1 < steps) {
+            load(c + 1);
+            fetch_fn(c + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const float* ft = s_fn + (c & 1) * HrCfg<RPB>::FN + og * kHrLd;
+        const float* rt = s_res + rg * kHrLd;
+#pragma unroll 2
+        for (int u = 0; u < QW; u += 4) {
+            const int k = (warp * QW + u + kq) * 4;
+            float4 b[6];
+#pragma unroll
+            for (int q = 0; q < 6; ++q) b[q] = *reinterpret_cast<const float4*>(ft + q * 4 * kHrLd + k);
+#pragma unroll
+            for (int i = 0; i < RL; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(rt + i * 2 * kHrLd + k);
+#pragma unroll
+                for (int q = 0; q < 6; ++q) acc[i][q] = fmaf(a.x, b[q].x, fmaf(a.y, b[q].y, fmaf(a.z, b[q].z, fmaf(a.w, b[q].w, acc[i][q]))));
+            }
+        }
+        __syncthreads();                                                   // the tiles are rewritten by the next step
+    }
+    // logits of a row: the warps' shares in order; lane o < 24 of the row's warp holds logit o
+    float* s_part = s_fn;
+#pragma unroll
+    for (int i = 0; i < RL; ++i)
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            float a = acc[i][q];
+            a += __shfl_xor_sync(0xffffffffu, a, 8);
+            a += __shfl_xor_sync(0xffffffffu, a, 16);
+            if (kq == 0) s_part[(warp * RPB + rg + 2 * i) * kHcOut + og + 4 * q] = a;
+        }
+    __syncthreads();
+    float m = 0.f;
+    if (lane < kHcOut)
+        for (int w = 0; w < RPB; ++w) m += s_part[(w * RPB + warp) * kHcOut + lane];
+    __syncthreads();                                                       // shared memory is free
+    ss = warp_sum(ss);
+    const float inv = rsqrtf(ss / (float)(N * hidden) + rms_eps);
+    {
+        const int t = lane & 15;                                           // element (t / 4, t % 4) of the mixing matrix, twice over
+        const float v = __shfl_sync(0xffffffffu, m, 2 * N + t) * inv * hc_scale[2] + hc_base[2 * N + t];
+        float mx = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float e = expf(v - mx);
+        float s = e + __shfl_xor_sync(0xffffffffu, e, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        float cm = e / s + hc_eps;
+        float cs = cm + __shfl_xor_sync(0xffffffffu, cm, 4);
+        cs += __shfl_xor_sync(0xffffffffu, cs, 8);
+        cm = cm / (cs + hc_eps);
+        for (int it = 1; it < iters; ++it) {
+            float rs = cm + __shfl_xor_sync(0xffffffffu, cm, 1);
+            rs += __shfl_xor_sync(0xffffffffu, rs, 2);
+            cm = cm / (rs + hc_eps);
+            cs = cm + __shfl_xor_sync(0xffffffffu, cm, 4);
+            cs += __shfl_xor_sync(0xffffffffu, cs, 8);
+            cm = cm / (cs + hc_eps);
+        }
+        if (live && lane < 16) comb[r * N * N + t] = cm;
+    }
+    float pre[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) pre[j] = sigmoidf_(__shfl_sync(0xffffffffu, m, j) * inv * hc_scale[0] + hc_base[j]) + hc_eps;
+    const float mp = __shfl_sync(0xffffffffu, m, N + (lane & (N - 1)));
+    if (live && lane < N) post[r * N + lane] = sigmoidf_(mp * inv * hc_scale[1] + hc_base[N + lane]) * post_mult;
+    if (!live) return;
+    // contraction and norm over what this thread has written; steps that fit shared memory are kept there between the two passes
+    const int kept = min(steps, HrCfg<RPB>::SMEM / (RPB * kHrCols * 4));
+    float* s_row = hsm + (size_t)warp * kept * kHrCols + lane * 4;
+    auto contract = [&](int c) {
+        float4 a = z4;
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const float4 v = *reinterpret_cast<const float4*>(rp + (size_t)j * hidden + c * kHrCols);
+            a.x += pre[j] * v.x; a.y += pre[j] * v.y; a.z += pre[j] * v.z; a.w += pre[j] * v.w;
+        }
+        return a;
+    };
+    ss = 0.f;
+#pragma unroll 4
+    for (int c = steps - 1; c >= 0; --c) {                                 // the columns written last are the nearest
+        const float4 a = contract(c);
+        ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+        if (c < kept) *reinterpret_cast<float4*>(s_row + c * kHrCols) = a;
+    }
+    const float ninv = rsqrtf(warp_sum(ss) / (float)hidden + rms_eps);
+#pragma unroll 4
+    for (int c = 0; c < steps; ++c) {
+        const float4 a = c < kept ? *reinterpret_cast<const float4*>(s_row + c * kHrCols) : contract(c);
+        const float4 w = __ldg(reinterpret_cast<const float4*>(norm_w + c * kHrCols + lane * 4));
+        bf162 o[2] = {__floats2bfloat162_rn(a.x * ninv * w.x, a.y * ninv * w.y), __floats2bfloat162_rn(a.z * ninv * w.z, a.w * ninv * w.w)};
+        *reinterpret_cast<uint2*>(out + (size_t)r * hidden + c * kHrCols + lane * 4) = *reinterpret_cast<uint2*>(o);
+    }
+}
+
 // ---- few-row (decode) variant: two launches instead of partial + one-block-per-row finalize -------------------------------
 // mhc_post_fused: same residual update and partial mixing logits as mhc_post_partial, plus the partial Gram matrix
 // G[j][j'] = sum_h res_j[h] res_j'[h] of the new residual streams.  The last block of a row to finish (atomic counter)
@@ -670,6 +846,24 @@ LSB_API int lsb_mhc_post_pre(void* out_x, void* residual, const void* x, void* p
                    iters, hc_eps, rms_eps, post_mult, comm_from_host(comm));
         launch_pdl((mhc_contract_kernel), dim3(rows, (hidden / 4 + 255) / 256), 256, 0, st, (bf16*)out_x, (const float*)residual, (const float*)prex,
                    (const float*)norm_w, hidden, n);
+        LSB_CHECK_LAUNCH();
+    }
+    // Whole rows per block, as many as keep the blocks to one wave.  The line against the two-launch form (one wave takes 76 us of 4096 columns
+    // whatever the rows, hidden / 128 steps of a load, an exchange and a product): 256 rows 76 against 66 us, 391 rows 76 against 95, 1024 rows
+    // 96 against 194, 2048 rows 168 against 371.
+    if (!comm && n == kHcMax && hidden % kHrCols == 0 && rows >= 352 && ((uintptr_t)norm_w & 15) == 0 && ((uintptr_t)fn & 15) == 0 && ((uintptr_t)x & 15) == 0
+        && ((uintptr_t)residual & 15) == 0 && ((uintptr_t)out_x & 7) == 0) {
+        auto go = [&](auto tag) {
+            constexpr int RPB = decltype(tag)::value;
+            static const cudaError_t attr = cudaFuncSetAttribute(mhc_rows_kernel<RPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, HrCfg<RPB>::SMEM);
+            (void)attr;
+            launch_pdl((mhc_rows_kernel<RPB>), (rows + RPB - 1) / RPB, RPB * 32, HrCfg<RPB>::SMEM, st, (bf16*)out_x, (float*)residual, (const float*)x, (float*)post,
+                       (float*)comb, (const float*)fn, (const float*)hc_scale, (const float*)hc_base, (const float*)norm_w, rows, hidden, mode, iters, hc_eps, rms_eps,
+                       post_mult);
+        };
+        if (rows > 8 * 148) go(std::integral_constant<int, 16>{});
+        else if (rows > 4 * 148) go(std::integral_constant<int, 8>{});
+        else go(std::integral_constant<int, 4>{});
         LSB_CHECK_LAUNCH();
     }
     const int rpb = rows >= 64 ? 16 : 1;      // many rows: amortise the mixing-matrix loads over 16 rows per block

@@ -543,3 +543,32 @@ def test_fp8_indexer_scores_over_the_cached_keys_match_the_cuda_core_kernel(R, I
             k = 64
             ta, tb = set(a.topk(k).indices.tolist()), set(b.topk(k).indices.tolist())
             assert len(ta & tb) >= 0.8 * k, len(ta & tb)
+
+
+@pytest.mark.parametrize("rows", [352, 592, 593, 1184, 1185])
+@pytest.mark.parametrize("H,mode", [(128, 1), (1152, 1), (4352, 1), (256, 0)])
+def test_hyper_connection_pass_of_many_rows(rows, H, mode):
+    """One launch for whole rows: 4, 8 and 16 rows per block, a last block that is not full, widths of one step and of more steps than shared memory keeps."""
+    from layerstorm_b200.ops import _native as nat
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, res, fn, base, nw = rnd(rows, H), rnd(rows, 4, H), rnd(24, 4 * H) * (0.3 / H ** 0.5), rnd(24) * 0.5, 1 + 0.1 * rnd(H)
+    scale, post, comb = torch.tensor([0.7, 1.1, 1.3], device="cuda"), torch.rand(rows, 4, generator=g, device="cuda"), torch.rand(rows, 4, 4, generator=g, device="cuda") / 4
+    x64, r64 = x.double(), res.double()
+    want_r = torch.einsum("tij,tih->tjh", comb.double(), r64) + post.double()[:, :, None] * x64[:, None] if mode else x64[:, None].repeat(1, 4, 1)
+    flat = want_r.flatten(1)
+    m = (flat @ fn.double().T) * torch.rsqrt(flat.square().mean(-1, keepdim=True) + 1e-5)
+    m = m * scale.double().repeat_interleave(torch.tensor([4, 4, 16], device="cuda")) + base.double()
+    k = torch.softmax(m[:, 8:].view(-1, 4, 4), -1) + 1e-6
+    k = k / (k.sum(-2, keepdim=True) + 1e-6)
+    for _ in range(19):
+        k = k / (k.sum(-1, keepdim=True) + 1e-6)
+        k = k / (k.sum(-2, keepdim=True) + 1e-6)
+    o = ((torch.sigmoid(m[:, :4]) + 1e-6)[:, :, None] * want_r).sum(1)
+    o = o * torch.rsqrt(o.square().mean(-1, keepdim=True) + 1e-5) * nw.double()
+    out = torch.zeros(rows, H, dtype=torch.bfloat16, device="cuda")
+    part, done, pre = torch.zeros(rows, max(H // 32, 1), 36, device="cuda"), torch.zeros(rows, dtype=torch.int32, device="cuda"), torch.zeros(rows, 8, device="cuda")
+    nat.call("lsb_mhc_post_pre", out, res, x, post, comb, fn, scale, base, nw, part, rows, H, 4, mode, 20, 1e-6, 1e-5, 2.0, done, pre, None)
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm())
+    # fp32 sums of up to 17408 products in runs of a few hundred: 2^-24 sqrt(17408) = 8e-6 at most; the output is rounded to bf16 (2^-9 at most)
+    assert rel(res, want_r) < 1e-6 and rel(post, torch.sigmoid(m[:, 4:8]) * 2) < 1e-5 and rel(comb, k) < 1e-5 and rel(out, o) < 3e-3
