@@ -23,6 +23,26 @@ namespace lsb {
 
 #include "kda_chunk.cuh"
 
+// acc[ii][jj] += sum_k A[ty + 16 ii][k] B[tx + 16 jj][k]  (both operands row-major with k contiguous, K a multiple of 4)
+template <int K>
+__device__ __forceinline__ void kda_mm_nt(const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb, float (&acc)[4][4],
+                                          int tx, int ty) {
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+        float4 a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            a[i] = *reinterpret_cast<const float4*>(A + (ty + 16 * i) * lda + k);
+            b[i] = *reinterpret_cast<const float4*>(B + (tx + 16 * i) * ldb + k);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                acc[i][j] = fmaf(a[i].x, b[j].x, fmaf(a[i].y, b[j].y, fmaf(a[i].z, b[j].z, fmaf(a[i].w, b[j].w, acc[i][j]))));
+    }
+}
+
 struct TmixParams {
     const float* proj;                       // [rows, ldp] fp32: r | k | v | g | w (rank of the decay) at the offsets below
     int ldp, off_r, off_k, off_v, off_g, off_w, rank;        // rank padded to a multiple of 8
