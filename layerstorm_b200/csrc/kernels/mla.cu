@@ -193,6 +193,7 @@ struct MlaDecodeParams {
     int H, dl, dr, page, kv_fmt, NS;
     float scale;
     const float* tq_centroids;   // kv_fmt 2: the 16 reconstruction levels
+    bf16* out;                   // one split and the shared-tile kernel: finished rows [R, H, dl] instead of partials (null: partials)
 };
 
 // Loads KT cache rows (token positions s_tok[0..KT), -1 = none) into the bf16 tile Ks[KT][DP]: latent part expanded
@@ -713,6 +714,21 @@ __global__ void __launch_bounds__(NG * 128) mla_decode_mma_shared_kernel(MlaDeco
         }
     }
     __syncthreads();
+    if (p.out) {
+        // the only split: divide by the sum here (2048 rows x 64 heads: 268 MB of fp32 partials not written and read again, one launch less)
+        const float i0 = s_l[hl0] > 0.f ? 1.f / s_l[hl0] : 0.f, i1 = s_l[hl1] > 0.f ? 1.f / s_l[hl1] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            if (j < ntile) {
+                const int col = sw * ncol + j * 8 + 2 * tq;
+                const int h0 = hb + hl0, h1 = hb + hl1;
+                if (h0 < p.H) *reinterpret_cast<bf162*>(p.out + ((size_t)r * p.H + h0) * p.dl + col) = __floats2bfloat162_rn(o[j][0] * i0, o[j][1] * i0);
+                if (h1 < p.H) *reinterpret_cast<bf162*>(p.out + ((size_t)r * p.H + h1) * p.dl + col) = __floats2bfloat162_rn(o[j][2] * i1, o[j][3] * i1);
+            }
+        }
+        pdl_launch_dependents();
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         if (j < ntile) {
@@ -851,7 +867,7 @@ LSB_API int lsb_mla_decode(const void* q, const void* cache, const void* block_t
     p.q = (const bf16*)q; p.cache = (const uint8_t*)cache; p.block_table = (const int*)block_table; p.max_pages = max_pages;
     p.row_seq = (const int*)row_seq; p.row_len = (const int*)row_len; p.sel_idx = (const int*)sel_idx; p.sel_cnt = (const int*)sel_cnt;
     p.sel_ld = sel_ld; p.o_part = (float*)o_part; p.ml_part = (float*)ml_part; p.H = H; p.dl = dl; p.dr = dr; p.page = page;
-    p.kv_fmt = kv_fmt; p.NS = NS; p.scale = scale; p.tq_centroids = (const float*)tq_centroids;
+    p.kv_fmt = kv_fmt; p.NS = NS; p.scale = scale; p.tq_centroids = (const float*)tq_centroids; p.out = nullptr;
     const int smem = lsb_mla_decode_smem_bytes(dl, dr);
     static bool attr_set = false;
     if (!attr_set) {
@@ -867,17 +883,20 @@ LSB_API int lsb_mla_decode(const void* q, const void* cache, const void* block_t
     static const int mma_min_rows = [] { const char* e = getenv("LSB_MLA_MMA_MIN_ROWS"); return e ? atoi(e) : 1; }();
     if (R >= mma_min_rows && dl % 64 == 0 && dl <= 512 && dr % 16 == 0) {
         // more than one 16-head group per query row: the groups of a row share each gathered K tile
+        if (NS == 1 && out && !lse && ((uintptr_t)out & 3) == 0 && H > kHG) p.out = (bf16*)out;
         if (H > 2 * kHG && mla_mma_shared_smem_bytes(dl, dr, 4) <= 200 * 1024)
             launch_pdl((mla_decode_mma_shared_kernel<4>), dim3(R, (H + 4 * kHG - 1) / (4 * kHG), NS), 512, (size_t)mla_mma_shared_smem_bytes(dl, dr, 4), st, p);
         else if (H > kHG && mla_mma_shared_smem_bytes(dl, dr, 2) <= 200 * 1024)
             launch_pdl((mla_decode_mma_shared_kernel<2>), dim3(R, (H + 2 * kHG - 1) / (2 * kHG), NS), 256, (size_t)mla_mma_shared_smem_bytes(dl, dr, 2), st, p);
-        else
+        else {
+            p.out = nullptr;
             launch_pdl((mla_decode_mma_kernel), dim3(R, (H + kHG - 1) / kHG, NS), 256, (size_t)lsb_mla_decode_mma_smem_bytes(dl, dr), st, p);
+        }
     } else {
         launch_pdl((mla_decode_kernel), dim3(R, (H + kHG - 1) / kHG, NS), 256, smem, st, p);
     }
     // out == null: the caller merges the partials itself (context-parallel attention combines them across ranks)
-    if (out) launch_pdl((mla_combine_kernel), dim3(R, H), dl >= 512 ? 512 : (dl >= 256 ? 256 : 128), 0, st, (bf16*)out, (float*)lse, (const float*)o_part, (const float*)ml_part, H, NS, dl);
+    if (out && !p.out) launch_pdl((mla_combine_kernel), dim3(R, H), dl >= 512 ? 512 : (dl >= 256 ? 256 : 128), 0, st, (bf16*)out, (float*)lse, (const float*)o_part, (const float*)ml_part, H, NS, dl);
     LSB_CHECK_LAUNCH();
 }
 
