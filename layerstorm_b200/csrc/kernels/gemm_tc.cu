@@ -38,18 +38,23 @@ struct GemmTcParams {
     PeerComm comm;
 };
 
-template <int BN> struct TcCfg {
+// A CTA computes MT weight tiles of 128 rows against one token tile.  MT = 2 (512 x 256 outputs of TMEM, one CTA per SM) brings a third less
+// through L2 per product than two CTAs of 128 x 256; MT = 1 has half the shared memory of an SM, so that two CTAs share one and the epilogue of
+// one runs under the main loop of the other.  Measured (one CTA of 128 x 256 per SM, MT = 1 at half an SM, MT = 2): 2048 x 24896 x 4096 534, 446,
+// 422 us; 2048 x 4096 x 12288 205, 182, 165 us; 391 x 16640 x 4096 119, 94, 89 us; MT = 1 with 64-row tiles and smaller: 32 x 24896 x 4096 66 -> 55 us.
+template <int BN, int MT> struct TcCfg {
     static constexpr int A_BYTES = BM * BK * 2;
     static constexpr int B_BYTES = BN * BK * 2;
-    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int STAGES = (BN >= 256) ? 4 : (BN >= 128 ? 6 : 8);
-    static constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
+    static constexpr int STAGE_BYTES = MT * A_BYTES + B_BYTES;
+    static constexpr int STAGES = MT == 2 ? 3 : (BN >= 256 ? 2 : (BN >= 128 ? 3 : 4));
+    static constexpr int TMEM_COLS = MT * (BN < 32 ? 32 : BN);
+    static constexpr int THREADS = 64 + 128 * MT;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
 
-template <int BN, bool BATCHED = false>
-__global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GemmTcParams p) {
-    using C = TcCfg<BN>;
+template <int BN, int MT = 1, bool BATCHED = false>
+__global__ void __launch_bounds__(TcCfg<BN, MT>::THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GemmTcParams p) {
+    using C = TcCfg<BN, MT>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
@@ -60,7 +65,7 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // token-row tiles are the fastest grid dimension: the blocks that share a weight tile run together, so the weight
     // matrix streams from DRAM once and the (much smaller) activation tiles stay in L2
-    const int n0 = blockIdx.y * BM, m0 = blockIdx.x * BN;
+    const int n0 = blockIdx.y * (BM * MT), m0 = blockIdx.x * BN;
     const int split = BATCHED ? 0 : blockIdx.z, batch = BATCHED ? blockIdx.z : 0;
     const int nkb_total = (p.K + BK - 1) / BK;
     const int kb0 = split * p.kb_per_split;
@@ -97,10 +102,11 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
             mbar_expect_tx(&full[s], C::STAGE_BYTES);
             if (BATCHED) {
                 tma_load_3d(a, &map_w, &full[s], (kb0 + it) * BK, n0, batch);
-                tma_load_3d(a + C::A_BYTES, &map_x, &full[s], (kb0 + it) * BK, m0, batch);
+                tma_load_3d(a + MT * C::A_BYTES, &map_x, &full[s], (kb0 + it) * BK, m0, batch);
             } else {
-                tma_load_2d(a, &map_w, &full[s], (kb0 + it) * BK, n0);
-                tma_load_2d(a + C::A_BYTES, &map_x, &full[s], (kb0 + it) * BK, m0);
+#pragma unroll
+                for (int m = 0; m < MT; ++m) tma_load_2d(a + m * C::A_BYTES, &map_w, &full[s], (kb0 + it) * BK, n0 + m * BM);
+                tma_load_2d(a + MT * C::A_BYTES, &map_x, &full[s], (kb0 + it) * BK, m0);
             }
             ++issued;
         }
@@ -108,27 +114,35 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
             // error path: let the loads already in flight land before this CTA's shared memory is released
             for (int it = max(0, issued - C::STAGES); it < issued; ++it) mbar_wait(&full[it % C::STAGES], (it / C::STAGES) & 1, nullptr, 0);
         }
-    } else if (warp == 1 && lane == 0) {
-        // ---------------- MMA issuer ----------------
+    } else if (warp == 1) {
+        // ---------------- MMA issuer: the whole warp walks the stages, so that the operands of the instructions are warp-uniform; one elected
+        // lane issues (a single thread's own loop takes about 90 cycles per instruction, more than the MMAs of a 256-row tile) ----------------
         constexpr uint32_t idesc = idesc_f16(BM, BN, 1);
+        const uint32_t d = __reduce_max_sync(0xffffffffu, tmem_d);
         bool ok = true;
+        uint32_t s = 0, ph = 0;
         for (int it = 0; it < nkb; ++it) {
-            const int s = it % C::STAGES;
-            const uint32_t ph = (it / C::STAGES) & 1;
-            ok = mbar_wait(&full[s], ph, p.err, 2);
+            ok = __all_sync(0xffffffffu, mbar_wait(&full[s], ph, p.err, 2));
             if (!ok) break;
             tc_fence_after();
             const uint8_t* a = smem + s * C::STAGE_BYTES;
-            const uint64_t da = smem_desc_sw128(a), db = smem_desc_sw128(a + C::A_BYTES);
+            const uint64_t da = smem_desc_sw128(a), db = smem_desc_sw128(a + MT * C::A_BYTES);
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < BK / 16; ++k) umma_f16(tmem_d, da + 2 * k, db + 2 * k, idesc, (it > 0 || k > 0) ? 1u : 0u);
-            umma_commit(&empty[s]);
+                for (int k = 0; k < BK / 16; ++k)
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) umma_f16(d + m * BN, da + m * (C::A_BYTES >> 4) + 2 * k, db + 2 * k, idesc, (it > 0 || k > 0) ? 1u : 0u);
+                umma_commit(&empty[s]);
+            }
+            __syncwarp();
+            if (++s == C::STAGES) { s = 0; ph ^= 1u; }
         }
-        if (ok) umma_commit(acc_full);
+        if (ok && elect_one()) umma_commit(acc_full);
+        __syncwarp();
     } else if (warp >= 2) {
         // ---------------- epilogue ----------------
-        const int q = warp & 3;
-        const int n = n0 + q * 32 + lane;
+        const int q = warp & 3, mt = (warp - 2) >> 2;
+        const int n = n0 + mt * BM + q * 32 + lane;
         bool ok = nkb > 0 ? mbar_wait(acc_full, 0, p.err, 3) : true;
         tc_fence_after();
         if (ok) {
@@ -136,7 +150,7 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 16) {
                 float v[16];
-                if (nkb > 0) tmem_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
+                if (nkb > 0) tmem_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(mt * BN + c0), v);
                 else {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] = 0.f;
@@ -261,23 +275,23 @@ int cached_map_2d(CUtensorMap* out, const void* ptr, CUtensorMapDataType dt, int
     return 0;
 }
 
-template <int BN>
+template <int BN, int MT = 1>
 static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTcParams& p, cudaStream_t st) {
-    using C = TcCfg<BN>;
+    using C = TcCfg<BN, MT>;
     static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM); attr = true; }
-    dim3 grid((p.M + BN - 1) / BN, (p.N + BM - 1) / BM, p.splits);
-    launch_pdl((gemm_tc_kernel<BN>), grid, 192, C::SMEM, st, mw, mx, p);
+    if (!attr) { cudaFuncSetAttribute(gemm_tc_kernel<BN, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM); attr = true; }
+    dim3 grid((p.M + BN - 1) / BN, (p.N + BM * MT - 1) / (BM * MT), p.splits);
+    launch_pdl((gemm_tc_kernel<BN, MT>), grid, C::THREADS, C::SMEM, st, mw, mx, p);
     return (int)cudaGetLastError();
 }
 
 template <int BN>
 static int launch_tc_batched(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTcParams& p, int batch, cudaStream_t st) {
-    using C = TcCfg<BN>;
+    using C = TcCfg<BN, 1>;
     static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(gemm_tc_kernel<BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM); attr = true; }
+    if (!attr) { cudaFuncSetAttribute(gemm_tc_kernel<BN, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM); attr = true; }
     dim3 grid((p.M + BN - 1) / BN, (p.N + BM - 1) / BM, batch);
-    launch_pdl((gemm_tc_kernel<BN, true>), grid, 192, C::SMEM, st, mw, mx, p);
+    launch_pdl((gemm_tc_kernel<BN, 1, true>), grid, C::THREADS, C::SMEM, st, mw, mx, p);
     return (int)cudaGetLastError();
 }
 
@@ -364,7 +378,8 @@ LSB_API int lsb_gemm_bf16_tc(void* out, const void* x, const void* w, const void
         case 32: rc = launch_tc<32>(mw, mx, p, st); break;
         case 64: rc = launch_tc<64>(mw, mx, p, st); break;
         case 128: rc = launch_tc<128>(mw, mx, p, st); break;
-        default: rc = launch_tc<256>(mw, mx, p, st); break;
+        // Two weight tiles per CTA pay from a reduction of 2048 on (K = 1536 and below: the same; a short one leaves the longer epilogue bare)
+        default: rc = K >= 2048 && !comm ? launch_tc<256, 2>(mw, mx, p, st) : launch_tc<256>(mw, mx, p, st); break;
     }
     if (rc) return rc;
     if (p.splits > 1) {

@@ -82,3 +82,35 @@ def test_quantised_linear_tensor_core_path(fmt, M, N, K):
     lin(few, x, 4)                                       # GEMV path on the first rows
     torch.cuda.synchronize()
     assert float((few - ref[:4]).abs().max() / ref.abs().max()) < 3e-3
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 8, 2048), (257, 200, 2056), (513, 384, 2112), (300, 1000, 2048), (700, 30000, 2048)])
+@pytest.mark.parametrize("ob", [0, 1])
+def test_two_weight_tiles_per_cta(M, N, K, ob):
+    """Reductions from 2048 on over more than 128 rows: a second weight tile that is empty or not full, token tiles and stages that are not full, with and without
+    split reductions, a bias, nothing written beyond the matrix."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = (torch.randn(n, K, generator=g, device="cuda").bfloat16() for n in (M, N))
+    bias = torch.randn(N, generator=g, device="cuda")
+    out = torch.zeros(M + 1, N + 8, device="cuda", dtype=torch.bfloat16 if ob else torch.float32)
+    part, err = torch.zeros(1 << 24, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    nat.call("lsb_gemm_bf16_tc", out, x, w, bias, M, N, K, K, K, N + 8, ob, part, part.numel(), err, None)
+    want = x.double() @ w.double().T + bias.double()
+    assert int(err) == 0 and float(out[M:].abs().sum()) == 0.0 and float(out[:M, N:].abs().sum()) == 0.0
+    # fp32 sums (2^-24 sqrt(K) = 3e-6), rounded to bf16 (2^-9) where asked
+    assert float((out[:M, :N].double() - want).norm() / want.norm()) < (3e-3 if ob else 1e-5)
+
+
+@pytest.mark.parametrize("M", [4, 5, 7, 8])
+@pytest.mark.parametrize("N,K", [(8, 64), (72, 136), (1040, 4096)])
+def test_bf16_linear_of_few_rows(M, N, K):
+    """Both sides of the line between the weight-streaming kernel and the tensor-core GEMM."""
+    from layerstorm_b200.models.device_model import QLinear
+    g = torch.Generator().manual_seed(N + M)
+    lin = QLinear.from_float(torch.randn(N, K, generator=g), "bf16", "cuda")
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16).cuda()
+    for dt in (torch.float32, torch.bfloat16):
+        out = torch.zeros(M, N, device="cuda", dtype=dt)
+        lin(out, x, M)
+        want = x.double() @ lin.w.double().T
+        assert float((out.double() - want).norm() / want.norm()) < (1e-5 if dt == torch.float32 else 3e-3)
