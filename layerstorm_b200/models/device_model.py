@@ -105,7 +105,16 @@ def expert_layout(fmt: str, H: int, F: int, down_fmt: Optional[str] = None, gate
 
 
 F32_SPLIT_MIN_ROWS = 128  # rows from which an fp32 matrix (the router) runs as a split-bf16 tensor-core GEMM instead of the CUDA-core SGEMM
-TC_MOE_MIN_ROWS = 16      # rows per step from which the routed experts run on the tensor-core grouped GEMM
+TC_MOE_MIN_ROWS = 16      # rows per step from which the routed experts run on the tensor-core grouped GEMM whatever their format
+# ... and from which by storage format (0 bf16, 1 FP8, 2 NVFP4 beyond the steps whose pairs stream their experts one by one, 3 Q4_K): where sort, gather and
+# grouped GEMM together take less than the 4-row weight-streaming kernels.  Microseconds, streaming against grouped, on a B200: FP8 (256 + 1 experts of
+# 7168 x 2048, top 8) 1 row 162 / 126, 6 rows 665 / 379, 15 rows 1502 / 791; bf16 (64 of 4096 x 2048) 1 row 108 / 113, 2 rows 174 / 173, 4 rows 289 / 254,
+# 12 rows 609 / 457; NVFP4 (288 + 1 of 4096 x 2048) 10 rows 543 / 301; Q4_K (64 + 1 of 6144 x 2048) 1 row 201 / 143, 8 rows 951 / 533.  The hidden
+# activations are fp16 there, bf16 in the streaming kernels: 2e-4 off 64 bits against 1.7e-3.
+TC_MOE_FROM = {0: 3, 1: 1, 2: 1, 3: 1}
+# rows from which a bf16 matrix runs on the tensor-core GEMM: above four rows the weight-streaming kernel reads the matrix twice (5 rows of 24896 x 4096:
+# 108 us against 55 us)
+TC_GEMM_MIN_ROWS = 5
 # router projection + top-k in one launch for decode-sized steps (switch: LSB_ROUTER_FUSED=1).  Off by default: measured on the
 # GLM-5.3-Flash shape the fused kernel (one block per expert, last block selects) gives 7.21 ms per decode step against 7.12 ms for
 # the split-K GEMV + top-k pair, whose second launch already overlaps the first through programmatic dependent launch
@@ -371,7 +380,7 @@ class QLinear:
             if self.fmt != "f32" or ob or bias is not None or comm is not None:
                 raise RuntimeError("fp32 activations need fp32 weights and an fp32 output on one GPU")
             nat.call("lsb_gemm_f32", out, x, self.w, M, self.N, self.K, ldx, self.K, ldo)
-        elif self.fmt == "bf16" and M >= 8:
+        elif self.fmt == "bf16" and M >= TC_GEMM_MIN_ROWS:
             sc = TcScratch.get(self.w.device)
             nat.call("lsb_gemm_bf16_tc", out, x, self.w, bias, M, self.N, self.K, ldx, self.K, ldo, ob, sc.partial, sc.cap, sc.err, comm)
         elif (self.fmt == "nvfp4" and MOE_BLOCK_SCALED and M >= 16 and comm is None and bias is None and ldx == self.K and self.K % 256 == 0
@@ -565,7 +574,7 @@ class MoeBuffers:
         self.y = z(R * S, H)
         self.miss = z(1, dtype=i32)
         # tensor-core grouped path (many rows): expert-sorted fp16 operands and the device-built tile list
-        self.tc_ok = tc and R >= TC_MOE_MIN_ROWS and H % 128 == 0 and F % 128 == 0
+        self.tc_ok = tc and H % 128 == 0 and F % 128 == 0
         self.bs_ok = self.bs_fp8 = False
         if self.tc_ok:
             P = R * S
@@ -745,10 +754,11 @@ class ModelBase:
 
     # ------------------------------------------------------------------ routed experts of a step
     def moe_mode(self, arena: "ExpertArena", ws, R: int) -> str:
-        if getattr(ws, "tc_ok", False) and R >= TC_MOE_MIN_ROWS and arena.ef.fmt <= 3 and not arena.ef.fmt_down1:
+        fast_fp4 = arena.ef.fmt == 2 and arena.ef.F % 128 == 0 and arena.ef.H % 128 == 0 and R * ws.S <= 72
+        if getattr(ws, "tc_ok", False) and arena.ef.fmt <= 3 and not arena.ef.fmt_down1 and (
+                R >= TC_MOE_MIN_ROWS or (R >= TC_MOE_FROM[arena.ef.fmt] and not fast_fp4 and not ws.bs_ok)):
             return "tc"
-        fast_fp4 = arena.ef.fmt == 2 and arena.ef.F % 128 == 0 and arena.ef.H % 128 == 0
-        return "pairs" if (fast_fp4 and R * ws.S <= 72) else "groups"
+        return "pairs" if fast_fp4 else "groups"
 
     def moe_prepare(self, arena: "ExpertArena", ws, x, R: int, E: int):
         """Group the step's (row, slot) pairs by expert (once per layer, independent of residency).  Ids outside [0, E) take no part."""

@@ -143,3 +143,40 @@ def test_widths_that_end_inside_boxes_and_operand_stages(fmt, H, F, BN):
         # a hidden value rounded to fp16, at most 2^-11 relative per term (NVFP4, FP8 and bf16 weights are exact in fp16).  Q4_K weights are d sc v - dmin m
         # with both products rounded to fp16, 2^-11 of terms up to 15 d sc and 8 d sc in size around weights of 4.6 d sc rms: 2.4e-3 at most
         assert float((got[r * 2 + k] - want).norm() / want.norm()) < (3e-3 if fmt == "gguf_q4_k" else 1e-3), e
+
+
+@pytest.mark.parametrize("fmt,first", [("bf16", 3), ("fp8_e4m3", 1), ("nvfp4", 13), ("gguf_q4_k", 1)])
+def test_steps_of_few_rows(fmt, first):
+    """Both sides of the row count from which a format's experts run on the grouped kernel (NVFP4: more than 72 pairs), an id that takes no part among them."""
+    from layerstorm_b200.models.device_model import ModelBase, MoeBuffers
+    dev = torch.device("cuda")
+    H, F, E, S = 256, 256, 9, 6
+    arena, ref = _setup(fmt, H, F, E, n_missing=0, seed=5)
+    m = ModelBase()
+    m.device, m.tp_size, m.expert_shard = dev, 1, "ep"
+    z = lambda *s, dtype=torch.float32: torch.zeros(*s, dtype=dtype, device=dev)
+    for R in sorted({1, 2, max(1, first - 1), first, 15, 16}):
+        g = torch.Generator(device="cpu").manual_seed(R)
+        x = torch.randn(R, H, generator=g).to(torch.bfloat16).to(dev)
+        ids = torch.stack([torch.randperm(E, generator=g)[:S] for _ in range(R)])
+        mb = MoeBuffers()
+        mb.alloc_moe(z, R, S, E, E, H, F, tc=True)
+        mb.tc_xs, mb.tc_act = z(R * S, H, dtype=torch.float16), z(R * S, F, dtype=torch.float16)
+        mb.ids.copy_(ids.int())
+        mb.ids[R - 1, 2] = -1
+        assert (m.moe_mode(arena, mb, R) == "tc") == (R >= first)
+        mb.bs_ok = True                                  # block-scaled steps of few rows stay on the streaming kernels
+        assert (m.moe_mode(arena, mb, R) == "tc") == (R >= 16)
+        mb.bs_ok = False
+        m.moe_prepare(arena, mb, x, R, E)
+        m.moe_experts(arena, mb, x, R, E, 0.0, mb.miss)
+        got, xd = mb.y.view(R, S, H).double().cpu(), x.double().cpu()
+        for r in range(R):
+            for k in range(S):
+                if (r, k) == (R - 1, 2):
+                    continue
+                gate, up, down = ref[int(ids[r, k])]
+                want = down @ (torch.nn.functional.silu(gate @ xd[r]) * (up @ xd[r]))
+                # a hidden value in bf16 (2^-9 at most, averaged out) on the streaming kernels; Q4_K weights as above
+                assert float((got[r, k] - want).norm() / want.norm()) < 4e-3, (R, r, k)
+        assert int(mb.miss) == 0
