@@ -62,11 +62,21 @@ __global__ void __launch_bounds__(1024) moe_tc_sort_kernel(const int* __restrict
         if (e >= 0 && e < E_total) atomicAdd(&cnt[e], 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    // first pair and first tile of every expert: a warp takes 32 experts at a time (one thread over 289 of them: 13 us)
+    if (threadIdx.x < 32) {
         int o = 0, t = 0;
-        for (int e = 0; e < E_total; ++e) { off[e] = o; tb[e] = t; o += cnt[e]; t += (cnt[e] + BN - 1) / BN; }
-        off[E_total] = o; tb[E_total] = t;
-        counters[0] = t; counters[1] = o;
+        for (int e0 = 0; e0 < E_total; e0 += 32) {
+            const int e = e0 + threadIdx.x, c = e < E_total ? cnt[e] : 0, nt = (c + BN - 1) / BN;
+            int so = c, st = nt;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, so, d), b = __shfl_up_sync(0xffffffffu, st, d);
+                if ((int)threadIdx.x >= d) { so += a; st += b; }
+            }
+            if (e < E_total) { off[e] = o + so - c; tb[e] = t + st - nt; }
+            o += __shfl_sync(0xffffffffu, so, 31); t += __shfl_sync(0xffffffffu, st, 31);
+        }
+        if (threadIdx.x == 0) { off[E_total] = o; tb[E_total] = t; counters[0] = t; counters[1] = o; }
     }
     __syncthreads();
     for (int e = threadIdx.x; e < E_total; e += blockDim.x) {
@@ -100,6 +110,18 @@ __global__ void __launch_bounds__(128) moe_tc_gather_kernel(const bf16* __restri
         *reinterpret_cast<uint4*>(dst + k) = *reinterpret_cast<uint4*>(h);
     }
     pdl_launch_dependents();
+}
+
+// The same with the rows as they are (bf16).
+__global__ void __launch_bounds__(128) moe_tc_gather_bf16_kernel(const bf16* __restrict__ x, const int* __restrict__ sorted_pair,
+                                                                 const int* __restrict__ counters, bf16* __restrict__ xs, int S, int H) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int pos = blockIdx.x;
+    if (pos >= counters[1]) return;
+    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(sorted_pair[pos] / S) * H);
+    uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)pos * H);
+    for (int k = threadIdx.x; k < H / 8; k += blockDim.x) dst[k] = __ldg(src + k);
 }
 
 // ------------------------------------------------------------------------------------------ converters
@@ -254,7 +276,10 @@ struct MoeTcParams {
     int up;               // one-matrix form of the kernel over the up matrices of experts without a gate: relu(up x)^2 into `act`
 };
 
-template <int FMT, int BN, bool GATEUP> struct MoeTcCfg {
+// DIRECT (bf16 gate / up over bf16 tokens): nothing to convert, the weight boxes in shared memory are the MMA's A operand as TMA wrote them; tensor
+// memory holds accumulators only, two sets of them.
+template <int FMT, int BN, bool GATEUP, bool DIRECT = false> struct MoeTcCfg {
+    static_assert(!DIRECT || (FMT == 0 && GATEUP), "direct operands: bf16 gate / up");
     static constexpr int A_TILES = GATEUP ? 2 : 1;
     static constexpr int NH = GATEUP ? 1 : 2;                             // converter threads per (row, stage): gate/up = one per matrix
     using CV = RowConv<FMT, NH>;
@@ -275,17 +300,17 @@ template <int FMT, int BN, bool GATEUP> struct MoeTcCfg {
 #ifndef LSB_MOE_NBUF1_COLS
 #define LSB_MOE_NBUF1_COLS 128
 #endif
-    static constexpr int NBUF = ACC_COLS > LSB_MOE_NBUF1_COLS ? 1 : 2;
+    static constexpr int NBUF = ACC_COLS > LSB_MOE_NBUF1_COLS && !DIRECT ? 1 : 2;
     static constexpr int A_COLS = 32 * A_TILES * KS;
     static constexpr int A_BASE = NBUF * ACC_COLS;
-    static constexpr int S_FIT = (512 - A_BASE) / A_COLS;
+    static constexpr int S_FIT = DIRECT ? 2 : (512 - A_BASE) / A_COLS;
     static constexpr int S = S_FIT > 3 ? 3 : S_FIT;                       // operand stages: weights in tensor memory, tokens in shared memory
     static constexpr int TMEM_COLS = 512;
     // 8 converter warps cover one sub-stage (4 lane quarters x 2 parts); two sets of them take the sub-stages in turns, so that a warp has
     // two sub-stage times for its serial read -> convert -> store chain
     static constexpr int CONV_SETS = 2;
     static constexpr int SET_WARPS = 8;
-    static constexpr int CONV_WARPS = SET_WARPS * CONV_SETS;
+    static constexpr int CONV_WARPS = DIRECT ? 0 : SET_WARPS * CONV_SETS;
     static_assert(KS % CONV_SETS == 0, "both sets have part in every operand stage");
     static constexpr int EPI_WARPS = 4;
     static constexpr int RAW_WARP = 2 + CONV_WARPS + EPI_WARPS;           // last warp: TMA producer of the raw weight ring
@@ -301,7 +326,7 @@ template <int FMT, int BN, bool GATEUP> struct MoeTcCfg {
     // One CTA per SM by construction (the CTA owns all of tensor memory): ask for more than half of the SM's shared memory.
     static constexpr int SMEM_NEED = S * KS * B_BYTES + RD * RAW_STAGE + BAR_BYTES + 1024;
     static constexpr int SMEM = SMEM_NEED < 120 * 1024 ? 120 * 1024 : SMEM_NEED;
-    static_assert(S >= 2 && A_BASE + S * A_COLS <= 512, "tensor memory budget");
+    static_assert(S >= 2 && A_BASE + (DIRECT ? 0 : S * A_COLS) <= 512, "tensor memory budget");
     static_assert(RD >= 3 && SMEM <= 227 * 1024, "shared memory budget");
     static_assert((3 * S + 2 * RD + 4) * 8 + 8 <= BAR_BYTES, "barrier area");
 };
@@ -344,11 +369,11 @@ template <int N> struct RingPos {
     __device__ __forceinline__ void skip(uint32_t n) { i += n; if (i >= N) { i -= N; ph ^= 1u; } }       // n <= N
 };
 
-template <int FMT, int BN, bool GATEUP>
-__global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS, 1) moe_tc_ffn_kernel(const __grid_constant__ CUtensorMap map_b,
+template <int FMT, int BN, bool GATEUP, bool DIRECT = false>
+__global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1) moe_tc_ffn_kernel(const __grid_constant__ CUtensorMap map_b,
                                                                                        const __grid_constant__ CUtensorMap map_w0,
                                                                                        const __grid_constant__ CUtensorMap map_w1, MoeTcParams p) {
-    using C = MoeTcCfg<FMT, BN, GATEUP>;
+    using C = MoeTcCfg<FMT, BN, GATEUP, DIRECT>;
     using CV = typename C::CV;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -371,8 +396,8 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS, 1) moe_tc_
     const int nkb = K / kTBK, nops = (nkb + C::KS - 1) / C::KS;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::S; ++s) { mbar_init(&full_a[s], C::CONV_WARPS); mbar_init(&full_b[s], 1); mbar_init(&empty[s], 1); }
-        for (int s = 0; s < C::RD; ++s) { mbar_init(&full_r[s], 1); mbar_init(&empty_r[s], C::SUB == 1 ? C::SET_WARPS : C::CONV_WARPS); }
+        for (int s = 0; s < C::S; ++s) { mbar_init(&full_a[s], DIRECT ? 1 : C::CONV_WARPS); mbar_init(&full_b[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < C::RD; ++s) { mbar_init(&full_r[s], 1); mbar_init(&empty_r[s], DIRECT ? 1 : (C::SUB == 1 ? C::SET_WARPS : C::CONV_WARPS)); }
         for (int b = 0; b < C::NBUF; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], C::EPI_WARPS); }
         fence_barrier_init();
         fence_proxy_async();
@@ -471,10 +496,11 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS, 1) moe_tc_
         // ---------------- MMA issuer: A (weights) from tensor memory, B (tokens) from shared memory ----------------
         // The whole warp walks the list (loop bounds and ring positions stay warp-uniform, so the operands of the instructions are uniform
         // registers) and one elected lane issues.
-        constexpr uint32_t idesc = idesc_f16(kTBM, BN, 0);
+        constexpr uint32_t idesc = idesc_f16(kTBM, BN, DIRECT ? 1 : 0);
         const int utotal = __reduce_max_sync(0xffffffffu, total), untiles = __reduce_max_sync(0xffffffffu, ntiles);
         const uint32_t ut = __reduce_max_sync(0xffffffffu, tmem_d);
         RingPos<C::S> r;
+        RingPos<C::RD> rr;                                     // (direct: raw entries)
         uint32_t lt = 0;
         bool ok = true;
         PROF_DECL();
@@ -490,6 +516,33 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP>::THREADS, 1) moe_tc_
             const uint32_t acc = ut + buf * C::ACC_COLS;
             for (int o = 0; o < nops; ++o, r.next()) {
                 PROF_SCOPE(1, ok = mbar_wait(&full_b[r.i], r.ph, p.err, 12));
+                if constexpr (DIRECT) {
+                    ok = __all_sync(0xffffffffu, ok);
+                    const int n = min(C::KS, nkb - o * C::KS);
+                    for (int j = 0; j < n && ok; ++j, rr.next()) {
+                        PROF_SCOPE(2, ok = mbar_wait(&full_r[rr.i], rr.ph, p.err, 12));
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint8_t* a = smem_r + rr.i * C::RAW_STAGE;
+                        const uint64_t dg = smem_desc_sw128(a), du = smem_desc_sw128(a + C::W_TILE), db = smem_desc_sw128(smem_b + (r.i * C::KS + j) * C::B_BYTES);
+                        PROF_SCOPE(3, {
+                        if (elect_one()) {
+#pragma unroll
+                            for (int k = 0; k < kTBK / 16; ++k) {
+                                const uint32_t accum = (o > 0 || j > 0 || k > 0) ? 1u : 0u;
+                                umma_f16(acc, dg + 2 * k, db + 2 * k, idesc, accum);
+                                umma_f16(acc + BN, du + 2 * k, db + 2 * k, idesc, accum);
+                            }
+                            umma_commit(&empty_r[rr.i]);
+                        }
+                        __syncwarp(); });
+                    }
+                    if (!ok) break;
+                    if (elect_one()) umma_commit(&empty[r.i]);
+                    __syncwarp();
+                    continue;
+                }
                 if (ok) PROF_SCOPE(2, ok = mbar_wait(&full_a[r.i], r.ph, p.err, 12));
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
@@ -734,7 +787,7 @@ static int sm_count() {
     return n;
 }
 
-template <int FMT, int BN, bool GATEUP>
+template <int FMT, int BN, bool GATEUP, bool DIRECT = false>
 static int launch_moe_tc(const CUtensorMap& mb, const MoeTcParams& p, int nout, int max_tiles, cudaStream_t st) {
     const int Kred = GATEUP || p.up ? p.ef.H : p.ef.F;
     CUtensorMap mw0, mw1;
@@ -749,12 +802,12 @@ static int launch_moe_tc(const CUtensorMap& mb, const MoeTcParams& p, int nout, 
         if (GATEUP) { rc = cached_map_w(&mw1, p.arena + p.ef.off_up, pitch, (uint64_t)nout, sstride, nslots); if (rc) return rc; }
         else mw1 = mw0;
     }
-    using C = MoeTcCfg<FMT, BN, GATEUP>;
+    using C = MoeTcCfg<FMT, BN, GATEUP, DIRECT>;
     static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(moe_tc_ffn_kernel<FMT, BN, GATEUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM); attr = true; }
+    if (!attr) { cudaFuncSetAttribute(moe_tc_ffn_kernel<FMT, BN, GATEUP, DIRECT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM); attr = true; }
     const long long work = (long long)(nout / kTBM) * max_tiles;
     const int grid = (int)(work < sm_count() ? (work > 0 ? work : 1) : sm_count());
-    launch_pdl((moe_tc_ffn_kernel<FMT, BN, GATEUP>), grid, C::THREADS, C::SMEM, st, mb, mw0, mw1, p);
+    launch_pdl((moe_tc_ffn_kernel<FMT, BN, GATEUP, DIRECT>), grid, C::THREADS, C::SMEM, st, mb, mw0, mw1, p);
     return (int)cudaGetLastError();
 }
 
@@ -803,6 +856,12 @@ LSB_API int lsb_moe_tc_gather(const void* x, const void* sorted_pair, const void
     LSB_CHECK_LAUNCH();
 }
 
+LSB_API int lsb_moe_tc_gather_bf16(const void* x, const void* sorted_pair, const void* counters, void* xs, int npairs, int S, int H, void* stream) {
+    if (H % 8 || (((uintptr_t)x | (uintptr_t)xs) & 15)) return -1;
+    launch_pdl((moe_tc_gather_bf16_kernel), npairs, 128, 0, (cudaStream_t)stream, (const bf16*)x, (const int*)sorted_pair, (const int*)counters, (bf16*)xs, S, H);
+    LSB_CHECK_LAUNCH();
+}
+
 // gateup != 0: act[pos][f] = SwiGLU(xs[pos] . Wgate[f], xs[pos] . Wup[f]) for every sorted position (fp16, [cap_rows, F]).
 // gateup == 0: y[pair][h] = act[pos] . Wdown[h]  (fp32, [npairs, H], rows in pair order).
 // gateup == 2: act[pos][f] = relu(xs[pos] . Wup[f])^2 (experts without a gate).
@@ -810,7 +869,7 @@ LSB_API int lsb_moe_tc_gather(const void* x, const void* sorted_pair, const void
 static int moe_tc_ffn(int gateup, const void* b, int cap_rows, const void* arena, const void* slot_of, const void* fmt_struct,
                            const void* tile_expert, const void* tile_row0, const void* tile_n, const void* counters,
                            const void* sorted_pair, void* out, int BN, int max_tiles, GluAct ga, void* miss_flag, void* err,
-                           const void* ep, void* stream) {
+                           const void* ep, void* stream, bool direct = false) {
     const ExpertFmt* ef = (const ExpertFmt*)fmt_struct;
     const int K = gateup ? ef->H : ef->F, nout = gateup ? ef->F : ef->H;
     if (gateup == 2 && ep) return -1;
@@ -829,7 +888,14 @@ static int moe_tc_ffn(int gateup, const void* b, int cap_rows, const void* arena
     if (ep) p.ep = *(const EpComm*)ep; else { memset(&p.ep, 0, sizeof(p.ep)); }
     p.ldo = nout; p.out_bf16 = 0; p.down_scale = 0.f; p.up = gateup == 2;
     cudaStream_t st = (cudaStream_t)stream;
-    if (gateup == 1) {
+    if (direct) {
+        if (gateup != 1 || ef->fmt != 0 || ep) return -1;
+        switch (BN) {
+            case 32: return launch_moe_tc<0, 32, true, true>(mb, p, nout, max_tiles, st);
+            case 64: return launch_moe_tc<0, 64, true, true>(mb, p, nout, max_tiles, st);
+            case 128: return launch_moe_tc<0, 128, true, true>(mb, p, nout, max_tiles, st);
+        }
+    } else if (gateup == 1) {
         switch (BN) {
             case 32: return dispatch_fmt<32, true>(ef->fmt, mb, p, nout, max_tiles, st);
             case 64: return dispatch_fmt<64, true>(ef->fmt, mb, p, nout, max_tiles, st);
@@ -851,6 +917,17 @@ LSB_API int lsb_moe_tc_ffn(int gateup, const void* b, int cap_rows, const void* 
                            const void* ep, void* stream) {
     return moe_tc_ffn(gateup, b, cap_rows, arena, slot_of, fmt_struct, tile_expert, tile_row0, tile_n, counters, sorted_pair, out, BN, max_tiles,
                       GluAct{limit, 1.f, 0.f, nullptr}, miss_flag, err, ep, stream);
+}
+
+// The gate/up half over bf16 experts and bf16 token rows (lsb_moe_tc_gather_bf16): both go to the tensor core as they are, which is exact where the other
+// form rounds weights outside fp16's normal range, and needs no converters.  1500 rows x top-8 of 64 experts of 4096 x 2048: 832 us through the converters,
+// 505 us so (bound by shared memory: 112 KB of operands read and written per 64 elements, 875 cycles beside 512 of MMA).
+LSB_API int lsb_moe_tc_gateup_bf16(const void* b, int cap_rows, const void* arena, const void* slot_of, const void* fmt_struct,
+                                   const void* tile_expert, const void* tile_row0, const void* tile_n, const void* counters,
+                                   const void* sorted_pair, void* out, int BN, int max_tiles, float limit, float alpha, float shift, const void* in_scale,
+                                   void* miss_flag, void* err, void* stream) {
+    return moe_tc_ffn(1, b, cap_rows, arena, slot_of, fmt_struct, tile_expert, tile_row0, tile_n, counters, sorted_pair, out, BN, max_tiles,
+                      GluAct{limit, alpha, shift, (const float*)in_scale}, miss_flag, err, nullptr, stream, true);
 }
 
 // The gate/up half with another gated unit (GluAct): in_scale [npairs] in pair order, or null.

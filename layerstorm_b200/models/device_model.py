@@ -760,6 +760,11 @@ class ModelBase:
             return "tc"
         return "pairs" if fast_fp4 else "groups"
 
+    @staticmethod
+    def _moe_direct(arena: "ExpertArena") -> bool:
+        """bf16 gate and up matrices meet bf16 rows on the tensor core as they are (the row buffer then holds bf16)."""
+        return arena.ef.fmt == 0 and arena.ef.off_up != arena.ef.off_gate
+
     def moe_prepare(self, arena: "ExpertArena", ws, x, R: int, E: int):
         """Group the step's (row, slot) pairs by expert (once per layer, independent of residency).  Ids outside [0, E) take no part."""
         S, H = ws.S, arena.ef.H
@@ -771,7 +776,7 @@ class ModelBase:
                 nat.call("lsb_quant_fp8_tiles" if ws.bs_fp8 else "lsb_quant_nvfp4_tiles", x, 0, ws.tc_sorted, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt,
                          S, H, ws.tc_bn, min(ws.tc_tiles, P // ws.tc_bn + E + 1), ws.bs_xq, ws.bs_xsf, ws.bs_xa)
             else:
-                nat.call("lsb_moe_tc_gather", x, ws.tc_sorted, ws.tc_cnt, ws.tc_xs, P, S, H)
+                nat.call("lsb_moe_tc_gather_bf16" if self._moe_direct(arena) else "lsb_moe_tc_gather", x, ws.tc_sorted, ws.tc_cnt, ws.tc_xs, P, S, H)
         elif mode == "groups":
             nat.call("lsb_moe_build_groups", ws.ids, R * S, E, ws.group_expert, ws.group_n, ws.group_pairs, ws.n_groups, ws.counts)
 
@@ -804,7 +809,9 @@ class ModelBase:
                 return
             up = (ws.tc_xs, ws.tc_xs.shape[0], arena.data, arena.slot_of, efp, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, ws.tc_sorted, ws.tc_act,
                   ws.tc_bn, tiles, limit)
-            if act is None or act == "relu2":
+            if self._moe_direct(arena) and act != "relu2":
+                nat.call("lsb_moe_tc_gateup_bf16", *up, *((1.0, 0.0, None) if act is None else act), miss, err)
+            elif act is None or act == "relu2":
                 nat.call("lsb_moe_tc_ffn", 1 if act is None else 2, *up, miss, err, None)
             else:
                 nat.call("lsb_moe_tc_gateup_act", *up, *act, miss, err)

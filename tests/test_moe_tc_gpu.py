@@ -180,3 +180,51 @@ def test_steps_of_few_rows(fmt, first):
                 # a hidden value in bf16 (2^-9 at most, averaged out) on the streaming kernels; Q4_K weights as above
                 assert float((got[r, k] - want).norm() / want.norm()) < 4e-3, (R, r, k)
         assert int(mb.miss) == 0
+
+
+@pytest.mark.parametrize("H,F", [(128, 384), (640, 128), (1152, 256)])
+@pytest.mark.parametrize("BN", [32, 64, 128])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_bf16_rows_meet_bf16_experts_directly(H, F, BN, scaled):
+    """Reductions of two sub-stages, that end inside an operand stage and that wrap the rings; an expert that is not resident; another gated unit with a factor
+    per pair; weights and rows outside fp16's normal range."""
+    from layerstorm_b200.ops import _native as nat
+    dev = torch.device("cuda")
+    E, R = 20, 2 * BN + 1
+    arena, ref = _setup("bf16", H, F, E, n_missing=1, seed=6)
+    g = torch.Generator(device="cpu").manual_seed(7)
+    x = torch.randn(R, H, generator=g) * 0.5
+    x[:, 0], x[:, 1] = 1e5, 1e-7                          # beyond fp16: the columns of the weights that meet them are as small and as large
+    x = x.to(torch.bfloat16).to(dev)
+    for e in range(1, E):
+        v = arena.data[int(arena.slot_of[e])]
+        for off in (arena.ef.off_gate, arena.ef.off_up):
+            w = v[off: off + F * H * 2].view(torch.bfloat16).view(F, H)
+            w[:, 0] *= 1e-6
+            w[:, 1] *= 1e6
+        ref[e] = [m.double().cpu() for m in arena.read_expert(int(arena.slot_of[e]), "bf16")]
+    ids = torch.stack([torch.full((R,), E - 1), torch.arange(R) % (E - 1)], 1).int().to(dev).contiguous()
+    P, tiles = R * 2, R * 2 // BN + E + 1
+    i32 = dict(dtype=torch.int32, device=dev)
+    srt, te, tr, tn, cnt, err, miss = (torch.zeros(n, **i32) for n in (P, tiles, tiles, tiles, 2, 1, 1))
+    xs, act = torch.zeros(P, H, dtype=torch.bfloat16, device=dev), torch.zeros(P, F, dtype=torch.float16, device=dev)
+    fac = torch.rand(P, generator=g).to(dev) if scaled else None
+    limit, alpha, shift = (1.1, 1.702, 1.0) if scaled else (0.0, 1.0, 0.0)
+    efp = ctypes.addressof(arena.ef)
+    nat.call("lsb_moe_tc_sort", ids, P, E, BN, srt, te, tr, tn, cnt)
+    nat.call("lsb_moe_tc_gather_bf16", x, srt, cnt, xs, P, 2, H)
+    nat.call("lsb_moe_tc_gateup_bf16", xs, P, arena.data, arena.slot_of, efp, te, tr, tn, cnt, srt, act, BN, tiles, limit, alpha, shift, fac, miss, err)
+    torch.cuda.synchronize()
+    assert int(err) == 0 and int(miss) == 1
+    pair, xd, got = srt.cpu().long(), x.double().cpu(), act.double().cpu()
+    for pos in range(0, P, 7):
+        r, e = int(pair[pos]) // 2, int(ids.view(-1)[int(pair[pos])])
+        if e < 1:
+            continue
+        c = float(fac[int(pair[pos])]) if scaled else 1.0
+        gv, uv = ref[e][0] @ xd[r] * c, ref[e][1] @ xd[r] * c
+        if limit:
+            gv, uv = gv.clamp(max=limit), uv.clamp(-limit, limit)
+        want = gv * torch.sigmoid(alpha * gv) * (uv + shift)
+        # fp32 sums, the unit rounded to fp16 (2^-11 relative at most)
+        assert float((got[pos] - want).norm() / want.norm()) < 1e-3, (pos, e)
