@@ -505,15 +505,13 @@ class Engine:
         # read it has completed, so the host can run ahead of the device by several steps
         if not hasattr(ws, "h_ring"):
             ws.h_ring = [torch.zeros(ws.inp.shape[0], ws.R, dtype=torch.int32).pin_memory() for _ in range(4)]
-            ws.h_np = [h.numpy() for h in ws.h_ring]          # filled through numpy: a tenth of a tensor operation's cost per call
-            ws.h_ev = [torch.cuda.Event() for _ in range(4)] if self.dev.type == "cuda" else [None] * 4
-            ws.h_used = [False] * 4
+            ws.h_ev = [None] * 4
             ws.h_i = 0
         k = ws.h_i
         ws.h_i = (k + 1) % 4
-        if ws.h_used[k]:
+        if ws.h_ev[k] is not None:
             ws.h_ev[k].synchronize()
-        h = ws.h_np[k]
+        h = ws.h_ring[k].numpy()                                     # filled through numpy: a tenth of a tensor operation's cost per call
         h[...] = 0
         h[1] = -1
         if rows:
@@ -535,8 +533,9 @@ class Engine:
         ws.seq_end = [rows[r0 + n - 1][2] + 1 for (r0, n, _) in seq_groups]
         ws.single_seq = len(seq_groups) == 1 and len({slot for (_, slot, _) in rows}) == 1
         ws.inp.copy_(ws.h_ring[k], non_blocking=True)
+        if ws.h_ev[k] is None:
+            ws.h_ev[k] = torch.cuda.Event()
         ws.h_ev[k].record(torch.cuda.current_stream())
-        ws.h_used[k] = True
         self.h2d_bytes += ws.inp.numel() * 4
 
     def _ws_decode(self, B: int) -> StepBuffers:
