@@ -561,6 +561,21 @@ class MoeBuffers:
     """Buffers of a routed feed-forward over up to ``R`` rows with ``S`` slots per row and ``E`` expert ids: routing, the 4-row groups of the
     weight-streaming kernels and - with ``tc`` - the expert-sorted operands of the tensor-core grouped kernel."""
 
+    @staticmethod
+    def tile_rows(P: int, E: int) -> int:
+        """Rows per token tile for ``P`` pairs over ``E`` experts: the smallest tile that most experts' rows fit, since every tile converts its expert's weights
+        anew (2048 rows x 9 of 289 NVFP4 experts of 4096 x 2048, gate/up: 920 us in tiles of 64, 1372 in 32, 1171 in 128), and a smaller one leaves tensor memory
+        for more weight stages (32 rows: 378 us in tiles of 32, 538 in 64)."""
+        avg = P / max(1, min(E, P))
+        return 32 if avg <= 32 else (64 if avg <= 96 else 128)
+
+    def step_tiles(self, P: int, E: int) -> tuple:
+        """(rows per tile, tiles at most) of a step of ``P`` pairs; the block-scaled operands are laid out for the workspace's own tiles."""
+        if self.bs_ok:
+            return self.tc_bn, min(self.tc_tiles, P // self.tc_bn + E + 1)
+        bn = self.tile_rows(P, E)
+        return bn, P // bn + E + 1
+
     def alloc_moe(self, z, R: int, S: int, E: int, n_logits: int, H: int, F: int, tc: bool, act_dtype=torch.bfloat16):
         i32 = torch.int32
         self.S = S
@@ -578,12 +593,12 @@ class MoeBuffers:
         self.bs_ok = self.bs_fp8 = False
         if self.tc_ok:
             P = R * S
-            avg = P / max(1, min(E, P))
-            self.tc_bn = 32 if avg <= 32 else (64 if avg <= 96 else 128)
+            self.tc_bn = self.tile_rows(P, E)
             self.tc_tiles = P // self.tc_bn + E + 1
+            n = P // 32 + E + 1                               # tiles of a step whose rows make smaller ones
             self.tc_sorted = z(P, dtype=i32)
-            self.tc_tile_e = z(self.tc_tiles, dtype=i32); self.tc_tile_r0 = z(self.tc_tiles, dtype=i32)
-            self.tc_tile_n = z(self.tc_tiles, dtype=i32); self.tc_cnt = z(2, dtype=i32)
+            self.tc_tile_e = z(n, dtype=i32); self.tc_tile_r0 = z(n, dtype=i32)
+            self.tc_tile_n = z(n, dtype=i32); self.tc_cnt = z(2, dtype=i32)
 
 
 class Workspace(StepBuffers, MoeBuffers):
@@ -771,10 +786,11 @@ class ModelBase:
         mode = self.moe_mode(arena, ws, R)
         if mode == "tc":
             P = R * S
-            nat.call("lsb_moe_tc_sort", ws.ids, P, E, ws.tc_bn, ws.tc_sorted, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt)
+            bn, tiles = ws.step_tiles(P, E)
+            nat.call("lsb_moe_tc_sort", ws.ids, P, E, bn, ws.tc_sorted, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt)
             if ws.bs_ok:
                 nat.call("lsb_quant_fp8_tiles" if ws.bs_fp8 else "lsb_quant_nvfp4_tiles", x, 0, ws.tc_sorted, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt,
-                         S, H, ws.tc_bn, min(ws.tc_tiles, P // ws.tc_bn + E + 1), ws.bs_xq, ws.bs_xsf, ws.bs_xa)
+                         S, H, bn, tiles, ws.bs_xq, ws.bs_xsf, ws.bs_xa)
             else:
                 nat.call("lsb_moe_tc_gather_bf16" if self._moe_direct(arena) else "lsb_moe_tc_gather", x, ws.tc_sorted, ws.tc_cnt, ws.tc_xs, P, S, H)
         elif mode == "groups":
@@ -791,24 +807,24 @@ class ModelBase:
         if mode == "tc":
             P = R * S
             err = TcScratch.get(self.device).err
-            tiles = min(ws.tc_tiles, P // ws.tc_bn + E + 1)
+            bn, tiles = ws.step_tiles(P, E)
             if ws.bs_ok and ws.bs_fp8:
                 wsf, og, ou, od = arena.bs_scale_atoms()
                 a = (arena.data, arena.slot_of, efp, wsf, wsf.shape[1], og, ou, od, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, ws.tc_sorted)
-                nat.call("lsb_moe_bs_ffn_fp8", 1, ws.bs_xq, ws.bs_xsf, ws.bs_xa, *a, ws.bs_act, ws.tc_bn, tiles, limit, miss, err)
-                nat.call("lsb_quant_fp8_tiles", ws.bs_act, 1, None, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, S, arena.ef.F, ws.tc_bn, tiles,
+                nat.call("lsb_moe_bs_ffn_fp8", 1, ws.bs_xq, ws.bs_xsf, ws.bs_xa, *a, ws.bs_act, bn, tiles, limit, miss, err)
+                nat.call("lsb_quant_fp8_tiles", ws.bs_act, 1, None, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, S, arena.ef.F, bn, tiles,
                          ws.bs_aq, ws.bs_asf, ws.bs_aa)
-                nat.call("lsb_moe_bs_ffn_fp8", 0, ws.bs_aq, ws.bs_asf, ws.bs_aa, *a, ws.y, ws.tc_bn, tiles, 0.0, None, err)
+                nat.call("lsb_moe_bs_ffn_fp8", 0, ws.bs_aq, ws.bs_asf, ws.bs_aa, *a, ws.y, bn, tiles, 0.0, None, err)
                 return
             if ws.bs_ok:
                 a = (arena.data, arena.slot_of, efp, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, ws.tc_sorted)
-                nat.call("lsb_moe_bs_ffn", 1, ws.bs_xq, ws.bs_xsf, ws.bs_xa, *a, ws.bs_act, ws.tc_bn, tiles, limit, miss, err)
-                nat.call("lsb_quant_nvfp4_tiles", ws.bs_act, 1, None, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, S, arena.ef.F, ws.tc_bn, tiles,
+                nat.call("lsb_moe_bs_ffn", 1, ws.bs_xq, ws.bs_xsf, ws.bs_xa, *a, ws.bs_act, bn, tiles, limit, miss, err)
+                nat.call("lsb_quant_nvfp4_tiles", ws.bs_act, 1, None, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, S, arena.ef.F, bn, tiles,
                          ws.bs_aq, ws.bs_asf, ws.bs_aa)
-                nat.call("lsb_moe_bs_ffn", 0, ws.bs_aq, ws.bs_asf, ws.bs_aa, *a, ws.y, ws.tc_bn, tiles, 0.0, None, err)
+                nat.call("lsb_moe_bs_ffn", 0, ws.bs_aq, ws.bs_asf, ws.bs_aa, *a, ws.y, bn, tiles, 0.0, None, err)
                 return
             up = (ws.tc_xs, ws.tc_xs.shape[0], arena.data, arena.slot_of, efp, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, ws.tc_sorted, ws.tc_act,
-                  ws.tc_bn, tiles, limit)
+                  bn, tiles, limit)
             if self._moe_direct(arena) and act != "relu2":
                 nat.call("lsb_moe_tc_gateup_bf16", *up, *((1.0, 0.0, None) if act is None else act), miss, err)
             elif act is None or act == "relu2":
@@ -816,7 +832,7 @@ class ModelBase:
             else:
                 nat.call("lsb_moe_tc_gateup_act", *up, *act, miss, err)
             nat.call("lsb_moe_tc_ffn", 0, ws.tc_act, ws.tc_act.shape[0], arena.data, arena.slot_of, efp, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n,
-                     ws.tc_cnt, ws.tc_sorted, ws.y, ws.tc_bn, tiles, 0.0, None, err, None)
+                     ws.tc_cnt, ws.tc_sorted, ws.y, bn, tiles, 0.0, None, err, None)
         elif mode == "pairs":
             # small batch: every (row, slot) pair streams its expert on its own - no grouping pass
             # blocks per expert: finer when this GPU holds only a share of the step's experts (expert parallel), see the kernels

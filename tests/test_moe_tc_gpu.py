@@ -228,3 +228,31 @@ def test_bf16_rows_meet_bf16_experts_directly(H, F, BN, scaled):
         want = gv * torch.sigmoid(alpha * gv) * (uv + shift)
         # fp32 sums, the unit rounded to fp16 (2^-11 relative at most)
         assert float((got[pos] - want).norm() / want.norm()) < 1e-3, (pos, e)
+
+
+@pytest.mark.parametrize("R", [16, 97, 340, 700])
+def test_steps_of_fewer_rows_than_the_workspace(R):
+    """The token tile follows the step's rows, not the workspace's: 32, 64 and 128 rows of a workspace whose own tile is 128."""
+    from layerstorm_b200.models.device_model import ModelBase, MoeBuffers
+    dev = torch.device("cuda")
+    H, F, E, S = 128, 256, 8, 2
+    arena, ref = _setup("nvfp4", H, F, E, n_missing=0, seed=8)
+    m, mb = ModelBase(), MoeBuffers()
+    m.device, m.tp_size, m.expert_shard = dev, 1, "ep"
+    z = lambda *s, dtype=torch.float32: torch.zeros(*s, dtype=dtype, device=dev)
+    mb.alloc_moe(z, 700, S, E, E, H, F, tc=True)
+    mb.tc_xs, mb.tc_act = z(700 * S, H, dtype=torch.float16), z(700 * S, F, dtype=torch.float16)
+    assert mb.tc_bn == 128 and mb.step_tiles(R * S, E)[0] == {16: 32, 97: 32, 340: 64, 700: 128}[R]
+    g = torch.Generator(device="cpu").manual_seed(R)
+    x = torch.randn(R, H, generator=g).to(torch.bfloat16).to(dev)
+    ids = torch.stack([torch.randperm(E, generator=g)[:S] for _ in range(R)])
+    mb.ids[:R].copy_(ids.int())
+    m.moe_prepare(arena, mb, x, R, E)
+    m.moe_experts(arena, mb, x, R, E, 0.0, mb.miss)
+    got, xd = mb.y.view(700, S, H)[:R].double().cpu(), x.double().cpu()
+    for e in range(E):
+        gate, up, down = ref[e]
+        r, k = (ids == e).nonzero(as_tuple=True)
+        want = (torch.nn.functional.silu(xd[r] @ gate.T) * (xd[r] @ up.T)) @ down.T
+        assert float((got[r, k] - want).norm() / want.norm()) < 1e-3, e
+    assert float(mb.y.view(700, S, H)[R:].abs().sum()) == 0.0
