@@ -575,7 +575,7 @@ def test_hyper_connection_pass_of_many_rows(rows, H, mode):
 
 
 @pytest.mark.parametrize("rows", [1, 148, 149])
-@pytest.mark.parametrize("dim", [4, 124, 4096, 7168, 12288, 130])
+@pytest.mark.parametrize("dim", [4, 124, 4096, 7168, 12252, 130])
 def test_rms_norm_row_forms(rows, dim):
     """Widths that end inside a warp's quads, the widest row, an odd one on the general form; with and without the residual."""
     g = torch.Generator(device="cuda").manual_seed(dim + rows)
@@ -601,3 +601,36 @@ def test_fp32_matrix_over_groups_of_rows(M, N):
         nat.call("lsb_gemv_f32w", out, x, w, None, M, N, 1024, 1024, 1024, N + 2, 1.0, int(dt == torch.bfloat16))
         want = x.double() @ w.double().T
         assert float((out[:M, :N].double() - want).norm() / want.norm()) < tol and float(out[M:].abs().sum() + out[:, N:].abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("R,H,off", [(1, 4, 0), (3, 4096, 0), (3, 4096, 1), (2, 12252, 0), (149, 4096, 0), (149, 132, 0), (2, 130, 0)])
+def test_contract_norm_vector_and_general_rows(R, H, off):
+    """One and four quads per thread, the widest row, and what the general kernel keeps (widths that quads do not cover, mixing rows off 16 bytes)."""
+    n, eps = 4, 1e-6
+    resid, x, nw = rnd(R, n, H, seed=1), rnd(R, H, seed=2), rnd(H, seed=3)
+    post, comb = torch.empty(R * n + off, device=DEV)[off:], rnd(R, n, n, seed=5)
+    post.copy_(rnd(R * n, seed=4))
+    out = torch.full((R, H), float("nan"), device=DEV, dtype=torch.bfloat16)
+    nat.call("lsb_mhc_contract_norm", out, resid, x, post, comb, nw, R, H, n, eps, None)
+    torch.cuda.synchronize()
+    d = [t.double() for t in (resid, x, post.view(R, n), comb, nw)]
+    v = (d[2].sum(1)[:, None] * d[1] + torch.einsum("ri,rih->rh", d[3].sum(2), d[0])) / n
+    want = v * torch.rsqrt(v.pow(2).mean(1, keepdim=True) + eps) * d[4]
+    # half a bf16 step of the result, and 20 fp32 roundings of the terms of v, which may cancel (2**-20 of a row's largest)
+    assert bool(((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -20 * want.abs().amax(1, keepdim=True) * 8).all())
+
+
+@pytest.mark.parametrize("H", [8, 264, 4096, 9216, 36])
+@pytest.mark.parametrize("scale", [1.0, 2.75])
+def test_embedding_vector_and_general_rows(H, scale):
+    """Rows of 16-byte pieces (one and two rounds a thread) and others; ids on both sides of the shard's range give zeros.  Exact."""
+    table = rnd(30, H, seed=7).bfloat16()
+    ids = torch.tensor([5, 34, 4, 35, -1, 20, 2 ** 31 - 1], device=DEV, dtype=torch.int32)
+    f, b = torch.full((7, H), float("nan"), device=DEV), torch.full((7, H), float("nan"), device=DEV, dtype=torch.bfloat16)
+    nat.call("lsb_embedding_scaled", f, b, table, ids, 7, H, 5, 35, scale)
+    torch.cuda.synchronize()
+    want = torch.zeros(7, H, device=DEV)
+    for r, i in enumerate(ids.tolist()):
+        if 5 <= i < 35:
+            want[r] = table[i - 5].float() * scale
+    assert torch.equal(f, want) and torch.equal(b, want.bfloat16())
