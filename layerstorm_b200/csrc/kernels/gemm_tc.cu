@@ -41,7 +41,8 @@ struct GemmTcParams {
 // A CTA computes MT weight tiles of 128 rows against one token tile.  MT = 2 (512 x 256 outputs of TMEM, one CTA per SM) brings a third less
 // through L2 per product than two CTAs of 128 x 256; MT = 1 has half the shared memory of an SM, so that two CTAs share one and the epilogue of
 // one runs under the main loop of the other.  Measured (one CTA of 128 x 256 per SM, MT = 1 at half an SM, MT = 2): 2048 x 24896 x 4096 534, 446,
-// 422 us; 2048 x 4096 x 12288 205, 182, 165 us; 391 x 16640 x 4096 119, 94, 89 us; MT = 1 with 64-row tiles and smaller: 32 x 24896 x 4096 66 -> 55 us.
+// 422 us; 2048 x 4096 x 12288 205, 182, 165 us; 391 x 16640 x 4096 119, 94, 89 us; MT = 1 with 64-row tiles and smaller: 32 x 24896 x 4096 66 -> 55 us.  (All with a slower epilogue
+// than now: see its comment for what the same sizes take.)
 template <int BN, int MT> struct TcCfg {
     static constexpr int A_BYTES = BM * BK * 2;
     static constexpr int B_BYTES = BN * BK * 2;
