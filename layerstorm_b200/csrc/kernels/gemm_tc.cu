@@ -41,8 +41,7 @@ struct GemmTcParams {
 // A CTA computes MT weight tiles of 128 rows against one token tile.  MT = 2 (512 x 256 outputs of TMEM, one CTA per SM) brings a third less
 // through L2 per product than two CTAs of 128 x 256; MT = 1 has half the shared memory of an SM, so that two CTAs share one and the epilogue of
 // one runs under the main loop of the other.  Measured (one CTA of 128 x 256 per SM, MT = 1 at half an SM, MT = 2): 2048 x 24896 x 4096 534, 446,
-// 422 us; 2048 x 4096 x 12288 205, 182, 165 us; 391 x 16640 x 4096 119, 94, 89 us; MT = 1 with 64-row tiles and smaller: 32 x 24896 x 4096 66 -> 55 us.  (All with a slower epilogue
-// than now: see its comment for what the same sizes take.)
+// 422 us; 2048 x 4096 x 12288 205, 182, 165 us; 391 x 16640 x 4096 119, 94, 89 us; MT = 1 with 64-row tiles and smaller: 32 x 24896 x 4096 66 -> 55 us.
 template <int BN, int MT> struct TcCfg {
     static constexpr int A_BYTES = BM * BK * 2;
     static constexpr int B_BYTES = BN * BK * 2;
@@ -148,42 +147,26 @@ __global__ void __launch_bounds__(TcCfg<BN, MT>::THREADS) gemm_tc_kernel(const _
         tc_fence_after();
         if (ok) {
             const float b = (p.bias && n < p.N && p.splits == 1) ? p.bias[n] : 0.f;
-            const int rows = min(BN, p.M - m0);
-            // 16 token rows at a time through `put`; a piece with all its rows has no test per row
-            auto tile = [&](auto put) {
 #pragma unroll 1
-                for (int c0 = 0; c0 < rows; c0 += 16) {
-                    float v[16];
-                    if (nkb > 0) tmem_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(mt * BN + c0), v);
-                    else {
+            for (int c0 = 0; c0 < BN; c0 += 16) {
+                float v[16];
+                if (nkb > 0) tmem_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(mt * BN + c0), v);
+                else {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) v[j] = 0.f;
-                    }
-                    if (n >= p.N) continue;
-                    if (c0 + 16 <= rows) {
+                    for (int j = 0; j < 16; ++j) v[j] = 0.f;
+                }
+                if (n < p.N) {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) put(c0 + j, v[j] + b);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (c0 + j < rows) put(c0 + j, v[j] + b);
+                    for (int j = 0; j < 16; ++j) {
+                        const int m = m0 + c0 + j;
+                        if (m < p.M) {
+                            if (p.comm.nranks) comm_push(p.comm, next_epoch, (size_t)m * p.ldo + n, v[j]);
+                            else if (p.splits > 1) p.partial[((size_t)split * p.M + m) * p.N + n] = v[j];
+                            else if (p.out_bf16) reinterpret_cast<bf16*>(p.out)[(size_t)batch * p.out_bs + (size_t)m * p.ldo + n] = __float2bfloat16(v[j] + b);
+                            else reinterpret_cast<float*>(p.out)[(size_t)batch * p.out_bs + (size_t)m * p.ldo + n] = v[j] + b;
+                        }
                     }
                 }
-            };
-            // Where the results go is settled once, and a row is a pointer step: 25 instructions per output when both were worked out for each
-            // (with one epilogue warp per scheduler their latency was the kernel's time at small K).  64 products of 2048 x 512 x 256: 234 us,
-            // 80 now; 2048 x 24896 x 4096: 420 us, 313 (1335 TFLOP/s) now; 391 x 16640 x 4096: 90, 68; 32 x 4096 x 8192: 37, 32.
-            if (p.comm.nranks) {
-                tile([&](int r, float y) { comm_push(p.comm, next_epoch, (size_t)(m0 + r) * p.ldo + n, y); });
-            } else if (p.splits > 1 || !p.out_bf16) {
-                const size_t step = p.splits > 1 ? (size_t)p.N : (size_t)p.ldo;
-                float* o = p.splits > 1 ? p.partial + ((size_t)split * p.M + m0) * p.N + n
-                                        : reinterpret_cast<float*>(p.out) + (size_t)batch * p.out_bs + (size_t)m0 * p.ldo + n;
-                tile([&](int, float y) { *o = y; o += step; });
-            } else {
-                const size_t step = (size_t)p.ldo;
-                bf16* o = reinterpret_cast<bf16*>(p.out) + (size_t)batch * p.out_bs + (size_t)m0 * p.ldo + n;
-                tile([&](int, float y) { *o = __float2bfloat16(y); o += step; });
             }
         }
     }

@@ -696,12 +696,6 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
 #pragma unroll
             for (int g = 0; g < BN / 32; ++g)
                 in_scale[g] = scaled && g * 32 + lane < ncols ? p.ga.in_scale[p.sorted_pair[row0 + g * 32 + lane]] : 1.f;
-            // pair that each column of the down projection belongs to, likewise (a load per output between the stores, which it has to stay
-            // behind, would be a chain as long as the tile's MMAs)
-            const bool scatter = !GATEUP && !up && !ep_mode;
-            int pair[BN / 32];
-#pragma unroll
-            for (int g = 0; g < BN / 32; ++g) pair[g] = scatter && g * 32 + lane < ncols ? p.sorted_pair[row0 + g * 32 + lane] : 0;
             int okw = 1;
             if (lane == 0) { if (q == 0) PROF_SCOPE(0, okw = mbar_wait_relaxed(&acc_full[buf], (lt / C::NBUF) & 1u, p.err, 14) ? 1 : 0); else okw = mbar_wait_relaxed(&acc_full[buf], (lt / C::NBUF) & 1u, p.err, 14) ? 1 : 0; }
             ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
@@ -717,45 +711,34 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                     sg = su = kFp8Unscale;
                 }
                 const uint32_t lane_addr = tmem_d + buf * C::ACC_COLS + ((uint32_t)(q * 32) << 16);
-                // 16 columns at a time through `put(column, index there, gate or only product, up product)`; a piece with all its columns has no
-                // test per column
-                auto tile = [&](const auto& per_col, auto put) {
 #pragma unroll 1
-                    for (int c0 = 0; c0 < ncols; c0 += 16) {
-                        float gq[16], uq[16];
-                        tmem_ld16(lane_addr + (uint32_t)c0, gq);
-                        if (GATEUP) tmem_ld16(lane_addr + (uint32_t)(BN + c0), uq);
-                        auto cs = per_col[0];                              // this group of 32 columns, one per lane
+                for (int c0 = 0; c0 < BN; c0 += 16) {
+                    if (c0 >= ncols) break;
+                    float gq[16], uq[16];
+                    tmem_ld16(lane_addr + (uint32_t)c0, gq);
+                    if (GATEUP) tmem_ld16(lane_addr + (uint32_t)(BN + c0), uq);
+                    float cs = in_scale[0];                                // factors of this group of 32 columns, one per lane
 #pragma unroll
-                        for (int g = 1; g < BN / 32; ++g) cs = (c0 >> 5) == g ? per_col[g] : cs;
-                        const bool whole = c0 + 16 <= ncols;
+                    for (int g = 1; g < BN / 32; ++g) cs = (c0 >> 5) == g ? in_scale[g] : cs;
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const auto c = __shfl_sync(0xffffffffu, cs, (c0 + j) & 31);
-                            if ((whole || c0 + j < ncols) && n < NOUT) put(c0 + j, c, gq[j], GATEUP ? uq[j] : 0.f);
+                    for (int j = 0; j < 16; ++j) {
+                        const float c = GATEUP && scaled ? __shfl_sync(0xffffffffu, cs, (c0 + j) & 31) : 1.f;
+                        if (c0 + j < ncols && n < NOUT) {
+                            if (GATEUP) {
+                                p.act[(size_t)(row0 + c0 + j) * NOUT + n] = __float2half_rn(glu_act(gq[j] * sg * c, uq[j] * su * c, p.ga));
+                            } else if (up) {
+                                // (fp16 range: far outside what normed inputs reach, kept finite all the same)
+                                p.act[(size_t)(row0 + c0 + j) * NOUT + n] = __float2half_rn(fminf(relu2_act(gq[j] * sg), 65504.f));
+                            } else if (ep_mode) {
+                                const int2 ra = p.ep.ret[p.ep.rank][row0 + c0 + j];      // (token owner, pair index there)
+                                p.ep.y[ra.x][(size_t)ra.y * NOUT + n] = gq[j] * sg;       // NVLink store into the owner's buffer
+                            } else if (p.out_bf16) {
+                                reinterpret_cast<bf16*>(p.y)[(size_t)p.sorted_pair[row0 + c0 + j] * p.ldo + n] = __float2bfloat16(gq[j] * sg);
+                            } else {
+                                p.y[(size_t)p.sorted_pair[row0 + c0 + j] * p.ldo + n] = gq[j] * sg;
+                            }
                         }
                     }
-                };
-                // Where the results go is settled once for the tile.  Down projection, before and now: bf16, 1500 rows over 64 experts (one accumulator
-                // set, so the MMAs wait for this) 532 -> 393 us; NVFP4, 2048 rows over 288 experts 643 -> 596; tiles of 32 columns the same.
-                __half* act = p.act + (size_t)row0 * NOUT + n;
-                if (GATEUP) {
-                    const GluAct ga = p.ga;
-                    tile(in_scale, [&](int col, float c, float g, float u) { act[(size_t)col * NOUT] = __float2half_rn(glu_act(g * sg * c, u * su * c, ga)); });
-                } else if (up) {
-                    // (fp16 range: far outside what normed inputs reach, kept finite all the same)
-                    tile(pair, [&](int col, int, float g, float) { act[(size_t)col * NOUT] = __float2half_rn(fminf(relu2_act(g * sg), 65504.f)); });
-                } else if (ep_mode) {
-                    tile(pair, [&](int col, int, float g, float) {
-                        const int2 ra = p.ep.ret[p.ep.rank][row0 + col];      // (token owner, pair index there)
-                        p.ep.y[ra.x][(size_t)ra.y * NOUT + n] = g * sg;       // NVLink store into the owner's buffer
-                    });
-                } else if (p.out_bf16) {
-                    bf16* y = reinterpret_cast<bf16*>(p.y) + n;
-                    tile(pair, [&](int, int to, float g, float) { y[(size_t)to * p.ldo] = __float2bfloat16(g * sg); });
-                } else {
-                    float* y = p.y + n;
-                    tile(pair, [&](int, int to, float g, float) { y[(size_t)to * p.ldo] = g * sg; });
                 }
             }
             tc_fence_before();
