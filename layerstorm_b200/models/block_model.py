@@ -268,7 +268,8 @@ class BlockWorkspace(StepBuffers):
             if b.experts and m.moe_key(i) not in self.moe:
                 arena = m.layers[i]["arena"]
                 mb = MoeBuffers()
-                mb.alloc_moe(z, R, b.top, b.experts, b.experts + b.identity, arena.ef.H, arena.ef.F, tc=not m.f32, act_dtype=act)
+                mb.alloc_moe(z, R, b.top, b.experts, b.experts + b.identity, arena.ef.H, arena.ef.F, tc=not m.f32 and R >= m.moe_grouped_from(arena.ef),
+                             act_dtype=act)
                 if mb.tc_ok:
                     mb.tc_xs = z(R * b.top, arena.ef.H, dtype=torch.float16)
                     mb.tc_act = z(R * b.top, arena.ef.F, dtype=torch.float16)

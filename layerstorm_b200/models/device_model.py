@@ -105,13 +105,15 @@ def expert_layout(fmt: str, H: int, F: int, down_fmt: Optional[str] = None, gate
 
 
 F32_SPLIT_MIN_ROWS = 128  # rows from which an fp32 matrix (the router) runs as a split-bf16 tensor-core GEMM instead of the CUDA-core SGEMM
-TC_MOE_MIN_ROWS = 16      # rows per step from which the routed experts run on the tensor-core grouped GEMM whatever their format
-# ... and from which by storage format (0 bf16, 1 FP8, 2 NVFP4 beyond the steps whose pairs stream their experts one by one, 3 Q4_K): where sort, gather and
-# grouped GEMM together take less than the 4-row weight-streaming kernels.  Microseconds, streaming against grouped, on a B200: FP8 (256 + 1 experts of
-# 7168 x 2048, top 8) 1 row 162 / 126, 6 rows 665 / 379, 15 rows 1502 / 791; bf16 (64 of 4096 x 2048) 1 row 108 / 113, 2 rows 174 / 173, 4 rows 289 / 254,
-# 12 rows 609 / 457; NVFP4 (288 + 1 of 4096 x 2048) 10 rows 543 / 301; Q4_K (64 + 1 of 6144 x 2048) 1 row 201 / 143, 8 rows 951 / 533.  The hidden
-# activations are fp16 there, bf16 in the streaming kernels: 2e-4 off 64 bits against 1.7e-3.
-TC_MOE_FROM = {0: 3, 1: 1, 2: 1, 3: 1}
+# Rows per step from which the routed experts run on the tensor-core grouped GEMM.  Sort, gather and grouped GEMM take less than the weight-streaming kernels
+# from fewer rows on (FP8, 256 + 1 experts of 7168 x 2048, top 8: 1 row 126 against 162 us, 6 rows 379 / 665, 15 rows 791 / 1502; Q4_K, 64 + 1 of 6144 x 2048:
+# 1 row 143 / 201, 8 rows 533 / 951; NVFP4, 288 + 1 of 4096 x 2048: 10 rows 301 / 543), but few rows stay on those: FP8 and Q4_K keep their scales in fp32 and the
+# rows and hidden values the range of bf16 there, where the grouped kernel's operands are fp16, and a row's expert outputs are the same bits whatever up to 14
+# others share its step (an answer's tokens and the check of a draft of them).
+TC_MOE_MIN_ROWS = 16
+# ... and gated bf16 experts, whose gate and up matrices and rows go to the tensor core as they are (64 of 4096 x 2048: 1 row 108 against 113 us, 2 rows 174 / 173,
+# 4 rows 289 / 254, 12 rows 609 / 457)
+TC_MOE_BF16_ROWS = 3
 # rows from which a bf16 matrix runs on the tensor-core GEMM: above four rows the weight-streaming kernel reads the matrix twice (5 rows of 24896 x 4096:
 # 108 us against 55 us)
 TC_GEMM_MIN_ROWS = 5
@@ -673,7 +675,8 @@ class Workspace(StepBuffers, MoeBuffers):
         if cfg.n_routed > 0:
             S = cfg.top_k + cfg.n_shared
             E_total = cfg.n_routed + cfg.n_shared
-            self.alloc_moe(z, R, S, E_total, cfg.n_routed, H, cfg.moe_inter, tc=m.Fe % 128 == 0)
+            first = min((m.moe_grouped_from(L["arena"].ef) for L in m.layers if L.get("arena") is not None), default=TC_MOE_MIN_ROWS)
+            self.alloc_moe(z, R, S, E_total, cfg.n_routed, H, cfg.moe_inter, tc=m.Fe % 128 == 0 and R >= first)
             if self.tc_ok:
                 # block-scaled path (NVFP4 experts): both operands stay 4-bit, the activations are quantised in tile order
                 fmts = {L["arena"].ef.fmt for L in m.layers if L.get("arena") is not None}
@@ -769,16 +772,21 @@ class ModelBase:
 
     # ------------------------------------------------------------------ routed experts of a step
     def moe_mode(self, arena: "ExpertArena", ws, R: int) -> str:
-        fast_fp4 = arena.ef.fmt == 2 and arena.ef.F % 128 == 0 and arena.ef.H % 128 == 0 and R * ws.S <= 72
-        if getattr(ws, "tc_ok", False) and arena.ef.fmt <= 3 and not arena.ef.fmt_down1 and (
-                R >= TC_MOE_MIN_ROWS or (R >= TC_MOE_FROM[arena.ef.fmt] and not fast_fp4 and not ws.bs_ok)):
+        if (getattr(ws, "tc_ok", False) and R >= (TC_MOE_MIN_ROWS if ws.bs_ok else self.moe_grouped_from(arena.ef)) and arena.ef.fmt <= 3
+                and not arena.ef.fmt_down1):
             return "tc"
-        return "pairs" if fast_fp4 else "groups"
+        fast_fp4 = arena.ef.fmt == 2 and arena.ef.F % 128 == 0 and arena.ef.H % 128 == 0
+        return "pairs" if (fast_fp4 and R * ws.S <= 72) else "groups"
 
     @staticmethod
-    def _moe_direct(arena: "ExpertArena") -> bool:
+    def moe_grouped_from(ef: ExpertFmt) -> int:
+        """Rows per step from which experts of this layout run on the grouped kernel."""
+        return TC_MOE_BF16_ROWS if ModelBase._moe_direct(ef) else TC_MOE_MIN_ROWS
+
+    @staticmethod
+    def _moe_direct(ef: ExpertFmt) -> bool:
         """bf16 gate and up matrices meet bf16 rows on the tensor core as they are (the row buffer then holds bf16)."""
-        return arena.ef.fmt == 0 and arena.ef.off_up != arena.ef.off_gate
+        return ef.fmt == 0 and ef.off_up != ef.off_gate
 
     def moe_prepare(self, arena: "ExpertArena", ws, x, R: int, E: int):
         """Group the step's (row, slot) pairs by expert (once per layer, independent of residency).  Ids outside [0, E) take no part."""
@@ -792,7 +800,7 @@ class ModelBase:
                 nat.call("lsb_quant_fp8_tiles" if ws.bs_fp8 else "lsb_quant_nvfp4_tiles", x, 0, ws.tc_sorted, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt,
                          S, H, bn, tiles, ws.bs_xq, ws.bs_xsf, ws.bs_xa)
             else:
-                nat.call("lsb_moe_tc_gather_bf16" if self._moe_direct(arena) else "lsb_moe_tc_gather", x, ws.tc_sorted, ws.tc_cnt, ws.tc_xs, P, S, H)
+                nat.call("lsb_moe_tc_gather_bf16" if self._moe_direct(arena.ef) else "lsb_moe_tc_gather", x, ws.tc_sorted, ws.tc_cnt, ws.tc_xs, P, S, H)
         elif mode == "groups":
             nat.call("lsb_moe_build_groups", ws.ids, R * S, E, ws.group_expert, ws.group_n, ws.group_pairs, ws.n_groups, ws.counts)
 
@@ -825,7 +833,7 @@ class ModelBase:
                 return
             up = (ws.tc_xs, ws.tc_xs.shape[0], arena.data, arena.slot_of, efp, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, ws.tc_sorted, ws.tc_act,
                   bn, tiles, limit)
-            if self._moe_direct(arena) and act != "relu2":
+            if self._moe_direct(arena.ef) and act != "relu2":
                 nat.call("lsb_moe_tc_gateup_bf16", *up, *((1.0, 0.0, None) if act is None else act), miss, err)
             elif act is None or act == "relu2":
                 nat.call("lsb_moe_tc_ffn", 1 if act is None else 2, *up, miss, err, None)

@@ -8,7 +8,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _setup(fmt, H, F, E, n_missing, seed):
+def _setup(fmt, H, F, E, n_missing, seed, size=1.0):
+    """``size``: factor on the gate and up matrices."""
     from layerstorm_b200.models.device_model import ExpertArena, QLinear, expert_layout
     dev = torch.device("cuda")
     g = torch.Generator(device="cpu").manual_seed(seed)
@@ -19,7 +20,7 @@ def _setup(fmt, H, F, E, n_missing, seed):
     for e in range(E):
         if e < n_missing:
             continue                                   # experts 0..n_missing-1 are not resident
-        mats = [torch.randn(F, H, generator=g) * 0.05, torch.randn(F, H, generator=g) * 0.05, torch.randn(H, F, generator=g) * 0.05]
+        mats = [torch.randn(F, H, generator=g) * 0.05 * size, torch.randn(F, H, generator=g) * 0.05 * size, torch.randn(H, F, generator=g) * 0.05]
         arena.write_expert(slot, *(QLinear.from_float(m.to(dev), fmt, dev) for m in mats))
         arena.slot_of[e] = slot
         ref[e] = [m.double().cpu() for m in arena.read_expert(slot, fmt)]
@@ -145,9 +146,10 @@ def test_widths_that_end_inside_boxes_and_operand_stages(fmt, H, F, BN):
         assert float((got[r * 2 + k] - want).norm() / want.norm()) < (3e-3 if fmt == "gguf_q4_k" else 1e-3), e
 
 
-@pytest.mark.parametrize("fmt,first", [("bf16", 3), ("fp8_e4m3", 1), ("nvfp4", 13), ("gguf_q4_k", 1)])
+@pytest.mark.parametrize("fmt,first", [("bf16", 3), ("fp8_e4m3", 16), ("nvfp4", 16), ("gguf_q4_k", 16)])
 def test_steps_of_few_rows(fmt, first):
-    """Both sides of the row count from which a format's experts run on the grouped kernel (NVFP4: more than 72 pairs), an id that takes no part among them."""
+    """Both sides of the row count from which a format's experts run on the grouped kernel and (NVFP4: 12 rows of 6 pairs) from which they run in groups, an id
+    that takes no part among them."""
     from layerstorm_b200.models.device_model import ModelBase, MoeBuffers
     dev = torch.device("cuda")
     H, F, E, S = 256, 256, 9, 6
@@ -155,7 +157,7 @@ def test_steps_of_few_rows(fmt, first):
     m = ModelBase()
     m.device, m.tp_size, m.expert_shard = dev, 1, "ep"
     z = lambda *s, dtype=torch.float32: torch.zeros(*s, dtype=dtype, device=dev)
-    for R in sorted({1, 2, max(1, first - 1), first, 15, 16}):
+    for R in sorted({1, 2, first - 1, first, 12, 13, 15, 16}):
         g = torch.Generator(device="cpu").manual_seed(R)
         x = torch.randn(R, H, generator=g).to(torch.bfloat16).to(dev)
         ids = torch.stack([torch.randperm(E, generator=g)[:S] for _ in range(R)])
@@ -180,6 +182,92 @@ def test_steps_of_few_rows(fmt, first):
                 # a hidden value in bf16 (2^-9 at most, averaged out) on the streaming kernels; Q4_K weights as above
                 assert float((got[r, k] - want).norm() / want.norm()) < 4e-3, (R, r, k)
         assert int(mb.miss) == 0
+
+
+@pytest.mark.parametrize("fmt,rows", [("fp8_e4m3", (1, 2, 9, 15)), ("gguf_q4_k", (1, 2, 9, 15)), ("bf16", (1, 2))])
+def test_steps_of_few_rows_keep_the_range_of_bf16(fmt, rows):
+    """Hidden values of about 1e6, FP8 block scales that are no powers of two and above 0.57 (where 256 of them times 448 passes fp16's largest number), and a
+    row of activations beyond it."""
+    from layerstorm_b200.models.device_model import ModelBase, MoeBuffers
+    dev = torch.device("cuda")
+    H, F, E, S = 256, 256, 9, 6
+    arena, ref = _setup(fmt, H, F, E, n_missing=0, seed=9, size=2000.0)
+    if fmt == "fp8_e4m3":
+        for e in range(E):
+            for off in (arena.ef.off_sg, arena.ef.off_su, arena.ef.off_sd):
+                sc = arena.data[e][off: off + 16].view(torch.float32)
+                sc *= 1.37
+            assert float(arena.data[e][arena.ef.off_sg:][:16].view(torch.float32).min()) > 0.57
+            ref[e] = [w.double().cpu() for w in arena.read_expert(e, fmt)]
+    m = ModelBase()
+    m.device, m.tp_size, m.expert_shard = dev, 1, "ep"
+    z = lambda *s, dtype=torch.float32: torch.zeros(*s, dtype=dtype, device=dev)
+    for R in rows:
+        g = torch.Generator(device="cpu").manual_seed(R)
+        x = torch.randn(R, H, generator=g)
+        x[R - 1] *= 1e5
+        x = x.to(torch.bfloat16).to(dev)
+        ids = torch.stack([torch.randperm(E, generator=g)[:S] for _ in range(R)])
+        mb = MoeBuffers()
+        mb.alloc_moe(z, R, S, E, E, H, F, tc=True)
+        mb.tc_xs, mb.tc_act = z(R * S, H, dtype=torch.float16), z(R * S, F, dtype=torch.float16)
+        mb.ids.copy_(ids.int())
+        m.moe_prepare(arena, mb, x, R, E)
+        m.moe_experts(arena, mb, x, R, E, 0.0, mb.miss)
+        got, xd = mb.y.view(R, S, H).double().cpu(), x.double().cpu()
+        for r in range(R):
+            for k in range(S):
+                gate, up, down = ref[int(ids[r, k])]
+                want = down @ (torch.nn.functional.silu(gate @ xd[r]) * (up @ xd[r]))
+                # fp32 sums and a hidden value in bf16: 2^-9 of it at most, averaged out over 256 of them
+                assert float((got[r, k] - want).norm() / want.norm()) < 4e-3, (R, r, k)
+
+
+@pytest.mark.parametrize("fmt", ["nvfp4", "fp8_e4m3", "gguf_q4_k"])
+def test_a_row_of_few_gets_the_same_experts_outputs_in_any_company(fmt):
+    """Bit for bit, whatever the other rows of the step are: a draft's rows are checked together and were answered one by one."""
+    from layerstorm_b200.models.device_model import ModelBase, MoeBuffers
+    dev = torch.device("cuda")
+    H, F, E, S, most = 256, 512, 20, 8, 15
+    arena, _ = _setup(fmt, H, F, E, n_missing=0, seed=12)
+    m = ModelBase()
+    m.device, m.tp_size, m.expert_shard = dev, 1, "ep"
+    z = lambda *s, dtype=torch.float32: torch.zeros(*s, dtype=dtype, device=dev)
+    g = torch.Generator(device="cpu").manual_seed(13)
+    x = torch.randn(most, H, generator=g).to(torch.bfloat16).to(dev)
+    ids = torch.stack([torch.randperm(E, generator=g)[:S] for _ in range(most)]).int()
+    alone = None
+    for R in (1, 2, 5, 9, 10, 12, 15):
+        for first in {0, most - R}:
+            mb = MoeBuffers()
+            mb.alloc_moe(z, R, S, E, E, H, F, tc=True)
+            mb.tc_xs, mb.tc_act = z(R * S, H, dtype=torch.float16), z(R * S, F, dtype=torch.float16)
+            mb.ids.copy_(ids[first: first + R])
+            rows = x[first: first + R].contiguous()
+            m.moe_prepare(arena, mb, rows, R, E)
+            m.moe_experts(arena, mb, rows, R, E, 0.0, mb.miss)
+            y = mb.y.view(R, S, H)
+            if R == 1:
+                alone = {**(alone or {}), first: y[0].clone()}
+            for row, want in alone.items():
+                if first <= row < first + R:
+                    assert torch.equal(y[row - first], want), (R, first, row)
+
+
+def test_steps_of_few_rows_take_no_grouped_buffers():
+    """A workspace whose steps all stream their experts has neither the grouped kernel's buffers nor the block-scaled ones."""
+    from layerstorm_b200.models.config import get_preset
+    from layerstorm_b200.models.device_model import DeviceModel, Workspace
+    from layerstorm_b200.models.weights import init_weights
+    cfg = get_preset("tiny-glm5-next")
+    w = init_weights(cfg, 5)
+    for eq, first in (("nvfp4", 16), ("fp8_e4m3", 16), ("bf16", 3)):
+        m = DeviceModel.from_state_dict(cfg, w, "cuda", kv_fmt="bf16", page=16, expert_quant=eq)
+        for R in (1, 2, 3, 15, 16):
+            ws = Workspace(m, R, 1, 64)
+            assert ws.set_block_scaled(True) in (False, R >= 16)
+            grouped = [n for n in ("tc_xs", "tc_act", "tc_sorted", "bs_xq", "bs_act") if hasattr(ws, n)]
+            assert bool(grouped) == (R >= first and ws.tc_ok), (eq, R, grouped)
 
 
 @pytest.mark.parametrize("H,F", [(128, 384), (640, 128), (1152, 256)])
