@@ -263,7 +263,7 @@ struct MoeTcParams {
     const uint8_t* arena; const int* slot_of; ExpertFmt ef;
     const int* tile_expert; const int* tile_row0; const int* tile_n; const int* counters;
     const int* sorted_pair;
-    __half* act;          // gate/up output, [pairs, F] fp16 in sorted order
+    __half* act;          // gate/up output, [pairs, F] fp16 (kDirectBf16: bf16) in sorted order
     float* y;             // down output, [npairs, H] fp32 in pair order
     GluAct ga;
     int* miss_flag; int* err;
@@ -276,10 +276,11 @@ struct MoeTcParams {
     int up;               // one-matrix form of the kernel over the up matrices of experts without a gate: relu(up x)^2 into `act`
 };
 
-// DIRECT (bf16 gate / up over bf16 tokens): nothing to convert, the weight boxes in shared memory are the MMA's A operand as TMA wrote them; tensor
-// memory holds accumulators only, two sets of them.
-template <int FMT, int BN, bool GATEUP, bool DIRECT = false> struct MoeTcCfg {
-    static_assert(!DIRECT || (FMT == 0 && GATEUP), "direct operands: bf16 gate / up");
+// DIRECT (bf16 weights over bf16 tokens): nothing to convert, the weight boxes in shared memory are the MMA's A operand as TMA wrote them; tensor
+// memory holds accumulators only, two sets of them.  kDirect: gate / up with fp16 hidden values; kDirectBf16: both halves, hidden values in bf16.
+constexpr int kDirect = 1, kDirectBf16 = 2;
+template <int FMT, int BN, bool GATEUP, int DIRECT = 0> struct MoeTcCfg {
+    static_assert(!DIRECT || (FMT == 0 && (GATEUP || DIRECT == kDirectBf16)), "direct operands: bf16 weights and tokens");
     static constexpr int A_TILES = GATEUP ? 2 : 1;
     static constexpr int NH = GATEUP ? 1 : 2;                             // converter threads per (row, stage): gate/up = one per matrix
     using CV = RowConv<FMT, NH>;
@@ -369,7 +370,7 @@ template <int N> struct RingPos {
     __device__ __forceinline__ void skip(uint32_t n) { i += n; if (i >= N) { i -= N; ph ^= 1u; } }       // n <= N
 };
 
-template <int FMT, int BN, bool GATEUP, bool DIRECT = false>
+template <int FMT, int BN, bool GATEUP, int DIRECT = 0>
 __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1) moe_tc_ffn_kernel(const __grid_constant__ CUtensorMap map_b,
                                                                                        const __grid_constant__ CUtensorMap map_w0,
                                                                                        const __grid_constant__ CUtensorMap map_w1, MoeTcParams p) {
@@ -532,7 +533,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                             for (int k = 0; k < kTBK / 16; ++k) {
                                 const uint32_t accum = (o > 0 || j > 0 || k > 0) ? 1u : 0u;
                                 umma_f16(acc, dg + 2 * k, db + 2 * k, idesc, accum);
-                                umma_f16(acc + BN, du + 2 * k, db + 2 * k, idesc, accum);
+                                if (GATEUP) umma_f16(acc + BN, du + 2 * k, db + 2 * k, idesc, accum);
                             }
                             umma_commit(&empty_r[rr.i]);
                         }
@@ -724,7 +725,9 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                     for (int j = 0; j < 16; ++j) {
                         const float c = GATEUP && scaled ? __shfl_sync(0xffffffffu, cs, (c0 + j) & 31) : 1.f;
                         if (c0 + j < ncols && n < NOUT) {
-                            if (GATEUP) {
+                            if (GATEUP && DIRECT == kDirectBf16) {
+                                reinterpret_cast<bf16*>(p.act)[(size_t)(row0 + c0 + j) * NOUT + n] = __float2bfloat16(glu_act(gq[j] * c, uq[j] * c, p.ga));
+                            } else if (GATEUP) {
                                 p.act[(size_t)(row0 + c0 + j) * NOUT + n] = __float2half_rn(glu_act(gq[j] * sg * c, uq[j] * su * c, p.ga));
                             } else if (up) {
                                 // (fp16 range: far outside what normed inputs reach, kept finite all the same)
@@ -787,7 +790,7 @@ static int sm_count() {
     return n;
 }
 
-template <int FMT, int BN, bool GATEUP, bool DIRECT = false>
+template <int FMT, int BN, bool GATEUP, int DIRECT = 0>
 static int launch_moe_tc(const CUtensorMap& mb, const MoeTcParams& p, int nout, int max_tiles, cudaStream_t st) {
     const int Kred = GATEUP || p.up ? p.ef.H : p.ef.F;
     CUtensorMap mw0, mw1;
@@ -869,7 +872,7 @@ LSB_API int lsb_moe_tc_gather_bf16(const void* x, const void* sorted_pair, const
 static int moe_tc_ffn(int gateup, const void* b, int cap_rows, const void* arena, const void* slot_of, const void* fmt_struct,
                            const void* tile_expert, const void* tile_row0, const void* tile_n, const void* counters,
                            const void* sorted_pair, void* out, int BN, int max_tiles, GluAct ga, void* miss_flag, void* err,
-                           const void* ep, void* stream, bool direct = false) {
+                           const void* ep, void* stream, int direct = 0) {
     const ExpertFmt* ef = (const ExpertFmt*)fmt_struct;
     const int K = gateup ? ef->H : ef->F, nout = gateup ? ef->F : ef->H;
     if (gateup == 2 && ep) return -1;
@@ -888,12 +891,15 @@ static int moe_tc_ffn(int gateup, const void* b, int cap_rows, const void* arena
     if (ep) p.ep = *(const EpComm*)ep; else { memset(&p.ep, 0, sizeof(p.ep)); }
     p.ldo = nout; p.out_bf16 = 0; p.down_scale = 0.f; p.up = gateup == 2;
     cudaStream_t st = (cudaStream_t)stream;
-    if (direct) {
+    if (direct == kDirectBf16) {
+        if (gateup < 0 || gateup > 1 || ef->fmt != 0 || BN != 32 || ep) return -1;
+        return gateup ? launch_moe_tc<0, 32, true, kDirectBf16>(mb, p, nout, max_tiles, st) : launch_moe_tc<0, 32, false, kDirectBf16>(mb, p, nout, max_tiles, st);
+    } else if (direct) {
         if (gateup != 1 || ef->fmt != 0 || ep) return -1;
         switch (BN) {
-            case 32: return launch_moe_tc<0, 32, true, true>(mb, p, nout, max_tiles, st);
-            case 64: return launch_moe_tc<0, 64, true, true>(mb, p, nout, max_tiles, st);
-            case 128: return launch_moe_tc<0, 128, true, true>(mb, p, nout, max_tiles, st);
+            case 32: return launch_moe_tc<0, 32, true, kDirect>(mb, p, nout, max_tiles, st);
+            case 64: return launch_moe_tc<0, 64, true, kDirect>(mb, p, nout, max_tiles, st);
+            case 128: return launch_moe_tc<0, 128, true, kDirect>(mb, p, nout, max_tiles, st);
         }
     } else if (gateup == 1) {
         switch (BN) {
@@ -927,7 +933,17 @@ LSB_API int lsb_moe_tc_gateup_bf16(const void* b, int cap_rows, const void* aren
                                    const void* sorted_pair, void* out, int BN, int max_tiles, float limit, float alpha, float shift, const void* in_scale,
                                    void* miss_flag, void* err, void* stream) {
     return moe_tc_ffn(1, b, cap_rows, arena, slot_of, fmt_struct, tile_expert, tile_row0, tile_n, counters, sorted_pair, out, BN, max_tiles,
-                      GluAct{limit, alpha, shift, (const float*)in_scale}, miss_flag, err, nullptr, stream, true);
+                      GluAct{limit, alpha, shift, (const float*)in_scale}, miss_flag, err, nullptr, stream, kDirect);
+}
+
+// Both halves over bf16 experts with hidden values in bf16 (`act` [cap_rows, F] bf16: out of gateup = 1, `b` of gateup = 0), in tiles of 32 rows: the roundings
+// and the range of the weight-streaming kernels, for steps of few rows.
+LSB_API int lsb_moe_tc_ffn_bf16(int gateup, const void* b, int cap_rows, const void* arena, const void* slot_of, const void* fmt_struct,
+                                const void* tile_expert, const void* tile_row0, const void* tile_n, const void* counters,
+                                const void* sorted_pair, void* out, int BN, int max_tiles, float limit, float alpha, float shift, const void* in_scale,
+                                void* miss_flag, void* err, void* stream) {
+    return moe_tc_ffn(gateup, b, cap_rows, arena, slot_of, fmt_struct, tile_expert, tile_row0, tile_n, counters, sorted_pair, out, BN, max_tiles,
+                      GluAct{limit, alpha, shift, (const float*)in_scale}, miss_flag, err, nullptr, stream, kDirectBf16);
 }
 
 // The gate/up half with another gated unit (GluAct): in_scale [npairs] in pair order, or null.

@@ -111,8 +111,8 @@ F32_SPLIT_MIN_ROWS = 128  # rows from which an fp32 matrix (the router) runs as 
 # rows and hidden values the range of bf16 there, where the grouped kernel's operands are fp16, and a row's expert outputs are the same bits whatever up to 14
 # others share its step (an answer's tokens and the check of a draft of them).
 TC_MOE_MIN_ROWS = 16
-# ... and gated bf16 experts, whose gate and up matrices and rows go to the tensor core as they are (64 of 4096 x 2048: 1 row 108 against 113 us, 2 rows 174 / 173,
-# 4 rows 289 / 254, 12 rows 609 / 457)
+# ... and gated bf16 experts, whose matrices and rows go to the tensor core as they are and whose hidden values are bf16 below that, as in the streaming kernels
+# (streaming against grouped, 64 experts of 4096 x 2048, top 8: 1 row 121 / 130 us, 2 rows 182 / 183, 3 rows 239 / 222, 4 rows 296 / 253, 12 rows 624 / 441)
 TC_MOE_BF16_ROWS = 3
 # rows from which a bf16 matrix runs on the tensor-core GEMM: above four rows the weight-streaming kernel reads the matrix twice (5 rows of 24896 x 4096:
 # 108 us against 55 us)
@@ -572,10 +572,10 @@ class MoeBuffers:
         return 32 if avg <= 32 else (64 if avg <= 96 else 128)
 
     def step_tiles(self, P: int, E: int) -> tuple:
-        """(rows per tile, tiles at most) of a step of ``P`` pairs; the block-scaled operands are laid out for the workspace's own tiles."""
+        """(rows per tile, tiles at most) of a step of ``P`` pairs; the block-scaled operands are laid out for the workspace's own tiles, few rows take tiles of 32."""
         if self.bs_ok:
             return self.tc_bn, min(self.tc_tiles, P // self.tc_bn + E + 1)
-        bn = self.tile_rows(P, E)
+        bn = 32 if P < TC_MOE_MIN_ROWS * self.S else self.tile_rows(P, E)
         return bn, P // bn + E + 1
 
     def alloc_moe(self, z, R: int, S: int, E: int, n_logits: int, H: int, F: int, tc: bool, act_dtype=torch.bfloat16):
@@ -833,6 +833,12 @@ class ModelBase:
                 return
             up = (ws.tc_xs, ws.tc_xs.shape[0], arena.data, arena.slot_of, efp, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, ws.tc_sorted, ws.tc_act,
                   bn, tiles, limit)
+            if R < TC_MOE_MIN_ROWS:
+                unit = (1.0, 0.0, None) if act is None else act
+                nat.call("lsb_moe_tc_ffn_bf16", 1, *up, *unit, miss, err)
+                nat.call("lsb_moe_tc_ffn_bf16", 0, ws.tc_act, ws.tc_act.shape[0], arena.data, arena.slot_of, efp, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n,
+                         ws.tc_cnt, ws.tc_sorted, ws.y, bn, tiles, 0.0, *(1.0, 0.0, None), None, err)
+                return
             if self._moe_direct(arena.ef) and act != "relu2":
                 nat.call("lsb_moe_tc_gateup_bf16", *up, *((1.0, 0.0, None) if act is None else act), miss, err)
             elif act is None or act == "relu2":

@@ -184,10 +184,10 @@ def test_steps_of_few_rows(fmt, first):
         assert int(mb.miss) == 0
 
 
-@pytest.mark.parametrize("fmt,rows", [("fp8_e4m3", (1, 2, 9, 15)), ("gguf_q4_k", (1, 2, 9, 15)), ("bf16", (1, 2))])
+@pytest.mark.parametrize("fmt,rows", [("fp8_e4m3", (1, 2, 9, 15)), ("gguf_q4_k", (1, 2, 9, 15)), ("bf16", (1, 2, 3, 9, 15))])
 def test_steps_of_few_rows_keep_the_range_of_bf16(fmt, rows):
     """Hidden values of about 1e6, FP8 block scales that are no powers of two and above 0.57 (where 256 of them times 448 passes fp16's largest number), and a
-    row of activations beyond it."""
+    row of activations beyond it (bf16 experts: on the grouped kernel with bf16 hidden values from 3 rows)."""
     from layerstorm_b200.models.device_model import ModelBase, MoeBuffers
     dev = torch.device("cuda")
     H, F, E, S = 256, 256, 9, 6
@@ -316,6 +316,52 @@ def test_bf16_rows_meet_bf16_experts_directly(H, F, BN, scaled):
         want = gv * torch.sigmoid(alpha * gv) * (uv + shift)
         # fp32 sums, the unit rounded to fp16 (2^-11 relative at most)
         assert float((got[pos] - want).norm() / want.norm()) < 1e-3, (pos, e)
+
+
+@pytest.mark.parametrize("H,F", [(128, 384), (640, 128), (1152, 640)])
+@pytest.mark.parametrize("R", [1, 15])
+@pytest.mark.parametrize("scaled", [False, True])
+def test_few_rows_keep_bf16_hidden_values_over_bf16_experts(H, F, R, scaled):
+    """Both halves of the direct form: reductions that end inside an operand stage and that wrap the rings, a full and a nearly empty tile, an expert that is not
+    resident, another gated unit with a factor per pair, hidden values and down weights outside fp16's range."""
+    from layerstorm_b200.ops import _native as nat
+    dev = torch.device("cuda")
+    E, S, BN = 20, 2, 32
+    arena, ref = _setup("bf16", H, F, E, n_missing=1, seed=14, size=1.0 if scaled else 2000.0)
+    for e in range(1, E):
+        w = arena.data[int(arena.slot_of[e])][arena.ef.off_down:][: F * H * 2].view(torch.bfloat16)
+        w *= 1e-7
+        ref[e] = [m.double().cpu() for m in arena.read_expert(int(arena.slot_of[e]), "bf16")]
+    g = torch.Generator(device="cpu").manual_seed(15)
+    x = torch.randn(R, H, generator=g).to(torch.bfloat16).to(dev)
+    ids = torch.stack([torch.full((R,), E - 1), torch.arange(R) % (E - 1)], 1).int().to(dev).contiguous()
+    P, tiles = R * S, R * S // BN + E + 1
+    i32 = dict(dtype=torch.int32, device=dev)
+    srt, te, tr, tn, cnt, err, miss = (torch.zeros(n, **i32) for n in (P, tiles, tiles, tiles, 2, 1, 1))
+    xs, act, y = torch.zeros(P, H, dtype=torch.bfloat16, device=dev), torch.zeros(P, F, dtype=torch.bfloat16, device=dev), torch.full((P, H), float("nan"), device=dev)
+    fac = torch.rand(P, generator=g).to(dev) if scaled else None
+    limit, alpha, shift = (1.1, 1.702, 1.0) if scaled else (0.0, 1.0, 0.0)
+    efp = ctypes.addressof(arena.ef)
+    nat.call("lsb_moe_tc_sort", ids, P, E, BN, srt, te, tr, tn, cnt)
+    nat.call("lsb_moe_tc_gather_bf16", x, srt, cnt, xs, P, S, H)
+    tl = (P, arena.data, arena.slot_of, efp, te, tr, tn, cnt, srt)
+    nat.call("lsb_moe_tc_ffn_bf16", 1, xs, *tl, act, BN, tiles, limit, alpha, shift, fac, miss, err)
+    nat.call("lsb_moe_tc_ffn_bf16", 0, act, *tl, y, BN, tiles, 0.0, 1.0, 0.0, None, None, err)
+    torch.cuda.synchronize()
+    assert int(err) == 0 and int(miss) == 1
+    xd, got = x.double().cpu(), y.double().cpu()
+    for p in range(P):
+        r, e = p // S, int(ids.view(-1)[p])
+        if e < 1:
+            assert bool(got[p].isnan().all())
+            continue
+        c = float(fac[p]) if scaled else 1.0
+        gv, uv = ref[e][0] @ xd[r] * c, ref[e][1] @ xd[r] * c
+        if limit:
+            gv, uv = gv.clamp(max=limit), uv.clamp(-limit, limit)
+        want = ref[e][2] @ (gv * torch.sigmoid(alpha * gv) * (uv + shift))
+        # fp32 sums and a hidden value in bf16: 2^-9 of it at most, averaged out over F of them
+        assert float((got[p] - want).norm() / want.norm()) < 4e-3, (p, e)
 
 
 @pytest.mark.parametrize("R", [16, 97, 340, 700])
