@@ -268,7 +268,7 @@ class BlockWorkspace(StepBuffers):
             if b.experts and m.moe_key(i) not in self.moe:
                 arena = m.layers[i]["arena"]
                 mb = MoeBuffers()
-                mb.alloc_moe(z, R, b.top, b.experts, b.experts + b.identity, arena.ef.H, arena.ef.F, tc=not m.f32 and R >= m.moe_grouped_from(arena.ef),
+                mb.alloc_moe(z, R, b.top, b.experts, b.experts + b.identity, arena.ef.H, arena.ef.F, tc=not m.f32 and m.moe_grouped(arena, b.top, R),
                              act_dtype=act)
                 if mb.tc_ok:
                     mb.tc_xs = z(R * b.top, arena.ef.H, dtype=torch.float16)

@@ -111,9 +111,12 @@ F32_SPLIT_MIN_ROWS = 128  # rows from which an fp32 matrix (the router) runs as 
 # rows and hidden values the range of bf16 there, where the grouped kernel's operands are fp16, and a row's expert outputs are the same bits whatever up to 14
 # others share its step (an answer's tokens and the check of a draft of them).
 TC_MOE_MIN_ROWS = 16
-# ... and gated bf16 experts, whose matrices and rows go to the tensor core as they are and whose hidden values are bf16 below that, as in the streaming kernels
-# (streaming against grouped, 64 experts of 4096 x 2048, top 8: 1 row 121 / 130 us, 2 rows 182 / 183, 3 rows 239 / 222, 4 rows 296 / 253, 12 rows 624 / 441)
-TC_MOE_BF16_ROWS = 3
+# ... and gated bf16 experts, whose matrices and rows go to the tensor core as they are and whose hidden values are bf16 below that, as in the streaming kernels,
+# from 3 rows where the step's experts are at least so many bytes: the grouped kernel streams faster, but takes 50 us whatever there is to do.  Streaming against
+# grouped, us: 64 experts of 4096 x 2048, top 8: 2 rows (730 MB) 182 / 183, 3 rows (1.0 GB) 239 / 222, 12 rows 624 / 441; an eighth of them resident, 8 rows (240 MB)
+# 107 / 122, 15 rows (380 MB) 175 / 162; 128 of 2048 x 768: 4 rows (270 MB) 91 / 103, 8 rows (480 MB) 138 / 138, 15 rows (750 MB) 209 / 173; 8 of 4096 x 14336, top
+# 2: 1 row (700 MB) 159 / 184, 3 rows (1.6 GB) 372 / 347; 16 of 1024 x 512: 15 rows (45 MB) 46 / 54.
+TC_MOE_BF16_ROWS, TC_MOE_BF16_BYTES = 3, 500e6
 # rows from which a bf16 matrix runs on the tensor-core GEMM: above four rows the weight-streaming kernel reads the matrix twice (5 rows of 24896 x 4096:
 # 108 us against 55 us)
 TC_GEMM_MIN_ROWS = 5
@@ -675,8 +678,8 @@ class Workspace(StepBuffers, MoeBuffers):
         if cfg.n_routed > 0:
             S = cfg.top_k + cfg.n_shared
             E_total = cfg.n_routed + cfg.n_shared
-            first = min((m.moe_grouped_from(L["arena"].ef) for L in m.layers if L.get("arena") is not None), default=TC_MOE_MIN_ROWS)
-            self.alloc_moe(z, R, S, E_total, cfg.n_routed, H, cfg.moe_inter, tc=m.Fe % 128 == 0 and R >= first)
+            self.alloc_moe(z, R, S, E_total, cfg.n_routed, H, cfg.moe_inter,
+                           tc=m.Fe % 128 == 0 and any(m.moe_grouped(L["arena"], S, R) for L in m.layers if L.get("arena") is not None))
             if self.tc_ok:
                 # block-scaled path (NVFP4 experts): both operands stay 4-bit, the activations are quantised in tile order
                 fmts = {L["arena"].ef.fmt for L in m.layers if L.get("arena") is not None}
@@ -772,16 +775,22 @@ class ModelBase:
 
     # ------------------------------------------------------------------ routed experts of a step
     def moe_mode(self, arena: "ExpertArena", ws, R: int) -> str:
-        if (getattr(ws, "tc_ok", False) and R >= (TC_MOE_MIN_ROWS if ws.bs_ok else self.moe_grouped_from(arena.ef)) and arena.ef.fmt <= 3
-                and not arena.ef.fmt_down1):
+        if (getattr(ws, "tc_ok", False) and arena.ef.fmt <= 3 and not arena.ef.fmt_down1
+                and (R >= TC_MOE_MIN_ROWS if ws.bs_ok else self.moe_grouped(arena, ws.S, R))):
             return "tc"
         fast_fp4 = arena.ef.fmt == 2 and arena.ef.F % 128 == 0 and arena.ef.H % 128 == 0
         return "pairs" if (fast_fp4 and R * ws.S <= 72) else "groups"
 
     @staticmethod
-    def moe_grouped_from(ef: ExpertFmt) -> int:
-        """Rows per step from which experts of this layout run on the grouped kernel."""
-        return TC_MOE_BF16_ROWS if ModelBase._moe_direct(ef) else TC_MOE_MIN_ROWS
+    def moe_grouped(arena: "ExpertArena", S: int, R: int) -> bool:
+        """Whether steps of ``R`` rows with ``S`` slots each run on the grouped kernel (then those of more rows do, too)."""
+        if R >= TC_MOE_MIN_ROWS:
+            return True
+        if R < TC_MOE_BF16_ROWS or not ModelBase._moe_direct(arena.ef):
+            return False
+        E = arena.slot_of.numel()
+        hit = E * (1.0 - (1.0 - min(1.0, S / E)) ** R)               # experts that independent rows ask for
+        return hit * min(1.0, arena.n_slots / E) * arena.ef.stride >= TC_MOE_BF16_BYTES
 
     @staticmethod
     def _moe_direct(ef: ExpertFmt) -> bool:

@@ -147,10 +147,12 @@ def test_widths_that_end_inside_boxes_and_operand_stages(fmt, H, F, BN):
 
 
 @pytest.mark.parametrize("fmt,first", [("bf16", 3), ("fp8_e4m3", 16), ("nvfp4", 16), ("gguf_q4_k", 16)])
-def test_steps_of_few_rows(fmt, first):
+def test_steps_of_few_rows(fmt, first, monkeypatch):
     """Both sides of the row count from which a format's experts run on the grouped kernel and (NVFP4: 12 rows of 6 pairs) from which they run in groups, an id
     that takes no part among them."""
+    from layerstorm_b200.models import device_model
     from layerstorm_b200.models.device_model import ModelBase, MoeBuffers
+    monkeypatch.setattr(device_model, "TC_MOE_BF16_BYTES", 0)
     dev = torch.device("cuda")
     H, F, E, S = 256, 256, 9, 6
     arena, ref = _setup(fmt, H, F, E, n_missing=0, seed=5)
@@ -185,10 +187,12 @@ def test_steps_of_few_rows(fmt, first):
 
 
 @pytest.mark.parametrize("fmt,rows", [("fp8_e4m3", (1, 2, 9, 15)), ("gguf_q4_k", (1, 2, 9, 15)), ("bf16", (1, 2, 3, 9, 15))])
-def test_steps_of_few_rows_keep_the_range_of_bf16(fmt, rows):
+def test_steps_of_few_rows_keep_the_range_of_bf16(fmt, rows, monkeypatch):
     """Hidden values of about 1e6, FP8 block scales that are no powers of two and above 0.57 (where 256 of them times 448 passes fp16's largest number), and a
     row of activations beyond it (bf16 experts: on the grouped kernel with bf16 hidden values from 3 rows)."""
+    from layerstorm_b200.models import device_model
     from layerstorm_b200.models.device_model import ModelBase, MoeBuffers
+    monkeypatch.setattr(device_model, "TC_MOE_BF16_BYTES", 0)
     dev = torch.device("cuda")
     H, F, E, S = 256, 256, 9, 6
     arena, ref = _setup(fmt, H, F, E, n_missing=0, seed=9, size=2000.0)
@@ -254,8 +258,21 @@ def test_a_row_of_few_gets_the_same_experts_outputs_in_any_company(fmt):
                     assert torch.equal(y[row - first], want), (R, first, row)
 
 
-def test_steps_of_few_rows_take_no_grouped_buffers():
+@pytest.mark.parametrize("E,H,F,S,slots,first", [(64, 4096, 2048, 8, 64, 3), (64, 4096, 2048, 8, 8, 16), (128, 2048, 768, 8, 128, 9), (8, 4096, 14336, 2, 8, 3),
+                                                 (16, 1024, 512, 2, 16, 16), (64, 4096, 2048, 8, 16, 8)])
+def test_few_rows_run_grouped_where_their_experts_are_many_bytes(E, H, F, S, slots, first):
+    import types
+    from layerstorm_b200.models.device_model import ModelBase, expert_layout
+    fake = types.SimpleNamespace(ef=expert_layout("bf16", H, F), slot_of=torch.empty(E), n_slots=slots)
+    assert [R for R in range(1, 40) if ModelBase.moe_grouped(fake, S, R)] == list(range(first, 40))
+    fake.ef = expert_layout("bf16", H, F, gated=False)
+    assert not ModelBase.moe_grouped(fake, S, 15) and ModelBase.moe_grouped(fake, S, 16)
+
+
+def test_steps_of_few_rows_take_no_grouped_buffers(monkeypatch):
     """A workspace whose steps all stream their experts has neither the grouped kernel's buffers nor the block-scaled ones."""
+    from layerstorm_b200.models import device_model
+    monkeypatch.setattr(device_model, "TC_MOE_BF16_BYTES", 0)
     from layerstorm_b200.models.config import get_preset
     from layerstorm_b200.models.device_model import DeviceModel, Workspace
     from layerstorm_b200.models.weights import init_weights
