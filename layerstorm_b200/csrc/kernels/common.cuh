@@ -70,6 +70,10 @@ __device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u 
 __device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 
 // 8 bf16 (one 16-byte vector) -> 8 floats
+// fp16 operands made of wider numbers: finite ones stay finite (the nearest that there is), infinities and NaN stay what they are.
+__device__ __forceinline__ float half_range(float v) { return fabsf(v) < __int_as_float(0x7f800000) ? fminf(fmaxf(v, -65504.f), 65504.f) : v; }
+__device__ __forceinline__ __half2 half2_finite(float a, float b) { return __floats2half2_rn(half_range(a), half_range(b)); }
+
 __device__ __forceinline__ void unpack_bf16x8(const uint4& v, float* f) {
     f[0] = bf16_lo(v.x); f[1] = bf16_hi(v.x);
     f[2] = bf16_lo(v.y); f[3] = bf16_hi(v.y);

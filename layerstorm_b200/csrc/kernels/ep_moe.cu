@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(128) ep_dispatch_kernel(const bf16* __restrict
             unpack_bf16x8(__ldg(reinterpret_cast<const uint4*>(src + k)), f);
             __half2 h[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) h[q] = __floats2half2_rn(f[2 * q], f[2 * q + 1]);
+            for (int q = 0; q < 4; ++q) h[q] = half2_finite(f[2 * q], f[2 * q + 1]);
             *reinterpret_cast<uint4*>(dst + k) = *reinterpret_cast<uint4*>(h);       // 16-byte store over NVLink when o != rank
         }
     }

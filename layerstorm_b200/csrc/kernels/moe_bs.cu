@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(MoeBsCfg<BN, GATEUP, FMT>::THREADS) moe_bs_ffn
                             if (GATEUP) {
                                 float gv = gq[j] * sg * ax, uv = uq[j] * su * ax;
                                 if (p.limit > 0.f) { gv = fminf(gv, p.limit); uv = fminf(fmaxf(uv, -p.limit), p.limit); }
-                                p.act[((size_t)t * BN + c0 + j) * NOUT + n] = __float2half_rn(siluf_(gv) * uv);
+                                p.act[((size_t)t * BN + c0 + j) * NOUT + n] = __float2half_rn(half_range(siluf_(gv) * uv));
                             } else {
                                 if (p.out_bf16) reinterpret_cast<bf16*>(p.y)[(size_t)orow * p.ldo + n] = __float2bfloat16(gq[j] * sg * ax);
                                 else reinterpret_cast<float*>(p.y)[(size_t)orow * p.ldo + n] = gq[j] * sg * ax;

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(1024) moe_tc_sort_kernel(const int* __restrict
     pdl_launch_dependents();
 }
 
-// xs[pos][:] = fp16(x[sorted_pair[pos] / S][:])
+// xs[pos][:] = fp16(x[sorted_pair[pos] / S][:]), finite numbers beyond fp16 as its largest
 __global__ void __launch_bounds__(128) moe_tc_gather_kernel(const bf16* __restrict__ x, const int* __restrict__ sorted_pair,
                                                             const int* __restrict__ counters, __half* __restrict__ xs, int S, int H) {
     pdl_wait();
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(128) moe_tc_gather_kernel(const bf16* __restri
         unpack_bf16x8(__ldg(reinterpret_cast<const uint4*>(src + k)), f);
         __half2 h[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
+        for (int i = 0; i < 4; ++i) h[i] = half2_finite(f[2 * i], f[2 * i + 1]);
         *reinterpret_cast<uint4*>(dst + k) = *reinterpret_cast<uint4*>(h);
     }
     pdl_launch_dependents();
@@ -187,7 +187,7 @@ template <int NH> struct RowConv<1, NH> {     // FP8 e4m3 with 128 x 128 block s
         for (int i = 0; i < NV; ++i) r.v[i] = ld_shared_16(swz_chunk(tile, row, sub * 4 + h * NV + i));
     }
     static __device__ __forceinline__ void convert(const Raw& r, uint32_t* out, int, int) {
-        // block scales of small weights sit near the bottom of the fp16 range: carry them times 2^8 (exact)
+        // block scales of small weights sit near the bottom of the fp16 range: carry them times 2^8 (exact; block scales up to 146 / 256, weights up to 255)
         // and take the factor out again in the fp32 epilogue (kFp8Unscale)
         const __half2 s2 = __float2half2_rn(r.sc * 256.f);
 #pragma unroll
@@ -728,7 +728,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                             if (GATEUP && DIRECT == kDirectBf16) {
                                 reinterpret_cast<bf16*>(p.act)[(size_t)(row0 + c0 + j) * NOUT + n] = __float2bfloat16(glu_act(gq[j] * c, uq[j] * c, p.ga));
                             } else if (GATEUP) {
-                                p.act[(size_t)(row0 + c0 + j) * NOUT + n] = __float2half_rn(glu_act(gq[j] * sg * c, uq[j] * su * c, p.ga));
+                                p.act[(size_t)(row0 + c0 + j) * NOUT + n] = __float2half_rn(half_range(glu_act(gq[j] * sg * c, uq[j] * su * c, p.ga)));
                             } else if (up) {
                                 // (fp16 range: far outside what normed inputs reach, kept finite all the same)
                                 p.act[(size_t)(row0 + c0 + j) * NOUT + n] = __float2half_rn(fminf(relu2_act(gq[j] * sg), 65504.f));

@@ -381,6 +381,47 @@ def test_few_rows_keep_bf16_hidden_values_over_bf16_experts(H, F, R, scaled):
         assert float((got[p] - want).norm() / want.norm()) < 4e-3, (p, e)
 
 
+@pytest.mark.parametrize("fmt", ["nvfp4", "fp8_e4m3", "bf16", "gguf_q4_k"])
+def test_many_rows_stay_finite_beyond_fp16(fmt):
+    """Hidden values of 4e4 rms, some of them beyond fp16, and a row of activations of 1e6 (hidden values of 1e15) count as fp16's largest number; a row with a NaN
+    and one with an infinity give no numbers, and none of them touches its neighbours."""
+    from layerstorm_b200.models.device_model import ModelBase, MoeBuffers
+    dev = torch.device("cuda")
+    H, F, E, S, R = 256, 256, 5, 2, 40
+    arena, ref = _setup(fmt, H, F, E, n_missing=0, seed=16, size=300.0)
+    m, mb = ModelBase(), MoeBuffers()
+    m.device, m.tp_size, m.expert_shard = dev, 1, "ep"
+    z = lambda *s, dtype=torch.float32: torch.zeros(*s, dtype=dtype, device=dev)
+    mb.alloc_moe(z, R, S, E, E, H, F, tc=True)
+    mb.tc_xs, mb.tc_act = z(R * S, H, dtype=torch.float16), z(R * S, F, dtype=torch.float16)
+    g = torch.Generator(device="cpu").manual_seed(17)
+    x = torch.randn(R, H, generator=g) * 0.8
+    x[7] *= 1.25e6
+    x[9, 3], x[11, 5] = float("nan"), float("inf")
+    x = x.to(torch.bfloat16).to(dev)
+    ids = torch.stack([torch.randperm(E, generator=g)[:S] for _ in range(R)])
+    mb.ids.copy_(ids.int())
+    m.moe_prepare(arena, mb, x, R, E)
+    m.moe_experts(arena, mb, x, R, E, 0.0, mb.miss)
+    got, xd = mb.y.view(R, S, H).double().cpu(), x.double().cpu()
+    if fmt != "bf16":
+        xd = xd.clamp(-65504.0, 65504.0)
+    for r in range(R):
+        for k in range(S):
+            if r in (9, 11):
+                assert not bool(got[r, k].isfinite().any()), (r, k)
+                continue
+            gate, up, down = ref[int(ids[r, k])]
+            want = down @ (torch.nn.functional.silu(gate @ xd[r]) * (up @ xd[r])).clamp(-65504.0, 65504.0)
+            if r == 7 and fmt == "gguf_q4_k":                 # every hidden value is at the limit, its sign that of sums whose weights are rounded
+                assert bool(got[r, k].isfinite().all())
+                continue
+            # hidden values in fp16, 2^-11 at most of each; Q4_K weights d sc v - dmin m with both products rounded to fp16: 2^-11 of terms up to 15 d sc and 8 d sc
+            # beside weights of 4.6 d sc rms is 2.4e-3 at most a matrix, three of them 4.2e-3 (most hidden values are inside the range: an error of those beyond it
+            # would count against a norm that the limit has cut)
+            assert float((got[r, k] - want).norm() / want.norm()) < (4.2e-3 if fmt == "gguf_q4_k" else 1e-3), (r, k)
+
+
 @pytest.mark.parametrize("R", [16, 97, 340, 700])
 def test_steps_of_fewer_rows_than_the_workspace(R):
     """The token tile follows the step's rows, not the workspace's: 32, 64 and 128 rows of a workspace whose own tile is 128."""
