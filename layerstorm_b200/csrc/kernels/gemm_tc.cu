@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(TcCfg<BN, MT>::THREADS) gemm_tc_kernel(const _
         // ---------------- epilogue ----------------
         const int q = warp & 3, mt = (warp - 2) >> 2;
         const int n = n0 + mt * BM + q * 32 + lane;
-        bool ok = nkb > 0 ? mbar_wait(acc_full, 0, p.err, 3) : true;
+        const bool ok = __all_sync(0xffffffffu, nkb > 0 ? mbar_wait(acc_full, 0, p.err, 3) : true);      // one answer for the warp: its loads are warp-wide
         tc_fence_after();
         if (ok) {
             const float b = (p.bias && n < p.N && p.splits == 1) ? p.bias[n] : 0.f;

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(192) indexer_score_tc_kernel(const __grid_cons
         } else if (warp >= 2) {
             const int q = warp & 3;
             const int n = k0 + q * 32 + lane;                               // this thread's key
-            const bool ok = mbar_wait_relaxed(acc_full, 0, p.err, 32);
+            const bool ok = __all_sync(0xffffffffu, mbar_wait_relaxed(acc_full, 0, p.err, 32));
             tc_fence_after();
             if (ok) {
                 const float ks = n < ne_tile ? p.kscale[n] : 0.f;
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(192) indexer_score_f8_kernel(const __grid_cons
                 const int pg = p.block_table[(size_t)seq * p.max_pages + n / p.page];
                 ks = *reinterpret_cast<const float*>(p.cache + ((size_t)pg * p.page + n % p.page) * kScEntry + kScD);
             }
-            const bool ok = mbar_wait_relaxed(acc_full, 0, p.err, 34);
+            const bool ok = __all_sync(0xffffffffu, mbar_wait_relaxed(acc_full, 0, p.err, 34));
             tc_fence_after();
             if (ok) {
                 float sum = 0.f;

@@ -101,6 +101,28 @@ def test_two_weight_tiles_per_cta(M, N, K, ob):
     assert float((out[:M, :N].double() - want).norm() / want.norm()) < (3e-3 if ob else 1e-5)
 
 
+@pytest.mark.parametrize("N", [72, 144, 1000])
+@pytest.mark.parametrize("M", [5, 12, 40, 100, 142, 398])
+def test_matrices_that_end_inside_a_warps_rows(M, N):
+    """Lanes with and without a row of the matrix side by side in every token tile, split reduction, bias and both output types; and as a batch."""
+    K = 4096
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w = (torch.randn(n, K, generator=g, device="cuda").bfloat16() for n in (M, N))
+    bias, part, err = torch.randn(N, generator=g, device="cuda"), torch.zeros(1 << 24, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = x.double() @ w.double().T
+    # fp32 sums (2^-24 sqrt(K) = 4e-6), rounded to bf16 (2^-9) where asked
+    for split in (False, True):
+        for dt, tol in ((torch.float32, 1e-5), (torch.bfloat16, 3e-3)):
+            out = torch.zeros(M + 1, N + 8, device="cuda", dtype=dt)
+            nat.call("lsb_gemm_bf16_tc", out, x, w, bias, M, N, K, K, K, N + 8, int(dt == torch.bfloat16), part if split else None, part.numel() if split else 0, err, None)
+            assert int(err) == 0 and float(out[M:].abs().sum()) == 0.0 and float(out[:M, N:].abs().sum()) == 0.0
+            assert float((out[:M, :N].double() - want - bias.double()).norm() / want.norm()) < tol
+    B, out = 4, torch.zeros(4, M, N, device="cuda")
+    nat.call("lsb_gemm_bf16_tc_batched", out, x, w, M, N, K // B, B, K, K // B, K, K // B, N, M * N, 0, err)
+    parts = torch.stack([x[:, b * K // B: (b + 1) * K // B].double() @ w[:, b * K // B: (b + 1) * K // B].double().T for b in range(B)])
+    assert int(err) == 0 and float((out.double() - parts).norm() / parts.norm()) < 1e-5
+
+
 @pytest.mark.parametrize("M", [4, 5, 7, 8])
 @pytest.mark.parametrize("N,K", [(8, 64), (72, 136), (1040, 4096)])
 def test_bf16_linear_of_few_rows(M, N, K):
