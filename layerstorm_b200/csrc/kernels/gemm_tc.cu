@@ -23,6 +23,7 @@ namespace lsb {
 using namespace tc;
 
 constexpr int BM = 128;   // weight rows per tile (UMMA M)
+constexpr int kSms = 148;
 constexpr int BK = 64;    // bf16 elements per stage row = 128 bytes = one swizzle span
 
 struct GemmTcParams {
@@ -42,19 +43,20 @@ struct GemmTcParams {
 // through L2 per product than two CTAs of 128 x 256; MT = 1 has half the shared memory of an SM, so that two CTAs share one and the epilogue of
 // one runs under the main loop of the other.  Measured (one CTA of 128 x 256 per SM, MT = 1 at half an SM, MT = 2): 2048 x 24896 x 4096 534, 446,
 // 422 us; 2048 x 4096 x 12288 205, 182, 165 us; 391 x 16640 x 4096 119, 94, 89 us; MT = 1 with 64-row tiles and smaller: 32 x 24896 x 4096 66 -> 55 us.
-template <int BN, int MT> struct TcCfg {
+// DEEP: MT = 1 with twice the stages, for grids that give an SM one CTA at a time anyway.
+template <int BN, int MT, bool DEEP = false> struct TcCfg {
     static constexpr int A_BYTES = BM * BK * 2;
     static constexpr int B_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = MT * A_BYTES + B_BYTES;
-    static constexpr int STAGES = MT == 2 ? 3 : (BN >= 256 ? 2 : (BN >= 128 ? 3 : 4));
+    static constexpr int STAGES = MT == 2 ? 3 : (BN >= 256 ? 2 : (BN >= 128 ? 3 : 4)) * (DEEP ? 2 : 1);
     static constexpr int TMEM_COLS = MT * (BN < 32 ? 32 : BN);
     static constexpr int THREADS = 64 + 128 * MT;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
 
-template <int BN, int MT = 1, bool BATCHED = false>
-__global__ void __launch_bounds__(TcCfg<BN, MT>::THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GemmTcParams p) {
-    using C = TcCfg<BN, MT>;
+template <int BN, int MT = 1, bool BATCHED = false, bool DEEP = false>
+__global__ void __launch_bounds__(TcCfg<BN, MT, DEEP>::THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GemmTcParams p) {
+    using C = TcCfg<BN, MT, DEEP>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE_BYTES);
@@ -275,15 +277,16 @@ int cached_map_2d(CUtensorMap* out, const void* ptr, CUtensorMapDataType dt, int
     return 0;
 }
 
-template <int BN, int MT = 1>
+template <int BN, int MT = 1, bool DEEP = false>
 static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTcParams& p, cudaStream_t st) {
-    using C = TcCfg<BN, MT>;
+    using C = TcCfg<BN, MT, DEEP>;
     static bool attr = false;
-    if (!attr) { cudaFuncSetAttribute(gemm_tc_kernel<BN, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM); attr = true; }
+    if (!attr) { cudaFuncSetAttribute(gemm_tc_kernel<BN, MT, false, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM); attr = true; }
     dim3 grid((p.M + BN - 1) / BN, (p.N + BM * MT - 1) / (BM * MT), p.splits);
-    launch_pdl((gemm_tc_kernel<BN, MT>), grid, C::THREADS, C::SMEM, st, mw, mx, p);
+    launch_pdl((gemm_tc_kernel<BN, MT, false, DEEP>), grid, C::THREADS, C::SMEM, st, mw, mx, p);
     return (int)cudaGetLastError();
 }
+
 
 template <int BN>
 static int launch_tc_batched(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTcParams& p, int batch, cudaStream_t st) {
@@ -365,21 +368,29 @@ LSB_API int lsb_gemm_bf16_tc(void* out, const void* x, const void* w, const void
     const int nkb = (K + BK - 1) / BK;
     const int tiles = ((N + BM - 1) / BM) * ((M + BN - 1) / BN);
     int splits = 1;
-    if (partial && tiles < 148) {
-        splits = (148 + tiles - 1) / tiles;
+    if (partial && tiles < kSms) {
+        splits = (kSms + tiles - 1) / tiles;
         if (splits > 16) splits = 16;
         if (splits > nkb / 4) splits = nkb / 4 > 0 ? nkb / 4 : 1;
         while (splits > 1 && (long long)splits * M * N > partial_cap) --splits;
     }
     p.kb_per_split = (nkb + splits - 1) / splits;
     p.splits = (nkb + p.kb_per_split - 1) / p.kb_per_split;
+    const int ctas = tiles * p.splits;                     // of one weight tile each
     switch (BN) {
         case 16: rc = launch_tc<16>(mw, mx, p, st); break;
         case 32: rc = launch_tc<32>(mw, mx, p, st); break;
         case 64: rc = launch_tc<64>(mw, mx, p, st); break;
         case 128: rc = launch_tc<128>(mw, mx, p, st); break;
-        // Two weight tiles per CTA pay from a reduction of 2048 on (K = 1536 and below: the same; a short one leaves the longer epilogue bare)
-        default: rc = K >= 2048 && !comm ? launch_tc<256, 2>(mw, mx, p, st) : launch_tc<256>(mw, mx, p, st); break;
+        // (one CTA of 128 x 256 per SM before there was a choice, one weight tile, one and deep, two; us).  A grid that one CTA per SM takes in one wave is deep:
+        // 160 x 576 x 4096 27.8, 26.4, 25.9, 28.9; 256 x 2048 x 2048 36.6, 35.1, 33.8, 38.1.  So is one of two to three such waves over a long reduction, which
+        // takes CTAs of two tiles two waves: 1500 x 7168 x 12288 298, 334, 291, 306; 391 x 24896 x 12288 304, 343, 301, 312, but 391 x 24896 x 4096 146, 139, 143,
+        // 130 and 1000 x 24896 x 12288 (780 CTAs) 659, 554, 645, 518.  Two weight tiles per CTA pay from a reduction of 2048 on (K = 1536 and below: the same; a
+        // short one leaves the longer epilogue bare) unless half the grid no longer covers the SMs: 300 x 576 x 4096 (150 CTAs) 36.6, 37.1, -, 40.2.
+        default:
+            if (ctas <= kSms || (K >= 8192 && ctas > 2 * kSms && ctas <= 3 * kSms)) rc = launch_tc<256, 1, true>(mw, mx, p, st);
+            else rc = K >= 2048 && !comm && ctas >= 160 ? launch_tc<256, 2>(mw, mx, p, st) : launch_tc<256>(mw, mx, p, st);
+            break;
     }
     if (rc) return rc;
     if (p.splits > 1) {

@@ -84,11 +84,13 @@ def test_quantised_linear_tensor_core_path(fmt, M, N, K):
     assert float((few - ref[:4]).abs().max() / ref.abs().max()) < 3e-3
 
 
-@pytest.mark.parametrize("M,N,K", [(129, 8, 2048), (257, 200, 2056), (513, 384, 2112), (300, 1000, 2048), (700, 30000, 2048)])
+@pytest.mark.parametrize("M,N,K", [(129, 8, 2048), (257, 200, 2056), (513, 384, 2112), (300, 1000, 2048), (700, 30000, 2048), (300, 2000, 2056), (1100, 576, 4096),
+                                   (300, 19000, 8200), (513, 12600, 8192)])
 @pytest.mark.parametrize("ob", [0, 1])
 def test_two_weight_tiles_per_cta(M, N, K, ob):
-    """Reductions from 2048 on over more than 128 rows: a second weight tile that is empty or not full, token tiles and stages that are not full, with and without
-    split reductions, a bias, nothing written beyond the matrix."""
+    """Reductions from 2048 on over more than 128 rows, in every form that they run in (one weight tile per CTA: one wave, just above it, three waves of a long
+    reduction; two tiles): a last weight tile that is empty or not full, token tiles and stages that are not full, with and without split reductions, a bias,
+    nothing written beyond the matrix."""
     g = torch.Generator(device="cuda").manual_seed(M)
     x, w = (torch.randn(n, K, generator=g, device="cuda").bfloat16() for n in (M, N))
     bias = torch.randn(N, generator=g, device="cuda")
