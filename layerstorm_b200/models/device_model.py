@@ -117,9 +117,10 @@ TC_MOE_MIN_ROWS = 16
 # 107 / 122, 15 rows (380 MB) 175 / 162; 128 of 2048 x 768: 4 rows (270 MB) 91 / 103, 8 rows (480 MB) 138 / 138, 15 rows (750 MB) 209 / 173; 8 of 4096 x 14336, top
 # 2: 1 row (700 MB) 159 / 184, 3 rows (1.6 GB) 372 / 347; 16 of 1024 x 512: 15 rows (45 MB) 46 / 54.
 TC_MOE_BF16_ROWS, TC_MOE_BF16_BYTES = 3, 500e6
-# rows from which a bf16 matrix runs on the tensor-core GEMM: above four rows the weight-streaming kernel reads the matrix twice (5 rows of 24896 x 4096:
-# 108 us against 55 us)
-TC_GEMM_MIN_ROWS = 5
+# rows from which a bf16 matrix runs on the tensor-core GEMM: above four rows the weight-streaming kernel reads the matrix twice, above six three times.  Streaming
+# against GEMM, us: 5 rows of 24896 x 4096 101 / 52, of 1536 x 4096 10.6 / 9.6; but a small matrix is in L2 the second time, and the GEMM is two launches: 5 rows
+# of 72 x 4096 5.8 / 7.4, of 1024 x 4096 7.9 / 8.7, of 2048 x 2048 8.1 / 8.2, of 4096 x 512 6.1 / 7.0; 7 rows of those 7.8 / 7.8, 10.9 / 9.0, 11.2 / 8.4, 9.1 / 7.2
+TC_GEMM_MIN_ROWS, TC_GEMM_MIN_ROWS_SMALL, TC_GEMM_SMALL = 5, 7, 4 << 20
 # router projection + top-k in one launch for decode-sized steps (switch: LSB_ROUTER_FUSED=1).  Off by default: measured on the
 # GLM-5.3-Flash shape the fused kernel (one block per expert, last block selects) gives 7.21 ms per decode step against 7.12 ms for
 # the split-K GEMV + top-k pair, whose second launch already overlaps the first through programmatic dependent launch
@@ -385,7 +386,7 @@ class QLinear:
             if self.fmt != "f32" or ob or bias is not None or comm is not None:
                 raise RuntimeError("fp32 activations need fp32 weights and an fp32 output on one GPU")
             nat.call("lsb_gemm_f32", out, x, self.w, M, self.N, self.K, ldx, self.K, ldo)
-        elif self.fmt == "bf16" and M >= TC_GEMM_MIN_ROWS:
+        elif self.fmt == "bf16" and M >= (TC_GEMM_MIN_ROWS if self.N * self.K > TC_GEMM_SMALL else TC_GEMM_MIN_ROWS_SMALL):
             sc = TcScratch.get(self.w.device)
             nat.call("lsb_gemm_bf16_tc", out, x, self.w, bias, M, self.N, self.K, ldx, self.K, ldo, ob, sc.partial, sc.cap, sc.err, comm)
         elif (self.fmt == "nvfp4" and MOE_BLOCK_SCALED and M >= 16 and comm is None and bias is None and ldx == self.K and self.K % 256 == 0

@@ -125,11 +125,13 @@ def test_matrices_that_end_inside_a_warps_rows(M, N):
     assert int(err) == 0 and float((out.double() - parts).norm() / parts.norm()) < 1e-5
 
 
-@pytest.mark.parametrize("M", [4, 5, 7, 8])
-@pytest.mark.parametrize("N,K", [(8, 64), (72, 136), (1040, 4096)])
-def test_bf16_linear_of_few_rows(M, N, K):
-    """Both sides of the line between the weight-streaming kernel and the tensor-core GEMM."""
+@pytest.mark.parametrize("M", [4, 5, 6, 7, 8])
+@pytest.mark.parametrize("N,K", [(8, 64), (72, 136), (1024, 4096), (1040, 4096)])
+def test_bf16_linear_of_few_rows(M, N, K, monkeypatch):
+    """Both sides of the lines between the weight-streaming kernel and the tensor-core GEMM: five rows, seven for small matrices."""
     from layerstorm_b200.models.device_model import QLinear
+    called, call = [], nat.call
+    monkeypatch.setattr(nat, "call", lambda name, *a: (called.append(name), call(name, *a))[1])
     g = torch.Generator().manual_seed(N + M)
     lin = QLinear.from_float(torch.randn(N, K, generator=g), "bf16", "cuda")
     x = torch.randn(M, K, generator=g).to(torch.bfloat16).cuda()
@@ -138,3 +140,4 @@ def test_bf16_linear_of_few_rows(M, N, K):
         lin(out, x, M)
         want = x.double() @ lin.w.double().T
         assert float((out.double() - want).norm() / want.norm()) < (1e-5 if dt == torch.float32 else 3e-3)
+    assert called == ["lsb_gemm_bf16_tc" if M >= (5 if N == 1040 else 7) else "lsb_gemv_bf16"] * 2
