@@ -436,10 +436,13 @@ struct KdaTail {
 };
 
 // One warp per (row, head), four channels a lane, eight of them per block.  2048 rows of 64 heads: 138 us with a block of 128 threads per (row, head),
-// 24 us now (traffic at DRAM's rate: 26 us).
+// 24 us now (traffic at DRAM's rate: 26 us).  VEC: the caller's norm weights are 16-byte and its rows 8-byte aligned (the scratch always is: the recurrence reads
+// it in 16-byte pieces); else they are taken one by one.
+template <bool VEC>
 __global__ void __launch_bounds__(256) kda_out_kernel(KdaParams p, KdaScratch w, int total) {
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;                 // i = row * H + head
-    const float4 ow = *reinterpret_cast<const float4*>(p.onorm_w + lane * 4);
+    const float* nw = p.onorm_w + lane * 4;
+    const float4 ow = VEC ? *reinterpret_cast<const float4*>(nw) : make_float4(nw[0], nw[1], nw[2], nw[3]);
     pdl_wait();
     pdl_launch_dependents();
     if (i >= total) return;
@@ -447,7 +450,8 @@ __global__ void __launch_bounds__(256) kda_out_kernel(KdaParams p, KdaScratch w,
     const float4 o = *reinterpret_cast<const float4*>(w.vo + at), g = *reinterpret_cast<const float4*>(w.gate + at);
     const float inv = rsqrtf(warp_sum(o.x * o.x + o.y * o.y + o.z * o.z + o.w * o.w) / (float)kD + p.eps);
     bf162 b[2] = {__floats2bfloat162_rn(o.x * inv * ow.x * g.x, o.y * inv * ow.y * g.y), __floats2bfloat162_rn(o.z * inv * ow.z * g.z, o.w * inv * ow.w * g.w)};
-    *reinterpret_cast<uint2*>(p.out + at) = *reinterpret_cast<uint2*>(b);
+    if (VEC) *reinterpret_cast<uint2*>(p.out + at) = *reinterpret_cast<uint2*>(b);
+    else { p.out[at] = b[0].x; p.out[at + 1] = b[0].y; p.out[at + 2] = b[1].x; p.out[at + 3] = b[1].y; }
 }
 
 }  // namespace lsb
@@ -521,7 +525,8 @@ static int kda_forward_impl(const void* proj, int ldp, int off_q, int off_k, int
         } else {
             launch_pdl((kda_recur_kernel), dim3(nseq, H), kD, 0, st, p, w);
         }
-        launch_pdl((kda_out_kernel), (total_rows * H + 7) / 8, 256, 0, st, p, w, total_rows * H);
+        if ((((uintptr_t)onorm_w & 15) | ((uintptr_t)out & 7)) == 0) launch_pdl((kda_out_kernel<true>), (total_rows * H + 7) / 8, 256, 0, st, p, w, total_rows * H);
+        else launch_pdl((kda_out_kernel<false>), (total_rows * H + 7) / 8, 256, 0, st, p, w, total_rows * H);
     } else {
         const int gate_smem = 2 * kD * kda_gate_row_bytes(rank);
         static bool gate_attr = false;

@@ -634,3 +634,29 @@ def test_embedding_vector_and_general_rows(H, scale):
         if 5 <= i < 35:
             want[r] = table[i - 5].float() * scale
     assert torch.equal(f, want) and torch.equal(b, want.bfloat16())
+
+
+@pytest.mark.parametrize("norm_at,out_at", [(0, 1), (1, 0), (3, 3)])
+def test_kda_rows_of_any_alignment(norm_at, out_at):
+    """Norm weights and output rows that start anywhere: the same bits as aligned ones, nothing written around them."""
+    H, D, rank, rows = 3, 128, 8, (7, 5)
+    C, R = H * D, sum(rows)
+    ldp = 3 * C + H + 2 * rank + 1
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    proj, fb, gb = rnd(R, ldp, seed=1), rnd(C, rank, dtype=torch.bfloat16, seed=2), rnd(C, rank, dtype=torch.bfloat16, seed=3)
+    conv = [rnd(C, 4, s=0.5, seed=4 + j) for j in range(3)]
+    a_exp, dt, norm = rnd(H, seed=7).exp(), rnd(C, seed=8), 1 + 0.1 * rnd(D, seed=9)
+    got = []
+    for n_at, o_at in ((0, 0), (norm_at, out_at)):
+        state, hist = rnd(2, H, D, D, s=0.1, seed=10), rnd(2, 3, C, 3, seed=11)
+        nbuf, obuf = torch.zeros(D + 8, device=DEV), torch.full((R * C + 16,), 7.0, dtype=torch.bfloat16, device=DEV)
+        nw, out = nbuf[n_at: n_at + D], obuf[o_at: o_at + R * C]
+        nw.copy_(norm)
+        scratch = torch.zeros(7 * R * C + R * H + 2 * R * rank + 16, device=DEV)
+        nat.call("lsb_kda_forward", proj, ldp, 0, C, 2 * C, 3 * C, 3 * C + H, 3 * C + H + rank, rank, fb, gb, None, None, *conv, a_exp, dt, nw, state, hist,
+                 i32(0, rows[0]), i32(*rows), i32(1, 0), out, 2, H, D, D ** -0.5, -5.0, 1e-5, R, scratch)
+        torch.cuda.synchronize()
+        assert bool((obuf[:o_at] == 7.0).all()) and bool((obuf[o_at + R * C:] == 7.0).all())
+        got.append((out.clone(), state, hist))
+    assert bool(got[0][0].isfinite().all()) and float(got[0][0].float().norm()) > 1.0
+    assert all(torch.equal(a, b) for a, b in zip(*got))
