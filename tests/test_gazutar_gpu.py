@@ -192,7 +192,7 @@ class Delta:
 
 
 @pytest.mark.parametrize("f32", [True, False])
-@pytest.mark.parametrize("H,G,dk,dv,taps", [(4, 2, 32, 64, 4), (3, 3, 24, 20, 3), (2, 1, 48, 96, 1), (6, 2, 64, 40, 2), (2, 2, 128, 128, 4), (2, 1, 100, 130, 5),
+@pytest.mark.parametrize("H,G,dk,dv,taps", [(4, 2, 32, 64, 4), (3, 3, 24, 20, 3), (2, 1, 48, 96, 1), (6, 2, 64, 40, 2), (2, 2, 128, 128, 4), (6, 2, 128, 128, 4), (2, 1, 100, 130, 5),
                                             (1, 1, 160, 72, 4), (3, 1, 20, 256, 6)])
 def test_delta_rule_forms_agree_with_the_recurrence(H, G, dk, dv, taps, f32):
     """Whole runs token by token and chunk-parallel, a cut in every short length, and the one-kernel form, on interleaved state slots."""

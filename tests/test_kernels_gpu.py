@@ -318,6 +318,62 @@ def test_mla_decode_attention(R, sparse, H):
         close(out[i], pr @ k[:, :dl], 2e-2, 2e-2, f"mla attention row {i}")
 
 
+@pytest.mark.parametrize("H", [24, 64, 72, 128])
+@pytest.mark.parametrize("NS", [1, 2])
+@pytest.mark.parametrize("dl,dr,fmt", [(128, 0, 1), (128, 16, 1), (512, 64, 1), (512, 0, 1), (128, 16, 0)])
+@pytest.mark.parametrize("sparse", [False, True])
+def test_mla_attention_over_head_groups(H, NS, dl, dr, fmt, sparse):
+    """Two and four head groups that share a key tile, FP8 rows fetched a tile ahead (bf16 rows beside them), one split (finished rows) and two: rows that see no
+    key, less than a tile, whole tiles and one key more, pages out of order, absent keys in a selection.  What no row sees is NaN."""
+    page, n_seq, max_pages, ctx = 16, 2, 20, 300
+    g = torch.Generator().manual_seed(H + dl + dr)
+    lens = [0, 1, 15, 63, 64, 65, 127, 128, 129, 193, 300]
+    R, rb = len(lens), (dl + 16 if fmt else 2 * dl) + 2 * dr
+    raw = torch.full(((n_seq * max_pages + 1) * page, rb), 255, dtype=torch.uint8)                 # NaN in every format
+    bt = (1 + torch.randperm(n_seq * max_pages, generator=g)).int().view(n_seq, max_pages)       # page 0 belongs to nobody
+    latent, rope = torch.randn(n_seq, ctx, dl, generator=g), (torch.randn(n_seq, ctx, dr, generator=g) * 0.5).to(torch.bfloat16)
+    at = bt.long()[:, torch.arange(ctx) // page] * page + torch.arange(ctx) % page
+    if fmt:
+        codes, scale8 = latent.to(torch.float8_e4m3fn), 0.2 + 0.6 * torch.rand(n_seq, ctx, generator=g)
+        latent = codes.double() * scale8[..., None].double()
+        raw[at] = torch.cat([codes.view(torch.uint8), scale8[..., None].contiguous().view(torch.uint8), torch.zeros(n_seq, ctx, 12, dtype=torch.uint8),
+                             rope.view(torch.uint8).view(n_seq, ctx, 2 * dr)], 2)
+    else:
+        raw[at] = torch.cat([(latent * 0.5).to(torch.bfloat16).view(torch.uint8).view(n_seq, ctx, 2 * dl), rope.view(torch.uint8).view(n_seq, ctx, 2 * dr)], 2)
+        latent = (latent * 0.5).to(torch.bfloat16).double()
+    q = (torch.randn(R, H, dl + dr, generator=g) * 0.5).to(torch.bfloat16)
+    seq = torch.tensor([i % n_seq for i in range(R)], dtype=torch.int32)
+    sel_ld = 208
+    sel, cnt = torch.full((R, sel_ld), -1, dtype=torch.int32), torch.zeros(R, dtype=torch.int32)
+    for i, n in enumerate(lens):
+        pick = torch.randperm(ctx, generator=g)[: min(n, sel_ld)].int()
+        pick[1::5] = -1
+        sel[i, : len(pick)], cnt[i] = pick, len(pick)
+    out = torch.full((R * H * dl + 64,), float("nan"), dtype=torch.bfloat16, device=DEV)
+    lse, o_part, ml_part = torch.zeros(R, H, device=DEV), torch.full((R, H, NS, dl), float("nan"), device=DEV), torch.full((R, H, NS, 2), float("nan"), device=DEV)
+    scale = (dl + dr) ** -0.5
+    args = (q.to(DEV), raw.to(DEV), bt.to(DEV), max_pages, seq.to(DEV), torch.tensor(lens, dtype=torch.int32).to(DEV), sel.to(DEV) if sparse else None,
+            cnt.to(DEV) if sparse else None, sel_ld if sparse else 0)
+    nat.call("lsb_mla_decode", *args, out, None, o_part, ml_part, R, H, dl, dr, page, fmt, NS, scale, None)
+    again = torch.full((R, H, dl), float("nan"), dtype=torch.bfloat16, device=DEV)                 # with the log sums: through partials and their merge
+    nat.call("lsb_mla_decode", *args, again, lse, o_part, ml_part, R, H, dl, dr, page, fmt, NS, scale, None)
+    torch.cuda.synchronize()
+    assert bool(out[R * H * dl:].isnan().all())
+    got = out[: R * H * dl].view(R, H, dl)
+    for i, n in enumerate(lens):
+        pos = sel[i, : int(cnt[i])].long() if sparse else torch.arange(n)
+        pos, s = pos[pos >= 0], int(seq[i])
+        sc = (q[i, :, :dl].double() @ latent[s, pos].T + q[i, :, dl:].double() @ rope[s, pos].double().T) * scale
+        want = torch.softmax(sc, -1) @ latent[s, pos] if len(pos) else torch.zeros(H, dl, dtype=torch.float64)
+        for o in (got, again):
+            # weights and rows in bf16: 2^-9 each of what they are, 2^-9 of the result
+            assert float((o[i].double().cpu() - want).norm()) <= 6e-3 * float(want.norm()), i
+        if len(pos):
+            assert float((lse[i].double().cpu() - torch.logsumexp(sc, -1)).abs().max()) < 1e-3 * max(1.0, float(sc.abs().max())), i
+        else:
+            assert bool((lse[i] == -math.inf).all()), i
+
+
 def test_sampling_kernels():
     R, V = 4, 5000
     logits = rnd(R, V, s=3.0)
