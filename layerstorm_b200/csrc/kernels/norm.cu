@@ -976,7 +976,7 @@ LSB_API int lsb_mhc_post_pre(void* out_x, void* residual, const void* x, void* p
     }
     // Whole rows per block, as many as keep the blocks to one wave.  The line against the two-launch form (one wave takes 76 us of 4096 columns
     // whatever the rows, hidden / 128 steps of a load, an exchange and a product): 256 rows 76 against 66 us, 391 rows 76 against 95, 1024 rows
-    // 96 against 194, 2048 rows 168 against 371.
+    // 96 against 194, 2048 rows 168 against 371.  352 rows of 1024, 2048, 6144, 7168 columns: 27 against 42, 43 / 62, 104 / 112, 120 / 134.
     if (!comm && n == kHcMax && hidden % kHrCols == 0 && hidden <= kRowCols && rows >= 352 && ((uintptr_t)norm_w & 15) == 0 && ((uintptr_t)fn & 15) == 0 && ((uintptr_t)x & 15) == 0
         && ((uintptr_t)residual & 15) == 0 && ((uintptr_t)out_x & 7) == 0) {
         auto go = [&](auto tag) {

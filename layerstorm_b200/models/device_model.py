@@ -203,7 +203,7 @@ def fp8_scale_atoms(scales: torch.Tensor) -> Optional[torch.Tensor]:
 
 class QLinear:
     """A weight matrix [N, K] in a device storage format, applied to bf16 activations.
-    Up to 4 rows (decode) stream the weights through the CUDA-core GEMV; larger row counts with
+    Up to 4 rows (decode; 6 over small matrices) stream the weights through the CUDA-core GEMV; larger row counts with
     bf16 weights run on the tcgen05 tensor-core GEMM."""
 
     def __init__(self, fmt: str, N: int, K: int, w: torch.Tensor, scales: Optional[torch.Tensor] = None, alpha: float = 1.0):

@@ -141,7 +141,8 @@ def test_widths_that_end_inside_boxes_and_operand_stages(fmt, H, F, BN):
         gate, up, down = ref[e]
         r, k = (idc == e).nonzero(as_tuple=True)
         want = (torch.nn.functional.silu(xd[r] @ gate.T) * (xd[r] @ up.T)) @ down.T
-        # a hidden value rounded to fp16, at most 2^-11 relative per term (NVFP4, FP8 and bf16 weights are exact in fp16).  Q4_K weights are d sc v - dmin m
+        # a hidden value rounded to fp16, at most 2^-11 relative per term (NVFP4 weights, bf16 weights of this size and FP8 weights with power-of-two block scales,
+        # as `_setup` makes them, are exact in fp16).  Q4_K weights are d sc v - dmin m
         # with both products rounded to fp16, 2^-11 of terms up to 15 d sc and 8 d sc in size around weights of 4.6 d sc rms: 2.4e-3 at most
         assert float((got[r * 2 + k] - want).norm() / want.norm()) < (3e-3 if fmt == "gguf_q4_k" else 1e-3), e
 
