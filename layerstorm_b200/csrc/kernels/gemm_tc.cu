@@ -8,8 +8,8 @@
 //              multi-stage shared-memory ring, completion on mbarriers
 //     warp 1   allocates tensor memory; one thread issues tcgen05.mma (kind::f16, fp32 accumulate
 //              in TMEM) and tcgen05.commit to release stages / publish the accumulator
-//     warps 2-5 epilogue: tcgen05.ld the accumulator (one TMEM lane = one output column n),
-//              optional bias, fp32 or bf16 store, coalesced over n
+//     warps 2-5 epilogue: tcgen05.ld the accumulator (one TMEM lane = one output column n), optional bias; bf16 rows of
+//              16-byte pitch through shared memory and TMA, others and fp32 by stores coalesced over n
 // This replaces the reference's CUDA-core tiled GEMM (src/compute/kernels/sm120/gemm/bf16_gemm.cu:156)
 // and the external FP8 GEMM launcher (G/sm120/gemm/fp8/fp8_gemm.h) for every M > 4.
 #include "tc_common.cuh"
@@ -33,6 +33,7 @@ struct GemmTcParams {
     int M, N, K, out_bf16, splits, kb_per_split;
     int* err;
     long long out_bs;              // batched mode: elements between consecutive batches of `out` (blockIdx.z = batch)
+    int tma_out;                   // bf16 rows that TMA can store (map_o)
     // fused all-reduce epilogue (row-parallel layers under tensor parallelism): instead of a local store, every tile of
     // the fp32 partial is stored into this rank's slot of every peer's receive buffer over NVLink; the last CTA
     // publishes the epoch.  The consuming kernel sums the slots in rank order.
@@ -42,7 +43,8 @@ struct GemmTcParams {
 // A CTA computes MT weight tiles of 128 rows against one token tile.  MT = 2 (512 x 256 outputs of TMEM, one CTA per SM) brings a third less
 // through L2 per product than two CTAs of 128 x 256; MT = 1 has half the shared memory of an SM, so that two CTAs share one and the epilogue of
 // one runs under the main loop of the other.  Measured (one CTA of 128 x 256 per SM, MT = 1 at half an SM, MT = 2): 2048 x 24896 x 4096 534, 446,
-// 422 us; 2048 x 4096 x 12288 205, 182, 165 us; 391 x 16640 x 4096 119, 94, 89 us; MT = 1 with 64-row tiles and smaller: 32 x 24896 x 4096 66 -> 55 us.
+// 422 us; 2048 x 4096 x 12288 205, 182, 165 us; 391 x 16640 x 4096 119, 94, 89 us; MT = 1 with 64-row tiles and smaller: 32 x 24896 x 4096 66 -> 55 us
+// (with an epilogue that took longer than the present one).
 // DEEP: MT = 1 with twice the stages, for grids that give an SM one CTA at a time anyway.
 template <int BN, int MT, bool DEEP = false> struct TcCfg {
     static constexpr int A_BYTES = BM * BK * 2;
@@ -55,7 +57,8 @@ template <int BN, int MT, bool DEEP = false> struct TcCfg {
 };
 
 template <int BN, int MT = 1, bool BATCHED = false, bool DEEP = false>
-__global__ void __launch_bounds__(TcCfg<BN, MT, DEEP>::THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GemmTcParams p) {
+__global__ void __launch_bounds__(TcCfg<BN, MT, DEEP>::THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                                                                                        const __grid_constant__ CUtensorMap map_o, GemmTcParams p) {
     using C = TcCfg<BN, MT, DEEP>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -143,31 +146,89 @@ __global__ void __launch_bounds__(TcCfg<BN, MT, DEEP>::THREADS) gemm_tc_kernel(c
         __syncwarp();
     } else if (warp >= 2) {
         // ---------------- epilogue ----------------
+        // Where the results go is settled once per tile, and lanes never part: what a lane must not store is a predicate of the store.  Worked out for
+        // every output, the destination took 25 dependent instructions with one or two warps per scheduler - a quarter of the kernel's time at K = 4096 and
+        // most of it at K = 256.  bf16 rows leave through shared memory (the stages, which nothing reads any more): 16 x 8 pieces of the accumulator
+        // are packed and stored transposed by one instruction for 256 values, and TMA writes 64 columns of up to 64 rows and drops what lies
+        // outside the matrix.  Before, now (us): 2048 x 24896 x 4096 fp32 408, 297 (1406 TFLOP/s), bf16 390, 279 (1500); 2048 x 4096 x 12288 156, 133;
+        // 2048 x 20480 x 1536 bf16 207, 107; 391 x 16640 x 4096 bf16 80, 57; 64 products of 2048 x 512 x 256 207, 66; 128 of 777 x 512 x 128 176, 47.
         const int q = warp & 3, mt = (warp - 2) >> 2;
-        const int n = n0 + mt * BM + q * 32 + lane;
         const bool ok = __all_sync(0xffffffffu, nkb > 0 ? mbar_wait(acc_full, 0, p.err, 3) : true);      // one answer for the warp: its loads are warp-wide
         tc_fence_after();
-        if (ok) {
-            const float b = (p.bias && n < p.N && p.splits == 1) ? p.bias[n] : 0.f;
+        const int rows = min(BN, p.M - m0);
+        const uint32_t lane_addr = tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(mt * BN);
+        const bool has_bias = p.bias && p.splits == 1;
+        if (ok && p.tma_out) {
+            constexpr int CH = BN < 64 ? BN : 64;                          // rows of a store
+            const int nh = n0 + mt * BM + (q >> 1) * 64;                   // first column of this pair of warps
+            float b[2][2];                                                 // bias of the rows of the accumulator that this thread's pieces hold
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const int n = nh + (q & 1) * 32 + h * 16 + r * 8 + (lane >> 2);
+                    b[h][r] = has_bias && n < p.N ? p.bias[n] : 0.f;
+                }
+            uint8_t* stage = smem + (mt * 2 + (q >> 1)) * (BN * 128);
+            if (nh < p.N)
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 16) {
+            for (int c0 = 0; c0 < rows; c0 += CH) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t r[CH / 2];
+                    tmem_ld_pieces<CH>(lane_addr + ((uint32_t)(h * 16) << 16) + (uint32_t)c0, r);
+#pragma unroll
+                    for (int g = 0; g < CH / 16; ++g) {
+                        uint32_t v[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            v[i] = pack_bf16x2(__uint_as_float(r[8 * g + 2 * i]) + b[h][i & 1], __uint_as_float(r[8 * g + 2 * i + 1]) + b[h][i & 1]);
+                        const int m = c0 + g * 16 + (lane >> 4) * 8 + (lane & 7), c = (q & 1) * 4 + h * 2 + ((lane >> 3) & 1);
+                        stmatrix_x4_trans(smem_u32(stage) + (uint32_t)(m * 128 + ((c ^ (m & 7)) << 4)), v);
+                    }
+                }
+                fence_proxy_async();
+                bar_sync(1 + mt * 2 + (q >> 1), 64);
+                if (!(q & 1)) {
+                    if (elect_one()) {
+                        if (BATCHED) tma_store_3d(stage + c0 * 128, &map_o, nh, m0 + c0, batch);
+                        else tma_store_2d(stage + c0 * 128, &map_o, nh, m0 + c0);
+                    }
+                    __syncwarp();
+                }
+            }
+            if (!(q & 1)) {
+                bulk_commit_wait();                                        // (the group of the thread that stored is the only one that is not empty)
+                __syncwarp();
+            }
+        } else if (ok) {
+            const int n = n0 + mt * BM + q * 32 + lane;
+            const bool nin = n < p.N;
+            const float b = has_bias && nin ? p.bias[n] : 0.f;
+            const bool f32 = p.splits > 1 || !p.out_bf16 || p.comm.nranks;
+            const size_t step = p.splits > 1 ? (size_t)p.N : (size_t)p.ldo;
+            const size_t at = p.splits > 1 ? ((size_t)split * p.M + m0) * p.N + n : (size_t)batch * p.out_bs + (size_t)m0 * p.ldo + n;
+            float* of = (p.splits > 1 ? p.partial : reinterpret_cast<float*>(p.out)) + at;
+            bf16* oh = reinterpret_cast<bf16*>(p.out) + at;
+#pragma unroll 1
+            for (int c0 = 0; c0 < rows; c0 += 16) {
                 float v[16];
-                if (nkb > 0) tmem_ld16(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(mt * BN + c0), v);
-                else {
+                tmem_ld16(lane_addr + (uint32_t)c0, v);
+                if (nkb == 0) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] = 0.f;
                 }
-                if (n < p.N) {
+                if (p.comm.nranks) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int m = m0 + c0 + j;
-                        if (m < p.M) {
-                            if (p.comm.nranks) comm_push(p.comm, next_epoch, (size_t)m * p.ldo + n, v[j]);
-                            else if (p.splits > 1) p.partial[((size_t)split * p.M + m) * p.N + n] = v[j];
-                            else if (p.out_bf16) reinterpret_cast<bf16*>(p.out)[(size_t)batch * p.out_bs + (size_t)m * p.ldo + n] = __float2bfloat16(v[j] + b);
-                            else reinterpret_cast<float*>(p.out)[(size_t)batch * p.out_bs + (size_t)m * p.ldo + n] = v[j] + b;
-                        }
-                    }
+                    for (int j = 0; j < 16; ++j)
+                        if (nin && c0 + j < rows) comm_push(p.comm, next_epoch, (size_t)(m0 + c0 + j) * p.ldo + n, v[j]);
+                    __syncwarp();
+                } else if (f32) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) { st_global_if(of, v[j] + b, nin && c0 + j < rows); of += step; }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) { st_global_if(oh, __float2bfloat16(v[j] + b), nin && c0 + j < rows); oh += step; }
                 }
             }
         }
@@ -278,23 +339,23 @@ int cached_map_2d(CUtensorMap* out, const void* ptr, CUtensorMapDataType dt, int
 }
 
 template <int BN, int MT = 1, bool DEEP = false>
-static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTcParams& p, cudaStream_t st) {
+static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mo, const GemmTcParams& p, cudaStream_t st) {
     using C = TcCfg<BN, MT, DEEP>;
     static bool attr = false;
     if (!attr) { cudaFuncSetAttribute(gemm_tc_kernel<BN, MT, false, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM); attr = true; }
     dim3 grid((p.M + BN - 1) / BN, (p.N + BM * MT - 1) / (BM * MT), p.splits);
-    launch_pdl((gemm_tc_kernel<BN, MT, false, DEEP>), grid, C::THREADS, C::SMEM, st, mw, mx, p);
+    launch_pdl((gemm_tc_kernel<BN, MT, false, DEEP>), grid, C::THREADS, C::SMEM, st, mw, mx, mo, p);
     return (int)cudaGetLastError();
 }
 
 
 template <int BN>
-static int launch_tc_batched(const CUtensorMap& mw, const CUtensorMap& mx, const GemmTcParams& p, int batch, cudaStream_t st) {
+static int launch_tc_batched(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mo, const GemmTcParams& p, int batch, cudaStream_t st) {
     using C = TcCfg<BN, 1>;
     static bool attr = false;
     if (!attr) { cudaFuncSetAttribute(gemm_tc_kernel<BN, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM); attr = true; }
     dim3 grid((p.M + BN - 1) / BN, (p.N + BM - 1) / BM, batch);
-    launch_pdl((gemm_tc_kernel<BN, 1, true>), grid, C::THREADS, C::SMEM, st, mw, mx, p);
+    launch_pdl((gemm_tc_kernel<BN, 1, true>), grid, C::THREADS, C::SMEM, st, mw, mx, mo, p);
     return (int)cudaGetLastError();
 }
 
@@ -331,13 +392,16 @@ LSB_API int lsb_gemm_bf16_tc_batched(void* out, const void* x, const void* w, in
     GemmTcParams p;
     p.out = out; p.ldo = ldo; p.partial = nullptr; p.bias = nullptr; p.M = M; p.N = N; p.K = K; p.out_bf16 = out_bf16; p.err = (int*)err;
     p.splits = 1; p.kb_per_split = (K + BK - 1) / BK; p.out_bs = os_b; p.comm.nranks = 0;
+    p.tma_out = out_bf16 && K > 0 && ldo % 8 == 0 && os_b % 8 == 0 && ldo >= N && os_b > 0 && ((uintptr_t)out & 15) == 0;
+    CUtensorMap mo = mx;
+    if (p.tma_out && get(out, M, N, ldo, os_b, BN < 64 ? BN : 64, &mo) != 0) p.tma_out = 0;
     cudaStream_t st = (cudaStream_t)stream;
     switch (BN) {
-        case 16: return launch_tc_batched<16>(mw, mx, p, B, st);
-        case 32: return launch_tc_batched<32>(mw, mx, p, B, st);
-        case 64: return launch_tc_batched<64>(mw, mx, p, B, st);
-        case 128: return launch_tc_batched<128>(mw, mx, p, B, st);
-        default: return launch_tc_batched<256>(mw, mx, p, B, st);
+        case 16: return launch_tc_batched<16>(mw, mx, mo, p, B, st);
+        case 32: return launch_tc_batched<32>(mw, mx, mo, p, B, st);
+        case 64: return launch_tc_batched<64>(mw, mx, mo, p, B, st);
+        case 128: return launch_tc_batched<128>(mw, mx, mo, p, B, st);
+        default: return launch_tc_batched<256>(mw, mx, mo, p, B, st);
     }
 }
 
@@ -377,19 +441,22 @@ LSB_API int lsb_gemm_bf16_tc(void* out, const void* x, const void* w, const void
     p.kb_per_split = (nkb + splits - 1) / splits;
     p.splits = (nkb + p.kb_per_split - 1) / p.kb_per_split;
     const int ctas = tiles * p.splits;                     // of one weight tile each
+    p.tma_out = out_bf16 && K > 0 && p.splits == 1 && !comm && ldo % 8 == 0 && ldo >= N && ((uintptr_t)out & 15) == 0;
+    CUtensorMap mo = mx;
+    if (p.tma_out && cached_map_2d(&mo, out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, N, ldo, BN < 64 ? BN : 64, BK) != 0) p.tma_out = 0;
     switch (BN) {
-        case 16: rc = launch_tc<16>(mw, mx, p, st); break;
-        case 32: rc = launch_tc<32>(mw, mx, p, st); break;
-        case 64: rc = launch_tc<64>(mw, mx, p, st); break;
-        case 128: rc = launch_tc<128>(mw, mx, p, st); break;
+        case 16: rc = launch_tc<16>(mw, mx, mo, p, st); break;
+        case 32: rc = launch_tc<32>(mw, mx, mo, p, st); break;
+        case 64: rc = launch_tc<64>(mw, mx, mo, p, st); break;
+        case 128: rc = launch_tc<128>(mw, mx, mo, p, st); break;
         // (one CTA of 128 x 256 per SM before there was a choice, one weight tile, one and deep, two; us).  A grid that one CTA per SM takes in one wave is deep:
         // 160 x 576 x 4096 27.8, 26.4, 25.9, 28.9; 256 x 2048 x 2048 36.6, 35.1, 33.8, 38.1.  So is one of two to three such waves over a long reduction, which
         // takes CTAs of two tiles two waves: 1500 x 7168 x 12288 298, 334, 291, 306; 391 x 24896 x 12288 304, 343, 301, 312, but 391 x 24896 x 4096 146, 139, 143,
         // 130 and 1000 x 24896 x 12288 (780 CTAs) 659, 554, 645, 518.  Two weight tiles per CTA pay from a reduction of 2048 on (K = 1536 and below: the same; a
         // short one leaves the longer epilogue bare) unless half the grid no longer covers the SMs: 300 x 576 x 4096 (150 CTAs) 36.6, 37.1, -, 40.2.
         default:
-            if (ctas <= kSms || (K >= 8192 && ctas > 2 * kSms && ctas <= 3 * kSms)) rc = launch_tc<256, 1, true>(mw, mx, p, st);
-            else rc = K >= 2048 && !comm && ctas >= 160 ? launch_tc<256, 2>(mw, mx, p, st) : launch_tc<256>(mw, mx, p, st);
+            if (ctas <= kSms || (K >= 8192 && ctas > 2 * kSms && ctas <= 3 * kSms)) rc = launch_tc<256, 1, true>(mw, mx, mo, p, st);
+            else rc = K >= 2048 && !comm && ctas >= 160 ? launch_tc<256, 2>(mw, mx, mo, p, st) : launch_tc<256>(mw, mx, mo, p, st);
             break;
     }
     if (rc) return rc;

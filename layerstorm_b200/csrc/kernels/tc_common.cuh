@@ -94,6 +94,17 @@ __device__ __forceinline__ uint4 ld_shared_16(uint32_t addr) {
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
 }
+// Tile stores; bulk_commit_wait() by the thread that issued them returns when they have been written.
+__device__ __forceinline__ void tma_store_2d(const void* smem_src, const CUtensorMap* map, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%1, {%2, %3}], [%0];" ::"r"(smem_u32(smem_src)), "l"(map), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tma_store_3d(const void* smem_src, const CUtensorMap* map, int x, int y, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%1, {%2, %3, %4}], [%0];" ::"r"(smem_u32(smem_src)), "l"(map), "r"(x), "r"(y), "r"(z) : "memory");
+}
+__device__ __forceinline__ void bulk_commit_wait() {
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -122,6 +133,46 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 lanes x COLS fp32 columns as mma accumulator pieces of 16 x 8: registers 4 i + {0, 1} hold lane (thread / 4), columns 8 i + 2 (thread % 4) + {0, 1},
+// registers 4 i + {2, 3} the same columns of lane (thread / 4) + 8.  The lanes are those at `taddr`, a half of the warp's quarter.
+template <int COLS> __device__ __forceinline__ void tmem_ld_pieces(uint32_t taddr, uint32_t* r) {
+    static_assert(COLS == 16 || COLS == 32 || COLS == 64, "pieces");
+    __syncwarp();
+    if constexpr (COLS == 16) {
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+    } else if constexpr (COLS == 32) {
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+                       "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr) : "memory");
+    } else {
+        asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+                     "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+                       "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+                       "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
+                       "=r"(r[31]) : "r"(taddr) : "memory");
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// Four 8 x 8 pieces of 16-bit values, each stored transposed: shared-memory row i of piece p (16 bytes at the address that thread 8 p + i gives) receives
+// column i of the piece in register p.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t* v) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// Stores of lanes that take part by predicate, without a branch.
+__device__ __forceinline__ void st_global_if(float* p, float v, bool on) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n @p st.global.f32 [%0], %1;\n}" ::"l"(p), "f"(v), "r"((int)on) : "memory");
+}
+__device__ __forceinline__ void st_global_if(bf16* p, bf16 v, bool on) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n @p st.global.b16 [%0], %1;\n}" ::"l"(p), "h"(*reinterpret_cast<const uint16_t*>(&v)), "r"((int)on) : "memory");
 }
 
 // 32 / 16 consecutive 32-bit columns of this thread's TMEM lane, written from registers (operand staging: an fp16

@@ -125,6 +125,31 @@ def test_matrices_that_end_inside_a_warps_rows(M, N):
     assert int(err) == 0 and float((out.double() - parts).norm() / parts.norm()) < 1e-5
 
 
+@pytest.mark.parametrize("M", [5, 16, 17, 33, 64, 65, 127, 200, 256, 257, 321])
+@pytest.mark.parametrize("N", [8, 56, 64, 72, 136, 264])
+def test_bf16_rows_by_tma_and_by_stores_are_the_same(M, N):
+    """Rows of 16-byte pitch at a 16-byte address leave by TMA, others by stores: the same bits, nothing outside the matrix; and as a batch in [row, head] order."""
+    K = 128
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w = (torch.randn(n, K, generator=g, device="cuda").bfloat16() for n in (M, N))
+    bias, err = torch.randn(N, generator=g, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = x.double() @ w.double().T + bias.double()
+    got = []
+    for ld, at in ((N + 8, 0), (N + 3, 0), (N + 8, 1)):
+        buf = torch.zeros((M + 1) * ld + 8, device="cuda", dtype=torch.bfloat16)
+        nat.call("lsb_gemm_bf16_tc", buf[at:], x, w, bias, M, N, K, K, K, ld, 1, None, 0, err, None)
+        out = buf[at: at + (M + 1) * ld].view(M + 1, ld)
+        assert int(err) == 0 and float(out[M:].abs().sum()) == 0.0 and float(out[:M, N:].abs().sum()) == 0.0 and float(buf[:at].abs().sum()) == 0.0
+        got.append(out[:M, :N].clone())
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    assert float((got[0].double() - want).norm() / want.norm()) < 3e-3          # 2^-9, rounding to bf16
+    B, out = 2, torch.zeros(M + 1, 2, N + 8, device="cuda", dtype=torch.bfloat16)
+    nat.call("lsb_gemm_bf16_tc_batched", out, x, w, M, N, K // B, B, K, K // B, K, K // B, B * (N + 8), N + 8, 1, err)
+    parts = torch.stack([x[:, b * K // B: (b + 1) * K // B].double() @ w[:, b * K // B: (b + 1) * K // B].double().T for b in range(B)], 1)
+    assert int(err) == 0 and float(out[M:].abs().sum()) == 0.0 and float(out[:, :, N:].abs().sum()) == 0.0
+    assert float((out[:M, :, :N].double() - parts).norm() / parts.norm()) < 3e-3
+
+
 @pytest.mark.parametrize("M", [4, 5, 6, 7, 8])
 @pytest.mark.parametrize("N,K", [(8, 64), (72, 136), (1024, 4096), (1040, 4096)])
 def test_bf16_linear_of_few_rows(M, N, K, monkeypatch):
