@@ -111,10 +111,12 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
 
 // ---------------------------------------------------------------- tensor memory
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_holder, uint32_t ncols) {   // whole warp
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_holder)), "r"(ncols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {        // whole warp
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -171,13 +173,19 @@ __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("ba
 __device__ __forceinline__ void st_global_if(float* p, float v, bool on) {
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n @p st.global.f32 [%0], %1;\n}" ::"l"(p), "f"(v), "r"((int)on) : "memory");
 }
+__device__ __forceinline__ void st_global_if(__half* p, __half v, bool on) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n @p st.global.b16 [%0], %1;\n}" ::"l"(p), "h"(*reinterpret_cast<const uint16_t*>(&v)), "r"((int)on) : "memory");
+}
 __device__ __forceinline__ void st_global_if(bf16* p, bf16 v, bool on) {
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n @p st.global.b16 [%0], %1;\n}" ::"l"(p), "h"(*reinterpret_cast<const uint16_t*>(&v)), "r"((int)on) : "memory");
 }
 
 // 32 / 16 consecutive 32-bit columns of this thread's TMEM lane, written from registers (operand staging: an fp16
-// A matrix lives in TMEM as one row per lane, two consecutive reduction elements per column).
+// A matrix lives in TMEM as one row per lane, two consecutive reduction elements per column).  A store is one instruction of the whole warp like the
+// loads above: lanes meet in front of it, whatever stood there - a lane that has just released a shared-memory entry for the others may still be on
+// its way, and a store that finds the warp apart is undefined (a launch failure once in tens to hundreds of runs of the bf16 down projection in tiles of 64).
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
+    __syncwarp();
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
         "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
@@ -187,12 +195,13 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
           "r"(r[30]), "r"(r[31]) : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    __syncwarp();
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
           "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { __syncwarp(); asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---------------------------------------------------------------- descriptors
 // K-major operand tile in shared memory written by TMA with 128-byte swizzle: rows of 128
