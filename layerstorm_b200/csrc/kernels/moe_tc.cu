@@ -632,7 +632,11 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                             if (e < nent) hdr_next = __ldg(reinterpret_cast<const uint4*>(qrow + (size_t)e * 144));
                         }
                         // one lane polls the barrier, the warp sleeps at the sync: waiting warps leave the issue slots alone
-                        if (lane == 0 && mine) { if (warp == 2) PROF_SCOPE(0, okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0); else okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0; }
+                        // Over bf16 the sets are in entries of their own, and the slot's round before this one may have been the other set's: its bytes can still be on
+                        // their way while those of later entries are here, and a parity alone takes the round two before for this one (a set may be 12 sub-stages
+                        // ahead, the ring has 7 or 9 entries).  So that round is waited for, too.
+                        if (C::SUB == 1 && lane == 0 && mine) okw = mbar_wait(&full_r[re.i], re.ph ^ 1, p.err, 17) ? 1 : 0;
+                        if (lane == 0 && mine && okw) { if (warp == 2) PROF_SCOPE(0, okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0); else okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0; }
                         ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
                         if (!ok) break;
                     }

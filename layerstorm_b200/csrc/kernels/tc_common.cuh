@@ -183,7 +183,7 @@ __device__ __forceinline__ void st_global_if(bf16* p, bf16 v, bool on) {
 // 32 / 16 consecutive 32-bit columns of this thread's TMEM lane, written from registers (operand staging: an fp16
 // A matrix lives in TMEM as one row per lane, two consecutive reduction elements per column).  A store is one instruction of the whole warp like the
 // loads above: lanes meet in front of it, whatever stood there - a lane that has just released a shared-memory entry for the others may still be on
-// its way, and a store that finds the warp apart is undefined (a launch failure once in tens to hundreds of runs of the bf16 down projection in tiles of 64).
+// its way, and a store that finds the warp apart is undefined.
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
     __syncwarp();
     asm volatile(
