@@ -323,7 +323,10 @@ template <int FMT, int BN, bool GATEUP, int DIRECT = 0> struct MoeTcCfg {
     static constexpr int BAR_BYTES = 512;
     static constexpr int RAW_BUDGET = 224 * 1024 - S * KS * B_BYTES - BAR_BYTES - 1024;
     static constexpr int RD_FIT = (RAW_BUDGET > 144 * 1024 ? 144 * 1024 : RAW_BUDGET) / RAW_STAGE;
-    static constexpr int RD = RD_FIT > 12 ? 12 : RD_FIT;
+    // Where the converter sets are in entries of their own (SUB = 1), a slot is one set's: a set may be 12 sub-stages ahead, and coming to a slot whose round before
+    // is the other's and still on its way (copies out of L2 overtake), it would take the round two before for its own, as the parity is the same.
+    static constexpr int ADV = SUB == 1 && !DIRECT ? CONV_SETS : 1;
+    static constexpr int RD = (RD_FIT > 12 ? 12 : RD_FIT) / ADV * ADV;
     // One CTA per SM by construction (the CTA owns all of tensor memory): ask for more than half of the SM's shared memory.
     static constexpr int SMEM_NEED = S * KS * B_BYTES + RD * RAW_STAGE + BAR_BYTES + 1024;
     static constexpr int SMEM = SMEM_NEED < 120 * 1024 ? 120 * 1024 : SMEM_NEED;
@@ -607,6 +610,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
             if (FMT == 3) hdr_next = __ldg(reinterpret_cast<const uint4*>(qrow));
             const int nent = (nkb + C::SUB - 1) / C::SUB;
             typename CV::Raw raw;
+            const int own = C::ADV > 1 ? (set + (int)rr.i) % C::CONV_SETS : set;       // (an item of odd length leaves the sets' slots shifted by one)
             // Straight-line code for the sub-stages of whole entries and whole operand stages: the instructions around a sub-stage (ring
             // positions, which barrier is due) cost as much as its conversion when they are decided at run time.
             constexpr int BLK = C::SUB > C::KS ? C::SUB : C::KS;
@@ -615,7 +619,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
             for (int b0 = 0; b0 < nkb && ok; b0 += BLK) {
 #pragma unroll
                 for (int i = 0; i < BLK / C::CONV_SETS; ++i) {
-                    const int l0 = i * C::CONV_SETS, l = l0 + set;       // sub-stages of both sets; this warp's
+                    const int l0 = i * C::CONV_SETS, l = l0 + own;       // sub-stages of both sets; this warp's
                     if (b0 + l0 >= nkb) break;
                     const bool mine = C::SUB > 1 || b0 + l < nkb;        // (past an odd end: zeros into columns that no MMA reads, or no entry at all)
                     RingPos<C::RD> re = rr;
@@ -632,11 +636,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                             if (e < nent) hdr_next = __ldg(reinterpret_cast<const uint4*>(qrow + (size_t)e * 144));
                         }
                         // one lane polls the barrier, the warp sleeps at the sync: waiting warps leave the issue slots alone
-                        // Over bf16 the sets are in entries of their own, and the slot's round before this one may have been the other set's: its bytes can still be on
-                        // their way while those of later entries are here, and a parity alone takes the round two before for this one (a set may be 12 sub-stages
-                        // ahead, the ring has 7 or 9 entries).  So that round is waited for, too.
-                        if (C::SUB == 1 && lane == 0 && mine) okw = mbar_wait(&full_r[re.i], re.ph ^ 1, p.err, 17) ? 1 : 0;
-                        if (lane == 0 && mine && okw) { if (warp == 2) PROF_SCOPE(0, okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0); else okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0; }
+                        if (lane == 0 && mine) { if (warp == 2) PROF_SCOPE(0, okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0); else okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0; }
                         ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
                         if (!ok) break;
                     }
