@@ -14,11 +14,12 @@
 //                    write them with tcgen05.st into a ring of operand stages in tensor memory
 //        warp 22     TMA producer for the raw weight bytes
 //        warps 18-21 epilogue (tcgen05.ld -> SwiGLU(+clamp) -> fp16, or -> fp32 / bf16 rows, or NVLink stores)
-//     With few rows per expert the kernel is bound by the converters' instructions and by what the roles spend on barriers, not by DRAM or the
-//     tensor cores.  Measured (gate/up, down) with one converter set, a single thread walking the issue loop and 64 elements per operand
-//     stage: 32 rows x top-8 of 288 + 1 shared NVFP4 experts of 4096 x 2048 (169 hit) 773 and 590 us, 2048 rows 1508 and 1221 us, 777 rows
-//     over 256 FP8 experts of 7168 x 2048 2310 and 1717 us; as it is now 375 and 271, 920 and 633, 1373 and 867 us (weights at DRAM's rate:
-//     244 and 122, 417 and 208, 1153 and 577 us).
+//     With few rows per expert the kernel is bound by the converters' instructions and by what the roles spend on barriers, with some 60 rows by these and
+//     the traffic of tensor memory (operands stored, MMAs), not by DRAM or the tensor cores alone.  Measured (gate/up, down; us) with one converter set, a single
+//     thread walking the issue loop and 64 elements per operand stage: 32 rows x top-8 of 288 + 1 shared NVFP4 experts of 4096 x 2048 (173 hit) 773 and 590,
+//     2048 rows 1508 and 1221, 777 rows over 256 FP8 experts of 7168 x 2048 2310 and 1717; with two sets and stages of 128 and 256 elements 379 and 276, 910 and
+//     643, 1307 and 860; with a token ring as long as the weights', row sets for down and an epilogue that waits for nothing 329 and 219, 843 and 510, 1262 and 778
+//     (weights at DRAM's rate: 253 and 126, 422 and 211, 1168 and 584).  With nothing converted the first are 305 and 192, without MMAs 295 and 206.
 //     gate and up tiles share one token tile and accumulate into two TMEM regions, so SwiGLU is
 //     fused and the [tokens, 2F] intermediate never exists.
 // Per-tensor NVFP4 scales are applied in the epilogue in fp32.  Every wait is bounded and reports
@@ -161,6 +162,10 @@ template <int NH> struct RowConv<2, NH> {     // NVFP4: 32 bytes per row-stage; 
         for (int i = 0; i < NV; ++i) r.v[i] = ld_shared_16(swz_chunk(tile, row, sub * 2 + h * NV + i));
     }
     static __device__ __forceinline__ void convert(const Raw& r, uint32_t* out, int, int h) {
+        // two scales per conversion; the products take them as halves of a register (a conversion of each scale in both halves: 8 more instructions a scheduler
+        // has to place in every 64 elements of a warp, 133 cycles instead of 114)
+        const __half2 s01 = e4m3x2_to_half2((uint16_t)(NH == 2 && h ? r.sc >> 16 : r.sc));
+        const __half2 s23 = NH == 1 ? e4m3x2_to_half2((uint16_t)(r.sc >> 16)) : s01;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const uint32_t wv[4] = {r.v[i].x, r.v[i].y, r.v[i].z, r.v[i].w};
@@ -168,8 +173,8 @@ template <int NH> struct RowConv<2, NH> {     // NVFP4: 32 bytes per row-stage; 
             for (int j = 0; j < 4; ++j) {             // one word = 8 elements; 16-group index = word / 2
                 __half2 hh[4];
                 fp4x8_to_half2x4(wv[j], hh);
-                const int word = (NH == 1 ? 0 : 4 * h) + 4 * i + j;
-                const __half2 s2 = e4m3x2_to_half2((uint16_t)(((r.sc >> ((word >> 1) * 8)) & 0xffu) * 0x0101u));
+                const int grp = (4 * i + j) >> 1;
+                const __half2 s2 = grp == 0 ? __low2half2(s01) : (grp == 1 ? __high2half2(s01) : (grp == 2 ? __low2half2(s23) : __high2half2(s23)));
 #pragma unroll
                 for (int q = 0; q < 4; ++q) out[(4 * i + j) * 4 + q] = h2_bits(__hmul2(hh[q], s2));
             }
@@ -282,7 +287,7 @@ constexpr int kDirect = 1, kDirectBf16 = 2;
 template <int FMT, int BN, bool GATEUP, int DIRECT = 0> struct MoeTcCfg {
     static_assert(!DIRECT || (FMT == 0 && (GATEUP || DIRECT == kDirectBf16)), "direct operands: bf16 weights and tokens");
     static constexpr int A_TILES = GATEUP ? 2 : 1;
-    static constexpr int NH = GATEUP ? 1 : 2;                             // converter threads per (row, stage): gate/up = one per matrix
+    static constexpr int NH = GATEUP || FMT != 0 ? 1 : 2;                 // converter threads per (row, sub-stage) of a matrix; bf16 rows take too many registers for one
     using CV = RowConv<FMT, NH>;
     static constexpr int B_BYTES = BN * kTBK * 2;                         // token tile of a sub-stage
     // An operand stage is KS sub-stages of 64 reduction elements behind one pair of barriers: the issuing warp's waits and commit cost a few
@@ -293,7 +298,7 @@ template <int FMT, int BN, bool GATEUP, int DIRECT = 0> struct MoeTcCfg {
 #ifndef LSB_MOE_KS_DN
 #define LSB_MOE_KS_DN 4
 #endif
-    static constexpr int KS = GATEUP ? LSB_MOE_KS_GU : (BN <= 64 ? LSB_MOE_KS_DN : 2);
+    static constexpr int KS = GATEUP ? LSB_MOE_KS_GU : (BN <= 64 || FMT != 0 ? LSB_MOE_KS_DN : 2);
     static constexpr int ACC_COLS = A_TILES * BN;                         // one accumulator set (gate [+ up])
     // Tensor memory (512 columns): accumulator sets first, then the ring of converted weight stages
     // (32 columns = 64 fp16 per matrix and sub-stage).  Two accumulator sets let the epilogue of one item overlap the
@@ -305,14 +310,16 @@ template <int FMT, int BN, bool GATEUP, int DIRECT = 0> struct MoeTcCfg {
     static constexpr int A_COLS = 32 * A_TILES * KS;
     static constexpr int A_BASE = NBUF * ACC_COLS;
     static constexpr int S_FIT = DIRECT ? 2 : (512 - A_BASE) / A_COLS;
-    static constexpr int S = S_FIT > 3 ? 3 : S_FIT;                       // operand stages: weights in tensor memory, tokens in shared memory
+    static constexpr int S = S_FIT > 3 ? 3 : S_FIT;                       // operand stages of the weights, in tensor memory
     static constexpr int TMEM_COLS = 512;
-    // 8 converter warps cover one sub-stage (4 lane quarters x 2 parts); two sets of them take the sub-stages in turns, so that a warp has
-    // two sub-stage times for its serial read -> convert -> store chain
-    static constexpr int CONV_SETS = 2;
-    static constexpr int SET_WARPS = 8;
-    static constexpr int CONV_WARPS = DIRECT ? 0 : SET_WARPS * CONV_SETS;
-    static_assert(KS % CONV_SETS == 0, "both sets have part in every operand stage");
+    // A set of converter warps covers one sub-stage (4 lane quarters x gate and up, or x the parts of a row); the sets take the sub-stages in turns, so
+    // that a warp has as many sub-stage times for its serial read -> convert -> store chain.  Down over quantised weights: four sets whose threads take
+    // a whole row of 64 elements; two sets with half rows spent as much on barriers as on converting.
+    static constexpr int PARTS = GATEUP ? 2 : NH;
+    static constexpr int SET_WARPS = 4 * PARTS;
+    static constexpr int CONV_SETS = 16 / SET_WARPS;
+    static constexpr int CONV_WARPS = DIRECT ? 0 : 16;
+    static_assert(KS % CONV_SETS == 0, "all sets have part in every operand stage");
     static constexpr int EPI_WARPS = 4;
     static constexpr int RAW_WARP = 2 + CONV_WARPS + EPI_WARPS;           // last warp: TMA producer of the raw weight ring
     static constexpr int THREADS = (RAW_WARP + 1) * 32;
@@ -321,18 +328,23 @@ template <int FMT, int BN, bool GATEUP, int DIRECT = 0> struct MoeTcCfg {
     static constexpr int W_TILE = kTBM * kBoxBytes;
     static constexpr int RAW_STAGE = A_TILES * (W_TILE + SUB * CV::AUX);
     static constexpr int BAR_BYTES = 512;
-    static constexpr int RAW_BUDGET = 224 * 1024 - S * KS * B_BYTES - BAR_BYTES - 1024;
-    static constexpr int RD_FIT = (RAW_BUDGET > 144 * 1024 ? 144 * 1024 : RAW_BUDGET) / RAW_STAGE;
-    // Where the converter sets are in entries of their own (SUB = 1), a slot is one set's: a set may be 12 sub-stages ahead, and coming to a slot whose round before
+    // The token tiles have a ring of their own (SB operand stages) that reaches as far ahead as the raw weights': a copy of theirs waits in the SM's copy
+    // engine behind the weights that have been asked for, some 3000 cycles.  With as many stages as the weights have in tensor memory (3 of 128
+    // elements) the tensor core waited for tokens: 2048 rows of 288 NVFP4 experts, gate/up 600 cycles per 64 elements whether weights were converted or not.
+    static constexpr int BUDGET = 224 * 1024 - BAR_BYTES - 1024;
+    static constexpr int RD_FIT = BUDGET / (RAW_STAGE + SUB * B_BYTES);
+    // Where the converter sets are in entries of their own (ADV > 1), a slot is one set's: a set may be 12 sub-stages ahead, and coming to a slot whose round before
     // is the other's and still on its way (copies out of L2 overtake), it would take the round two before for its own, as the parity is the same.
-    static constexpr int ADV = SUB == 1 && !DIRECT ? CONV_SETS : 1;
-    static constexpr int RD = (RD_FIT > 12 ? 12 : RD_FIT) / ADV * ADV;
+    static constexpr int ADV = CONV_SETS > SUB && !DIRECT ? CONV_SETS / SUB : 1;
+    static constexpr int RD = (RD_FIT > 12 ? 12 : (RD_FIT < 3 ? 3 : RD_FIT)) / ADV * ADV;
+    static constexpr int SB_FIT = (BUDGET - RD * RAW_STAGE) / (KS * B_BYTES), SB_ALL = (RD * SUB + KS - 1) / KS;
+    static constexpr int SB = SB_FIT < SB_ALL ? SB_FIT : SB_ALL;
     // One CTA per SM by construction (the CTA owns all of tensor memory): ask for more than half of the SM's shared memory.
-    static constexpr int SMEM_NEED = S * KS * B_BYTES + RD * RAW_STAGE + BAR_BYTES + 1024;
+    static constexpr int SMEM_NEED = SB * KS * B_BYTES + RD * RAW_STAGE + BAR_BYTES + 1024;
     static constexpr int SMEM = SMEM_NEED < 120 * 1024 ? 120 * 1024 : SMEM_NEED;
     static_assert(S >= 2 && A_BASE + (DIRECT ? 0 : S * A_COLS) <= 512, "tensor memory budget");
-    static_assert(RD >= 3 && SMEM <= 227 * 1024, "shared memory budget");
-    static_assert((3 * S + 2 * RD + 4) * 8 + 8 <= BAR_BYTES, "barrier area");
+    static_assert(RD >= 3 && SB >= 2 && SMEM <= 227 * 1024, "shared memory budget");
+    static_assert((2 * S + 2 * SB + 2 * RD + 4) * 8 + 8 <= BAR_BYTES, "barrier area");
 };
 constexpr int kMaxSlots = 1 << 16;
 // Role-level time breakdown for tuning builds (-DLSB_MOE_PROFILE): block 0 accumulates the cycles each role spends
@@ -381,12 +393,13 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
     using CV = typename C::CV;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* smem_b = smem;                                   // [S][KS] token tiles
-    uint8_t* smem_r = smem + C::S * C::KS * C::B_BYTES;       // [RD] raw weight entries
+    uint8_t* smem_b = smem;                                   // [SB][KS] token tiles
+    uint8_t* smem_r = smem + C::SB * C::KS * C::B_BYTES;      // [RD] raw weight entries
     uint64_t* full_a = reinterpret_cast<uint64_t*>(smem_r + C::RD * C::RAW_STAGE);
-    uint64_t* full_b = full_a + C::S;
-    uint64_t* empty = full_b + C::S;             // both operands of a stage
-    uint64_t* full_r = empty + C::S;
+    uint64_t* empty_a = full_a + C::S;
+    uint64_t* full_b = empty_a + C::S;
+    uint64_t* empty_b = full_b + C::SB;
+    uint64_t* full_r = empty_b + C::SB;
     uint64_t* empty_r = full_r + C::RD;
     uint64_t* acc_full = empty_r + C::RD;        // [NBUF]
     uint64_t* acc_empty = acc_full + 2;          // [NBUF]
@@ -400,8 +413,9 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
     const int nkb = K / kTBK, nops = (nkb + C::KS - 1) / C::KS;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::S; ++s) { mbar_init(&full_a[s], DIRECT ? 1 : C::CONV_WARPS); mbar_init(&full_b[s], 1); mbar_init(&empty[s], 1); }
-        for (int s = 0; s < C::RD; ++s) { mbar_init(&full_r[s], 1); mbar_init(&empty_r[s], DIRECT ? 1 : (C::SUB == 1 ? C::SET_WARPS : C::CONV_WARPS)); }
+        for (int s = 0; s < C::S; ++s) { mbar_init(&full_a[s], DIRECT ? 1 : C::CONV_WARPS); mbar_init(&empty_a[s], 1); }
+        for (int s = 0; s < C::SB; ++s) { mbar_init(&full_b[s], 1); mbar_init(&empty_b[s], 1); }
+        for (int s = 0; s < C::RD; ++s) { mbar_init(&full_r[s], 1); mbar_init(&empty_r[s], DIRECT ? 1 : C::CONV_WARPS / C::ADV); }
         for (int b = 0; b < C::NBUF; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], C::EPI_WARPS); }
         fence_barrier_init();
         fence_proxy_async();
@@ -430,7 +444,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
     if (warp == 0) {
         if (lane == 0) {
             // ---------------- TMA producer: token tiles ----------------
-            RingPos<C::S> r;
+            RingPos<C::SB> r;
             uint32_t g = 0;
             bool ok = true;
             PROF_DECL();
@@ -444,7 +458,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                 }
                 const int row0 = p.tile_row0[t];
                 for (int o = 0; o < nops; ++o, ++g, r.next()) {
-                    PROF_SCOPE(0, ok = mbar_wait(&empty[r.i], r.ph ^ 1, p.err, 11));
+                    PROF_SCOPE(0, ok = mbar_wait(&empty_b[r.i], r.ph ^ 1, p.err, 11));
                     if (!ok) break;
                     const int n = min(C::KS, nkb - o * C::KS);
                     mbar_expect_tx(&full_b[r.i], (uint32_t)(n * C::B_BYTES));
@@ -455,7 +469,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
             PROF_FLUSH(0, 1);
             if (!ok) {
                 // loads in flight still write this CTA's shared memory: let them land (bounded, no error code)
-                for (uint32_t i = g > (uint32_t)C::S ? g - C::S : 0; i < g; ++i) mbar_wait(&full_b[i % C::S], (i / C::S) & 1, nullptr, 0);
+                for (uint32_t i = g > (uint32_t)C::SB ? g - C::SB : 0; i < g; ++i) mbar_wait(&full_b[i % C::SB], (i / C::SB) & 1, nullptr, 0);
             }
         }
     } else if (warp == C::RAW_WARP) {
@@ -503,7 +517,8 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
         constexpr uint32_t idesc = idesc_f16(kTBM, BN, DIRECT ? 1 : 0);
         const int utotal = __reduce_max_sync(0xffffffffu, total), untiles = __reduce_max_sync(0xffffffffu, ntiles);
         const uint32_t ut = __reduce_max_sync(0xffffffffu, tmem_d);
-        RingPos<C::S> r;
+        RingPos<C::S> ra;                                      // weights in tensor memory
+        RingPos<C::SB> r;                                      // token tiles
         RingPos<C::RD> rr;                                     // (direct: raw entries)
         uint32_t lt = 0;
         bool ok = true;
@@ -518,7 +533,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
             if (!ok) break;
             tc_fence_after();
             const uint32_t acc = ut + buf * C::ACC_COLS;
-            for (int o = 0; o < nops; ++o, r.next()) {
+            for (int o = 0; o < nops; ++o, r.next(), ra.next()) {
                 PROF_SCOPE(1, ok = mbar_wait(&full_b[r.i], r.ph, p.err, 12));
                 if constexpr (DIRECT) {
                     ok = __all_sync(0xffffffffu, ok);
@@ -543,15 +558,15 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                         __syncwarp(); });
                     }
                     if (!ok) break;
-                    if (elect_one()) umma_commit(&empty[r.i]);
+                    if (elect_one()) umma_commit(&empty_b[r.i]);
                     __syncwarp();
                     continue;
                 }
-                if (ok) PROF_SCOPE(2, ok = mbar_wait(&full_a[r.i], r.ph, p.err, 12));
+                if (ok) PROF_SCOPE(2, ok = mbar_wait(&full_a[ra.i], ra.ph, p.err, 12));
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t a_t = ut + C::A_BASE + r.i * C::A_COLS;
+                const uint32_t a_t = ut + C::A_BASE + ra.i * C::A_COLS;
                 const uint64_t db = smem_desc_sw128(smem_b + r.i * C::KS * C::B_BYTES);
                 const int n = min(C::KS, nkb - o * C::KS);
                 PROF_SCOPE(3, {
@@ -567,7 +582,8 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                             if (GATEUP) umma_f16_ts(acc + BN, a_t + j * 32 * C::A_TILES + 32 + 8 * k, b, idesc, accum);
                         }
                     }
-                    umma_commit(&empty[r.i]);
+                    umma_commit(&empty_a[ra.i]);
+                    umma_commit(&empty_b[r.i]);
                 }
                 __syncwarp(); });
             }
@@ -580,8 +596,8 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
         // ---------------- weight converters ----------------
         constexpr int NC = 32 / C::NH;
         const int q = warp & 3;                                // TMEM lane quarter this warp may access
-        const int part = ((warp - 2) >> 2) & 1;                // gate/up: matrix (0 gate, 1 up); down: half of the stage's K range
-        const int set = (warp - 2) >> 3;                       // this warp converts the sub-stages `it` with it % CONV_SETS == set
+        const int part = ((warp - 2) >> 2) % C::PARTS;         // gate/up: matrix (0 gate, 1 up); down: part of the sub-stage's elements
+        const int set = (warp - 2) / C::SET_WARPS;             // this warp converts the sub-stages `it` with it % CONV_SETS == set
         const int row = q * 32 + lane;                         // row of the 128-row weight tile = TMEM lane
         const int h = GATEUP ? 0 : part;
         const int mat = GATEUP ? part : 0;
@@ -604,30 +620,31 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
             // one stage ahead of their use
             const float* fsc = reinterpret_cast<const float*>(sf) + (size_t)(n >> 7) * ((K + 127) >> 7);
             const uint8_t* qrow = wm + (size_t)n * CV::pitch(K);
+            // this warp's place among the sub-stages that the sets take side by side (an item with an odd number of entries leaves the sets' slots shifted)
+            const int own = C::ADV > 1 ? ((set / C::SUB + C::ADV - (int)rr.i % C::ADV) % C::ADV) * C::SUB + set % C::SUB : set;
             float sc_next = 0.f;
             uint4 hdr_next = make_uint4(0, 0, 0, 0);
-            if (FMT == 1) sc_next = __ldg(fsc);
+            if (FMT == 1) sc_next = __ldg(fsc + (C::ADV > 1 && own / C::SUB < nkb / C::SUB ? own / C::SUB : 0));
             if (FMT == 3) hdr_next = __ldg(reinterpret_cast<const uint4*>(qrow));
             const int nent = (nkb + C::SUB - 1) / C::SUB;
             typename CV::Raw raw;
-            const int own = C::ADV > 1 ? (set + (int)rr.i) % C::CONV_SETS : set;       // (an item of odd length leaves the sets' slots shifted by one)
             // Straight-line code for the sub-stages of whole entries and whole operand stages: the instructions around a sub-stage (ring
             // positions, which barrier is due) cost as much as its conversion when they are decided at run time.
             constexpr int BLK = C::SUB > C::KS ? C::SUB : C::KS;
-            int okw = 1;
 #pragma unroll 1
             for (int b0 = 0; b0 < nkb && ok; b0 += BLK) {
 #pragma unroll
                 for (int i = 0; i < BLK / C::CONV_SETS; ++i) {
-                    const int l0 = i * C::CONV_SETS, l = l0 + own;       // sub-stages of both sets; this warp's
+                    const int l0 = i * C::CONV_SETS, l = l0 + own;       // sub-stages of all sets; this warp's
                     if (b0 + l0 >= nkb) break;
-                    const bool mine = C::SUB > 1 || b0 + l < nkb;        // (past an odd end: zeros into columns that no MMA reads, or no entry at all)
+                    // (past the end: zeros into columns that no MMA reads, or no entry at all)
+                    const bool mine = C::ADV == 1 || b0 + l / C::SUB * C::SUB < nkb;
                     RingPos<C::RD> re = rr;
-                    if (C::SUB == 1) re.skip(l);
-                    if (C::SUB == 1 || l0 % C::SUB == 0) {
+                    if (C::ADV > 1) re.skip(l / C::SUB);
+                    if (C::ADV > 1 || l0 % C::SUB == 0) {
                         if constexpr (FMT == 1) {
                             raw.sc = sc_next;
-                            const int e = (b0 + l0) / C::SUB + 1;
+                            const int e = (b0 + (C::ADV > 1 ? l : l0)) / C::SUB + C::ADV;
                             if (e < nent) sc_next = __ldg(fsc + e);
                         }
                         if constexpr (FMT == 3) {
@@ -635,9 +652,9 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                             const int e = (b0 + l0) / C::SUB + 1;
                             if (e < nent) hdr_next = __ldg(reinterpret_cast<const uint4*>(qrow + (size_t)e * 144));
                         }
-                        // one lane polls the barrier, the warp sleeps at the sync: waiting warps leave the issue slots alone
-                        if (lane == 0 && mine) { if (warp == 2) PROF_SCOPE(0, okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0); else okw = mbar_wait(&full_r[re.i], re.ph, p.err, 17) ? 1 : 0; }
-                        ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
+                        // (the warp polls as a whole: a lane's poll handed round by a shuffle is a longer chain, 556 instead of 512 cycles per 64 elements of 32 rows)
+                        if (mine) PROF_SCOPE(0, ok = mbar_wait(&full_r[re.i], re.ph, p.err, 17));
+                        ok = __all_sync(0xffffffffu, ok);
                         if (!ok) break;
                     }
                     uint32_t out[NC];
@@ -651,14 +668,14 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                         }
                         CV::convert(raw, out, (b0 + l) * kTBK, h);       // consumes every byte read above
                     }
-                    if (C::SUB == 1 || (l0 + C::CONV_SETS) % C::SUB == 0 || b0 + l0 + C::CONV_SETS >= nkb) {
+                    if (C::ADV > 1 || (l0 + C::CONV_SETS) % C::SUB == 0 || b0 + l0 + C::CONV_SETS >= nkb) {
                         __syncwarp();
                         if (lane == 0 && mine) mbar_arrive(&empty_r[re.i]);        // the raw entry may be refilled
-                        if (C::SUB > 1) rr.next();
+                        if (C::ADV == 1) rr.next();
                     }
                     if (l0 % C::KS == 0) {
-                        if (lane == 0) { if (warp == 2) PROF_SCOPE(1, okw = mbar_wait(&empty[ra.i], ra.ph ^ 1, p.err, 13) ? 1 : 0); else okw = mbar_wait(&empty[ra.i], ra.ph ^ 1, p.err, 13) ? 1 : 0; }
-                        ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
+                        PROF_SCOPE(1, ok = mbar_wait(&empty_a[ra.i], ra.ph ^ 1, p.err, 13));
+                        ok = __all_sync(0xffffffffu, ok);
                         if (!ok) break;
                         tc_fence_after();                      // the MMAs that read this operand stage have completed
                     }
@@ -675,7 +692,7 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                         ra.next();
                     }
                 }
-                if (C::SUB == 1) rr.skip(min(BLK, nkb - b0));
+                if (C::ADV > 1) rr.skip((min(BLK, nkb - b0) + C::SUB - 1) / C::SUB);
             }
         }
         if (warp == 2 && lane == 0) { PROF_FLUSH(0, 6); PROF_FLUSH(1, 8); PROF_FLUSH(2, 7); PROF_FLUSH(3, 9); PROF_TOTAL(10); }
@@ -695,12 +712,18 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
             const int n = jn * kTBM + q * 32 + lane;
             const uint8_t* base = p.arena + (size_t)slot * p.ef.stride;
             const uint32_t buf = lt % C::NBUF;
-            // the columns' factors on the experts' inputs, fetched while the tile is being computed
+            // what 32 columns need, a lane each, fetched while the tile or the 32 in front of them are worked on: the factor on the expert's input, or the output
+            // row of the down projection (read between the stores, which it has to stay behind as far as the compiler knows, the pair index made a chain of 64
+            // loads that took longer than the tile's MMAs: the down projection of 2048 rows of 288 NVFP4 experts waited for its epilogue a quarter of the time)
             const bool scaled = GATEUP && p.ga.in_scale != nullptr;
-            float in_scale[BN / 32];
-#pragma unroll
-            for (int g = 0; g < BN / 32; ++g)
-                in_scale[g] = scaled && g * 32 + lane < ncols ? p.ga.in_scale[p.sorted_pair[row0 + g * 32 + lane]] : 1.f;
+            const bool scatter = !GATEUP && !up && !ep_mode;
+            float cs = 1.f, cs_next = 1.f;
+            int ct = 0, ct_next = 0;
+            auto fetch = [&](int c) {
+                ct_next = (scaled || scatter) && c < ncols ? p.sorted_pair[row0 + c] : 0;
+                cs_next = scaled && c < ncols ? p.ga.in_scale[ct_next] : 1.f;
+            };
+            fetch(lane);
             int okw = 1;
             if (lane == 0) { if (q == 0) PROF_SCOPE(0, okw = mbar_wait_relaxed(&acc_full[buf], (lt / C::NBUF) & 1u, p.err, 14) ? 1 : 0); else okw = mbar_wait_relaxed(&acc_full[buf], (lt / C::NBUF) & 1u, p.err, 14) ? 1 : 0; }
             ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
@@ -716,34 +739,48 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                     sg = su = kFp8Unscale;
                 }
                 const uint32_t lane_addr = tmem_d + buf * C::ACC_COLS + ((uint32_t)(q * 32) << 16);
+                const GluAct ga = p.ga;
+                // (NOUT is whole tiles, so every lane has a row of the matrix; which columns are stored is a predicate of the store)
+                __half* act = p.act + (size_t)row0 * NOUT + n;
+                float* yf = p.y + n;
+                bf16* yh = reinterpret_cast<bf16*>(p.y) + n;
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 16) {
-                    if (c0 >= ncols) break;
+                for (int c0 = 0; c0 < ncols; c0 += 16) {
+                    if ((c0 & 31) == 0) { ct = ct_next; cs = cs_next; fetch(c0 + 32 + lane); }
                     float gq[16], uq[16];
                     tmem_ld16(lane_addr + (uint32_t)c0, gq);
                     if (GATEUP) tmem_ld16(lane_addr + (uint32_t)(BN + c0), uq);
-                    float cs = in_scale[0];                                // factors of this group of 32 columns, one per lane
+                    if (GATEUP) {
 #pragma unroll
-                    for (int g = 1; g < BN / 32; ++g) cs = (c0 >> 5) == g ? in_scale[g] : cs;
+                        for (int j = 0; j < 16; ++j, act += NOUT) {
+                            const float c = __shfl_sync(0xffffffffu, cs, (c0 + j) & 31);
+                            if (DIRECT == kDirectBf16) st_global_if(reinterpret_cast<bf16*>(act), __float2bfloat16(glu_act(gq[j] * c, uq[j] * c, ga)), c0 + j < ncols);
+                            else st_global_if(act, __float2half_rn(half_range(glu_act(gq[j] * sg * c, uq[j] * su * c, ga))), c0 + j < ncols);
+                        }
+                    } else if (up) {
+                        // (fp16 range: far outside what normed inputs reach, kept finite all the same)
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const float c = GATEUP && scaled ? __shfl_sync(0xffffffffu, cs, (c0 + j) & 31) : 1.f;
-                        if (c0 + j < ncols && n < NOUT) {
-                            if (GATEUP && DIRECT == kDirectBf16) {
-                                reinterpret_cast<bf16*>(p.act)[(size_t)(row0 + c0 + j) * NOUT + n] = __float2bfloat16(glu_act(gq[j] * c, uq[j] * c, p.ga));
-                            } else if (GATEUP) {
-                                p.act[(size_t)(row0 + c0 + j) * NOUT + n] = __float2half_rn(half_range(glu_act(gq[j] * sg * c, uq[j] * su * c, p.ga)));
-                            } else if (up) {
-                                // (fp16 range: far outside what normed inputs reach, kept finite all the same)
-                                p.act[(size_t)(row0 + c0 + j) * NOUT + n] = __float2half_rn(fminf(relu2_act(gq[j] * sg), 65504.f));
-                            } else if (ep_mode) {
-                                const int2 ra = p.ep.ret[p.ep.rank][row0 + c0 + j];      // (token owner, pair index there)
-                                p.ep.y[ra.x][(size_t)ra.y * NOUT + n] = gq[j] * sg;       // NVLink store into the owner's buffer
-                            } else if (p.out_bf16) {
-                                reinterpret_cast<bf16*>(p.y)[(size_t)p.sorted_pair[row0 + c0 + j] * p.ldo + n] = __float2bfloat16(gq[j] * sg);
-                            } else {
-                                p.y[(size_t)p.sorted_pair[row0 + c0 + j] * p.ldo + n] = gq[j] * sg;
-                            }
+                        for (int j = 0; j < 16; ++j, act += NOUT) st_global_if(act, __float2half_rn(fminf(relu2_act(gq[j] * sg), 65504.f)), c0 + j < ncols);
+                    } else if (ep_mode) {
+#pragma unroll 1
+                        for (int j = 0; j < 16 && c0 + j < ncols; ++j) {
+                            float v = gq[0];
+#pragma unroll
+                            for (int i = 1; i < 16; ++i) v = i == j ? gq[i] : v;
+                            const int2 ra = p.ep.ret[p.ep.rank][row0 + c0 + j];      // (token owner, pair index there)
+                            p.ep.y[ra.x][(size_t)ra.y * NOUT + n] = v * sg;           // NVLink store into the owner's buffer
+                        }
+                    } else if (p.out_bf16) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const int r = __shfl_sync(0xffffffffu, ct, (c0 + j) & 31);
+                            st_global_if(yh + (size_t)r * p.ldo, __float2bfloat16(gq[j] * sg), c0 + j < ncols);
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const int r = __shfl_sync(0xffffffffu, ct, (c0 + j) & 31);
+                            st_global_if(yf + (size_t)r * p.ldo, gq[j] * sg, c0 + j < ncols);
                         }
                     }
                 }

@@ -449,3 +449,40 @@ def test_steps_of_fewer_rows_than_the_workspace(R):
         want = (torch.nn.functional.silu(xd[r] @ gate.T) * (xd[r] @ up.T)) @ down.T
         assert float((got[r, k] - want).norm() / want.norm()) < 1e-3, e
     assert float(mb.y.view(700, S, H)[R:].abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("fmt", ["nvfp4", "fp8_e4m3", "bf16", "gguf_q4_k"])
+@pytest.mark.parametrize("BN", [32, 64, 128])
+@pytest.mark.parametrize("copies", [1, 12])
+def test_tiles_of_every_number_of_rows(fmt, BN, copies):
+    """One row, one below, at and above each piece of the epilogue, whole tiles and a remainder behind one, each beside experts with other numbers of rows; with
+    copies, several tiles per thread block and reductions that end at every place of the rings."""
+    from layerstorm_b200.ops import _native as nat
+    dev, H, F = torch.device("cuda"), 1024, 768
+    counts = [n for n in (1, 15, 16, 17, 31, 32, 33, 48, 63, 64, 65, 112, 127, 128, 129) if n <= BN + 1]
+    E = len(counts)
+    arena, ref = _setup(fmt, H, F, E, n_missing=0, seed=8)
+    arena.slot_of = arena.slot_of.repeat(copies)                     # more experts with the same weights
+    g = torch.Generator(device="cpu").manual_seed(9)
+    ids = torch.cat([torch.full((n,), e + E * c) for c in range(copies) for e, n in enumerate(counts)])
+    ids = ids[torch.randperm(len(ids), generator=g)].int()
+    P = len(ids)
+    x, tiles = torch.randn(P, H, generator=g).to(torch.bfloat16).to(dev), P // BN + E * copies + 1
+    i32 = dict(dtype=torch.int32, device=dev)
+    srt, te, tr, tn, cnt, err = (torch.zeros(n, **i32) for n in (P, tiles, tiles, tiles, 2, 1))
+    xs, act = torch.zeros(P, H, dtype=torch.float16, device=dev), torch.zeros(P + 1, F, dtype=torch.float16, device=dev)
+    y, efp = torch.zeros(P + 1, H, device=dev), ctypes.addressof(arena.ef)
+    nat.call("lsb_moe_tc_sort", ids.to(dev), P, E * copies, BN, srt, te, tr, tn, cnt)
+    nat.call("lsb_moe_tc_gather", x, srt, cnt, xs, P, 1, H)
+    nat.call("lsb_moe_tc_ffn", 1, xs, P, arena.data, arena.slot_of, efp, te, tr, tn, cnt, srt, act, BN, tiles, 0.0, None, err, None)
+    nat.call("lsb_moe_tc_ffn", 0, act, P, arena.data, arena.slot_of, efp, te, tr, tn, cnt, srt, y, BN, tiles, 0.0, None, err, None)
+    torch.cuda.synchronize()
+    assert int(err) == 0 and float(act[P].abs().sum()) == 0.0 and float(y[P].abs().sum()) == 0.0
+    for e in range(E):
+        r = (ids % E == e).nonzero()[:, 0].to(dev)
+        gate, up, down = (m.to(dev) for m in ref[e])
+        xd = x[r].double()
+        want = (torch.nn.functional.silu(xd @ gate.T) * (xd @ up.T)) @ down.T
+        # hidden values in fp16 (2^-11 each at most), bf16 weights converted to fp16 (the same); Q4_K weights are a scale times 0 .. 15 less an offset, both rounded
+        # to fp16: 2^-11 of up to 15 steps where the weights' rms is 4.3 of them, 1.7e-3, in each of the three matrices
+        assert float((y[r].double() - want).norm() / want.norm()) < (3 ** 0.5 * 1.7e-3 if fmt == "gguf_q4_k" else 1e-3), (e, counts[e])
