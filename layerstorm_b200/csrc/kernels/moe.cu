@@ -17,6 +17,7 @@
 #include "gemv_core.cuh"
 #include "comm.cuh"
 #include "moe_fmt.cuh"
+#include "fp8_rows.cuh"
 #include "router_core.cuh"
 
 namespace lsb {
@@ -176,6 +177,36 @@ __global__ void moe_build_groups_kernel(const int* __restrict__ ids, int npairs,
             group_expert[g + j] = e;
             group_n[g + j] = min(4, c - j * 4);
         }
+    }
+    pdl_launch_dependents();
+}
+
+// The same for few pairs, a thread each: a pair's place among those of its expert, and how many groups of lower experts there are, counted over ids in shared
+// memory.  (The walk over all experts above takes 12 to 20 us whatever there is to group: one thread adds up 257 counts, then threads walk the pairs one by one.)
+constexpr int kFewPairs = 256;
+__global__ void __launch_bounds__(kFewPairs) moe_build_few_groups_kernel(const int* __restrict__ ids, int npairs, int E_total, int* __restrict__ group_expert,
+                                                                         int* __restrict__ group_n, int* __restrict__ group_pairs, int* __restrict__ n_groups) {
+    __shared__ int s_id[kFewPairs], s_first[kFewPairs];                // a pair's expert; the same where the pair is a group's first
+    const int i = threadIdx.x;
+    pdl_wait();
+    pdl_launch_dependents();
+    int e = i < npairs ? ids[i] : -1;
+    if (e >= E_total) e = -1;
+    s_id[i] = e;
+    __syncthreads();
+    int before = 0, all = 0, base = 0;
+#pragma unroll 8
+    for (int j = 0; j < npairs; ++j) { const bool same = s_id[j] == e; all += same; before += same && j < i; }
+    const bool first = e >= 0 && (before & 3) == 0;
+    s_first[i] = first ? e : 0x7fffffff;
+    const int total = __syncthreads_count(first);
+#pragma unroll 8
+    for (int j = 0; j < npairs; ++j) base += s_first[j] < e;
+    if (i == 0) n_groups[0] = total;
+    if (e >= 0) {
+        const int g = base + (before >> 2);
+        group_pairs[g * 4 + (before & 3)] = i;
+        if (first) { group_expert[g] = e; group_n[g] = min(4, all - before); }
     }
     pdl_launch_dependents();
 }
@@ -633,9 +664,27 @@ LSB_API int lsb_router_hash(const void* logits, const void* tid2eid, const void*
 
 LSB_API int lsb_moe_build_groups(const void* ids, int npairs, int E_total, void* group_expert, void* group_n,
                                  void* group_pairs, void* n_groups, void* counts, void* stream) {
+    if (npairs > 0 && npairs <= kFewPairs) {
+        launch_pdl((moe_build_few_groups_kernel), 1, (npairs + 31) & ~31, 0, (cudaStream_t)stream, (const int*)ids, npairs, E_total, (int*)group_expert, (int*)group_n,
+                   (int*)group_pairs, (int*)n_groups);
+        LSB_CHECK_LAUNCH();
+    }
     launch_pdl((moe_build_groups_kernel), 1, 512, 0, (cudaStream_t)stream, (const int*)ids, npairs, E_total, (int*)group_expert, (int*)group_n,
                                                                (int*)group_pairs, (int*)n_groups, (int*)counts);
     LSB_CHECK_LAUNCH();
+}
+
+// FP8 experts whose matrices the few-row kernel takes (fp8_rows.cuh), a group's rows of `K` values staged together.
+static bool fp8_experts_ok(const ExpertFmt& ef, const void* x, const void* arena, int K) {
+    return ef.fmt == 1 && ef.down_fmt() == 1 && ef.H % 128 == 0 && ef.F % 128 == 0 && ef.H >= 1024 && 4 * (K + 8) * 2 <= kF8Rows
+           && ((ef.stride | ef.off_gate | ef.off_up | ef.off_down | (long long)(uintptr_t)x | (long long)(uintptr_t)arena) & 15) == 0;
+}
+static Fp8RowsArgs fp8_expert_args(const ExpertFmt& ef, const void* x, int N, int K, const void* arena, const void* slot_of, const void* group_expert,
+                                   const void* group_n, const void* group_pairs, const void* n_groups, void* out) {
+    Fp8RowsArgs a{};
+    a.x = (const bf16*)x; a.N = N; a.K = K; a.M = 4; a.out = out; a.arena = (const uint8_t*)arena; a.slot_of = (const int*)slot_of; a.ef = ef;
+    a.group_expert = (const int*)group_expert; a.group_n = (const int*)group_n; a.group_pairs = (const int*)group_pairs; a.n_groups = (const int*)n_groups;
+    return a;
 }
 
 // Pair mode (group_n == null): every (row, slot) pair is its own group - group_expert is the
@@ -673,6 +722,11 @@ static int moe_gateup(const void* x, const void* arena, const void* slot_of, con
         LSB_CHECK_LAUNCH();
     }
     if (!group_n) return -1;   // pair mode is only implemented for the NVFP4 fast path
+    if (fp8_experts_ok(ef, x, arena, ef.H)) {
+        Fp8RowsArgs a = fp8_expert_args(ef, x, ef.F, ef.H, arena, slot_of, group_expert, group_n, group_pairs, n_groups, act);
+        a.S = S; a.ga = ga; a.miss_flag = (int*)miss_flag;
+        return fp8_rows_launch<kF8GateUp>(a, max_groups, st);
+    }
     dim3 grid((ef.F + 7) / 8, max_groups);
 #define ARGS (const bf16*)x, (const uint8_t*)arena, (const int*)slot_of, ef, (const int*)group_expert, (const int*)group_n, \
              (const int*)group_pairs, (const int*)n_groups, (bf16*)act, S, ga, (int*)miss_flag
@@ -741,6 +795,8 @@ LSB_API int lsb_moe_down(const void* act, const void* arena, const void* slot_of
                    (const int*)group_expert, (const int*)group_n, (const int*)group_pairs, (const int*)n_groups, (float*)y, 1, GluAct{0.f, 1.f, 0.f, nullptr}, nullptr);
         LSB_CHECK_LAUNCH();
     }
+    if (ef.down_fmt() == 1 && fp8_experts_ok(ef, act, arena, ef.F))
+        return fp8_rows_launch<kF8Down>(fp8_expert_args(ef, act, ef.H, ef.F, arena, slot_of, group_expert, group_n, group_pairs, n_groups, y), max_groups, st);
     dim3 grid((ef.H + 15) / 16, max_groups);
 #define ARGS (const bf16*)act, (const uint8_t*)arena, (const int*)slot_of, ef, (const int*)group_expert, (const int*)group_n, \
              (const int*)group_pairs, (const int*)n_groups, (float*)y

@@ -716,3 +716,87 @@ def test_kda_rows_of_any_alignment(norm_at, out_at):
         got.append((out.clone(), state, hist))
     assert bool(got[0][0].isfinite().all()) and float(got[0][0].float().norm()) > 1.0
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("npairs,E", [(1, 1), (9, 257), (31, 4), (32, 3), (33, 40), (135, 257), (255, 7), (256, 300), (257, 300), (700, 20)])
+def test_expert_groups_of_any_number_of_pairs(npairs, E):
+    """Groups of up to four pairs in order of their experts, pairs in order inside; ids outside the range take no part; both sides of 256 pairs."""
+    from layerstorm_b200.ops import _native as nat
+    g = torch.Generator().manual_seed(npairs)
+    ids = torch.randint(-1, E + 1, (npairs,), generator=g).int()
+    mg = npairs // 4 + E + 1 + npairs
+    ge, gn, gp, ng, cn = (torch.full((n,), -7, dtype=torch.int32, device="cuda") for n in (mg, mg, 4 * mg, 1, 2 * E + 2))
+    nat.call("lsb_moe_build_groups", ids.cuda(), npairs, E, ge, gn, gp, ng, cn)
+    want = [(e, p[j: j + 4]) for e in range(E) for p in [(ids == e).nonzero()[:, 0].tolist()] for j in range(0, len(p), 4)]
+    assert int(ng) == len(want)
+    got = [(int(ge[k]), gp[4 * k: 4 * k + int(gn[k])].tolist()) for k in range(int(ng))]
+    assert got == want and int(ge[int(ng):].ne(-7).sum()) == 0
+
+
+@pytest.mark.parametrize("N,K", [(8192, 1536), (98304, 128), (16400, 1024), (1648, 8192), (6160, 2176), (784, 18432)])
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 9, 15])
+def test_fp8_rows_over_large_matrices(N, K, M):
+    """Few rows over FP8 weights by mma: last units and 16-row tiles that blocks share unevenly, one to 144 blocks of the reduction, rows in one and several passes,
+    strided rows, a bias, both output types; rows of very different sizes, of zeros and beyond fp16; nothing written outside."""
+    from layerstorm_b200.ops import _native as nat
+    assert N * K >= 12 << 20
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    w = torch.randn(N, K, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    sc = torch.rand((N + 127) // 128, K // 128, device="cuda", generator=g) * 0.01 + 0.01
+    x = torch.randn(M, K + 8, device="cuda", generator=g)
+    x *= torch.tensor([1.0, 3e-30, 1e30, 0.0, 1e-4, 7e4], device="cuda")[torch.arange(M, device="cuda") % 6][:, None]
+    x[:, 5] *= 300
+    x = x.bfloat16()
+    bias = torch.randn(N, device="cuda", generator=g)
+    sums = torch.zeros(M, N, dtype=torch.float64, device="cuda")
+    for k in range(0, K, 128):
+        sums += (x[:, k: k + 128].double() @ w[:, k: k + 128].double().T) * sc[:, k // 128].double().repeat_interleave(128)[:N]
+    for dt, b, tol in ((torch.float32, None, 5e-7), (torch.bfloat16, bias, 3e-3)):
+        out = torch.zeros(M + 1, N + 8, device="cuda", dtype=dt)
+        nat.call("lsb_gemv_fp8b", out, x, w, sc, b, M, N, K, K + 8, N + 8, 1.0, int(dt == torch.bfloat16), None)
+        want = sums if b is None else sums + b.double()
+        assert float(out[M:].abs().sum()) == 0.0 and float(out[:M, N:].abs().sum()) == 0.0
+        # products exact, fp32 sums (2^-24 sqrt(K) at most of what was added, which the result's norm is), rounded to bf16 (2^-9) where asked
+        for m in range(M):
+            assert float((out[m, :N].double() - want[m]).norm()) <= tol * float(want[m].norm()), m
+    if M > 2:                                             # infinities and NaN stay in their rows
+        x[1, 7], x[2, 9] = float("inf"), float("nan")
+        bad = torch.zeros(M, N + 8, device="cuda")
+        nat.call("lsb_gemv_fp8b", bad, x, w, sc, None, M, N, K, K + 8, N + 8, 1.0, 0, None)
+        assert not bool(bad[1, :N].isfinite().any()) or bool((w[:, 7].float() == 0).any())
+        assert bool(bad[2, :N].isnan().all()) and torch.equal(bad[0], torch.cat([bad[0, :N], torch.zeros(8, device="cuda")])) and bool(bad[0].isfinite().all())
+
+
+@pytest.mark.parametrize("H,F", [(1024, 512), (1152, 384), (2048, 128), (7168, 256)])
+@pytest.mark.parametrize("R", [1, 3, 7, 15])
+def test_fp8_experts_of_few_rows(H, F, R):
+    """Gate/up and down of every group: one to four rows, experts that are not resident, a unit with limits; against 64 bits."""
+    import ctypes
+    from layerstorm_b200.models.device_model import ExpertArena, QLinear, expert_layout
+    from layerstorm_b200.ops import _native as nat
+    E, S, dev = 9, 3, "cuda"
+    g = torch.Generator().manual_seed(H + R)
+    arena, ref = ExpertArena(expert_layout("fp8_e4m3", H, F), E - 1, E, torch.device(dev)), {}
+    for e in range(1, E):
+        arena.write_expert(e - 1, *(QLinear.from_float(torch.randn(o, i, generator=g).cuda() * i ** -0.5, "fp8_e4m3", dev) for o, i in ((F, H), (F, H), (H, F))))
+        arena.slot_of[e] = e - 1
+        ref[e] = [m.double().cuda() for m in arena.read_expert(e - 1, "fp8_e4m3")]
+    ids = torch.stack([torch.cat([torch.randperm(E - 1, generator=g)[: S - 1], torch.tensor([E - 1])]) for _ in range(R)]).int()
+    x, P, mg = torch.randn(R, H, generator=g).bfloat16().cuda(), R * S, R * S + E
+    ge, gn, gp, ng, cn, miss = (torch.zeros(n, dtype=torch.int32, device=dev) for n in (mg, mg, 4 * mg, 1, 2 * E + 2, 1))
+    act, y, efp = torch.zeros(P, F, dtype=torch.bfloat16, device=dev), torch.zeros(P, H, device=dev), ctypes.addressof(arena.ef)
+    nat.call("lsb_moe_build_groups", ids.cuda(), P, E, ge, gn, gp, ng, cn)
+    nat.call("lsb_moe_gateup", x, arena.data, arena.slot_of, efp, ge, gn, gp, ng, act, S, mg, 1.5, miss, 0)
+    nat.call("lsb_moe_down", act, arena.data, arena.slot_of, efp, ge, gn, gp, ng, y, mg, 0)
+    assert int(miss) == (1 if bool((ids == 0).any()) else 0)
+    for p in range(P):
+        e = int(ids.view(-1)[p])
+        if e == 0:
+            assert float(act[p].abs().sum()) == 0.0 and float(y[p].abs().sum()) == 0.0
+            continue
+        gate, up, down = ref[e]
+        gv, uv = (gate @ x[p // S].double()).clamp(max=1.5), (up @ x[p // S].double()).clamp(-1.5, 1.5)
+        want = torch.nn.functional.silu(gv) * uv
+        assert float((act[p].double() - want).norm() / want.norm()) < 3e-3          # rounded to bf16 (2^-9)
+        want = down @ act[p].double()
+        assert float((y[p].double() - want).norm() / want.norm()) < 5e-7            # products exact, fp32 sums
