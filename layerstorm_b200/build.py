@@ -45,7 +45,7 @@ CXX_FLAGS = ["-O2", "-g", "-std=c++20", "-fPIC", "-Wall", "-Wno-unused-function"
 # kernel files of a model family: models described layer by layer run without the MLA-family, indexer, hyper-connection and expert-parallel kernels, and
 # without those of the mixers that they do not have
 MIXER_FILES = {"delta": ("channel_delta", "head_delta"), "latent": ("latent_attention",), "tmix": ("time_mix",)}
-FAMILIES = {"blocks" + "".join(f"_{f}" for f in extra): ("attn", "gemm_tc", "gemv", "moe", "moe_tc", "norm", "sampling") + extra
+FAMILIES = {"blocks" + "".join(f"_{f}" for f in extra): ("attn", "gemm_tc", "gemv", "kv_rows", "moe", "moe_tc", "norm", "sampling") + extra
             for n in range(len(MIXER_FILES) + 1) for extra in itertools.combinations(MIXER_FILES, n)}
 
 

@@ -12,6 +12,26 @@
 
 namespace lsb {
 
+// Per-sequence slots of several tensors copied from one slot to another in one launch (a sequence that goes on from another's frontier: recurrent states,
+// convolution histories, open index pools).  A copy per tensor was bound by its launches: 125 us a sequence with three recurrent layers of 64 heads of 128 x 128 and
+// their histories, 80 us now (the page bookkeeping and the block table's copy; the bytes take 4 us).
+constexpr int kSlotTensors = 96;
+struct SlotCopy { uint8_t* base[kSlotTensors]; long long bytes[kSlotTensors]; };      // bytes: of a slot, and between slots
+__global__ void __launch_bounds__(256) copy_slots_kernel(const __grid_constant__ SlotCopy t, int from, int to) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const long long n = t.bytes[blockIdx.y];
+    const uint8_t* src = t.base[blockIdx.y] + from * n;
+    uint8_t* dst = t.base[blockIdx.y] + to * n;
+    const long long i0 = (long long)blockIdx.x * 256 + threadIdx.x, step = (long long)gridDim.x * 256;
+    if ((((uintptr_t)src | (uintptr_t)dst | (uintptr_t)n) & 15) == 0) {
+#pragma unroll 4
+        for (long long i = i0; i < n / 16; i += step) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+    } else {
+        for (long long i = i0; i < n; i += step) dst[i] = src[i];
+    }
+}
+
 // grid (ceil(sel_ld / 8), rows), 256 threads: a warp moves one row, 16 bytes per lane and pass
 __global__ void __launch_bounds__(256) kv_row_gather_kernel(const uint8_t* __restrict__ cache, const int* __restrict__ block_table, int max_pages,
                                                             const int* __restrict__ row_seq, const int* __restrict__ sel_idx,
@@ -55,6 +75,25 @@ __global__ void kv_rows_identity_kernel(int* __restrict__ sel_m, int sel_ld, int
 using namespace lsb;
 
 // out: [rows, out_rows, row_bytes] bytes; row_bytes a multiple of 16, all buffers 16-byte aligned.
+// `table` (host): n pairs {address, bytes per slot}; the slots of a tensor lie one behind the other.
+LSB_API int lsb_copy_slots(const void* table, int n, int from, int to, void* stream) {
+    const long long* t = (const long long*)table;
+    if (n < 0 || from < 0 || to < 0) return -1;
+    for (int k = 0; k < n && from != to; k += kSlotTensors) {
+        const int m = n - k < kSlotTensors ? n - k : kSlotTensors;
+        SlotCopy c{};
+        long long most = 0;
+        for (int i = 0; i < m; ++i) {
+            c.base[i] = (uint8_t*)t[2 * (k + i)];
+            c.bytes[i] = t[2 * (k + i) + 1];
+            if (c.bytes[i] > most) most = c.bytes[i];
+        }
+        const long long want = (most + 16383) / 16384;              // four 16-byte pieces a thread
+        launch_pdl((copy_slots_kernel), dim3(want < 1 ? 1 : (want > 256 ? 256 : (int)want), m), 256, 0, (cudaStream_t)stream, c, from, to);
+    }
+    LSB_CHECK_LAUNCH();
+}
+
 LSB_API int lsb_kv_row_gather(const void* cache, const void* block_table, int max_pages, const void* row_seq, const void* sel_idx,
                               const void* sel_cnt, int sel_ld, void* out, int out_rows, int rows, int page, int row_bytes, void* stream) {
     if (row_bytes % 16 || (((uintptr_t)cache | (uintptr_t)out) & 15) || rows <= 0) return -1;

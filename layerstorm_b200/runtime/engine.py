@@ -256,14 +256,25 @@ class Engine:
         self.seqs[slot] = cs
         with torch.cuda.stream(self.stream):
             m = self.model
-            for t in list(m.kda_state.values()) + list(m.kda_conv.values()) + list(m.idx_tail.values()):
-                t[slot].copy_(t[ps.slot])
+            self._copy_slot(ps.slot, slot)
             self._sync_block_table(cs)
             if self.mtp is not None:
                 self.mtp.on_fork(parent, slot, prefix_len)
             if self.aux_listener is not None:
                 self.aux_listener.on_fork(parent, slot, prefix_len)
         return slot
+
+    def _copy_slot(self, src: int, dst: int):
+        """What a sequence slot holds besides its pages (recurrent states, convolution histories, open index pools), from one slot to another."""
+        m = self.model
+        ts = [t for d in (m.kda_state, m.kda_conv, m.idx_tail) for t in d.values()]
+        if all(t.is_cuda and t.is_contiguous() for t in ts):
+            if ts:
+                table = np.array([(t.data_ptr(), t.stride(0) * t.element_size()) for t in ts], dtype=np.int64)
+                nat.call("lsb_copy_slots", table.ctypes.data, len(ts), src, dst)
+        else:
+            for t in ts:
+                t[dst].copy_(t[src])
 
     # ------------------------------------------------------------------ KV tiering (hibernate / resume)
     def enable_kv_tiering(self, cold_pages: int):
