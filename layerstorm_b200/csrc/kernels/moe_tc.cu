@@ -289,6 +289,9 @@ template <int FMT, int BN, bool GATEUP, int DIRECT = 0> struct MoeTcCfg {
     static constexpr int A_TILES = GATEUP ? 2 : 1;
     static constexpr int NH = GATEUP || FMT != 0 ? 1 : 2;                 // converter threads per (row, sub-stage) of a matrix; bf16 rows take too many registers for one
     using CV = RowConv<FMT, NH>;
+    // Token tiles of 256 rows (bf16 experts): a copy of 128 rows and an MMA of 128 columns where no more are there, else two and 256.  Half the weights per product
+    // through L2 and shared memory, which bound tiles of 128 (12.7 TB/s of L2); tensor memory then holds one accumulator set.
+    static constexpr int B_BOX = BN > 128 ? 128 : BN;
     static constexpr int B_BYTES = BN * kTBK * 2;                         // token tile of a sub-stage
     // An operand stage is KS sub-stages of 64 reduction elements behind one pair of barriers: the issuing warp's waits and commit cost a few
     // hundred cycles a stage beside the converters' instruction streams, which is more than the MMAs of 64 elements of a small token tile take.
@@ -298,7 +301,7 @@ template <int FMT, int BN, bool GATEUP, int DIRECT = 0> struct MoeTcCfg {
 #ifndef LSB_MOE_KS_DN
 #define LSB_MOE_KS_DN 4
 #endif
-    static constexpr int KS = GATEUP ? LSB_MOE_KS_GU : (BN <= 64 || FMT != 0 ? LSB_MOE_KS_DN : 2);
+    static constexpr int KS = GATEUP ? (BN > 128 ? 1 : LSB_MOE_KS_GU) : (BN <= 64 || FMT != 0 ? LSB_MOE_KS_DN : 2);
     static constexpr int ACC_COLS = A_TILES * BN;                         // one accumulator set (gate [+ up])
     // Tensor memory (512 columns): accumulator sets first, then the ring of converted weight stages
     // (32 columns = 64 fp16 per matrix and sub-stage).  Two accumulator sets let the epilogue of one item overlap the
@@ -306,7 +309,7 @@ template <int FMT, int BN, bool GATEUP, int DIRECT = 0> struct MoeTcCfg {
 #ifndef LSB_MOE_NBUF1_COLS
 #define LSB_MOE_NBUF1_COLS 128
 #endif
-    static constexpr int NBUF = ACC_COLS > LSB_MOE_NBUF1_COLS && !DIRECT ? 1 : 2;
+    static constexpr int NBUF = ACC_COLS > LSB_MOE_NBUF1_COLS && (!DIRECT || ACC_COLS > 256) ? 1 : 2;
     static constexpr int A_COLS = 32 * A_TILES * KS;
     static constexpr int A_BASE = NBUF * ACC_COLS;
     static constexpr int S_FIT = DIRECT ? 2 : (512 - A_BASE) / A_COLS;
@@ -319,7 +322,7 @@ template <int FMT, int BN, bool GATEUP, int DIRECT = 0> struct MoeTcCfg {
     static constexpr int SET_WARPS = 4 * PARTS;
     static constexpr int CONV_SETS = 16 / SET_WARPS;
     static constexpr int CONV_WARPS = DIRECT ? 0 : 16;
-    static_assert(KS % CONV_SETS == 0, "all sets have part in every operand stage");
+    static_assert(DIRECT || KS % CONV_SETS == 0, "all sets have part in every operand stage");
     static constexpr int EPI_WARPS = 4;
     static constexpr int RAW_WARP = 2 + CONV_WARPS + EPI_WARPS;           // last warp: TMA producer of the raw weight ring
     static constexpr int THREADS = (RAW_WARP + 1) * 32;
@@ -457,13 +460,17 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
                     continue;
                 }
                 const int row0 = p.tile_row0[t];
+                const int boxes = BN > 128 && p.tile_n[t] > 128 ? 2 : 1;
                 for (int o = 0; o < nops; ++o, ++g, r.next()) {
                     PROF_SCOPE(0, ok = mbar_wait(&empty_b[r.i], r.ph ^ 1, p.err, 11));
                     if (!ok) break;
                     const int n = min(C::KS, nkb - o * C::KS);
-                    mbar_expect_tx(&full_b[r.i], (uint32_t)(n * C::B_BYTES));
-                    for (int j = 0; j < n; ++j)
-                        tma_load_2d(smem_b + (r.i * C::KS + j) * C::B_BYTES, &map_b, &full_b[r.i], (o * C::KS + j) * kTBK, row0);
+                    mbar_expect_tx(&full_b[r.i], (uint32_t)(n * boxes * C::B_BOX * kTBK * 2));
+                    for (int j = 0; j < n; ++j) {
+                        uint8_t* dst = smem_b + (r.i * C::KS + j) * C::B_BYTES;
+                        tma_load_2d(dst, &map_b, &full_b[r.i], (o * C::KS + j) * kTBK, row0);
+                        if (BN > 128 && boxes > 1) tma_load_2d(dst + C::B_BOX * kTBK * 2, &map_b, &full_b[r.i], (o * C::KS + j) * kTBK, row0 + C::B_BOX);
+                    }
                 }
             }
             PROF_FLUSH(0, 1);
@@ -514,7 +521,6 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
         // ---------------- MMA issuer: A (weights) from tensor memory, B (tokens) from shared memory ----------------
         // The whole warp walks the list (loop bounds and ring positions stay warp-uniform, so the operands of the instructions are uniform
         // registers) and one elected lane issues.
-        constexpr uint32_t idesc = idesc_f16(kTBM, BN, DIRECT ? 1 : 0);
         const int utotal = __reduce_max_sync(0xffffffffu, total), untiles = __reduce_max_sync(0xffffffffu, ntiles);
         const uint32_t ut = __reduce_max_sync(0xffffffffu, tmem_d);
         RingPos<C::S> ra;                                      // weights in tensor memory
@@ -527,6 +533,9 @@ __global__ void __launch_bounds__(MoeTcCfg<FMT, BN, GATEUP, DIRECT>::THREADS, 1)
             int t, jn;
             work_item(w, untiles, NT, t, jn);
             if (!__reduce_or_sync(0xffffffffu, slot_ok(p.slot_of[p.tile_expert[t]]) ? 1u : 0u)) continue;
+            constexpr uint32_t idesc_all = idesc_f16(kTBM, BN, DIRECT ? 1 : 0), idesc_box = idesc_f16(kTBM, C::B_BOX, DIRECT ? 1 : 0);
+            uint32_t idesc = idesc_all;
+            if constexpr (BN > 128) idesc = __reduce_or_sync(0xffffffffu, p.tile_n[t] > C::B_BOX ? 1u : 0u) ? idesc_all : idesc_box;
             const uint32_t buf = lt % C::NBUF;
             PROF_SCOPE(0, ok = mbar_wait(&acc_empty[buf], ((lt / C::NBUF) & 1u) ^ 1u, p.err, 15));   // epilogue has drained this accumulator set
             ok = __all_sync(0xffffffffu, ok);
@@ -883,11 +892,11 @@ LSB_API int lsb_moe_tc_prof_read(void* out32, int reset, void* stream) {
 #endif
 }
 
-// Tiles of at most `BN` (32, 64 or 128) sorted rows.  tile_* arrays hold npairs / BN + E_total + 1 entries,
+// Tiles of at most `BN` (32, 64, 128; 256 over bf16 experts) sorted rows.  tile_* arrays hold npairs / BN + E_total + 1 entries,
 // counters 2 ints, sorted_pair npairs ints.
 LSB_API int lsb_moe_tc_sort(const void* ids, int npairs, int E_total, int BN, void* sorted_pair, void* tile_expert, void* tile_row0,
                             void* tile_n, void* counters, void* stream) {
-    if (E_total > 4000 || (BN != 32 && BN != 64 && BN != 128)) return -1;
+    if (E_total > 4000 || (BN != 32 && BN != 64 && BN != 128 && BN != 256)) return -1;
     launch_pdl((moe_tc_sort_kernel), 1, 1024, (size_t)(3 * E_total + 2) * 4, (cudaStream_t)stream, (const int*)ids, npairs, E_total, BN,
                (int*)sorted_pair, (int*)tile_expert, (int*)tile_row0, (int*)tile_n, (int*)counters);
     LSB_CHECK_LAUNCH();
@@ -921,7 +930,7 @@ static int moe_tc_ffn(int gateup, const void* b, int cap_rows, const void* arena
     if (ef->fmt == 1 && (K % 128)) return -1;
     if (ef->fmt == 3 && (K % 256)) return -1;
     CUtensorMap mb;
-    int rc = cached_map_2d(&mb, b, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)cap_rows, (uint64_t)K, (uint64_t)K, (uint32_t)BN, kTBK);
+    int rc = cached_map_2d(&mb, b, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)cap_rows, (uint64_t)K, (uint64_t)K, BN > 128 ? 128u : (uint32_t)BN, kTBK);
     if (rc) return rc;
     MoeTcParams p;
     p.arena = (const uint8_t*)arena; p.slot_of = (const int*)slot_of; p.ef = *ef;
@@ -941,6 +950,7 @@ static int moe_tc_ffn(int gateup, const void* b, int cap_rows, const void* arena
             case 32: return launch_moe_tc<0, 32, true, kDirect>(mb, p, nout, max_tiles, st);
             case 64: return launch_moe_tc<0, 64, true, kDirect>(mb, p, nout, max_tiles, st);
             case 128: return launch_moe_tc<0, 128, true, kDirect>(mb, p, nout, max_tiles, st);
+            case 256: return launch_moe_tc<0, 256, true, kDirect>(mb, p, nout, max_tiles, st);
         }
     } else if (gateup == 1) {
         switch (BN) {
@@ -953,6 +963,7 @@ static int moe_tc_ffn(int gateup, const void* b, int cap_rows, const void* arena
             case 32: return dispatch_fmt<32, false>(ef->fmt, mb, p, nout, max_tiles, st);
             case 64: return dispatch_fmt<64, false>(ef->fmt, mb, p, nout, max_tiles, st);
             case 128: return dispatch_fmt<128, false>(ef->fmt, mb, p, nout, max_tiles, st);
+            case 256: if (ef->fmt == 0 && !ep) return launch_moe_tc<0, 256, false>(mb, p, nout, max_tiles, st);
         }
     }
     return -1;

@@ -568,18 +568,23 @@ class MoeBuffers:
     weight-streaming kernels and - with ``tc`` - the expert-sorted operands of the tensor-core grouped kernel."""
 
     @staticmethod
-    def tile_rows(P: int, E: int) -> int:
+    def tile_rows(P: int, E: int, direct: bool = False) -> int:
         """Rows per token tile for ``P`` pairs over ``E`` experts: the smallest tile that most experts' rows fit, since every tile converts its expert's weights
         anew (2048 rows x 9 of 289 NVFP4 experts of 4096 x 2048, gate/up: 920 us in tiles of 64, 1372 in 32, 1171 in 128), and a smaller one leaves tensor memory
-        for more weight stages (32 rows: 378 us in tiles of 32, 538 in 64)."""
+        for more weight stages (32 rows: 378 us in tiles of 32, 538 in 64).  ``direct``: gated bf16 experts, which convert nothing in front of half of their
+        products: tiles of 64 only for as many rows, and of 256 where most experts' rows fit them and not 128 (64 experts of 4096 x 2048, gate/up + down, tiles of
+        64, 128, 256: 56 pairs an expert 553, 558, -; 69 574, 562, -; 137 754, 645, 670; 169 938, 888, 776; 225 1148, 879, 812; 256 1222, 904, 875; 375 1729,
+        1275, 1545)."""
         avg = P / max(1, min(E, P))
+        if direct:
+            return 32 if avg <= 32 else (64 if avg <= 64 else (256 if 140 < avg <= 260 else 128))
         return 32 if avg <= 32 else (64 if avg <= 96 else 128)
 
-    def step_tiles(self, P: int, E: int) -> tuple:
+    def step_tiles(self, P: int, E: int, direct: bool = False) -> tuple:
         """(rows per tile, tiles at most) of a step of ``P`` pairs; the block-scaled operands are laid out for the workspace's own tiles, few rows take tiles of 32."""
         if self.bs_ok:
             return self.tc_bn, min(self.tc_tiles, P // self.tc_bn + E + 1)
-        bn = 32 if P < TC_MOE_MIN_ROWS * self.S else self.tile_rows(P, E)
+        bn = 32 if P < TC_MOE_MIN_ROWS * self.S else self.tile_rows(P, E, direct)
         return bn, P // bn + E + 1
 
     def alloc_moe(self, z, R: int, S: int, E: int, n_logits: int, H: int, F: int, tc: bool, act_dtype=torch.bfloat16):
@@ -804,7 +809,7 @@ class ModelBase:
         mode = self.moe_mode(arena, ws, R)
         if mode == "tc":
             P = R * S
-            bn, tiles = ws.step_tiles(P, E)
+            bn, tiles = ws.step_tiles(P, E, self._moe_direct(arena.ef))
             nat.call("lsb_moe_tc_sort", ws.ids, P, E, bn, ws.tc_sorted, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt)
             if ws.bs_ok:
                 nat.call("lsb_quant_fp8_tiles" if ws.bs_fp8 else "lsb_quant_nvfp4_tiles", x, 0, ws.tc_sorted, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt,
@@ -825,7 +830,7 @@ class ModelBase:
         if mode == "tc":
             P = R * S
             err = TcScratch.get(self.device).err
-            bn, tiles = ws.step_tiles(P, E)
+            bn, tiles = ws.step_tiles(P, E, self._moe_direct(arena.ef))
             if ws.bs_ok and ws.bs_fp8:
                 wsf, og, ou, od = arena.bs_scale_atoms()
                 a = (arena.data, arena.slot_of, efp, wsf, wsf.shape[1], og, ou, od, ws.tc_tile_e, ws.tc_tile_r0, ws.tc_tile_n, ws.tc_cnt, ws.tc_sorted)

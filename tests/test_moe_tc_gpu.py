@@ -486,3 +486,36 @@ def test_tiles_of_every_number_of_rows(fmt, BN, copies):
         # hidden values in fp16 (2^-11 each at most), bf16 weights converted to fp16 (the same); Q4_K weights are a scale times 0 .. 15 less an offset, both rounded
         # to fp16: 2^-11 of up to 15 steps where the weights' rms is 4.3 of them, 1.7e-3, in each of the three matrices
         assert float((y[r].double() - want).norm() / want.norm()) < (3 ** 0.5 * 1.7e-3 if fmt == "gguf_q4_k" else 1e-3), (e, counts[e])
+
+
+@pytest.mark.parametrize("H,F", [(1024, 768), (128, 256)])
+def test_bf16_experts_in_tiles_of_256_rows(H, F):
+    """Gate/up over bf16 rows and down over fp16 hidden values in tiles of up to 256 rows: tiles of one and of two boxes of 128 side by side, whole, ragged and
+    behind a full one; several tiles per thread block."""
+    from layerstorm_b200.ops import _native as nat
+    dev, BN, copies = torch.device("cuda"), 256, 6
+    counts = [1, 127, 128, 129, 255, 256, 257, 300, 512, 513]
+    E = len(counts)
+    arena, ref = _setup("bf16", H, F, E, n_missing=0, seed=10)
+    arena.slot_of = arena.slot_of.repeat(copies)
+    g = torch.Generator(device="cpu").manual_seed(11)
+    ids = torch.cat([torch.full((n,), e + E * c) for c in range(copies) for e, n in enumerate(counts)])
+    ids = ids[torch.randperm(len(ids), generator=g)].int()
+    P = len(ids)
+    x, tiles = torch.randn(P, H, generator=g).to(torch.bfloat16).to(dev), P // BN + E * copies + 1
+    i32 = dict(dtype=torch.int32, device=dev)
+    srt, te, tr, tn, cnt, err, miss = (torch.zeros(n, **i32) for n in (P, tiles, tiles, tiles, 2, 1, 1))
+    xs, act = torch.zeros(P, H, dtype=torch.bfloat16, device=dev), torch.zeros(P + 1, F, dtype=torch.float16, device=dev)
+    y, efp = torch.zeros(P + 1, H, device=dev), ctypes.addressof(arena.ef)
+    nat.call("lsb_moe_tc_sort", ids.to(dev), P, E * copies, BN, srt, te, tr, tn, cnt)
+    nat.call("lsb_moe_tc_gather_bf16", x, srt, cnt, xs, P, 1, H)
+    nat.call("lsb_moe_tc_gateup_bf16", xs, P, arena.data, arena.slot_of, efp, te, tr, tn, cnt, srt, act, BN, tiles, 0.0, 1.0, 0.0, None, miss, err)
+    nat.call("lsb_moe_tc_ffn", 0, act, P, arena.data, arena.slot_of, efp, te, tr, tn, cnt, srt, y, BN, tiles, 0.0, None, err, None)
+    torch.cuda.synchronize()
+    assert int(err) == 0 and float(act[P].abs().sum()) == 0.0 and float(y[P].abs().sum()) == 0.0
+    for e in range(E):
+        r = (ids % E == e).nonzero()[:, 0].to(dev)
+        gate, up, down = (m.to(dev) for m in ref[e])
+        xd = x[r].double()
+        want = (torch.nn.functional.silu(xd @ gate.T) * (xd @ up.T)) @ down.T
+        assert float((y[r].double() - want).norm() / want.norm()) < 1e-3, counts[e]          # hidden values and down weights in fp16 (2^-11 each at most)
