@@ -605,6 +605,58 @@ __global__ void __launch_bounds__(RPB * 32, 1) mhc_rows_kernel(bf16* __restrict_
 constexpr int kHcGram = kHcMax * (kHcMax + 1) / 2;         // 10
 constexpr int kHcPart2 = kHcOut + kHcGram + 2;             // 36 floats per (row, chunk)
 
+// A row's gates from its logits and Gram sums in `mix` (shared memory), by one warp (lane t): mixing matrix, gates, norm of the contracted vector.
+__device__ __forceinline__ void hc_row_gates(const float* mix, int t, int r, float* __restrict__ post, float* __restrict__ comb, const float* __restrict__ hc_scale,
+                                             const float* __restrict__ hc_base, unsigned* __restrict__ done, float* __restrict__ prex, int hidden, int n, int iters,
+                                             float hc_eps, float rms_eps, float post_mult) {
+    // sum of squares of the residual streams = trace of the Gram matrix (diagonal entries 0, 4, 7, 9 for n = 4)
+    float tr = 0.f;
+    { int e = 0; for (int j = 0; j < kHcMax; ++j) for (int k = j; k < kHcMax; ++k, ++e) if (k == j && j < n) tr += mix[kHcOut + e]; }
+    const float inv = rsqrtf(tr / (float)(n * hidden) + rms_eps);
+    float cm = 0.f;
+    const int i = (t & 15) >> 2, j = t & 3;
+    const bool valid = t < 16 && i < n && j < n;
+    {
+        float v = valid ? mix[2 * n + i * n + j] * inv * hc_scale[2] + hc_base[2 * n + i * n + j] : -INFINITY;
+        float mx = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        float e = valid ? expf(v - mx) : 0.f;
+        float sm = e + __shfl_xor_sync(0xffffffffu, e, 1);
+        sm += __shfl_xor_sync(0xffffffffu, sm, 2);
+        cm = valid ? e / sm + hc_eps : 0.f;
+        float cs = cm + __shfl_xor_sync(0xffffffffu, cm, 4);
+        cs += __shfl_xor_sync(0xffffffffu, cs, 8);
+        cm = valid ? cm / (cs + hc_eps) : 0.f;
+        for (int it = 1; it < iters; ++it) {
+            float rs = cm + __shfl_xor_sync(0xffffffffu, cm, 1);
+            rs += __shfl_xor_sync(0xffffffffu, rs, 2);
+            cm = valid ? cm / (rs + hc_eps) : 0.f;
+            cs = cm + __shfl_xor_sync(0xffffffffu, cm, 4);
+            cs += __shfl_xor_sync(0xffffffffu, cs, 8);
+            cm = valid ? cm / (cs + hc_eps) : 0.f;
+        }
+    }
+    if (valid) comb[(r * n + i) * n + j] = cm;
+    // pre gates on lanes 16..19, post gates on lanes 20..23
+    float pre_v = 0.f;
+    if (t >= 16 && t < 16 + kHcMax && t - 16 < n) pre_v = sigmoidf_(mix[t - 16] * inv * hc_scale[0] + hc_base[t - 16]) + hc_eps;
+    if (t >= 20 && t < 20 + kHcMax && t - 20 < n) post[r * n + (t - 20)] = sigmoidf_(mix[n + t - 20] * inv * hc_scale[1] + hc_base[n + t - 20]) * post_mult;
+    float pj[kHcMax];
+#pragma unroll
+    for (int q = 0; q < kHcMax; ++q) pj[q] = __shfl_sync(0xffffffffu, pre_v, 16 + q);
+    if (t == 0) {
+        float quad = 0.f;
+        int e = 0;
+        for (int a = 0; a < kHcMax; ++a)
+            for (int b = a; b < kHcMax; ++b, ++e) quad += (a == b ? 1.f : 2.f) * pj[a] * pj[b] * mix[kHcOut + e];
+        float* px = prex + (size_t)r * 8;
+#pragma unroll
+        for (int q = 0; q < kHcMax; ++q) px[q] = pj[q];
+        px[4] = rsqrtf(fmaxf(quad, 0.f) / (float)hidden + rms_eps);
+        done[r] = 0;
+    }
+}
+
 __global__ void __launch_bounds__(128) mhc_post_fused_kernel(float* __restrict__ residual, const float* __restrict__ x,
                                                              float* __restrict__ post, float* __restrict__ comb,
                                                              const float* __restrict__ fn, const float* __restrict__ hc_scale,
@@ -700,54 +752,128 @@ __global__ void __launch_bounds__(128) mhc_post_fused_kernel(float* __restrict__
         mix[t] = a;
     }
     __syncthreads();
-    if (t < 32) {
-        // sum of squares of the residual streams = trace of the Gram matrix (diagonal entries 0, 4, 7, 9 for n = 4)
-        float tr = 0.f;
-        { int e = 0; for (int j = 0; j < kHcMax; ++j) for (int k = j; k < kHcMax; ++k, ++e) if (k == j && j < n) tr += mix[kHcOut + e]; }
-        const float inv = rsqrtf(tr / (float)(n * hidden) + rms_eps);
-        float cm = 0.f;
-        const int i = (t & 15) >> 2, j = t & 3;
-        const bool valid = t < 16 && i < n && j < n;
+    if (t < 32) hc_row_gates(mix, t, r, post, comb, hc_scale, hc_base, done, prex, hidden, n, iters, hc_eps, rms_eps, post_mult);
+}
+
+// The same for four streams on one GPU: 128 columns per block, four a lane, and `per` rows one after another, so that `fn` is read per block and not per row, the
+// loads of a row are under way while the one before is worked on, and the last block of a row adds up 32 partials (of 4096 columns) and not 128.  Nine sums a row
+// and warp go through one exchange of halves.
+constexpr int kHfCols = 128, kHfRows = 8;
+__global__ void __launch_bounds__(128, 3) mhc_post_few_kernel(float* __restrict__ residual, const float* __restrict__ x, float* __restrict__ post,
+                                                              float* __restrict__ comb, const float* __restrict__ fn, const float* __restrict__ hc_scale,
+                                                              const float* __restrict__ hc_base, float* __restrict__ part, unsigned* __restrict__ done,
+                                                              float* __restrict__ prex, int rows, int per, int hidden, int mode, int iters, float hc_eps,
+                                                              float rms_eps, float post_mult) {
+    constexpr int N = kHcMax;
+    __shared__ float mix[4][kHcPart2];
+    __shared__ int s_last[kHfRows];
+    const int c = blockIdx.x, nch = gridDim.x, t = threadIdx.x, lane = t & 31, og = t >> 5, r0 = blockIdx.y * per, nr = min(per, rows - r0);
+    const int h = c * kHfCols + lane * 4;
+    float4 f[kHcPerWarp][N];
+#pragma unroll
+    for (int i = 0; i < kHcPerWarp; ++i)
+#pragma unroll
+        for (int j = 0; j < N; ++j) f[i][j] = __ldg(reinterpret_cast<const float4*>(fn + ((size_t)(og * kHcPerWarp + i) * N + j) * hidden + h));
+    pdl_wait();
+    pdl_launch_dependents();
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 xv = z4, old[N];
+    auto load = [&](int r) {
+        xv = *reinterpret_cast<const float4*>(x + (size_t)r * hidden + h);
+#pragma unroll
+        for (int i = 0; i < N; ++i) old[i] = mode ? *reinterpret_cast<const float4*>(residual + ((size_t)r * N + i) * hidden + h) : z4;
+    };
+    load(r0);
+#pragma unroll 1
+    for (int k = 0; k < nr; ++k) {
+        const int r = r0 + k;
+        float4 res[N];
+        float pj[N], cj[N][N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            pj[j] = mode ? post[r * N + j] : 1.f;                      // mode 0: every stream starts as x
+#pragma unroll
+            for (int i = 0; i < N; ++i) cj[i][j] = mode ? comb[(r * N + i) * N + j] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            float4 a = make_float4(pj[j] * xv.x, pj[j] * xv.y, pj[j] * xv.z, pj[j] * xv.w);
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                a.x += cj[i][j] * old[i].x; a.y += cj[i][j] * old[i].y; a.z += cj[i][j] * old[i].z; a.w += cj[i][j] * old[i].w;
+            }
+            res[j] = a;
+        }
+        if (k + 1 < nr) load(r + 1);
+        auto dot = [](const float4& a, const float4& b, float s) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, s)))); };
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < kHcPerWarp; ++i) {
+            float a = 0.f;
+#pragma unroll
+            for (int j = 0; j < N; ++j) a = dot(res[j], f[i][j], a);
+            v[i] = a;
+        }
+        // Gram entries og, 4 + og, 8 + og of the ten (j <= j')
+        float g[12];
         {
-            float v = valid ? mix[2 * n + i * n + j] * inv * hc_scale[2] + hc_base[2 * n + i * n + j] : -INFINITY;
-            float mx = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            float e = valid ? expf(v - mx) : 0.f;
-            float sm = e + __shfl_xor_sync(0xffffffffu, e, 1);
-            sm += __shfl_xor_sync(0xffffffffu, sm, 2);
-            cm = valid ? e / sm + hc_eps : 0.f;
-            float cs = cm + __shfl_xor_sync(0xffffffffu, cm, 4);
-            cs += __shfl_xor_sync(0xffffffffu, cs, 8);
-            cm = valid ? cm / (cs + hc_eps) : 0.f;
-            for (int it = 1; it < iters; ++it) {
-                float rs = cm + __shfl_xor_sync(0xffffffffu, cm, 1);
-                rs += __shfl_xor_sync(0xffffffffu, rs, 2);
-                cm = valid ? cm / (rs + hc_eps) : 0.f;
-                cs = cm + __shfl_xor_sync(0xffffffffu, cm, 4);
-                cs += __shfl_xor_sync(0xffffffffu, cs, 8);
-                cm = valid ? cm / (cs + hc_eps) : 0.f;
+            int e = 0;
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+#pragma unroll
+                for (int q = j; q < N; ++q, ++e) g[e] = dot(res[j], res[q], 0.f);
+            g[10] = g[11] = 0.f;
+        }
+#pragma unroll
+        for (int m = 0; m < 3; ++m) v[kHcPerWarp + m] = og == 0 ? g[4 * m] : (og == 1 ? g[4 * m + 1] : (og == 2 ? g[4 * m + 2] : g[4 * m + 3]));
+#pragma unroll
+        for (int i = 9; i < 16; ++i) v[i] = 0.f;
+        // sums over the lanes by exchanging halves: lane l ends with sum l % 16
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int i = 0; i < o; ++i) {
+                const float send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
         }
-        if (valid) comb[(r * n + i) * n + j] = cm;
-        // pre gates on lanes 16..19, post gates on lanes 20..23
-        float pre_v = 0.f;
-        if (t >= 16 && t < 16 + kHcMax && t - 16 < n) pre_v = sigmoidf_(mix[t - 16] * inv * hc_scale[0] + hc_base[t - 16]) + hc_eps;
-        if (t >= 20 && t < 20 + kHcMax && t - 20 < n) post[r * n + (t - 20)] = sigmoidf_(mix[n + t - 20] * inv * hc_scale[1] + hc_base[n + t - 20]) * post_mult;
-        float pj[kHcMax];
-#pragma unroll
-        for (int q = 0; q < kHcMax; ++q) pj[q] = __shfl_sync(0xffffffffu, pre_v, 16 + q);
-        if (t == 0) {
-            float quad = 0.f;
-            int e = 0;
-            for (int a = 0; a < kHcMax; ++a)
-                for (int b = a; b < kHcMax; ++b, ++e) quad += (a == b ? 1.f : 2.f) * pj[a] * pj[b] * mix[kHcOut + e];
-            float* px = prex + (size_t)r * 8;
-#pragma unroll
-            for (int q = 0; q < kHcMax; ++q) px[q] = pj[q];
-            px[4] = rsqrtf(fmaxf(quad, 0.f) / (float)hidden + rms_eps);
-            done[r] = 0;
-        }
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
+        float* po = part + ((size_t)r * nch + c) * kHcPart2;
+        if (lane < kHcPerWarp) po[og * kHcPerWarp + lane] = v[0];
+        else if (lane < 9 && (lane - kHcPerWarp) * 4 + og < kHcGram) po[kHcOut + (lane - kHcPerWarp) * 4 + og] = v[0];
+        __syncthreads();                              // every warp has read the old streams (updated in place, a stream a warp)
+        const float4 mine = og == 0 ? res[0] : (og == 1 ? res[1] : (og == 2 ? res[2] : res[3]));
+        *reinterpret_cast<float4*>(residual + ((size_t)r * N + og) * hidden + h) = mine;
     }
+    // ---- the last block of a row finishes it, a warp a row ----
+    __threadfence();
+    __syncthreads();
+    if (t < nr) s_last[t] = atomicAdd(done + r0 + t, 1u) == (unsigned)(nch - 1);
+    __syncthreads();
+    for (int k = og; k < nr; k += 4) {
+        if (!s_last[k]) continue;                     // (the same for the warp)
+        __threadfence();
+        const int r = r0 + k;
+        const float* p = part + (size_t)r * nch * kHcPart2;
+        float a = 0.f, b = 0.f;
+        for (int c0 = 0; c0 < nch; c0 += 16) {
+            float v[16], w[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                v[u] = c0 + u < nch ? __ldcg(p + (size_t)(c0 + u) * kHcPart2 + lane) : 0.f;
+                w[u] = c0 + u < nch && lane < 2 ? __ldcg(p + (size_t)(c0 + u) * kHcPart2 + 32 + lane) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 16; ++u) { a += v[u]; b += w[u]; }
+        }
+        mix[og][lane] = a;
+        if (lane < 2) mix[og][32 + lane] = b;
+        __syncwarp();
+        hc_row_gates(mix[og], lane, r, post, comb, hc_scale, hc_base, done, prex, hidden, N, iters, hc_eps, rms_eps, post_mult);
+        __syncwarp();
+    }
+    pdl_launch_dependents();
 }
 
 __global__ void __launch_bounds__(256) mhc_contract_kernel(bf16* __restrict__ out, const float* __restrict__ residual, const float* __restrict__ prex,
@@ -964,12 +1090,25 @@ LSB_API int lsb_mhc_post_pre(void* out_x, void* residual, const void* x, void* p
     if (hidden % kHcChunk || n > kHcMax) return -1;
     cudaStream_t st = (cudaStream_t)stream;
     const int nchunks = hidden / kHcChunk;
-    if (done && prex && rows < 64 && hidden % 4 == 0) {
+    // part must hold rows * nchunks * 36 floats, done rows zero-initialised counters, prex rows * 8 floats
+    const bool few = done && prex && !comm && n == kHcMax && hidden % kHfCols == 0 && (((uintptr_t)fn | (uintptr_t)x | (uintptr_t)residual) & 15) == 0;
+    // Up to 351 rows of 4 x 4096, us: the kernels of few rows / with a block per 32 columns and row 9 rows 11.6 / 18.4, 32 14.1 / 32.3, 63 23.6 / 51.5; / partials by
+    // 16 rows and a block per row to finish 64 23.7 / 29.5, 96 28.0 / 30.2, 128 36.9 / 30.5, 192 38.3 / 49.9, 256 48.6 / 50.1, 350 58.2 / 77.9; whole rows by block 391
+    // 61.  Of 4 x 7168 32 rows 24.5 / 49.2, 350 84 / 134.
+    if (done && prex && hidden % 4 == 0 && (rows < 64 || (few && (rows <= 96 || (rows >= 160 && rows < 352))))) {
         // few rows: partials + finalize in one launch (last block per row), then a fully parallel contraction.
-        // part must hold rows * nchunks * 36 floats, done rows zero-initialised counters, prex rows * 8 floats.
-        launch_pdl((mhc_post_fused_kernel), dim3(rows, nchunks), 128, 0, st, (float*)residual, (const float*)x, (float*)post, (float*)comb,
-                   (const float*)fn, (const float*)hc_scale, (const float*)hc_base, (float*)part, (unsigned*)done, (float*)prex, hidden, n, mode,
-                   iters, hc_eps, rms_eps, post_mult, comm_from_host(comm));
+        if (few) {
+            // as many rows a block as make one wave of three blocks an SM, up to 8
+            const int nch = hidden / kHfCols;
+            int per = (rows * nch + 443) / 444;
+            per = per < 1 ? 1 : (per > kHfRows ? kHfRows : per);
+            launch_pdl((mhc_post_few_kernel), dim3(nch, (rows + per - 1) / per), 128, 0, st, (float*)residual, (const float*)x, (float*)post, (float*)comb, (const float*)fn,
+                       (const float*)hc_scale, (const float*)hc_base, (float*)part, (unsigned*)done, (float*)prex, rows, per, hidden, mode, iters, hc_eps, rms_eps, post_mult);
+        } else {
+            launch_pdl((mhc_post_fused_kernel), dim3(rows, nchunks), 128, 0, st, (float*)residual, (const float*)x, (float*)post, (float*)comb, (const float*)fn,
+                       (const float*)hc_scale, (const float*)hc_base, (float*)part, (unsigned*)done, (float*)prex, hidden, n, mode, iters, hc_eps, rms_eps, post_mult,
+                       comm_from_host(comm));
+        }
         launch_pdl((mhc_contract_kernel), dim3(rows, (hidden / 4 + 255) / 256), 256, 0, st, (bf16*)out_x, (const float*)residual, (const float*)prex,
                    (const float*)norm_w, hidden, n);
         LSB_CHECK_LAUNCH();

@@ -146,7 +146,8 @@ MOE_BLOCK_SCALED = os.environ.get("LSB_MOE_BLOCK_SCALED", "0") not in ("", "0")
 # LSB_MHC_CLUSTER=0: decode-sized hyper-connection passes fall back to the two-launch path (partials + last-block finalize, contraction)
 MHC_CLUSTER = os.environ.get("LSB_MHC_CLUSTER", "1") not in ("", "0")
 # rows of a step up to which the cluster kernel (one cluster per row) is used; above it the partial + last-block-finalize kernels, which
-# tile better over many rows (32 rows on a B200: 32.6 us per pass against 55.2 us for 32 clusters)
+# tile better over many rows (32 rows of 4 x 4096 on a B200: 14 us per pass against 55 us for 32 clusters).  On one GPU up to five rows: clusters of more
+# come in two waves (5 rows 11.2 us against 10.8, 8 rows 21.5 / 11.3)
 MHC_CLUSTER_MAX_ROWS = int(os.environ.get("LSB_MHC_CLUSTER_MAX_ROWS", "8"))
 # ablation switches of the two folds of the cluster kernel (router behind, MoE combine in front)
 MHC_FOLD_ROUTER = os.environ.get("LSB_MHC_FOLD_ROUTER", "0") not in ("", "0")
@@ -1601,7 +1602,7 @@ class DeviceModel(ModelBase):
         if cfg.mhc:
             nat.call("lsb_embedding", ws.sub, None, self.embed, ws.tok, R, H, 0, cfg.vocab)
             # decode-sized steps: one cluster kernel per post -> pre pass, with the MoE combine folded in front and the router behind
-            clus = R <= MHC_CLUSTER_MAX_ROWS and self._mhc_cluster_ok()
+            clus = R <= (MHC_CLUSTER_MAX_ROWS if self.comm is not None else min(5, MHC_CLUSTER_MAX_ROWS)) and self._mhc_cluster_ok()
             pending = None         # slot table of the MoE layer whose combine the next pass performs
             last_run = -1
             for i, L in enumerate(self.layers):

@@ -800,3 +800,33 @@ def test_fp8_experts_of_few_rows(H, F, R):
         assert float((act[p].double() - want).norm() / want.norm()) < 3e-3          # rounded to bf16 (2^-9)
         want = down @ act[p].double()
         assert float((y[p].double() - want).norm() / want.norm()) < 5e-7            # products exact, fp32 sums
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 9, 14, 27, 63, 64, 96, 97, 160, 351])
+@pytest.mark.parametrize("H", [128, 1152, 4096])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_hyper_connection_passes_of_few_rows(rows, H, mode):
+    """One to eight rows a block, a last block of fewer, one and several blocks of columns, both sides of the lines; twice, as the counters of a row start over."""
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, res0, fn, base, nw = rnd(rows, H), rnd(rows, 4, H), rnd(24, 4 * H) * (0.3 / H ** 0.5), rnd(24) * 0.5, 1 + 0.1 * rnd(H)
+    scale, post0, comb0 = torch.tensor([0.7, 1.1, 1.3], device="cuda"), torch.rand(rows, 4, generator=g, device="cuda"), torch.rand(rows, 4, 4, generator=g, device="cuda") / 4
+    want_r = torch.einsum("tij,tih->tjh", comb0.double(), res0.double()) + post0.double()[:, :, None] * x.double()[:, None] if mode else x.double()[:, None].repeat(1, 4, 1)
+    flat = want_r.flatten(1)
+    m = (flat @ fn.double().T) * torch.rsqrt(flat.square().mean(-1, keepdim=True) + 1e-5)
+    m = m * scale.double().repeat_interleave(torch.tensor([4, 4, 16], device="cuda")) + base.double()
+    k = torch.softmax(m[:, 8:].view(-1, 4, 4), -1) + 1e-6
+    k = k / (k.sum(-2, keepdim=True) + 1e-6)
+    for _ in range(19):
+        k = k / (k.sum(-1, keepdim=True) + 1e-6)
+        k = k / (k.sum(-2, keepdim=True) + 1e-6)
+    o = ((torch.sigmoid(m[:, :4]) + 1e-6)[:, :, None] * want_r).sum(1)
+    o = o * torch.rsqrt(o.square().mean(-1, keepdim=True) + 1e-5) * nw.double()
+    part, done, pre = torch.zeros(rows, max(H // 32, 1), 36, device="cuda"), torch.zeros(rows, dtype=torch.int32, device="cuda"), torch.zeros(rows, 8, device="cuda")
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm())
+    for _ in range(2):
+        out, res, post, comb = torch.zeros(rows, H, dtype=torch.bfloat16, device="cuda"), res0.clone(), post0.clone(), comb0.clone()
+        nat.call("lsb_mhc_post_pre", out, res, x, post, comb, fn, scale, base, nw, part, rows, H, 4, mode, 20, 1e-6, 1e-5, 2.0, done, pre, None)
+        # fp32 sums of up to 16384 products in runs of a few hundred: 2^-24 sqrt(16384) = 8e-6 at most; the output is rounded to bf16 (2^-9 at most)
+        assert rel(res, want_r) < 1e-6 and rel(post, torch.sigmoid(m[:, 4:8]) * 2) < 1e-5 and rel(comb, k) < 1e-5 and rel(out, o) < 3e-3
+        assert int(done.abs().sum()) == 0
