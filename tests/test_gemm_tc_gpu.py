@@ -166,3 +166,23 @@ def test_bf16_linear_of_few_rows(M, N, K, monkeypatch):
         want = x.double() @ lin.w.double().T
         assert float((out.double() - want).norm() / want.norm()) < (1e-5 if dt == torch.float32 else 3e-3)
     assert called == ["lsb_gemm_bf16_tc" if M >= (5 if N == 1040 else 7) else "lsb_gemv_bf16"] * 2
+
+
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 16, 17, 31, 33])
+@pytest.mark.parametrize("B,N,K,dr", [(5, 512, 128, 64), (3, 72, 512, 0), (16, 128, 8, 8), (2, 40, 264, 0)])
+def test_products_per_head_of_any_number_of_rows(M, B, N, K, dr):
+    """Per-head products of few and many rows with and without rotated tails; rows and heads of other tensors between them stay as they are."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w = torch.randn(M, B, K + dr, generator=g, device="cuda").bfloat16(), torch.randn(B, N, K, generator=g, device="cuda").bfloat16()
+    inv, pos = torch.rand(max(dr // 2, 1), generator=g, device="cuda"), torch.randint(0, 5000, (M,), generator=g, device="cuda", dtype=torch.int32)
+    out = torch.full((M + 1, B, N + dr + 8), 3.0, device="cuda", dtype=torch.bfloat16)
+    nat.call("lsb_batched_gemv_bf16", out, x, w, M, B, N, K, B * (K + dr), K + dr, B * (N + dr + 8), N + dr + 8, dr, inv if dr else None, pos)
+    want = torch.einsum("mbk,bnk->mbn", x[..., :K].double(), w.double())
+    assert float((out[:M, :, :N].double() - want).norm() / want.norm()) < 3e-3          # fp32 sums rounded to bf16 (2^-9)
+    assert bool((out[M:] == 3.0).all()) and bool((out[:, :, N + dr:] == 3.0).all())
+    if dr:
+        a = pos.double()[:, None, None] * inv.double()
+        e, o = x[..., K::2].double(), x[..., K + 1::2].double()
+        tail = torch.stack((e * a.cos() - o * a.sin(), e * a.sin() + o * a.cos()), -1).flatten(-2)
+        # angles of up to 5000 in fp32 (5000 x 2^-24 = 3e-4) and rounding to bf16 (2^-9)
+        assert float((out[:M, :, N: N + dr].double() - tail).norm() / tail.norm()) < 3e-3
