@@ -13,6 +13,7 @@
 // This replaces the reference's CUDA-core tiled GEMM (src/compute/kernels/sm120/gemm/bf16_gemm.cu:156)
 // and the external FP8 GEMM launcher (G/sm120/gemm/fp8/fp8_gemm.h) for every M > 4.
 #include "tc_common.cuh"
+#include "bf16_rows.cuh"
 #include "comm.cuh"
 
 #include <map>
@@ -413,11 +414,21 @@ LSB_API int lsb_gemm_tc_workspace_floats(int M, int N, int K) {
 // x bf16 [M, ldx], w bf16 [N, ldw], out fp32/bf16 [M, ldo]; K % 8 == 0; ldx, ldw % 8 == 0; pointers 16-byte aligned.
 // partial: fp32 scratch of partial_cap floats (split-K is limited to what fits) or null to disable split-K.
 // err: int error word (0 = ok; 1-3 = a bounded pipeline wait gave up).
+// out_bf16: 1 = bf16 output, + 2 = no kernel that may still run writes w, so that few-row products ask for their weights before they wait for the kernel in front
+// (weights of a model; 1 to 2 us per product).
 LSB_API int lsb_gemm_bf16_tc(void* out, const void* x, const void* w, const void* bias, int M, int N, int K, int ldx, int ldw,
                              int ldo, int out_bf16, void* partial, long long partial_cap, void* err, const void* comm, void* stream) {
+    const int steady = (out_bf16 >> 1) & 1;
+    out_bf16 &= 1;
     if (K % 8 || ldx % 8 || ldw % 8 || ((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return -1;
     if (comm) { partial = nullptr; if (out_bf16 || bias || (long long)M * ldo > ((const PeerComm*)comm)->cap) return -1; }
     cudaStream_t st = (cudaStream_t)stream;
+    if (!comm && bf16_rows_ok(M, N, K, ldx, ldw, x, w)) {
+        Bf16RowsArgs a{};
+        a.x = (const bf16*)x; a.ldx = ldx; a.w = (const bf16*)w; a.ldw = ldw; a.out = out; a.ldo = ldo; a.out_bf16 = out_bf16;
+        a.bias = (const float*)bias; a.M = M; a.N = N; a.K = K; a.steady = steady;
+        return bf16_rows_launch(a, st);
+    }
     int BN = 16;
     while (BN < 256 && BN < M) BN <<= 1;
     CUtensorMap mw, mx;

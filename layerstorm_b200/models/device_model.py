@@ -389,7 +389,7 @@ class QLinear:
             nat.call("lsb_gemm_f32", out, x, self.w, M, self.N, self.K, ldx, self.K, ldo)
         elif self.fmt == "bf16" and M >= (TC_GEMM_MIN_ROWS if self.N * self.K > TC_GEMM_SMALL else TC_GEMM_MIN_ROWS_SMALL):
             sc = TcScratch.get(self.w.device)
-            nat.call("lsb_gemm_bf16_tc", out, x, self.w, bias, M, self.N, self.K, ldx, self.K, ldo, ob, sc.partial, sc.cap, sc.err, comm)
+            nat.call("lsb_gemm_bf16_tc", out, x, self.w, bias, M, self.N, self.K, ldx, self.K, ldo, ob | 2, sc.partial, sc.cap, sc.err, comm)
         elif (self.fmt == "nvfp4" and MOE_BLOCK_SCALED and M >= 16 and comm is None and bias is None and ldx == self.K and self.K % 256 == 0
               and self.K <= 8192 and self.N % 128 == 0):
             # many rows over NVFP4 weights, block-scaled mode: the rows are quantised to NVFP4 and both operands stay 4-bit

@@ -186,3 +186,26 @@ def test_products_per_head_of_any_number_of_rows(M, B, N, K, dr):
         tail = torch.stack((e * a.cos() - o * a.sin(), e * a.sin() + o * a.cos()), -1).flatten(-2)
         # angles of up to 5000 in fp32 (5000 x 2^-24 = 3e-4) and rounding to bf16 (2^-9)
         assert float((out[:M, :, N: N + dr].double() - tail).norm() / tail.norm()) < 3e-3
+
+
+@pytest.mark.parametrize("M", [1, 5, 8, 9, 16, 17])
+@pytest.mark.parametrize("N,K", [(16, 64), (144, 448), (2320, 1536), (1040, 512), (576, 4096), (4752, 7168), (8192, 4096), (130, 512)])
+def test_few_rows_of_bf16_weights(M, N, K):
+    """Few-row form and, behind its limits, the tiles: both against 64 bits; rows with padding between them, bias, weights asked for early or late.
+
+    A sum of K products in fp32, each rounded once, is off at most K 2^-24 times the sum of the absolute products; the bf16 output by half a unit more.
+    """
+    g = torch.Generator().manual_seed(M * 1000 + N)
+    x = torch.randn(M, K + 8, generator=g).bfloat16().cuda()
+    w = torch.randn(N, K + 16, generator=g).bfloat16().cuda()
+    bias = torch.randn(N, generator=g).cuda()
+    err, part = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(16 * M * N, device="cuda")
+    xd, wd = x[:, :K].double(), w[:, :K].double()
+    want, size = xd @ wd.T + bias.double(), xd.abs() @ wd.abs().T + bias.double().abs()
+    for flag, dt in [(0, torch.float32), (2, torch.float32), (1, torch.bfloat16), (3, torch.bfloat16)]:
+        out = torch.full((M, N + 24), 7.0, device="cuda", dtype=dt)
+        nat.call("lsb_gemm_bf16_tc", out, x, w, bias, M, N, K, K + 8, K + 16, N + 24, flag, part, part.numel(), err, None)
+        bound = (K + 2) * 2.0 ** -24 * size + (want.abs() * 2.0 ** -8 if dt == torch.bfloat16 else 0)
+        assert bool(((out[:, :N].double() - want).abs() <= bound).all())
+        assert bool((out[:, N:] == 7).all())
+    assert int(err) == 0
