@@ -1,4 +1,4 @@
-// Five to sixteen rows over a large bf16 matrix: the scheme of fp8_rows.cuh without conversions.
+// Five to sixteen rows over a bf16 matrix: the scheme of fp8_rows.cuh without conversions.
 //
 // A warp owns 16 weight rows and every kw-th block of 64 reduction elements; a thread's 16-byte pieces, copied into a ring in shared memory and read by the thread that
 // copied them, are its fragments of four mma.sync (m16n8k16, fp32 sums) when the reduction is taken in another order (thread c of a row's four: elements

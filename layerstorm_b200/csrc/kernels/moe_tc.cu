@@ -979,7 +979,7 @@ LSB_API int lsb_moe_tc_ffn(int gateup, const void* b, int cap_rows, const void* 
 
 // The gate/up half over bf16 experts and bf16 token rows (lsb_moe_tc_gather_bf16): both go to the tensor core as they are, which is exact where the other
 // form rounds weights outside fp16's normal range, and needs no converters.  1500 rows x top-8 of 64 experts of 4096 x 2048: 832 us through the converters,
-// 505 us so (bound by shared memory: 112 KB of operands read and written per 64 elements, 875 cycles beside 512 of MMA).
+// 505 us so in tiles of 128 (bound by shared memory: 112 KB of operands read and written per 64 elements, 875 cycles beside 512 of MMA), 424 in tiles of 256.
 LSB_API int lsb_moe_tc_gateup_bf16(const void* b, int cap_rows, const void* arena, const void* slot_of, const void* fmt_struct,
                                    const void* tile_expert, const void* tile_row0, const void* tile_n, const void* counters,
                                    const void* sorted_pair, void* out, int BN, int max_tiles, float limit, float alpha, float shift, const void* in_scale,
