@@ -119,7 +119,7 @@ TC_MOE_MIN_ROWS = 16
 TC_MOE_BF16_ROWS, TC_MOE_BF16_BYTES = 3, 500e6
 # rows from which a bf16 matrix runs on the tensor-core GEMM: above four rows the weight-streaming kernel reads the matrix twice, above six three times.  Streaming
 # against GEMM, us: 5 rows of 24896 x 4096 101 / 52, of 1536 x 4096 10.6 / 9.6; but a small matrix is in L2 the second time, and the GEMM is two launches: 5 rows
-# of 72 x 4096 5.8 / 7.4, of 1024 x 4096 7.9 / 8.7, of 2048 x 2048 8.1 / 8.2, of 4096 x 512 6.1 / 7.0; 7 rows of those 7.8 / 7.8, 10.9 / 9.0, 11.2 / 8.4, 9.1 / 7.2
+# of 72 x 4096 5.8 / 7.4, 7 rows 7.8 / 7.8.  (Both entries take the mma.sync form of few rows where it is the faster one, bf16_rows_ok.)
 TC_GEMM_MIN_ROWS, TC_GEMM_MIN_ROWS_SMALL, TC_GEMM_SMALL = 5, 7, 4 << 20
 # router projection + top-k in one launch for decode-sized steps (switch: LSB_ROUTER_FUSED=1).  Off by default: measured on the
 # GLM-5.3-Flash shape the fused kernel (one block per expert, last block selects) gives 7.21 ms per decode step against 7.12 ms for
@@ -571,8 +571,9 @@ class MoeBuffers:
     @staticmethod
     def tile_rows(P: int, E: int, direct: bool = False) -> int:
         """Rows per token tile for ``P`` pairs over ``E`` experts: the smallest tile that most experts' rows fit, since every tile converts its expert's weights
-        anew (2048 rows x 9 of 289 NVFP4 experts of 4096 x 2048, gate/up: 920 us in tiles of 64, 1372 in 32, 1171 in 128), and a smaller one leaves tensor memory
-        for more weight stages (32 rows: 378 us in tiles of 32, 538 in 64).  ``direct``: gated bf16 experts, which convert nothing in front of half of their
+        anew, and a smaller one leaves tensor memory for more weight stages (32 rows x 9 of 289 NVFP4 experts of 4096 x 2048, gate/up: 378 us in tiles of 32, 538 in
+        64).  Both halves in tiles of 64, 128, us: those experts, 64 pairs an expert 1328, 1602; 68 1446, 1622; 72 1621, 1629; 76 1789, 1645; 81 1969, 1653; 257 FP8
+        experts of 7168 x 2048: 68 2713, 2825; 72 2989, 2824; 76 3249, 2868: both sides meet near 70 now, below the line of 96 from before weights were converted faster.  ``direct``: gated bf16 experts, which convert nothing in front of half of their
         products: tiles of 64 only for as many rows, and of 256 where most experts' rows fit them and not 128 (64 experts of 4096 x 2048, gate/up + down, tiles of
         64, 128, 256: 56 pairs an expert 553, 558, -; 69 574, 562, -; 137 754, 645, 670; 169 938, 888, 776; 225 1148, 879, 812; 256 1222, 904, 875; 375 1729,
         1275, 1545)."""
