@@ -7,6 +7,7 @@
 #include <type_traits>
 #include "gemv_core.cuh"
 #include "fp8_rows.cuh"
+#include "bf16_rows.cuh"
 #include "tc_common.cuh"
 #include "comm.cuh"
 
@@ -363,6 +364,14 @@ LSB_API int lsb_gemv_error() {
 LSB_API int lsb_gemv_bf16(void* out, const void* x, const void* w, const void* bias, int M, int N, int K, int ldx,
                           int ldw, int ldo, float alpha, int out_bf16, const void* comm, void* stream) {
     if (K % 8 || ldw % 8 || ldx % 8) return -1;
+    // Above four rows the streaming form reads the weights twice.  5 rows in it and on mma.sync, us: 576 x 4096 4.5, 3.6; 1024 x 4096 6.3, 3.7; 2048 x 2048 6.3, 3.5;
+    // 4096 x 512 4.1, 3.1; but smaller ones come from L2 the second time: 144 x 4096 3.5, 3.5; 256 x 7168 4.3, 5.1 (staging rows takes longest).
+    if (M > 4 && alpha == 1.f && !comm && (long long)N * K >= (2 << 20) && bf16_rows_ok(M, N, K, ldx, ldw, x, w)) {
+        Bf16RowsArgs a{};
+        a.x = (const bf16*)x; a.ldx = ldx; a.w = (const bf16*)w; a.ldw = ldw; a.out = out; a.ldo = ldo; a.out_bf16 = out_bf16;
+        a.bias = (const float*)bias; a.M = M; a.N = N; a.K = K; a.steady = 1;
+        return bf16_rows_launch(a, (cudaStream_t)stream);
+    }
     return launch_gemv(MatBf16{(const bf16*)w, ldw}, (const bf16*)x, ldx, out, ldo, M, N, K, alpha, (const float*)bias,
                        out_bf16, (cudaStream_t)stream, comm);
 }

@@ -208,4 +208,8 @@ def test_few_rows_of_bf16_weights(M, N, K):
         bound = (K + 2) * 2.0 ** -24 * size + (want.abs() * 2.0 ** -8 if dt == torch.bfloat16 else 0)
         assert bool(((out[:, :N].double() - want).abs() <= bound).all())
         assert bool((out[:, N:] == 7).all())
+        out.fill_(7.0)
+        nat.call("lsb_gemv_bf16", out, x, w, bias, M, N, K, K + 8, K + 16, N + 24, 1.0, flag & 1, None)
+        assert bool(((out[:, :N].double() - want).abs() <= bound).all())
+        assert bool((out[:, N:] == 7).all())
     assert int(err) == 0
