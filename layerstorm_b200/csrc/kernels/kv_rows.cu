@@ -74,26 +74,31 @@ __global__ void kv_rows_identity_kernel(int* __restrict__ sel_m, int sel_ld, int
 }  // namespace lsb
 using namespace lsb;
 
-// out: [rows, out_rows, row_bytes] bytes; row_bytes a multiple of 16, all buffers 16-byte aligned.
-// `table` (host): n pairs {address, bytes per slot}; the slots of a tensor lie one behind the other.
+// `table` (host): n pairs {address, bytes per slot}; the slots of a tensor lie one behind the other.  Tensors without bytes take no part, whatever their address.
 LSB_API int lsb_copy_slots(const void* table, int n, int from, int to, void* stream) {
     const long long* t = (const long long*)table;
     if (n < 0 || from < 0 || to < 0) return -1;
-    for (int k = 0; k < n && from != to; k += kSlotTensors) {
-        const int m = n - k < kSlotTensors ? n - k : kSlotTensors;
+    for (int i = 0; i < n; ++i)
+        if (t[2 * i + 1] < 0 || (t[2 * i + 1] > 0 && !t[2 * i])) return -1;
+    for (int k = 0; k < n && from != to;) {
         SlotCopy c{};
         long long most = 0;
-        for (int i = 0; i < m; ++i) {
-            c.base[i] = (uint8_t*)t[2 * (k + i)];
-            c.bytes[i] = t[2 * (k + i) + 1];
-            if (c.bytes[i] > most) most = c.bytes[i];
+        int m = 0;
+        for (; k < n && m < kSlotTensors; ++k) {
+            if (!t[2 * k + 1]) continue;
+            c.base[m] = (uint8_t*)t[2 * k];
+            c.bytes[m] = t[2 * k + 1];
+            if (c.bytes[m] > most) most = c.bytes[m];
+            ++m;
         }
+        if (!m) break;
         const long long want = (most + 16383) / 16384;              // four 16-byte pieces a thread
         launch_pdl((copy_slots_kernel), dim3(want < 1 ? 1 : (want > 256 ? 256 : (int)want), m), 256, 0, (cudaStream_t)stream, c, from, to);
     }
     LSB_CHECK_LAUNCH();
 }
 
+// out: [rows, out_rows, row_bytes] bytes; row_bytes a multiple of 16, all buffers 16-byte aligned.
 LSB_API int lsb_kv_row_gather(const void* cache, const void* block_table, int max_pages, const void* row_seq, const void* sel_idx,
                               const void* sel_cnt, int sel_ld, void* out, int out_rows, int rows, int page, int row_bytes, void* stream) {
     if (row_bytes % 16 || (((uintptr_t)cache | (uintptr_t)out) & 15) || rows <= 0) return -1;

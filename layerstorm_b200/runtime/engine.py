@@ -267,7 +267,8 @@ class Engine:
     def _copy_slot(self, src: int, dst: int):
         """What a sequence slot holds besides its pages (recurrent states, convolution histories, open index pools), from one slot to another."""
         m = self.model
-        ts = [t for d in (m.kda_state, m.kda_conv, m.idx_tail) for t in d.values()]
+        # (without tensors of no elements, such as the history of a convolution of one tap: they have no address, but strides)
+        ts = [t for d in (m.kda_state, m.kda_conv, m.idx_tail) for t in d.values() if t.numel()]
         if all(t.is_cuda and t.is_contiguous() for t in ts):
             if ts:
                 table = np.array([(t.data_ptr(), t.stride(0) * t.element_size()) for t in ts], dtype=np.int64)

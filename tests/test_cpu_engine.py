@@ -264,3 +264,29 @@ def test_performance_objective_sets_the_prefill_slice_of_the_batched_server():
     cfg["orchestrator"]["performance_objective"] = {"latency_weight": 0.2, "throughput_weight": 0.8}
     _, thr = serve.build_server(cfg, shape, ckpt, serve.build_engine(cfg, shape, ckpt, args), args)
     assert lat.prefill_slice == chunk and thr.prefill_slice == 8 * chunk
+
+
+def test_slot_copies_leave_out_tensors_without_elements(monkeypatch):
+    """What a fork hands to the copy kernel: addresses and sizes of the tensors that hold something.  A history of no steps (a convolution of one tap) has address 0
+    and strides like any other, so it must not be in the table."""
+    import ctypes
+    from types import SimpleNamespace
+
+    from layerstorm_b200.ops import _native as nat
+    from layerstorm_b200.runtime.engine import Engine
+
+    class OnDevice(torch.Tensor):
+        is_cuda = True
+
+    state, hist, none = (torch.zeros(*s).as_subclass(OnDevice) for s in ((3, 2, 8, 16), (3, 2, 24, 4), (3, 2, 24, 0)))
+    assert none.is_contiguous() and none.stride(0) > 0 and none.data_ptr() == 0
+    seen = []
+
+    def call(name, table, n, src, dst):
+        seen.extend([name, src, dst, list((ctypes.c_longlong * (2 * n)).from_address(table))])
+    monkeypatch.setattr(nat, "call", call)
+    Engine._copy_slot(SimpleNamespace(model=SimpleNamespace(kda_state={0: state}, kda_conv={0: none, 1: hist}, idx_tail={})), 0, 2)
+    assert seen == ["lsb_copy_slots", 0, 2, [state.data_ptr(), 2 * 8 * 16 * 4, hist.data_ptr(), 2 * 24 * 4 * 4]]
+    seen.clear()
+    Engine._copy_slot(SimpleNamespace(model=SimpleNamespace(kda_state={}, kda_conv={0: none}, idx_tail={})), 0, 2)
+    assert not seen

@@ -430,6 +430,21 @@ def test_forks_anchored_rewinds_and_hibernation_keep_the_state(tmp_path_factory)
     assert rms(eng.forward_rows(b, toks[0][72:75]), ref[0][72:75]) < 2e-4
 
 
+@pytest.mark.parametrize("name", ["attention first", "odd"])
+def test_a_fork_goes_on_like_its_parent(tmp_path_factory, name):
+    """Delta rules with a convolution of one tap, which keep no history, and of more: parent and fork go on together, and the parent alone behind the fork."""
+    c, m, toks, ref = load(tmp_path_factory, name, "float32")
+    eng = engine(m)
+    a = eng.create_sequence()
+    eng.prefill(a, toks[0][:40])
+    b = eng.fork_sequence(a)
+    for k in range(40, 44):
+        _, lg = eng.decode([b, a], [toks[0][k]] * 2, return_logits=True)
+        assert rms(lg, ref[0][k: k + 1].repeat(2, 1)) < TOL["float32"]
+    eng.free_sequence(b)
+    assert rms(eng.forward_rows(a, toks[0][44:50]), ref[0][44:50]) < TOL["float32"]
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_greedy_generation_through_the_server_scheduler(tmp_path_factory, dtype):
     """Requests that join, decode together and leave get the tokens of ``Engine.generate`` alone; in fp32 these are the oracle's."""
