@@ -16,11 +16,6 @@ struct Bf16RowsArgs {
     int steady;                                                        // the kernel before does not write w
 };
 
-__device__ __forceinline__ void b16_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // NC: sets of eight activation rows; NS: weight blocks in flight per warp.
 template <int NC, int NS>
 __global__ void __launch_bounds__(kF8Warps * 32, 1) bf16_rows_kernel(const Bf16RowsArgs a) {
@@ -77,8 +72,8 @@ __global__ void __launch_bounds__(kF8Warps * 32, 1) bf16_rows_kernel(const Bf16R
                 __syncwarp();
 #pragma unroll
                 for (int n = 0; n < NC; ++n) {
-                    b16_mma(tot[n], lo.x, hi.x, lo.y, hi.y, b[n].x, b[n].y);
-                    b16_mma(tot[n], lo.z, hi.z, lo.w, hi.w, b[n].z, b[n].w);
+                    rows_mma(tot[n], lo.x, hi.x, lo.y, hi.y, b[n].x, b[n].y);
+                    rows_mma(tot[n], lo.z, hi.z, lo.w, hi.w, b[n].z, b[n].w);
                 }
             }
         }

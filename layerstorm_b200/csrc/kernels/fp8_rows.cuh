@@ -1,14 +1,14 @@
 // Few rows over FP8 weights (e4m3, fp32 scales of 128 x 128 blocks): dense matrices and the experts of decode and verification steps.
 //
-// A warp owns 16 weight rows and every KW-th block of 128 reduction elements.  A thread's 16-byte loads are already its share of the mma fragments when
-// the reduction is taken in another order (thread c of a row's four: elements 16 c .. 16 c + 15 of 64), so weights go from DRAM to registers, through one
-// conversion per two (e4m3 -> fp16, exact) and into mma.sync (m16n8k16, fp32 sums) for up to eight activation rows at once; a block's sum is multiplied by its scale
-// in fp32.  Activation rows are staged as fp16 times a power of two per row that puts the row's largest at 2^14: exact but for elements below 2^-31 of it,
-// whose last bits lie under 2^-39 of it.
-// Bound by DRAM and, in small matrices, by the staging (3 us).  The form with a multiplication per weight and row took 8 scheduler cycles for two weights and one row
-// (conversion, two halves to floats, two FMAs), and read the weights again from the fifth row on.  Before, now (us), out of a clean cache: 36864 x 7168 1 row 64,
-// 54, 6 rows 203, 57 (DRAM's rate: 41); 7168 x 16384 36, 36 and 118, 50 (18); 256 + 1 experts of 7168 x 2048, top 8 + 1, gate/up and down: 1 row 94 and 59, 61 and 35 (41 and
-// 20), 6 rows 442 and 266, 290 and 150 (209 and 104).  Against 64 bits 36864 x 7168 is off 8e-8, 2e-7 before.
+// A warp owns 16 weight rows and every KW-th block of 128 reduction elements.  A thread's 16-byte pieces are already its share of the mma fragments when
+// the reduction is taken in another order (thread c of a row's four: elements 16 c .. 16 c + 15 of 64), so weights go from DRAM into a ring in shared memory, from there
+// to the registers of the thread that copied them, from e4m3 to bf16 (exact), and into mma.sync (m16n8k16, fp32 sums) for up to eight activation rows at once,
+// which are bf16 as they come; a block's sum is multiplied by its scale in fp32.  Products are exact, whatever lies beside them.
+// Bound by DRAM and, with several rows, by the warps' chains of conversions and products.  The form with a multiplication per weight and row took 8 scheduler cycles for two
+// weights and one row (conversion, two halves to floats, two FMAs), and read the weights again from the fifth row on.  Before, now (us), out of a clean cache: 36864 x 7168
+// 1 row 64, 57, 6 rows 203, 61 (DRAM's rate: 41); 7168 x 16384 36, 38 and 118, 55 (18); 256 + 1 experts of 7168 x 2048, top 8 + 1, gate/up and down: 1 row 94 and 59, 61 and 35
+// (41 and 20), 6 rows 442 and 266, 307 and 162 (209 and 104).  Against 64 bits 36864 x 7168 is off 8e-8, 2e-7 before.  fp16 operands, a conversion less per weight, take
+// 2 to 6 % less (54, 57; 36, 50; experts of 6 rows 300 and 156) but need a power of two per row, and what lies 2^-31 below a row's largest element loses bits.
 #pragma once
 #include "gemv_core.cuh"
 #include "moe_fmt.cuh"
@@ -33,13 +33,15 @@ struct Fp8RowsArgs {
     int S; GluAct ga; int* miss_flag;
 };
 
+// Two weights as bf16, which holds every e4m3 value, NaN among them.
 __device__ __forceinline__ uint32_t f8_pair(uint32_t two) {
     uint32_t r;
-    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(r) : "h"((uint16_t)two));
+    asm("{\n .reg .b32 h;\n .reg .b16 l, u;\n .reg .f32 fl, fu;\n cvt.rn.f16x2.e4m3x2 h, %1;\n mov.b32 {l, u}, h;\n cvt.f32.f16 fl, l;\n cvt.f32.f16 fu, u;\n"
+        " cvt.rn.bf16x2.f32 %0, fu, fl;\n}" : "=r"(r) : "h"((uint16_t)two));
     return r;
 }
-__device__ __forceinline__ void f8_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+__device__ __forceinline__ void rows_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
@@ -58,10 +60,8 @@ template <int MODE, int NS>
 __global__ void __launch_bounds__(kF8Warps * 32, 1) fp8_rows_kernel(const Fp8RowsArgs a) {
     constexpr int NT = kF8Warps * 32;
     extern __shared__ __align__(16) uint8_t f8_smem[];                 // [NS][warps][4][32] 16-byte pieces, then
-    __half* xs = reinterpret_cast<__half*>(f8_smem + NS * kF8Ring);    // [cols][K + 8]: rows 16 bytes apart in the banks
+    bf16* xs = reinterpret_cast<bf16*>(f8_smem + NS * kF8Ring);        // [cols][K + 8]: rows 16 bytes apart in the banks
     __shared__ float red[2][kF8Warps][16][kF8Cols];
-    __shared__ uint32_t rmax[kF8Warps];
-    __shared__ float s_inv[kF8Cols];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
     const int K = a.K, nkb = K >> 7, kw = a.kw, ks = warp % kw, sub = warp / kw, per = MODE == kF8GateUp ? 1 : kF8Warps / kw;
     // A block stages its rows once and takes every step-th unit of `per` tiles of 16 weight rows; what a warp asks for next runs on from one to the next.
@@ -109,57 +109,18 @@ __global__ void __launch_bounds__(kF8Warps * 32, 1) fp8_rows_kernel(const Fp8Row
         ncols = min(a.group_n[grp], 4);
     }
     auto pair_of = [&](int m) { return MODE == kF8Dense ? (int)(blockIdx.x % passes) * a.cols + m : a.group_pairs[blockIdx.y * 4 + m]; };
-    // ---- rows to fp16: some warps for each, all of a row's loads on their way together
-    const int wpr = kF8Warps / ncols, xm = warp / wpr, x0 = warp % wpr * 32 + lane;
-    const bool stages = xm < ncols;
-    const uint4* xp = nullptr;
-    if (stages) {
+    // ---- rows: some warps for each, a row's loads on their way together
+    const int wpr = kF8Warps / ncols, xm = warp / wpr;
+    if (xm < ncols) {
         const int p = pair_of(xm);
-        xp = reinterpret_cast<const uint4*>(MODE == kF8Dense ? a.x + (size_t)p * a.ldx : a.x + (size_t)(MODE == kF8GateUp ? p / a.S : p) * K);
-    }
-    // the row's largest finite value, as bf16 bits
-    auto largest = [&](bool finite) {
-        uint32_t b = 0;
-        if (stages) {
+        const uint4* xp = reinterpret_cast<const uint4*>(MODE == kF8Dense ? a.x + (size_t)p * a.ldx : a.x + (size_t)(MODE == kF8GateUp ? p / a.S : p) * K);
 #pragma unroll 8
-            for (int k = x0; k < K / 8; k += wpr * 32) {
-                const uint4 v = __ldg(xp + k);
-                uint32_t u[4] = {v.x & 0x7fff7fffu, v.y & 0x7fff7fffu, v.z & 0x7fff7fffu, v.w & 0x7fff7fffu};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (finite) u[i] &= ((u[i] & 0xffffu) < 0x7f80u ? 0xffffu : 0u) | ((u[i] >> 16) < 0x7f80u ? 0xffff0000u : 0u);
-                    b = __vmaxu2(b, u[i]);
-                }
-            }
-        }
-        __syncwarp();
-        b = __reduce_max_sync(0xffffffffu, max(b & 0xffffu, b >> 16));
-        if (lane == 0) rmax[warp] = b;
-        __syncthreads();
-        b = lane < wpr && stages ? rmax[xm * wpr + lane] : 0u;
-        return __reduce_max_sync(0xffffffffu, b);
-    };
-    uint32_t top = largest(false);
-    if (__syncthreads_or(top >= 0x7f80u)) top = largest(true);
-    // power of two that takes it to [2^14, 2^15): its exponent, at most 126
-    const int shift = top ? min(126, 141 - (int)(top >> 7)) : 0;
-    if (stages) {
-        const float f = __int_as_float((shift + 127) << 23);
-        if (x0 == 0) s_inv[xm] = __int_as_float((127 - shift) << 23);
-#pragma unroll 8
-        for (int k = x0; k < K / 8; k += wpr * 32) {
-            float v[8];
-            unpack_bf16x8(__ldg(xp + k), v);
-            __half2 h[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(v[2 * i] * f, v[2 * i + 1] * f);
-            *reinterpret_cast<uint4*>(xs + (size_t)xm * (K + 8) + k * 8) = *reinterpret_cast<uint4*>(h);
-        }
+        for (int k = warp % wpr * 32 + lane; k < K / 8; k += wpr * 32) *reinterpret_cast<uint4*>(xs + (size_t)xm * (K + 8) + k * 8) = __ldg(xp + k);
     }
     __syncthreads();
     // ---- products
     float tot[4] = {0.f, 0.f, 0.f, 0.f};
-    const __half* xb = xs + (size_t)min(g, ncols - 1) * (K + 8) + c * 16;
+    const bf16* xb = xs + (size_t)min(g, ncols - 1) * (K + 8) + c * 16;
     const bool have = g < ncols;
     int u = u0, kb = ks, par = 0;
     auto finish = [&]() {
@@ -178,12 +139,12 @@ __global__ void __launch_bounds__(kF8Warps * 32, 1) fp8_rows_kernel(const Fp8Row
             }
             const int pair = pair_of(m);
             if constexpr (MODE == kF8GateUp) {
-                const float f = s_inv[m] * glu_in_scale(a.ga, pair);
+                const float f = glu_in_scale(a.ga, pair);
                 reinterpret_cast<bf16*>(a.out)[(size_t)pair * a.N + n] = __float2bfloat16(glu_act(v * f, up * f, a.ga));
             } else if constexpr (MODE == kF8Down) {
-                reinterpret_cast<float*>(a.out)[(size_t)pair * a.N + n] = v * s_inv[m];
+                reinterpret_cast<float*>(a.out)[(size_t)pair * a.N + n] = v;
             } else {
-                float y = v * s_inv[m] * a.alpha;
+                float y = v * a.alpha;
                 if (a.bias) y += a.bias[n];
                 if (a.out_bf16) reinterpret_cast<bf16*>(a.out)[(size_t)pair * a.ldo + n] = __float2bfloat16(y);
                 else reinterpret_cast<float*>(a.out)[(size_t)pair * a.ldo + n] = y;
@@ -217,7 +178,7 @@ __global__ void __launch_bounds__(kF8Warps * 32, 1) fp8_rows_kernel(const Fp8Row
                 const uint32_t bb[8] = {b[0].x, b[0].y, b[0].z, b[0].w, b[1].x, b[1].y, b[1].z, b[1].w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    f8_mma(acc, f8_pair(wl[j]), f8_pair(wh[j]), f8_pair(wl[j] >> 16), f8_pair(wh[j] >> 16), bb[2 * j], bb[2 * j + 1]);
+                    rows_mma(acc, f8_pair(wl[j]), f8_pair(wh[j]), f8_pair(wl[j] >> 16), f8_pair(wh[j] >> 16), bb[2 * j], bb[2 * j + 1]);
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) tot[q] = fmaf(s, acc[q], tot[q]);

@@ -482,9 +482,10 @@ LSB_API int lsb_gemm_f32(void* out, const void* x, const void* w, int M, int N, 
 LSB_API int lsb_gemv_fp8b(void* out, const void* x, const void* w, const void* scales, const void* bias, int M, int N,
                           int K, int ldx, int ldo, float alpha, int out_bf16, const void* comm, void* stream) {
     if (K % 16 || ldx % 8) return -1;
-    // Small matrices are over before their rows are staged.  Here against there, us, for 1, 2, 4, 6, 12 rows: 576 x 7168 9, 10, 12, 17, 14 against 14, 14, 17, 17, 17;
-    // 1536 x 7168 10, 12, 14, 22, 27 / 14, 15, 17, 18, 18; 8192 x 1536 10, 12, 16, 22, 31 / 12, 12, 14, 14, 14; 2304 x 7168 12, 14, 20, 26, 35 / 14, 15, 18, 18, 19;
-    // 24576 x 1536 17, 21, 31, 46, 72 / 17, 18, 18, 18, 23; 7168 x 16384 36, 49, 76, 118, 197 / 36, 37, 48, 50, 80; 36864 x 7168 64, 85, 127, 203, 336 / 54, 54, 57, 57, 87.
+    // Small matrices are over before their rows are staged.  Streaming against mma.sync, one product behind another with weights out of DRAM, us, for 1, 2, 4, 6, 12 rows:
+    // 576 x 7168 3.5, 4.0, 5.3, 9.4, 8.2 / 6.6, 7.2, 7.9, 9.6, 9.5; 1536 x 7168 5.8, 6.5, 8.2, 14.4, 19.2 / 7.0, 7.7, 8.4, 10.0, 10.0; 8192 x 1536 5.3, 6.0, 8.6, 14.2, 22.9 / 5.5, 5.6,
+    // 5.9, 7.3, 7.9; 7168 x 2048 5.4, 6.9, 10.3, 16.8, 25.4 / 5.7, 5.7, 6.0, 6.4, 9.1; 2304 x 7168 6.4, 7.0, 12.3, 18.8, 27.8 / 7.4, 8.3, 8.9, 10.5, 10.4; 24576 x 1536 11.3, 15.2, 23.1,
+    // 37.3, 63.5 / 11.1, 11.3, 11.9, 13.0, 17.7; 7168 x 16384 31.5, 46, 71, 111, 191 / 33, 35, 50, 51, 84; 36864 x 7168 58, 80, 121, 196, 331 / 52, 53, 54, 57, 94.
     // One choice for all numbers of rows: a row's sums do not depend on its company.
     if (!comm && (long long)N * K >= 12 << 20 && fp8_rows_ok(x, ldx, w, N, K)) {
         Fp8RowsArgs a{};

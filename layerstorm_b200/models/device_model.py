@@ -106,7 +106,7 @@ def expert_layout(fmt: str, H: int, F: int, down_fmt: Optional[str] = None, gate
 
 F32_SPLIT_MIN_ROWS = 128  # rows from which an fp32 matrix (the router) runs as a split-bf16 tensor-core GEMM instead of the CUDA-core SGEMM
 # Rows per step from which the routed experts run on the tensor-core grouped GEMM.  Sort, gather and grouped GEMM take less than the weight-streaming kernels
-# from fewer rows on (FP8, 256 + 1 experts of 7168 x 2048, top 8: 6 rows 379 against 440 us, but 1 row 126 / 96; Q4_K, 64 + 1 of 6144 x 2048:
+# from fewer rows on (FP8, 256 + 1 experts of 7168 x 2048, top 8: 6 rows 379 against 469 us, but 1 row 126 / 96; Q4_K, 64 + 1 of 6144 x 2048:
 # 1 row 143 / 201, 8 rows 533 / 951; NVFP4, 288 + 1 of 4096 x 2048: 10 rows 301 / 543), but few rows stay on those: FP8 and Q4_K keep their scales in fp32 and the
 # rows and hidden values the range of bf16 there, where the grouped kernel's operands are fp16, and a row's expert outputs are the same bits whatever up to 14
 # others share its step (an answer's tokens and the check of a draft of them).

@@ -830,3 +830,55 @@ def test_hyper_connection_passes_of_few_rows(rows, H, mode):
         # fp32 sums of up to 16384 products in runs of a few hundred: 2^-24 sqrt(16384) = 8e-6 at most; the output is rounded to bf16 (2^-9 at most)
         assert rel(res, want_r) < 1e-6 and rel(post, torch.sigmoid(m[:, 4:8]) * 2) < 1e-5 and rel(comb, k) < 1e-5 and rel(out, o) < 3e-3
         assert int(done.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("M", [1, 5, 9])
+@pytest.mark.parametrize("N,K", [(8192, 1536), (1648, 8192)])
+def test_fp8_rows_keep_what_is_small_beside_a_large_element(N, K, M):
+    """A row's largest element meets zero weights: the others, 2^-45 of it and less, make up the result.  Rows near both ends of bf16's range."""
+    from layerstorm_b200.ops import _native as nat
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    w = torch.randn(N, K, device="cuda", generator=g)
+    w[:, 7] = 0.0
+    w = w.to(torch.float8_e4m3fn)
+    sc = torch.rand((N + 127) // 128, K // 128, device="cuda", generator=g) * 0.01 + 0.01
+    x = torch.randn(M, K, device="cuda", generator=g) * torch.tensor([2.0 ** -45, 2.0 ** -60, 2.0 ** -100], device="cuda")[torch.arange(M, device="cuda") % 3][:, None]
+    x[:, 7] = torch.tensor([1.0, 3e38], device="cuda")[torch.arange(M, device="cuda") % 2]
+    x, out = x.bfloat16(), torch.zeros(M, N, device="cuda")
+    want = torch.zeros(M, N, dtype=torch.float64, device="cuda")
+    for k in range(0, K, 128):
+        want += (x[:, k: k + 128].double() @ w[:, k: k + 128].double().T) * sc[:, k // 128].double().repeat_interleave(128)[:N]
+    nat.call("lsb_gemv_fp8b", out, x, w, sc, None, M, N, K, K, N, 1.0, 0, None)
+    for m in range(M):                                    # products exact, fp32 sums
+        assert float((out[m].double() - want[m]).norm()) <= 5e-7 * float(want[m].norm()), m
+
+
+def test_fp8_experts_keep_what_is_small_beside_a_large_element():
+    """The same for experts: token rows in gate/up and hidden values in down."""
+    import ctypes
+    from layerstorm_b200.models.device_model import ExpertArena, QLinear, expert_layout
+    from layerstorm_b200.ops import _native as nat
+    E, R, H, F, dev = 3, 5, 1024, 512, "cuda"
+    g = torch.Generator().manual_seed(4)
+    arena, ref = ExpertArena(expert_layout("fp8_e4m3", H, F), E, E, torch.device(dev)), []
+    for e in range(E):
+        ms = [torch.randn(o, i, generator=g).cuda() * i ** -0.5 for o, i in ((F, H), (F, H), (H, F))]
+        for m in ms:
+            m[:, 9] = 0.0
+        arena.write_expert(e, *(QLinear.from_float(m, "fp8_e4m3", dev) for m in ms))
+        arena.slot_of[e] = e
+        ref.append([m.double().cuda() for m in arena.read_expert(e, "fp8_e4m3")])
+    ids = torch.tensor([[0], [1], [0], [2], [0]]).int()
+    small = lambda n: torch.cat([torch.randn(R, 9, generator=g) * 2.0 ** -45, torch.ones(R, 1), torch.randn(R, n - 10, generator=g) * 2.0 ** -45], 1).bfloat16().cuda()
+    x, hid, mg = small(H), small(F), R + E
+    ge, gn, gp, ng, cn, miss = (torch.zeros(n, dtype=torch.int32, device=dev) for n in (mg, mg, 4 * mg, 1, 2 * E + 2, 1))
+    act, y, efp = torch.zeros(R, F, dtype=torch.bfloat16, device=dev), torch.zeros(R, H, device=dev), ctypes.addressof(arena.ef)
+    nat.call("lsb_moe_build_groups", ids.cuda(), R, E, ge, gn, gp, ng, cn)
+    nat.call("lsb_moe_gateup", x, arena.data, arena.slot_of, efp, ge, gn, gp, ng, act, 1, mg, 0.0, miss, 0)
+    nat.call("lsb_moe_down", hid, arena.data, arena.slot_of, efp, ge, gn, gp, ng, y, mg, 0)
+    for r in range(R):
+        gate, up, down = ref[int(ids[r])]
+        want = torch.nn.functional.silu(gate @ x[r].double()) * (up @ x[r].double())
+        assert float((act[r].double() - want).norm() / want.norm()) < 3e-3          # rounded to bf16 (2^-9)
+        want = down @ hid[r].double()
+        assert float((y[r].double() - want).norm() / want.norm()) < 5e-7            # products exact, fp32 sums
