@@ -213,6 +213,7 @@ template <int MODE, int NS> inline int fp8_rows_start(const Fp8RowsArgs& a, dim3
 }
 template <int MODE> inline int fp8_rows_launch(Fp8RowsArgs a, int max_groups, cudaStream_t st) {
     const int row = (a.K + 8) * 2, most = MODE == kF8Dense ? kF8Cols : 4, fit = kF8Rows / row;
+    if (MODE == kF8Dense ? a.M < 1 : max_groups < 1) return -1;
     if (MODE != kF8Dense && (fit < most || (MODE == kF8GateUp && a.K < 1024))) return -2;      // a group's rows are staged together; every warp has a block
     a.kw = MODE == kF8GateUp ? kF8Warps / 2 : fp8_rows_kw(a.N, a.K);
     a.cols = a.M < most ? a.M : most;

@@ -487,7 +487,7 @@ LSB_API int lsb_gemv_fp8b(void* out, const void* x, const void* w, const void* s
     // 5.9, 7.3, 7.9; 7168 x 2048 5.4, 6.9, 10.3, 16.8, 25.4 / 5.7, 5.7, 6.0, 6.4, 9.1; 2304 x 7168 6.4, 7.0, 12.3, 18.8, 27.8 / 7.4, 8.3, 8.9, 10.5, 10.4; 24576 x 1536 11.3, 15.2, 23.1,
     // 37.3, 63.5 / 11.1, 11.3, 11.9, 13.0, 17.7; 7168 x 16384 31.5, 46, 71, 111, 191 / 33, 35, 50, 51, 84; 36864 x 7168 58, 80, 121, 196, 331 / 52, 53, 54, 57, 94.
     // One choice for all numbers of rows: a row's sums do not depend on its company.
-    if (!comm && (long long)N * K >= 12 << 20 && fp8_rows_ok(x, ldx, w, N, K)) {
+    if (!comm && M > 0 && (long long)N * K >= 12 << 20 && fp8_rows_ok(x, ldx, w, N, K)) {
         Fp8RowsArgs a{};
         a.x = (const bf16*)x; a.ldx = ldx; a.N = N; a.K = K; a.M = M; a.w = (const uint8_t*)w; a.scales = (const float*)scales;
         a.out = out; a.ldo = ldo; a.out_bf16 = out_bf16; a.alpha = alpha; a.bias = (const float*)bias;
