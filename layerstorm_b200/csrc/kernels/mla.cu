@@ -875,10 +875,11 @@ LSB_API int lsb_mla_prep(const void* proj, int ldp, int off_qa, int q_lora, int 
     LSB_CHECK_LAUNCH();
 }
 
-// x: bf16 rows m with stride xs_m, batch stride xs_b; W: bf16 [B, N, K]; out bf16 (strides os_m, os_b).
-LSB_API int lsb_batched_gemv_bf16(void* out, const void* x, const void* w, int M, int B, int N, int K, long long xs_m,
-                                  long long xs_b, long long os_m, long long os_b, int dr, const void* inv_freq,
-                                  const void* row_pos, void* stream) {
+// x: bf16 rows m with stride xs_m, batch stride xs_b; W: bf16 [B, N, K]; out bf16 (strides os_m, os_b).  err: int error word (0 = ok; the GEMM's codes 1-3 = a
+// bounded pipeline wait gave up, and `out` is not what was asked for).
+LSB_API int lsb_head_products_bf16(void* out, const void* x, const void* w, int M, int B, int N, int K, long long xs_m,
+                                   long long xs_b, long long os_m, long long os_b, int dr, const void* inv_freq,
+                                   const void* row_pos, void* err, void* stream) {
     if (K % 8 || xs_m % 8 || xs_b % 8) return -1;
     cudaStream_t st = (cudaStream_t)stream;
     dim3 grid((N + 15) / 16, B);
@@ -887,7 +888,7 @@ LSB_API int lsb_batched_gemv_bf16(void* out, const void* x, const void* w, int M
         // to 31 rows while the GEMM's epilogue took as long.  Below, here (us, weights out of DRAM; the tail takes 2.5 more): 64 heads of 512 x 256, 2 rows 7.7, 5.7,
         // 4 rows 11.6, 5.7, 8 rows 21, 5.7, 31 rows 80, 5.7; 128 of 512 x 128 13.7, 7.4, 22, 7.5, 41, 7.5, 154, 7.8; 128 of 128 x 512 6.3, 5.8, 9.4, 5.7, 17, 5.8,
         // 61, 6.0.  One row stays below (with a tail 8.9 against 10 in a step's chain).
-        const int rc = lsb_gemm_bf16_tc_batched(out, x, w, M, N, K, B, (int)xs_m, xs_b, K, (long long)N * K, (int)os_m, os_b, 1, nullptr, stream);
+        const int rc = lsb_gemm_bf16_tc_batched(out, x, w, M, N, K, B, (int)xs_m, xs_b, K, (long long)N * K, (int)os_m, os_b, 1, err, stream);
         if (rc) return rc;
         if (dr > 0)
             launch_pdl((rope_tail_kernel), M, 256, (size_t)dr / 2 * sizeof(float2), st, (bf16*)out, (const bf16*)x, N, K, xs_m, xs_b, os_m, os_b, B, dr,
@@ -906,6 +907,13 @@ LSB_API int lsb_batched_gemv_bf16(void* out, const void* x, const void* w, int M
         m0 += mt;
     }
     LSB_CHECK_LAUNCH();
+}
+
+// The same for programs that keep no error word.
+LSB_API int lsb_batched_gemv_bf16(void* out, const void* x, const void* w, int M, int B, int N, int K, long long xs_m,
+                                  long long xs_b, long long os_m, long long os_b, int dr, const void* inv_freq,
+                                  const void* row_pos, void* stream) {
+    return lsb_head_products_bf16(out, x, w, M, B, N, K, xs_m, xs_b, os_m, os_b, dr, inv_freq, row_pos, nullptr, stream);
 }
 
 LSB_API int lsb_mla_decode_smem_bytes(int dl, int dr) {

@@ -1501,8 +1501,9 @@ class DeviceModel(ModelBase):
                  KV_FMT[self.kv_fmt], cfg.rms_eps, L.get("tq_rot_t"), self.tq_centroids, ws.row_store if self.dcp is not None else None)
         ldq = self.max_qb
         L["mla_qb"](ws.qproj, ws.q_c, R, ldo=ldq)
-        nat.call("lsb_batched_gemv_bf16", ws.q_abs, ws.qproj, L["k_b"], R, Hh, dl, dn, ldq, dn + dr, Hh * (dl + dr), dl + dr,
-                 dr, self.inv_freq, ws.row_pos)
+        err = TcScratch.get(self.device).err
+        nat.call("lsb_head_products_bf16", ws.q_abs, ws.qproj, L["k_b"], R, Hh, dl, dn, ldq, dn + dr, Hh * (dl + dr), dl + dr,
+                 dr, self.inv_freq, ws.row_pos, err)
         sel_idx = sel_cnt = None
         sel_ld = 0
         if cfg.has_indexer and not dense:
@@ -1514,12 +1515,12 @@ class DeviceModel(ModelBase):
                     # a prefill chunk: every row scores the same sequence's keys - one GEMM on the tensor cores
                     nat.call("lsb_indexer_score_tc", ws.q_idx, ws.idx_w, cfg.index_n_heads, self.idx_cache[i], self.idx_block_table,
                              self.max_pages, self.page // P, ws.row_seq, ws.n_entries, ws.scores, ws.max_entries, R, ws.ne_hint,
-                             ws.idx_kbf, ws.idx_kbf_rows, ws.idx_kscale, TcScratch.get(self.device).err)
+                             ws.idx_kbf, ws.idx_kbf_rows, ws.idx_kscale, err)
                 elif getattr(ws, "idx_f8", False):
                     # few rows over a long index row: FP8 x FP8 on the tensor cores straight over the cached keys
                     nat.call("lsb_indexer_score_f8", ws.q_idx, ws.idx_w, cfg.index_n_heads, self.idx_cache[i], self.idx_cache[i].shape[0],
                              self.idx_block_table, self.max_pages, self.page // P, ws.row_seq, ws.n_entries, ws.scores, ws.max_entries, R,
-                             ws.max_entries, TcScratch.get(self.device).err)
+                             ws.max_entries, err)
                 else:
                     nat.call("lsb_indexer_score", ws.q_idx, ws.idx_w, cfg.index_n_heads, self.idx_cache[i], self.idx_block_table,
                              self.max_pages, self.page // P, ws.row_seq, ws.n_entries, ws.scores, ws.max_entries, R, ws.max_entries)
@@ -1544,7 +1545,7 @@ class DeviceModel(ModelBase):
             nat.call("lsb_mla_decode", ws.q_abs, self.kv_cache[i], self.block_table, self.max_pages, ws.row_seq, ws.row_len,
                      sel_idx, sel_cnt, sel_ld, ws.o_lat, None, ws.o_part, ws.ml_part, R, Hh, dl, dr, self.page,
                      KV_FMT[self.kv_fmt], ws.NS, cfg.softmax_scale, self.tq_centroids)
-        nat.call("lsb_batched_gemv_bf16", ws.attn_v, ws.o_lat, L["v_b"], R, Hh, dv, dl, Hh * dl, dl, Hh * dv, dv, 0, None, None)
+        nat.call("lsb_head_products_bf16", ws.attn_v, ws.o_lat, L["v_b"], R, Hh, dv, dl, Hh * dl, dl, Hh * dv, dv, 0, None, None, err)
         L["mla_o"](ws.sub, ws.attn_v, R, comm=self._cp)
         self._reduce(ws, R)
 

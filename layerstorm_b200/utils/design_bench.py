@@ -203,7 +203,7 @@ def work(cfg, rows: int, ctx: int, batch: int) -> dict:
     if att is None:
         out["lsb_kda_forward"] = out["lsb_kda_forward_chunked"] = rec
         out["lsb_mla_decode"] = latent
-        out["lsb_batched_gemv_bf16"] = (absorb[0], (absorb[1] + up[1]) / 2)
+        out["lsb_head_products_bf16"] = (absorb[0], (absorb[1] + up[1]) / 2)
         out["lsb_add_rmsnorm"] = ("bytes", rows * H * 14)
         out["lsb_moe_combine"] = ("bytes", rows * H * (experts + 1) * 4)
         out["lsb_mla_prep"] = ("bytes", rows * (cfg.q_lora + lat + rot) * 6)

@@ -29,3 +29,31 @@ def test_no_groups_of_fp8_experts_are_refused(half):
     mid = {"gateup": "4096, 4, 0, 0.0, None, 0", "down": "4096, 0, 0"}[half]
     assert _alone("import ctypes; from layerstorm_b200.models.device_model import expert_layout; ef = expert_layout('fp8_e4m3', 1024, 512); "
                   f"print(n.load().lsb_moe_{half}(4096, 4096, 4096, ctypes.addressof(ef), 4096, 4096, 4096, 4096, {mid}, None) != 0)") == ["True"]
+
+
+@pytest.mark.parametrize("rows", [1, 2, 40])
+def test_per_head_products_of_a_latent_layer_report_to_the_error_word(rows, monkeypatch):
+    """Query absorption and value up-projection run on a pipelined product whose waits are bounded: the layer hands them the word that the engine reads behind a step,
+    and the launcher hands it on."""
+    from types import SimpleNamespace
+    from unittest.mock import MagicMock
+
+    from layerstorm_b200.models import device_model as dm
+
+    seen, word = [], object()
+
+    def call(name, *args):
+        assert len(args) == len(nat.SIGS[name][0]), name
+        seen.append((name, args))
+    monkeypatch.setattr(dm.nat, "call", call)
+    monkeypatch.setattr(dm.TcScratch, "get", classmethod(lambda cls, device: SimpleNamespace(err=word)))
+    cfg = SimpleNamespace(kv_lora=512, qk_rope=64, qk_nope=128, v_head=128, q_lora=1536, index_head_dim=0, index_n_heads=0, has_indexer=False, index_kpool=1, rms_eps=1e-6,
+                          softmax_scale=0.1)
+    me = MagicMock(cfg=cfg, Hh=16, max_proj=4096, max_qb=4096, max_pages=4, page=64, kv_fmt="fp8", dcp=None, row_tier=None)
+    L = {"mla_in": MagicMock(), "mla_qb": MagicMock(), "mla_o": MagicMock(), "qa_norm": 0, "kv_norm": 0, "k_b": "k_b", "v_b": "v_b"}
+    dm.DeviceModel._mla(me, 0, L, MagicMock(NS=4), rows)
+    products = [a for n, a in seen if L["k_b"] in a or L["v_b"] in a]
+    assert len(products) == 2 and all(a[-1] is word for a in products)
+    source = (ROOT / "layerstorm_b200/csrc/kernels/mla.cu").read_text()
+    calls = [c.split(";")[0] for c in source.split("= lsb_gemm_bf16_tc_batched(")[1:]]
+    assert calls and all(c.endswith("err, stream)") for c in calls)
