@@ -883,7 +883,9 @@ LSB_API int lsb_head_products_bf16(void* out, const void* x, const void* w, int 
     if (K % 8 || xs_m % 8 || xs_b % 8) return -1;
     cudaStream_t st = (cudaStream_t)stream;
     dim3 grid((N + 15) / 16, B);
-    if (M > 1 && os_b % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
+    // (what the GEMM's maps cannot describe streams: rows or heads that share memory, row strides beyond 32 bits)
+    const bool maps = xs_m > 0 && xs_b > 0 && os_m > 0 && xs_m <= 0x7fffffff && os_m <= 0x7fffffff && K > 0;
+    if (M > 1 && maps && os_b % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
         // One tensor-core GEMM per head ([M, K] x [N, K]^T), the rope tail on the side; the kernel below reads the weights again for every four rows and was kept for up
         // to 31 rows while the GEMM's epilogue took as long.  Below, here (us, weights out of DRAM; the tail takes 2.5 more): 64 heads of 512 x 256, 2 rows 7.7, 5.7,
         // 4 rows 11.6, 5.7, 8 rows 21, 5.7, 31 rows 80, 5.7; 128 of 512 x 128 13.7, 7.4, 22, 7.5, 41, 7.5, 154, 7.8; 128 of 128 x 512 6.3, 5.8, 9.4, 5.7, 17, 5.8,
@@ -896,7 +898,7 @@ LSB_API int lsb_head_products_bf16(void* out, const void* x, const void* w, int 
         LSB_CHECK_LAUNCH();
     }
     for (int m0 = 0; m0 < M;) {
-        const int rem = M - m0, mt = rem >= 4 ? 4 : (rem >= 2 ? 2 : 1);
+        const int rem = xs_m > 0x7fffffff ? 1 : M - m0, mt = rem >= 4 ? 4 : (rem >= 2 ? 2 : 1);      // (the kernel steps from row to row in 32 bits)
         bf16* o = (bf16*)out + (size_t)m0 * os_m;
         const bf16* xp = (const bf16*)x + (size_t)m0 * xs_m;
 #define ARGS o, xp, (const bf16*)w, N, K, xs_m, xs_b, os_m, os_b, dr, (const float*)inv_freq, (const int*)row_pos, m0

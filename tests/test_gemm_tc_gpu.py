@@ -213,3 +213,33 @@ def test_few_rows_of_bf16_weights(M, N, K):
         assert bool(((out[:, :N].double() - want).abs() <= bound).all())
         assert bool((out[:, N:] == 7).all())
     assert int(err) == 0
+
+
+@pytest.mark.parametrize("M", [1, 2, 5, 33])
+def test_products_per_head_of_rows_and_heads_that_share_memory(M):
+    """One row for all heads, one head's input for all rows: strides of zero, as the kernel that streams them took at any number of rows."""
+    B, N, K = 4, 72, 128
+    g = torch.Generator(device="cuda").manual_seed(M)
+    w = torch.randn(B, N, K, generator=g, device="cuda").bfloat16()
+    for xs_m, xs_b in ((K, 0), (0, K), (0, 0)):
+        x = torch.randn(max(M, B), K, generator=g, device="cuda").bfloat16()
+        rows = torch.as_strided(x, (M, B, K), (xs_m, xs_b, 1))
+        out, err = torch.full((M + 1, B, N), 3.0, device="cuda", dtype=torch.bfloat16), torch.zeros(1, dtype=torch.int32, device="cuda")
+        nat.call("lsb_head_products_bf16", out, x, w, M, B, N, K, xs_m, xs_b, B * N, N, 0, None, None, err)
+        want = torch.einsum("mbk,bnk->mbn", rows.double(), w.double())
+        assert int(err) == 0 and bool((out[M] == 3.0).all())
+        assert float((out[:M].double() - want).norm() / want.norm()) < 3e-3          # fp32 sums rounded to bf16 (2^-9)
+
+
+def test_products_per_head_of_rows_far_apart():
+    """Rows 2^32 + 8 elements apart: a stride that 32 bits cut down to 8."""
+    B, N, K, far = 2, 72, 128, 2 ** 32 + 8
+    g = torch.Generator(device="cuda").manual_seed(5)
+    big = torch.empty(far + B * K, dtype=torch.bfloat16, device="cuda")
+    big[: B * K + 8] = torch.randn(B * K + 8, generator=g, device="cuda").bfloat16()
+    big[far:] = torch.randn(B * K, generator=g, device="cuda").bfloat16()
+    w, err = torch.randn(B, N, K, generator=g, device="cuda").bfloat16(), torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.zeros(2, B, N, device="cuda", dtype=torch.bfloat16)
+    nat.call("lsb_head_products_bf16", out, big, w, 2, B, N, K, far, K, B * N, N, 0, None, None, err)
+    want = torch.einsum("mbk,bnk->mbn", torch.stack([big[: B * K], big[far:]]).view(2, B, K).double(), w.double())
+    assert int(err) == 0 and float((out.double() - want).norm() / want.norm()) < 3e-3
