@@ -885,11 +885,11 @@ LSB_API int lsb_head_products_bf16(void* out, const void* x, const void* w, int 
     dim3 grid((N + 15) / 16, B);
     // (what the GEMM's maps cannot describe streams: rows or heads that share memory, row strides beyond 32 bits)
     const bool maps = xs_m > 0 && xs_b > 0 && os_m > 0 && xs_m <= 0x7fffffff && os_m <= 0x7fffffff && K > 0;
-    if (M > 1 && maps && os_b % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
-        // One tensor-core GEMM per head ([M, K] x [N, K]^T), the rope tail on the side; the kernel below reads the weights again for every four rows and was kept for up
-        // to 31 rows while the GEMM's epilogue took as long.  Below, here (us, weights out of DRAM; the tail takes 2.5 more): 64 heads of 512 x 256, 2 rows 7.7, 5.7,
-        // 4 rows 11.6, 5.7, 8 rows 21, 5.7, 31 rows 80, 5.7; 128 of 512 x 128 13.7, 7.4, 22, 7.5, 41, 7.5, 154, 7.8; 128 of 128 x 512 6.3, 5.8, 9.4, 5.7, 17, 5.8,
-        // 61, 6.0.  One row stays below (with a tail 8.9 against 10 in a step's chain).
+    if (M > 0 && maps && os_b % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
+        // One tensor-core GEMM per head ([M, K] x [N, K]^T), the rope tail on the side, whatever the number of rows: a row's sums do not depend on its company.  The kernel
+        // below reads the weights again for every four rows.  Below, here (us, weights out of DRAM; the tail takes 2.5 more): 64 heads of 512 x 256, 2 rows 7.7, 5.7, 4 rows
+        // 11.6, 5.7, 8 rows 21, 5.7, 31 rows 80, 5.7; 128 of 512 x 128 13.7, 7.4, 22, 7.5, 41, 7.5, 154, 7.8; 128 of 128 x 512 6.3, 5.8, 9.4, 5.7, 17, 5.8, 61, 6.0.  For one row it is
+        // the slower one (with a tail 10 against 8.9 in a step's chain), but in another order of sums a user's answer would change as others come and go.
         const int rc = lsb_gemm_bf16_tc_batched(out, x, w, M, N, K, B, (int)xs_m, xs_b, K, (long long)N * K, (int)os_m, os_b, 1, err, stream);
         if (rc) return rc;
         if (dr > 0)

@@ -243,3 +243,17 @@ def test_products_per_head_of_rows_far_apart():
     nat.call("lsb_head_products_bf16", out, big, w, 2, B, N, K, far, K, B * N, N, 0, None, None, err)
     want = torch.einsum("mbk,bnk->mbn", torch.stack([big[: B * K], big[far:]]).view(2, B, K).double(), w.double())
     assert int(err) == 0 and float((out.double() - want).norm() / want.norm()) < 3e-3
+
+
+@pytest.mark.parametrize("B,N,K,dr", [(16, 512, 192, 64), (8, 256, 512, 0)])
+def test_products_per_head_of_a_row_do_not_depend_on_its_company(B, N, K, dr):
+    """The same bits for a row alone and beside any number of others: every number of rows sums in one order."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x, w = torch.randn(300, B, K + dr, generator=g, device="cuda").bfloat16(), torch.randn(B, N, K, generator=g, device="cuda").bfloat16()
+    inv, pos = torch.rand(max(dr // 2, 1), generator=g, device="cuda"), torch.randint(0, 5000, (300,), generator=g, device="cuda", dtype=torch.int32)
+    err, first = torch.zeros(1, dtype=torch.int32, device="cuda"), None
+    for M in (1, 2, 3, 4, 5, 8, 16, 17, 31, 32, 33, 65, 129, 300):
+        out = torch.zeros(M, B, N + dr, device="cuda", dtype=torch.bfloat16)
+        nat.call("lsb_head_products_bf16", out, x, w, M, B, N, K, B * (K + dr), K + dr, B * (N + dr), N + dr, dr, inv if dr else None, pos, err)
+        first = out if first is None else first
+        assert int(err) == 0 and torch.equal(out[0], first[0]), M
