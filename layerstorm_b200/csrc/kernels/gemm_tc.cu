@@ -154,7 +154,8 @@ __global__ void __launch_bounds__(TcCfg<BN, MT, DEEP>::THREADS) gemm_tc_kernel(c
         // outside the matrix.  Before, now (us): 2048 x 24896 x 4096 fp32 408, 297 (1406 TFLOP/s), bf16 390, 279 (1500); 2048 x 4096 x 12288 156, 133;
         // 2048 x 20480 x 1536 bf16 207, 107; 391 x 16640 x 4096 bf16 80, 57; 64 products of 2048 x 512 x 256 207, 66; 128 of 777 x 512 x 128 176, 47.
         const int q = warp & 3, mt = (warp - 2) >> 2;
-        const bool ok = __all_sync(0xffffffffu, nkb > 0 ? mbar_wait(acc_full, 0, p.err, 3) : true);      // one answer for the warp: its loads are warp-wide
+        bool ok = __all_sync(0xffffffffu, nkb > 0 ? mbar_wait(acc_full, 0, p.err, 3) : true);      // one answer for the warp: its loads are warp-wide
+        if (p.tma_out) ok = bar_all(1 + mt * 2 + (q >> 1), 64, ok);        // and for the pair of warps that store together: their limits end at different times
         tc_fence_after();
         const int rows = min(BN, p.M - m0);
         const uint32_t lane_addr = tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(mt * BN);

@@ -168,6 +168,12 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
+// Whether `ok` holds in all of the threads that meet.
+__device__ __forceinline__ bool bar_all(int id, int threads, bool ok) {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %3, 0;\n bar.red.and.pred q, %1, %2, p;\n selp.u32 %0, 1, 0, q;\n}" : "=r"(r) : "r"(id), "r"(threads), "r"((uint32_t)ok) : "memory");
+    return r != 0;
+}
 __device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 // Stores of lanes that take part by predicate, without a branch.
 __device__ __forceinline__ void st_global_if(float* p, float v, bool on) {
