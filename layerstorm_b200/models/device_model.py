@@ -146,9 +146,17 @@ MOE_BLOCK_SCALED = os.environ.get("LSB_MOE_BLOCK_SCALED", "0") not in ("", "0")
 # LSB_MHC_CLUSTER=0: decode-sized hyper-connection passes fall back to the two-launch path (partials + last-block finalize, contraction)
 MHC_CLUSTER = os.environ.get("LSB_MHC_CLUSTER", "1") not in ("", "0")
 # rows of a step up to which the cluster kernel (one cluster per row) is used; above it the partial + last-block-finalize kernels, which
-# tile better over many rows (32 rows of 4 x 4096 on a B200: 14 us per pass against 55 us for 32 clusters).  On one GPU up to five rows: clusters of more
-# come in two waves (5 rows 11.2 us against 10.8, 8 rows 21.5 / 11.3)
-MHC_CLUSTER_MAX_ROWS = int(os.environ.get("LSB_MHC_CLUSTER_MAX_ROWS", "8"))
+# tile better over many rows (32 rows of 4 x 4096 on a B200: 14 us per pass against 55 us for 32 clusters).  LSB_MHC_CLUSTER_MAX_ROWS is taken as given; without it 8 where
+# ranks exchange partials (the fused exchange is the cluster kernel's), else 5: more clusters come in two waves (5 rows 11.2 us in one launch against 10.8 in two, 8 rows
+# 21.5 / 11.3)
+MHC_CLUSTER_MAX_ROWS = int(os.environ["LSB_MHC_CLUSTER_MAX_ROWS"]) if os.environ.get("LSB_MHC_CLUSTER_MAX_ROWS") else None
+
+
+def mhc_cluster_rows(peers: bool) -> int:
+    """Rows of a step up to which hyper-connection passes run on the cluster kernel, alone or among tensor-parallel ranks."""
+    return MHC_CLUSTER_MAX_ROWS if MHC_CLUSTER_MAX_ROWS is not None else (8 if peers else 5)
+
+
 # ablation switches of the two folds of the cluster kernel (router behind, MoE combine in front)
 MHC_FOLD_ROUTER = os.environ.get("LSB_MHC_FOLD_ROUTER", "0") not in ("", "0")
 MHC_FOLD_COMBINE = os.environ.get("LSB_MHC_FOLD_COMBINE", "0") not in ("", "0")
@@ -1595,7 +1603,7 @@ class DeviceModel(ModelBase):
         if self.comm is not None:
             # fewer than 8 rows: the kernel that consumes a cross-rank sum exchanges the partials itself (one flag per CTA) instead of
             # the producer's last block copying them to every peer; needs the cluster form of the hyper-connection pass where there is one
-            xchg = COMM_XCHG if (self._fused and R < 8 and R <= MHC_CLUSTER_MAX_ROWS and self.dcp is None and (not cfg.mhc or self._mhc_cluster_ok())) else 0
+            xchg = COMM_XCHG if (self._fused and R < 8 and R <= mhc_cluster_rows(True) and self.dcp is None and (not cfg.mhc or self._mhc_cluster_ok())) else 0
             if xchg == 2 and R * H > self.comm.ll_cap:
                 xchg = 1
             self.comm.struct.xchg = xchg
@@ -1604,7 +1612,7 @@ class DeviceModel(ModelBase):
         if cfg.mhc:
             nat.call("lsb_embedding", ws.sub, None, self.embed, ws.tok, R, H, 0, cfg.vocab)
             # decode-sized steps: one cluster kernel per post -> pre pass, with the MoE combine folded in front and the router behind
-            clus = R <= (MHC_CLUSTER_MAX_ROWS if self.comm is not None else min(5, MHC_CLUSTER_MAX_ROWS)) and self._mhc_cluster_ok()
+            clus = R <= mhc_cluster_rows(self.comm is not None) and self._mhc_cluster_ok()
             pending = None         # slot table of the MoE layer whose combine the next pass performs
             last_run = -1
             for i, L in enumerate(self.layers):

@@ -57,3 +57,12 @@ def test_per_head_products_of_a_latent_layer_report_to_the_error_word(rows, monk
     source = (ROOT / "layerstorm_b200/csrc/kernels/mla.cu").read_text()
     calls = [c.split(";")[0] for c in source.split("= lsb_gemm_bf16_tc_batched(")[1:]]
     assert calls and all(c.endswith("err, stream)") for c in calls)
+
+
+@pytest.mark.parametrize("given,alone,peers", [(None, 5, 8), ("", 5, 8), ("8", 8, 8), ("3", 3, 3), ("0", 0, 0)])
+def test_the_row_limit_of_the_cluster_kernel_is_taken_as_given(given, alone, peers):
+    import os
+    env = {k: v for k, v in os.environ.items() if k != "LSB_MHC_CLUSTER_MAX_ROWS"} | ({} if given is None else {"LSB_MHC_CLUSTER_MAX_ROWS": given})
+    code = "from layerstorm_b200.models import device_model as m; print(m.mhc_cluster_rows(False), m.mhc_cluster_rows(True))"
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+    assert r.stdout.split() == [str(alone), str(peers)], r.stderr[-500:]
