@@ -126,7 +126,7 @@ def test_matrices_that_end_inside_a_warps_rows(M, N):
 
 
 @pytest.mark.parametrize("M", [5, 16, 17, 33, 64, 65, 127, 200, 256, 257, 321])
-@pytest.mark.parametrize("N", [8, 56, 64, 72, 136, 264])
+@pytest.mark.parametrize("N", [8, 12, 56, 64, 72, 100, 136, 264])
 def test_bf16_rows_by_tma_and_by_stores_are_the_same(M, N):
     """Rows of 16-byte pitch at a 16-byte address leave by TMA, others by stores: the same bits, nothing outside the matrix; and as a batch in [row, head] order."""
     K = 128
@@ -134,8 +134,8 @@ def test_bf16_rows_by_tma_and_by_stores_are_the_same(M, N):
     x, w = (torch.randn(n, K, generator=g, device="cuda").bfloat16() for n in (M, N))
     bias, err = torch.randn(N, generator=g, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
     want = x.double() @ w.double().T + bias.double()
-    got = []
-    for ld, at in ((N + 8, 0), (N + 3, 0), (N + 8, 1)):
+    got, even = [], (N + 15) // 8 * 8
+    for ld, at in ((even, 0), (N + 3, 0), (even, 1)):
         buf = torch.zeros((M + 1) * ld + 8, device="cuda", dtype=torch.bfloat16)
         nat.call("lsb_gemm_bf16_tc", buf[at:], x, w, bias, M, N, K, K, K, ld, 1, None, 0, err, None)
         out = buf[at: at + (M + 1) * ld].view(M + 1, ld)
@@ -143,8 +143,8 @@ def test_bf16_rows_by_tma_and_by_stores_are_the_same(M, N):
         got.append(out[:M, :N].clone())
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
     assert float((got[0].double() - want).norm() / want.norm()) < 3e-3          # 2^-9, rounding to bf16
-    B, out = 2, torch.zeros(M + 1, 2, N + 8, device="cuda", dtype=torch.bfloat16)
-    nat.call("lsb_gemm_bf16_tc_batched", out, x, w, M, N, K // B, B, K, K // B, K, K // B, B * (N + 8), N + 8, 1, err)
+    B, out = 2, torch.zeros(M + 1, 2, even, device="cuda", dtype=torch.bfloat16)
+    nat.call("lsb_gemm_bf16_tc_batched", out, x, w, M, N, K // B, B, K, K // B, K, K // B, B * even, even, 1, err)
     parts = torch.stack([x[:, b * K // B: (b + 1) * K // B].double() @ w[:, b * K // B: (b + 1) * K // B].double().T for b in range(B)], 1)
     assert int(err) == 0 and float(out[M:].abs().sum()) == 0.0 and float(out[:, :, N:].abs().sum()) == 0.0
     assert float((out[:M, :, :N].double() - parts).norm() / parts.norm()) < 3e-3
@@ -188,7 +188,7 @@ def test_products_per_head_of_any_number_of_rows(M, B, N, K, dr):
         assert float((out[:M, :, N: N + dr].double() - tail).norm() / tail.norm()) < 3e-3
 
 
-@pytest.mark.parametrize("M", [1, 5, 8, 9, 16, 17])
+@pytest.mark.parametrize("M", [1, 5, 8, 9, 11, 12, 14, 16, 17])
 @pytest.mark.parametrize("N,K", [(16, 64), (144, 448), (2320, 1536), (1040, 512), (576, 4096), (4752, 7168), (8192, 4096), (130, 512)])
 def test_few_rows_of_bf16_weights(M, N, K):
     """Few-row form and, behind its limits, the tiles: both against 64 bits; rows with padding between them, bias, weights asked for early or late.

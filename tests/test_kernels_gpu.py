@@ -763,7 +763,7 @@ def test_fp8_rows_over_large_matrices(N, K, M):
         x[1, 7], x[2, 9] = float("inf"), float("nan")
         bad = torch.zeros(M, N + 8, device="cuda")
         nat.call("lsb_gemv_fp8b", bad, x, w, sc, None, M, N, K, K + 8, N + 8, 1.0, 0, None)
-        assert not bool(bad[1, :N].isfinite().any()) or bool((w[:, 7].float() == 0).any())
+        assert not bool(bad[1, :N].isfinite().any())          # (zero weights make NaN of an infinity)
         assert bool(bad[2, :N].isnan().all()) and torch.equal(bad[0], torch.cat([bad[0, :N], torch.zeros(8, device="cuda")])) and bool(bad[0].isfinite().all())
 
 

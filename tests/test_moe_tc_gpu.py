@@ -116,7 +116,7 @@ def test_engine_prefill_uses_grouped_path_and_matches_oracle():
                                      ("bf16", 1152, 128), ("gguf_q4_k", 256, 768), ("gguf_q4_k", 1280, 256)])
 @pytest.mark.parametrize("BN", [32, 64, 128])
 def test_widths_that_end_inside_boxes_and_operand_stages(fmt, H, F, BN):
-    """Reduction lengths shorter than a weight box, that end inside one, inside an operand stage, and that wrap the rings; more work items than CTAs."""
+    """Reduction lengths shorter than a weight box, that end inside one, inside an operand stage, and that wrap the rings."""
     from layerstorm_b200.ops import _native as nat
     dev = torch.device("cuda")
     E, R = 20, 2 * BN + 1
@@ -519,3 +519,37 @@ def test_bf16_experts_in_tiles_of_256_rows(H, F):
         xd = x[r].double()
         want = (torch.nn.functional.silu(xd @ gate.T) * (xd @ up.T)) @ down.T
         assert float((y[r].double() - want).norm() / want.norm()) < 1e-3, counts[e]          # hidden values and down weights in fp16 (2^-11 each at most)
+
+
+@pytest.mark.parametrize("H,F", [(640, 384), (384, 128), (128, 640)])
+@pytest.mark.parametrize("BN", [32, 64, 128])
+def test_fp8_reductions_of_an_odd_number_of_blocks_over_many_items(H, F, BN):
+    """Each thread block computes several tiles one after another whose reductions end on an odd block of 128: what a converter set takes moves on by one each time."""
+    from layerstorm_b200.ops import _native as nat
+    dev = torch.device("cuda")
+    E, copies = 12, 40 if H > 128 else 160
+    arena, ref = _setup("fp8_e4m3", H, F, E, n_missing=0, seed=12)
+    arena.slot_of = arena.slot_of.repeat(copies)                     # more experts with the same weights
+    g = torch.Generator(device="cpu").manual_seed(13)
+    ids = torch.arange(E * copies).repeat(2)[: 2 * E * copies - 5]
+    ids = ids[torch.randperm(len(ids), generator=g)].int()
+    P = len(ids)
+    x, tiles = torch.randn(P, H, generator=g).to(torch.bfloat16).to(dev), P // BN + E * copies + 1
+    i32 = dict(dtype=torch.int32, device=dev)
+    srt, te, tr, tn, cnt, err = (torch.zeros(n, **i32) for n in (P, tiles, tiles, tiles, 2, 1))
+    xs, act = torch.zeros(P, H, dtype=torch.float16, device=dev), torch.zeros(P + 1, F, dtype=torch.float16, device=dev)
+    y, efp = torch.zeros(P + 1, H, device=dev), ctypes.addressof(arena.ef)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert E * copies * min(H, F) // 128 > 3 * sms                   # items of either half
+    nat.call("lsb_moe_tc_sort", ids.to(dev), P, E * copies, BN, srt, te, tr, tn, cnt)
+    nat.call("lsb_moe_tc_gather", x, srt, cnt, xs, P, 1, H)
+    nat.call("lsb_moe_tc_ffn", 1, xs, P, arena.data, arena.slot_of, efp, te, tr, tn, cnt, srt, act, BN, tiles, 0.0, None, err, None)
+    nat.call("lsb_moe_tc_ffn", 0, act, P, arena.data, arena.slot_of, efp, te, tr, tn, cnt, srt, y, BN, tiles, 0.0, None, err, None)
+    torch.cuda.synchronize()
+    assert int(err) == 0 and float(act[P].abs().sum()) == 0.0 and float(y[P].abs().sum()) == 0.0
+    for e in range(E):
+        r = (ids % E == e).nonzero()[:, 0].to(dev)
+        gate, up, down = (m.to(dev) for m in ref[e])
+        xd = x[r].double()
+        want = (torch.nn.functional.silu(xd @ gate.T) * (xd @ up.T)) @ down.T
+        assert float((y[r].double() - want).norm() / want.norm()) < 1e-3, e          # hidden values in fp16 (2^-11 at most)
