@@ -11,7 +11,8 @@
 //     warps 2-5 epilogue: tcgen05.ld the accumulator (one TMEM lane = one output column n), optional bias; bf16 rows of
 //              16-byte pitch through shared memory and TMA, others and fp32 by stores coalesced over n
 // This replaces the reference's CUDA-core tiled GEMM (src/compute/kernels/sm120/gemm/bf16_gemm.cu:156)
-// and the external FP8 GEMM launcher (G/sm120/gemm/fp8/fp8_gemm.h) for every M > 4.
+// and the external FP8 GEMM launcher (G/sm120/gemm/fp8/fp8_gemm.h).  Up to 16 rows of suitable matrices run on the few-row
+// form of bf16_rows.cuh instead.
 #include "tc_common.cuh"
 #include "bf16_rows.cuh"
 #include "comm.cuh"

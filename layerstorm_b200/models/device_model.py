@@ -212,8 +212,8 @@ def fp8_scale_atoms(scales: torch.Tensor) -> Optional[torch.Tensor]:
 
 class QLinear:
     """A weight matrix [N, K] in a device storage format, applied to bf16 activations.
-    Up to 4 rows (decode; 6 over small matrices) stream the weights through the CUDA-core GEMV; larger row counts with
-    bf16 weights run on the tcgen05 tensor-core GEMM."""
+    Up to 4 rows (decode; 6 over small matrices) of bf16 weights stream through the CUDA-core GEMV; larger row counts run on the tensor cores (up to
+    16 rows of suitable matrices, and few rows over large FP8 matrices, on mma.sync, others on tcgen05)."""
 
     def __init__(self, fmt: str, N: int, K: int, w: torch.Tensor, scales: Optional[torch.Tensor] = None, alpha: float = 1.0):
         self.fmt, self.N, self.K, self.w, self.scales, self.alpha = fmt, N, K, w, scales, alpha
@@ -581,10 +581,10 @@ class MoeBuffers:
         """Rows per token tile for ``P`` pairs over ``E`` experts: the smallest tile that most experts' rows fit, since every tile converts its expert's weights
         anew, and a smaller one leaves tensor memory for more weight stages (32 rows x 9 of 289 NVFP4 experts of 4096 x 2048, gate/up: 378 us in tiles of 32, 538 in
         64).  Both halves in tiles of 64, 128, us: those experts, 64 pairs an expert 1328, 1602; 68 1446, 1622; 72 1621, 1629; 76 1789, 1645; 81 1969, 1653; 257 FP8
-        experts of 7168 x 2048: 68 2713, 2825; 72 2989, 2824; 76 3249, 2868: both sides meet near 70 now, below the line of 96 from before weights were converted faster.  ``direct``: gated bf16 experts, which convert nothing in front of half of their
-        products: tiles of 64 only for as many rows, and of 256 where most experts' rows fit them and not 128 (64 experts of 4096 x 2048, gate/up + down, tiles of
-        64, 128, 256: 56 pairs an expert 553, 558, -; 69 574, 562, -; 137 754, 645, 670; 169 938, 888, 776; 225 1148, 879, 812; 256 1222, 904, 875; 375 1729,
-        1275, 1545)."""
+        experts of 7168 x 2048: 68 2713, 2825; 72 2989, 2824; 76 3249, 2868.  Both sides meet near 70; the line of 96 is from before weights were converted faster and has not
+        been moved yet.  ``direct``: gated bf16 experts, which convert nothing in front of half of their products: tiles of 64 only for as many rows, and of 256 where most
+        experts' rows fit them and not 128 (64 experts of 4096 x 2048, gate/up + down, tiles of 64, 128, 256: 56 pairs an expert 553, 558, -; 69 574, 562, -; 137 754, 645, 670;
+        169 938, 888, 776; 225 1148, 879, 812; 256 1222, 904, 875; 375 1729, 1275, 1545)."""
         avg = P / max(1, min(E, P))
         if direct:
             return 32 if avg <= 32 else (64 if avg <= 64 else (256 if 140 < avg <= 260 else 128))
